@@ -7,17 +7,17 @@
 namespace gzgpu {
 
 constexpr int kRingWarps = 1;      // ring kernel: warps per CTA (64 KB ring each)
-constexpr int kPageWarps = 8;      // page kernel: warps per CTA (tables only)
-constexpr int kDistBits = 8;       // distance LUT index bits
+constexpr uint32_t kCtaThreads = 256;  // page kernel: threads per CTA (one chunk each)
+constexpr int kDistBits = 8;       // distance LUT index bits (ring kernel, sync-start search)
 
 template <int LB>
 size_t inflate_smem_bytes(bool ring);
-// page kernel: `ctas` (3 or 4) CTAs of kPageWarps warps per SM; registers are
-// sized for that many (80 or 64 per thread)
+// page kernel: `ctas` (3 or 4) CTAs per SM; registers are sized for that many
+// (80 or 64 per thread)
 template <int LB>
 int inflate_blocks_per_sm(bool ring, int ctas);
 template <int LB>
-// sync: the job has sync starts (selects the kernel variant that handles them)
+// sync: the job has sync starts (successors are watched mid-block)
 cudaError_t launch_inflate(bool ring, int ctas, bool sync, const uint8_t* in, ChunkDesc* descs,
                            ChunkResult* results, const uint32_t* work, const uint32_t* n_work,
                            uint32_t* work_counter, const PagePool& pool, int blocks,

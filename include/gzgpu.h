@@ -58,10 +58,11 @@ typedef struct {
                          bucket, share of streams whose first block is fixed-Huffman)
                          is decoded once per candidate and the fastest is kept for
                          later jobs of that kind; overrides the three fields */
-  int ring_history;   /* 1 = decode history in a shared-memory ring (3 warps/SM) instead
-                         of the output pages in HBM (24 or 32 warps/SM, the default) */
-  int ctas_per_sm;    /* page-history decoder: 3 (24 warps/SM, 80 registers; default) or
-                         4 (32 warps/SM, 64 registers); 0 = default */
+  int ring_history;   /* 1 = decode history in a shared-memory ring (one warp per chunk, 3
+                         per SM) instead of the output pages in HBM (one CTA of 256 threads
+                         per chunk, the default) */
+  int ctas_per_sm;    /* page-history decoder: 3 (80 registers per thread; default) or
+                         4 (64 registers); 0 = default */
   int fine_split;     /* 1 = cut partitions whose first blocks promise a high output
                          ratio into pieces and give pieces without a block start a
                          sync start inside their dynamic block; 0 = off (default:
@@ -72,13 +73,8 @@ typedef struct {
                          contexts' streams (running blocks are not preempted) */
   int work_order;     /* order in which the persistent decoder takes chunks: 0 = longest
                          expected decode first (default), 1 = in stream order */
-  int decoder;        /* Huffman block bodies: 0 = default (4), 1 = lane-parallel 32-bit steps
-                         (each lane decodes a whole candidate symbol at one bit offset),
-                         2 = warp-uniform serial decode, 3 = lane-parallel 64-bit steps (each
-                         lane looks up literal codes at two bit offsets; length, end and
-                         long codes are decoded on the chain walk by the whole warp),
-                         4 = chosen per block: 3 where length codes take under 0.3 of the
-                         code space (literal-heavy data), else 1 */
+  int decoder;        /* accepted (0 to 4) and without effect: the page-history kernel has one
+                         block decoder */
 } gzgpu_config;
 
 typedef struct {
@@ -198,7 +194,7 @@ int gzgpu_decompress_batch_device(gzgpu_ctx *ctx, const void *d_in, const uint64
  * every GPU loading this library holds until the process exits; so the
  * output of one call is limited to GZGPU_NOALLOC_MAX_OUT bytes (4 MiB, all
  * members together) and larger streams return GZGPU_NOALLOC_TOO_LARGE.  One
- * warp decodes the members in order (no speculative chunks): made for small
+ * CTA decodes the members in order (no speculative chunks): made for small
  * streams, not throughput.  The first call on a device looks the array's
  * address up (cudaGetSymbolAddress); make that first call before any stream
  * capture.  All calls share the array: calls whose work overlaps on the GPU
