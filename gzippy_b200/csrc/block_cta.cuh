@@ -2,18 +2,20 @@
 //
 // Block body.  A Huffman-coded block is decoded in rounds of up to
 // kCtaThreads bit ranges of `r` bits each, one range per thread:
-//   1. every thread decodes its range from a guessed start (its first bit).
-//      Prefix codes resynchronise: a decode that starts off a symbol boundary
-//      falls into step with the true one, so most ranges end at the right
-//      bit although they started at a wrong one.
-//   2. each range is decoded again from where the range before it ended, and
+//   1. every thread walks its range from a guessed start (its first bit),
+//      following symbol lengths only.  Prefix codes resynchronise: a walk that
+//      starts off a symbol boundary falls into step with the true one, so most
+//      ranges end at the right bit although they started at a wrong one.
+//   2. each range is walked again from where the range before it ended, and
 //      again while that end moves, until no start changes (or all ranges up
 //      to one that met the end of the block agree).  By induction from the
 //      first range, whose start is exact, the joined ranges are the serial
-//      decode.  Each pass confirms at least one more range.
-//   3. a block scan of the ranges' symbol counts gives each its place in the
+//      decode.  Each pass confirms at least one more range.  A walk leaves
+//      the first boundary past each quarter of its range, and the lookups from
+//      there to its end; a later walk that meets one of them is done.
+//   3. a block scan of the ranges' lookup counts gives each its place in the
 //      round's token list (a literal: one slot; a match: length, then
-//      distance), written in one more decode pass.
+//      distance), written by one decode of each range.
 //   4. the tokens are expanded in windows of kWin output positions (see
 //      expand_tokens), which leave as coalesced stores to the pages.
 // What bounds a block is its serial chain of code lookups; the ranges cut
@@ -40,29 +42,30 @@ constexpr uint32_t kWin = 2048;       // output positions expanded at a time (di
 constexpr uint32_t kWinPer = kWin / kCtaThreads;
 constexpr uint32_t kTokPer = 4;       // token slots per thread and batch
 constexpr uint32_t kCtaDistBits = 9;  // distance LUT index bits
-constexpr uint32_t kInWords = kCtaThreads * kRangeMax / 32 + 8;
+constexpr uint32_t kSegs = 4;           // a range is walked in quarters
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 
-// table entry: [4:0] bits of the code and its extra bits, bit 5 = length code,
-// bit 6 = not a literal, length or distance (end of block, or, by value:
-// invalid, or not in the LUT), bit 7 = literal, [23:8] token value without the
-// extra bits, [31:28] code length
-enum : uint32_t { kEntLen = 0x20, kEntStop = 0x40, kEntLit = 0x80 };
+// Table entry: [4:0] bits of the code and its extra bits, bit 5 = length code,
+// [23:8] token value without the extra bits, [30:27] code length; bit 31 =
+// not a literal, length or distance: end of block, or, by value, invalid, or
+// not in the LUT ([4:0] = 0).  The shift amounts sit where the shifts read them, so the
+// chain from one lookup to the next is mask, load, shift.
+enum : uint32_t { kEntLen = 0x20, kEntStop = 0x80000000u };
 enum : uint32_t { kStopEob = 0, kStopBad = 1, kStopLong = 2 };
 constexpr uint32_t kTokMatch = 0x8000u;  // a match's first slot: flag and length
 
 __device__ __forceinline__ uint32_t tok_lit_entry(uint32_t sym, uint32_t L) {
-  if (sym < 256) return L << 28 | sym << 8 | kEntLit | L;
-  if (sym == 256) return L << 28 | kStopEob << 8 | kEntStop | L;
+  if (sym < 256) return L << 27 | sym << 8 | L;
+  if (sym == 256) return kEntStop | L << 27 | kStopEob << 8;
   if (sym <= 285) {
     const uint32_t k = sym - 257;
-    return L << 28 | (kTokMatch + c_len_base[k]) << 8 | kEntLen | (L + c_len_extra[k]);
+    return L << 27 | (kTokMatch + c_len_base[k]) << 8 | kEntLen | (L + c_len_extra[k]);
   }
-  return L << 28 | kStopBad << 8 | kEntStop | L;
+  return kEntStop | kStopBad << 8;
 }
 __device__ __forceinline__ uint32_t tok_dist_entry(uint32_t sym, uint32_t L) {
-  if (sym < 30) return L << 28 | (uint32_t)(c_dist_base[sym] - 1) << 8 | (L + c_dist_extra[sym]);
-  return L << 28 | kStopBad << 8 | kEntStop | L;
+  if (sym < 30) return L << 27 | (uint32_t)(c_dist_base[sym] - 1) << 8 | (L + c_dist_extra[sym]);
+  return kEntStop | kStopBad << 8;
 }
 
 // the chunk's state, written by thread 0 (or warp 0) and read by all after a barrier
@@ -82,156 +85,303 @@ struct CtaCtl {
   uint32_t build_ok[2];
   uint32_t page_cur, page_prev, page_seq, n_pages;
   uint32_t min_need[2], min_term[2];
-  uint32_t round_slots, round_out, round_lanes, round_kind, round_pos;
+  uint32_t round_slots, round_lanes, round_kind, round_pos;
   int32_t carry_ms;         // match reaching into the next window: start (relative to it)
   uint32_t carry_len, carry_dist;
   uint32_t any_match, bad_dist, mark_max;
 };
 
+// A code beside its LUT: codes are canonical, so the length of the code at the
+// head of a 15-bit window (first bit = MSB) is the number of lengths l with
+// window >= lim[l], plus one, and its place among the codes sorted by length
+// and symbol is (window >> (15 - length)) + base[length].
+struct CodeIndex {
+  uint32_t lim[16], base[16];
+  uint16_t count[16], first[16], offs[16], next[16];
+};
+
 template <int LB>
 struct alignas(16) CtaSmem {
-  uint32_t lit_lut[1 << LB];
-  uint32_t dist_lut[1 << kCtaDistBits];
+  // literal/length LUT, then the distance LUT (at a power of two, so that its
+  // offset joins an index by OR)
+  uint32_t lut[(1 << LB) + (1 << kCtaDistBits)];
   uint16_t tok[kTokCap + 8];
   union {
-    HeaderScratch h;                           // block header
-    uint32_t in[kInWords + kInWords / 32 + 4]; // decode: the round's input words (padded by skew)
-    struct {                                   // expansion
-      uint32_t stage[kWin];
-      uint32_t bm[kWin / 32];                  // match starts
-      int32_t lastm[kWin / 32];                // last match start before each word's positions
+    HeaderScratch h;  // block header
+    struct {          // expansion
+      alignas(16) uint32_t stage[kWin];
+      uint32_t bm[kWin / 32];  // match starts
     };
   };
-  uint16_t lit_sorted[288], dist_sorted[32];
-  uint16_t lit_count[16], lit_first[16], lit_offs[16];
-  uint16_t dist_count[16], dist_first[16], dist_offs[16];
-  uint16_t dist_next[16];
+  uint32_t lit_ent[288], dist_ent[32];  // entries in canonical order
+  CodeIndex lit, dist;
   uint32_t end[kCtaThreads];
-  uint32_t scan_a[2][kCtaThreads / 32], scan_b[2][kCtaThreads / 32];
+  // per quarter of each range (but the last): [9:0] first boundary at or past
+  // its end, relative to the range's first bit, [31:10] lookups from there
+  uint32_t cp[kSegs - 1][kCtaThreads];
+  uint32_t scan[2][kCtaThreads / 32];
   CtaCtl c;
 };
 
-// word j of the round's input, skewed so that threads at the same place of
-// their ranges read different banks
-__device__ __forceinline__ uint32_t in_at(uint32_t j) { return j + (j >> 5); }
-
-// exclusive prefix sums of a and b over the CTA; totals in ta, tb.  One
-// barrier; `par` alternates between calls (0, 1, 0, ...).
+// exclusive prefix sum of a over the CTA, total in ta.  One barrier; `par`
+// alternates between calls (0, 1, 0, ...).
 template <int LB>
-__device__ __forceinline__ void cta_scan2(CtaSmem<LB>* S, uint32_t par, uint32_t& a, uint32_t& b,
-                                          uint32_t& ta, uint32_t& tb) {
+__device__ __forceinline__ uint32_t cta_scan(CtaSmem<LB>* S, uint32_t par, uint32_t a, uint32_t& ta) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t x = a, y = b;
+  uint32_t x = a;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, x, d), v = __shfl_up_sync(0xFFFFFFFFu, y, d);
-    if (lane >= d) {
-      x += u;
-      y += v;
-    }
+    const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, x, d);
+    if (lane >= d) x += u;
   }
-  if (lane == 31) {
-    S->scan_a[par][warp] = x;
-    S->scan_b[par][warp] = y;
-  }
+  if (lane == 31) S->scan[par][warp] = x;
   __syncthreads();
-  uint32_t pa = 0, pb = 0;
-  ta = tb = 0;
+  uint32_t pa = 0;
+  ta = 0;
 #pragma unroll
-  for (int w = 0; w < kCtaThreads / 32; w++) {
-    const uint32_t u = S->scan_a[par][w], v = S->scan_b[par][w];
-    if (w < warp) {
-      pa += u;
-      pb += v;
-    }
+  for (int w = 0; w < (int)kCtaThreads / 32; w++) {
+    const uint32_t u = S->scan[par][w];
+    if (w < warp) pa += u;
     ta += u;
-    tb += v;
   }
-  a = pa + x - a;
-  b = pb + y - b;
+  return pa + x - a;
 }
 
-// Codes longer than the LUT, or invalid: canonical search.  Returns the entry.
+// The entry of a code longer than the LUT, or kStopBad.
 template <int LB>
 __device__ __noinline__ uint32_t long_entry(const CtaSmem<LB>* S, uint32_t x, bool dist) {
+  const CodeIndex& I = dist ? S->dist : S->lit;
   const uint32_t rev = __brev(x) >> 17;  // 15 code bits, first bit = MSB
-  const uint16_t* count = dist ? S->dist_count : S->lit_count;
-  const uint16_t* first = dist ? S->dist_first : S->lit_first;
-  for (int L = 1; L <= 15; L++) {
-    const uint32_t idx = (rev >> (15 - L)) - first[L];
-    if (idx < count[L])
-      return dist ? tok_dist_entry(S->dist_sorted[S->dist_offs[L] + idx], (uint32_t)L)
-                  : tok_lit_entry(S->lit_sorted[S->lit_offs[L] + idx], (uint32_t)L);
-  }
-  return kStopBad << 8 | kEntStop;
+  uint32_t L = 1;
+#pragma unroll
+  for (int l = 1; l <= 15; l++) L += rev >= I.lim[l] ? 1u : 0u;
+  if (L > 15) return kEntStop | kStopBad << 8;
+  const uint32_t i = (rev >> (15 - L)) + I.base[L];
+  return dist ? S->dist_ent[i] : S->lit_ent[i];
 }
 
-// What one range decoded to.  A range that meets the end of the block or an
-// invalid code has term set; slots and outs then count up to there.
-struct RangeOut {
-  uint32_t end, slots, outs, term, term_pos;
-};
-enum : uint32_t { kTermNone = 0, kTermEob = 1, kTermBad = 2 };
+// One thread's bits: the next `q - p + 30` stream bits at bit 2 of hi:lo
+// (indexes into the LUT are byte offsets), the word after them in w.  No
+// branches: a divergent one costs about as much as a lookup.
+struct RangeBits {
+  const uint32_t* next;  // word after w
+  uint32_t lo, hi, w;
+  uint32_t p, q;  // position; refill when p >= q, which leaves 30 bits at least
 
-// Decode the symbols that start in [p, e) (bits relative to the staged
-// input).  One table lookup per iteration: a literal or a length code, or the
-// distance code of the length just read, so threads at literals and threads
-// inside matches run the same instructions.  guess: p may be no symbol
-// boundary; decode on past an end of block or an invalid code (from its next
-// bit) to find a likely end for the range.  kTok: write the tokens.
-template <int LB, bool kTok>
-__device__ __forceinline__ void walk_range(const CtaSmem<LB>* S, uint32_t p, uint32_t e, bool guess,
-                                           RangeOut& r, uint16_t* tok) {
-  constexpr uint32_t LM = (1u << LB) - 1, DM = (1u << kCtaDistBits) - 1;
-  uint32_t j = p >> 5, sh = p & 31;
-  uint32_t w0 = S->in[in_at(j)], w1 = S->in[in_at(j + 1)], w2 = S->in[in_at(j + 2)];
-  j += 3;
-  uint32_t slots = 0, outs = 0, is_len = 0;
-  uint32_t term = kTermNone, t_slots = 0, t_outs = 0, t_pos = 0;
-  while (is_len || p < e) {
-    const uint32_t x = __funnelshift_r(w0, w1, sh);
-    const uint32_t* t = is_len ? S->dist_lut + (x & DM) : S->lit_lut + (x & LM);
-    uint32_t ent = *t;
-    if (ent & kEntStop) {
-      if (((ent >> 8) & 3) == kStopLong) ent = long_entry<LB>(S, x, is_len != 0);
-      if (ent & kEntStop) {
-        if (kTok) break;  // the range's last symbol is the end of the block
-        if (term == kTermNone) {
-          const bool eob = ((ent >> 8) & 3) == kStopEob;
-          term = eob ? kTermEob : kTermBad;
-          t_slots = slots;
-          t_outs = outs;
-          t_pos = p + (eob ? ent & 31 : 0u);
+  __device__ __forceinline__ void refill_if_due() {
+#ifdef __CUDA_ARCH__
+    // 2 + the bits left (2 .. 32) is where the next word goes
+    asm("{\n\t"
+        ".reg .pred due;\n\t"
+        ".reg .u32 s, a, b;\n\t"
+        "setp.ge.u32 due, %4, %3;\n\t"
+        "sub.u32 s, %3, %4;\n\t"
+        "add.u32 s, s, 32;\n\t"
+        "shf.l.clamp.b32 a, 0, %2, s;\n\t"
+        "shf.l.clamp.b32 b, %2, 0, s;\n\t"
+        "@due or.b32 %0, %0, a;\n\t"
+        "@due or.b32 %1, %1, b;\n\t"
+        "@due add.u32 %3, %3, 32;\n\t"
+        "@due ld.global.u32 %2, [%5];\n\t"
+        "@due add.u64 %5, %5, 4;\n\t"
+        "}"
+        : "+r"(lo), "+r"(hi), "+r"(w), "+r"(q), "+r"(p), "+l"(next));
+#else
+    if (p < q) return;
+    const uint32_t s = q + 32 - p;
+    lo |= __funnelshift_lc(0, w, s);
+    hi |= __funnelshift_lc(w, 0, s);
+    q += 32;
+    w = *next++;
+#endif
+  }
+  // base: the word of position 0
+  __device__ __forceinline__ void seek(const uint32_t* base, uint32_t pos) {
+    const uint32_t* a = base + (pos >> 5);
+    const uint32_t x = a[0] >> (pos & 31);
+    w = a[1];
+    next = a + 2;
+    lo = x << 2;
+    hi = x >> 30;
+    p = pos;
+    q = (pos & ~31u) + 2;  // 32 - (pos & 31) bits in place
+    refill_if_due();
+  }
+  __device__ __forceinline__ void take(uint32_t ent) {  // ent[4:0] bits
+    lo = __funnelshift_r(lo, hi, ent);
+    hi = __funnelshift_r(hi, 0, ent);
+    p += ent & 31;
+    refill_if_due();
+  }
+};
+
+// what ended a range's walk before its end
+enum : uint32_t { kTermNone = 0, kTermEob = 1, kTermBad = 2 };
+constexpr uint32_t kNoCp = 0x3FFu;  // a quarter without a recorded boundary
+
+// One thread's range of a round: where it starts and ends, and the lookups
+// between (a literal is one, a match two).
+struct Range {
+  uint32_t start, end, slots;
+  uint32_t term, term_pos;  // met the end of the block or an invalid code there
+  bool guessed_on;          // walked on from a guess past a stop: starts nowhere
+};
+
+// Walk the range [first, first + r) (cut at e) from r.start on, positions
+// relative to `base`.  One table lookup per iteration: a literal or a length
+// code, or the distance code of the length just read, so threads at literals
+// and threads inside matches run the same instructions.  guess: the start may
+// be no symbol boundary; go on past a stop (from the next bit) to find a
+// likely end for the range.  Otherwise a stop ends the walk.  again: an earlier
+// walk of this round left its boundaries, and meeting one ends this walk: from
+// there on they agree.
+template <int LB>
+__device__ __forceinline__ void walk_range(CtaSmem<LB>* S, const uint32_t* base, uint32_t first,
+                                           uint32_t len, uint32_t e, bool guess, bool again,
+                                           Range& r) {
+  constexpr uint32_t LM = ((1u << LB) - 1) << 2, DM = ((1u << kCtaDistBits) - 1) << 2;
+  const uint32_t tid = threadIdx.x;
+  const char* lut = reinterpret_cast<const char*>(S->lut);
+  RangeBits b;
+  b.seek(base, r.start);
+  uint32_t slots = 0, valid_from = 0, seg = 0;
+  uint32_t mask = LM, off = 0;
+  r.term = kTermNone;
+  r.guessed_on = false;
+  bool met = false;
+  for (;; seg++) {
+    uint32_t es = seg == kSegs - 1 ? e : min(e, first + (seg + 1) * (len / kSegs));
+    if (b.p < es) do {
+      uint32_t ent = *reinterpret_cast<const uint32_t*>(lut + ((b.lo & mask) | off));
+      if (__builtin_expect((int32_t)ent < 0, 0)) {
+        if (((ent >> 8) & 3) == kStopLong) ent = long_entry<LB>(S, b.lo >> 2, off != 0);
+        if ((int32_t)ent < 0) {
+          if (guess) {
+            r.guessed_on = true;
+            valid_from = seg;  // boundaries before the stop lead to it
+            ent = 1;           // one bit on
+          } else {
+            const bool eob = ((ent >> 8) & 3) == kStopEob;
+            r.term = eob ? kTermEob : kTermBad;
+            r.term_pos = b.p + (eob ? (ent >> 27) & 15 : 0u);
+            slots--;
+            ent = 0;
+            es = 0;  // ends the walk
+          }
         }
-        if (!guess) break;
-        ent = 1;  // go on at the next bit
+      }
+      b.take(ent);
+      slots++;
+      mask = ent & kEntLen ? DM : LM;
+      off = ent & kEntLen ? 4u << LB : 0u;
+    } while (b.p < (off ? kNone : es));
+    if (r.term || seg == kSegs - 1) break;
+    const uint32_t at = b.p - first;
+    if (again) {
+      const uint32_t old = S->cp[seg][tid];
+      if ((old & 0x3FFu) == at) {
+        slots += old >> 10;
+        met = true;
+        break;
       }
     }
-    const uint32_t n = ent & 31;
-    const uint32_t v = (ent >> 8) + ((x & ~(0xFFFFFFFFu << n)) >> (ent >> 28));
-    if (kTok) tok[slots] = (uint16_t)v;
-    is_len = ent & kEntLen;
-    slots++;
-    outs += is_len ? (v & 0x1FFu) : (ent >> 7) & 1u;
-    p += n;
-    sh += n;
-    if (sh >= 32) {
-      sh -= 32;
-      w0 = w1;
-      w1 = w2;
-      w2 = S->in[in_at(j)];
-      j++;
-    }
+    S->cp[seg][tid] = at | slots << 10;
   }
-  r.end = p;
-  r.term = term;
-  r.slots = term ? t_slots : slots;
-  r.outs = term ? t_outs : outs;
-  r.term_pos = t_pos;
+  // seg quarters were passed; their lookups become those left to the end
+  for (uint32_t k = 0; k < kSegs - 1; k++) {
+    if (r.term || (guess && k < valid_from)) S->cp[k][tid] = kNoCp;
+    else if (k < seg) S->cp[k][tid] = (S->cp[k][tid] & 0x3FFu) | (slots - (S->cp[k][tid] >> 10)) << 10;
+  }
+  r.slots = slots;
+  if (!r.term && !met) r.end = b.p;
+}
+
+// The tokens of the symbols that start in [start, e), n of them, to tok.
+template <int LB>
+__device__ __forceinline__ void write_tokens(const CtaSmem<LB>* S, const uint32_t* base,
+                                             uint32_t start, uint32_t n, uint16_t* tok) {
+  constexpr uint32_t LM = ((1u << LB) - 1) << 2, DM = ((1u << kCtaDistBits) - 1) << 2;
+  const char* lut = reinterpret_cast<const char*>(S->lut);
+  RangeBits b;
+  b.seek(base, start);
+  uint32_t mask = LM, off = 0;
+  for (uint32_t i = 0; i < n; i++) {
+    uint32_t ent = *reinterpret_cast<const uint32_t*>(lut + ((b.lo & mask) | off));
+    if (__builtin_expect((int32_t)ent < 0, 0)) ent = long_entry<LB>(S, b.lo >> 2, off != 0);
+    // value + extra bits: the code's bits cut off the front of what it takes
+    const uint32_t x = (b.lo >> 2) & ~(0xFFFFFFFFu << (ent & 31));
+    tok[i] = (uint16_t)((ent >> 8) + (x >> (ent >> 27)));
+    b.take(ent);
+    mask = ent & kEntLen ? DM : LM;
+    off = ent & kEntLen ? 4u << LB : 0u;
+  }
+}
+
+// A code's index by one warp: counts, first codes, limits, and the symbols'
+// entries in canonical order.  lens[0..n) in shared memory, n <= 320.
+// Acceptance follows zlib (canon_build).
+template <typename EntryFn>
+__device__ __noinline__ bool index_code(const uint8_t* lens, int n, CodeIndex* I, uint32_t* ent,
+                                        int lane, EntryFn entry) {
+  if (lane < 16) I->count[lane] = 0;
+  __syncwarp();
+  // rank of each symbol among those of its length, in symbol order
+  uint32_t rank[10], len[10];
+#pragma unroll
+  for (int g = 0; g < 10; g++) {
+    const int s = 32 * g + lane;
+    len[g] = s < n ? lens[s] : 0;
+    rank[g] = 0;
+    if (32 * g >= n) continue;
+    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, len[g]);
+    const uint32_t before = I->count[len[g]];
+    rank[g] = before + __popc(peers & ((1u << lane) - 1));
+    __syncwarp();
+    if (len[g] && (__ffs(peers) - 1) == lane) I->count[len[g]] = (uint16_t)(before + __popc(peers));
+    __syncwarp();
+  }
+  // lane L: first code, offset and limit of length L; Kraft sum in units of 2^-15
+  const uint32_t cnt = lane >= 1 && lane <= 15 ? I->count[lane] : 0;
+  uint32_t first = 0, offs = 0, kraft = 0, maxl = 0;
+#pragma unroll
+  for (int l = 1; l <= 15; l++) {
+    const uint32_t c = __shfl_sync(0xFFFFFFFFu, cnt, l);
+    if (l < lane) {
+      first += c << ((lane - l) & 31);
+      offs += c;
+    }
+    kraft += c << (15 - l);
+    if (c) maxl = l;
+  }
+  if (lane >= 1 && lane <= 15) {
+    I->lim[lane] = (first + cnt) << (15 - lane);
+    I->base[lane] = offs - first;
+    I->offs[lane] = (uint16_t)offs;
+  }
+  const bool ok = kraft <= 1u << 15 && (kraft == 1u << 15 || maxl <= 1);
+  __syncwarp();
+  if (!ok) return false;
+#pragma unroll
+  for (int g = 0; g < 10; g++)
+    if (len[g]) ent[I->offs[len[g]] + rank[g]] = entry(32u * g + lane, len[g]);
+  __syncwarp();
+  return true;
+}
+
+// LUT entry i: the entry of the code at the head of i's low TB bits
+template <int TB>
+__device__ __forceinline__ uint32_t lut_value(uint32_t i, const uint32_t* lim, const CodeIndex* I,
+                                              const uint32_t* ent) {
+  const uint32_t rev = __brev(i) >> 17;
+  uint32_t L = 1;
+#pragma unroll
+  for (int l = 1; l <= TB; l++) L += rev >= lim[l] ? 1u : 0u;
+  if (L > TB) return kEntStop | kStopLong << 8;
+  return ent[(rev >> (15 - L)) + I->base[L]];
 }
 
 // Both code tables from h.lens (whole CTA).  Warp 0 sorts the
-// literal/length code, warp 1 the distance code, all threads fill the LUTs.
+// literal/length code, warp 1 the distance code, all threads fill the LUT.
 // Distance lengths sit at lens + 288.
 template <int LB>
 __device__ __forceinline__ bool cta_build_tables(CtaSmem<LB>* S) {
@@ -239,25 +389,22 @@ __device__ __forceinline__ bool cta_build_tables(CtaSmem<LB>* S) {
   if (warp < 2) {
     bool ok;
     if (warp == 0)
-      ok = canon_build(S->h.lens, (int)S->c.nlen, S->lit_count, S->lit_first, S->lit_offs,
-                       S->lit_sorted, S->h.next, lane);
+      ok = index_code(S->h.lens, (int)S->c.nlen, &S->lit, S->lit_ent, lane, tok_lit_entry);
     else
-      ok = canon_build(S->h.lens + 288, (int)S->c.ndist, S->dist_count, S->dist_first, S->dist_offs,
-                       S->dist_sorted, S->dist_next, lane);
+      ok = index_code(S->h.lens + 288, (int)S->c.ndist, &S->dist, S->dist_ent, lane, tok_dist_entry);
     if (lane == 0) S->c.build_ok[warp] = ok;
   }
   __syncthreads();
   if (!S->c.build_ok[0] || !S->c.build_ok[1]) return false;
-  for (uint32_t i = threadIdx.x; i < (1u << LB); i += kCtaThreads) {
-    const uint32_t e = lut_entry<LB>(i, S->lit_count, S->lit_first, S->lit_offs, S->lit_sorted,
-                                     tok_lit_entry);
-    S->lit_lut[i] = e ? e : kStopLong << 8 | kEntStop;
-  }
-  for (uint32_t i = threadIdx.x; i < (1u << kCtaDistBits); i += kCtaThreads) {
-    const uint32_t e = lut_entry<(int)kCtaDistBits>(i, S->dist_count, S->dist_first, S->dist_offs,
-                                                    S->dist_sorted, tok_dist_entry);
-    S->dist_lut[i] = e ? e : kStopLong << 8 | kEntStop;
-  }
+  uint32_t lim[LB + 1];
+#pragma unroll
+  for (int l = 1; l <= LB; l++) lim[l] = S->lit.lim[l];
+  for (uint32_t i = threadIdx.x; i < (1u << LB); i += kCtaThreads)
+    S->lut[i] = lut_value<LB>(i, lim, &S->lit, S->lit_ent);
+#pragma unroll
+  for (int l = 1; l <= (int)kCtaDistBits; l++) lim[l] = S->dist.lim[l];
+  for (uint32_t i = threadIdx.x; i < (1u << kCtaDistBits); i += kCtaThreads)
+    S->lut[(1u << LB) + i] = lut_value<(int)kCtaDistBits>(i, lim, &S->dist, S->dist_ent);
   __syncthreads();
   return true;
 }
@@ -287,24 +434,26 @@ __device__ __forceinline__ bool cta_page(CtaSmem<LB>* S, const PagePool& pool, u
   return S->c.page_cur != kNoPage;
 }
 
-// Expand a round's tokens (slots [0, n), total_out entries) after the
-// chunk's entry position S->c.o.  Output goes in windows of kWin positions
+// Expand a round's tokens (slots [0, n)) after the chunk's entry position
+// S->c.o, and move that on (thread 0, before a barrier).  Output goes in windows of kWin positions
 // aligned to kWin, so a window lies in one page.  Batches of kTokPer slots a
 // thread get their positions from a block scan; literals and match records go
 // to the window's stage (a match's record at its first position, a bit in
-// bm).  Then every position finds the last match start at or before it, and a
-// position that the match covers takes its source: the history in the pages
-// (or the marker / zero before the chunk), or a position of this window,
-// followed by pointer jumping through the stage.  All positions of a window
-// resolve in parallel, and a window without matches goes out as it is.
+// bm).  Then every thread takes kWinPer positions in a row, finds the match
+// that reaches into them and those that start in them, and gives each covered
+// position its source: the history in the pages (or the marker / zero before
+// the chunk), or a position of this window, followed by pointer jumping
+// through the stage.  Neighbours mostly share a match, so a match is looked at
+// once per thread, its sources are loaded from one address, and the window
+// leaves in 16-byte stores; a window without matches goes out as it is.
 // Returns kOk, kBadDeflate (a distance beyond the window) or kPoolExhausted.
 template <int LB>
 __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool& pool, uint32_t n,
-                                                 uint32_t total_out, bool zero_window) {
+                                                 bool zero_window) {
   const uint32_t tid = threadIdx.x;
   const uint64_t o = S->c.o;
   const uint64_t base = o & ~(uint64_t)(kWin - 1);  // positions below are relative to this
-  const uint32_t rel0 = (uint32_t)(o - base), rel_end = rel0 + total_out;
+  const uint32_t rel0 = (uint32_t)(o - base);
   uint32_t lo = rel0;          // next position to write
   uint32_t b0 = 0;             // first slot of the batch
   uint32_t bpos = rel0, bend;  // positions of the batch
@@ -337,15 +486,15 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
       pos[k] = sum;
       sum += len[k];
     }
-    uint32_t a = sum, z = 0, ta, tz;
-    cta_scan2(S, par, a, z, ta, tz);
+    uint32_t ta;
+    const uint32_t a = cta_scan(S, par, sum, ta);
     par ^= 1;
 #pragma unroll
     for (uint32_t k = 0; k < kTokPer; k++) pos[k] += bpos + a;
     bend = bpos + ta;
   };
   load_batch();
-  while (lo < rel_end) {
+  for (;;) {
     const uint32_t wbase = lo & ~(kWin - 1), wend = wbase + kWin;
     if (!cta_page(S, pool, base + wbase)) return kPoolExhausted;
     for (;;) {
@@ -370,110 +519,155 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
       load_batch();
     }
     __syncthreads();
-    const uint32_t hi = min(wend, rel_end) - wbase, l0 = lo - wbase;
+    const uint32_t hi = min(wend, bend) - wbase, l0 = lo - wbase;
     uint16_t* page = pool.data + (size_t)S->c.page_cur * kPageEntries +
                      ((uint32_t)(base + wbase) & (kPageEntries - 1));
     const bool matches = S->c.any_match != 0 || S->c.carry_len != 0;
+    // this thread's positions: e0 .. e0 + 7
+    const uint32_t e0 = kWinPer * tid;
+    uint32_t st[kWinPer];  // a position's value, or (bit 31) a reference into the window
+    {
+      const uint4 a = reinterpret_cast<const uint4*>(S->stage)[2 * tid];
+      const uint4 b = reinterpret_cast<const uint4*>(S->stage)[2 * tid + 1];
+      st[0] = a.x, st[1] = a.y, st[2] = a.z, st[3] = a.w;
+      st[4] = b.x, st[5] = b.y, st[6] = b.z, st[7] = b.w;
+    }
     if (matches) {
-      const uint16_t* pprev = pool.data + (size_t)S->c.page_prev * kPageEntries;
-      const uint16_t* pcur = pool.data + (size_t)S->c.page_cur * kPageEntries;
+      const int lane = tid & 31;
       const int32_t page_off = (int32_t)((uint32_t)(base + wbase) & (kPageEntries - 1));
+      const uint16_t* pprev = pool.data + (size_t)S->c.page_prev * kPageEntries + kPageEntries;
+      const uint16_t* pcur = pool.data + (size_t)S->c.page_cur * kPageEntries;
       const int64_t wabs = (int64_t)(base + wbase);
       const int32_t c_ms = S->c.carry_ms;
       const uint32_t c_len = S->c.carry_len, c_dist = S->c.carry_dist;
-      if (tid < kWin / 32) {
-        int32_t m = -1;
-        // a match is at most 258 long: nine words back
-        for (int32_t w = (int32_t)tid - 1; w >= 0 && w + 9 >= (int32_t)tid; w--)
-          if (S->bm[w]) {
-            m = 32 * w + 31 - __clz(S->bm[w]);
-            break;
-          }
-        S->lastm[tid] = m;
+      // the last match start before e0: in this warp, else in the nine words
+      // before the warp's (a match is at most 258 long), else the match that
+      // reaches in from the window before
+      uint32_t bits = (S->bm[tid >> 2] >> (8 * (tid & 3))) & 0xFFu;
+      const int32_t own = (int32_t)e0 + 31 - __clz(bits | 1u);
+      const uint32_t have = __ballot_sync(0xFFFFFFFFu, bits != 0);
+      const int32_t wi = (int32_t)(tid >> 5) * 8 - 1 - lane;
+      const uint32_t pw = lane < 9 && wi >= 0 ? S->bm[wi] : 0u;
+      const uint32_t havep = __ballot_sync(0xFFFFFFFFu, pw != 0);
+      const int32_t far = __shfl_sync(0xFFFFFFFFu, 32 * wi + 31 - __clz(pw | 1u), __ffs(havep | 0x80000000u) - 1);
+      const uint32_t below = have & ((1u << lane) - 1);
+      const int32_t near = __shfl_sync(0xFFFFFFFFu, own, 31 - __clz(below | 1u));
+      const int32_t at = below ? near : (havep ? far : -1);
+      int32_t ms = at >= 0 ? at : c_ms;
+      uint32_t ml = c_len, md = c_dist;
+      if (at >= 0) {
+        const uint32_t d = S->stage[at];
+        ml = d >> 16;
+        md = (d & 0xFFFFu) + 1;
       }
-      __syncthreads();
-      // each position's new state: a value, or (bit 31) a reference into the window
-      uint32_t st[kWinPer];
-      uint32_t todo = 0;  // bit k: position k is covered by a match
-#pragma unroll
-      for (uint32_t k = 0; k < kWinPer; k++) {
-        const uint32_t e = tid + kCtaThreads * k;
-        st[k] = 0;
-        if (e < l0 || e >= hi) continue;
-        const uint32_t m = S->bm[e >> 5] & (0xFFFFFFFFu >> (31 - (e & 31)));
-        int32_t ms = m ? (int32_t)((e & ~31u) + 31 - __clz(m)) : S->lastm[e >> 5];
-        uint32_t ml, md;
-        if (ms >= 0) {
-          const uint32_t d = S->stage[ms];
-          ml = d >> 16;
-          md = (d & 0xFFFFu) + 1;
-        } else {
-          ms = c_ms;
-          ml = c_len;
-          md = c_dist;
-        }
-        const uint32_t jj = (uint32_t)((int32_t)e - ms);
-        if (e + 1 == hi) {  // a match that goes on in the next window
-          const bool more = jj < ml && (uint32_t)((int32_t)hi - ms) < ml;
-          S->c.carry_ms = ms - (int32_t)kWin;
-          S->c.carry_len = more ? ml : 0u;
-          S->c.carry_dist = md;
-        }
-        if (jj >= ml) continue;
-        todo |= 1u << k;
-        // every entry of an overlapping match maps to one before the match
-        const int32_t src = md < ml ? ms - (int32_t)md + (int32_t)(md == 1 ? 0u : jj % md)
-                                    : (int32_t)e - (int32_t)md;
-        if (src >= (int32_t)l0) {
-          st[k] = 0x80000000u | (uint32_t)src;
-        } else if (wabs + src >= 0) {
-          const int32_t q = page_off + src;
-          st[k] = q >= 0 ? pcur[q] : pprev[q + (int32_t)kPageEntries];
-        } else {
-          st[k] = zero_window ? 0u : (uint32_t)((int64_t)(kMarkerBase + kWindow) + wabs + src) & 0xFFFFu;
-        }
-      }
-      __syncthreads();
-#pragma unroll
-      for (uint32_t k = 0; k < kWinPer; k++)
-        if ((todo >> k) & 1) S->stage[tid + kCtaThreads * k] = st[k];
-      // references: a position takes its source's value, or the source's own
-      // reference (always further back), until none is left
+      uint32_t cover = 0;  // bit i: position e0 + i is inside a match
       for (;;) {
-        uint32_t left = 0;
+        // positions [x0, x1) of this thread's eight that the match covers
+        const uint32_t nx = bits ? (uint32_t)__ffs(bits) - 1 : kWinPer;
+        const int32_t x0 = max(0, ms - (int32_t)e0);
+        const int32_t x1 = min((int32_t)min(nx, hi - min(hi, e0)), ms + (int32_t)ml - (int32_t)e0);
+        if (x0 < x1) {
+          const uint32_t jj = (uint32_t)((int32_t)e0 + x0 - ms), cnt = (uint32_t)(x1 - x0);
+          // every entry of an overlapping match maps to one before the match:
+          // its place mod the distance (the quotient is exact for jj < 258)
+          uint32_t r = jj;
+          if (md < ml) r -= (uint32_t)__fdividef((float)jj + 0.5f, (float)md) * md;
+          const int32_t s0 = ms - (int32_t)md + (int32_t)r, s1 = s0 + (int32_t)cnt - 1;
+          const uint32_t mine = ((1u << x1) - 1) & ~((1u << x0) - 1);
+          cover |= mine;
+          const bool wrap = r + cnt > md;
+          if (!wrap && (s0 >= (int32_t)l0 || wabs + s1 < 0)) {
+            // references into the window, or markers (zeros) before the chunk
+            const bool ref = s0 >= (int32_t)l0;
+            const uint32_t v0 = ref ? 0x80000000u | (uint32_t)s0
+                                    : (uint32_t)((int64_t)(kMarkerBase + kWindow) + wabs + s0);
+            const bool zero = !ref && zero_window;
 #pragma unroll
-        for (uint32_t k = 0; k < kWinPer; k++) left |= st[k];
-        if (!__syncthreads_or((int)(left >> 31))) break;
+            for (uint32_t i = 0; i < kWinPer; i++)
+              if ((mine >> i) & 1) st[i] = zero ? 0u : v0 + i - (uint32_t)x0;
+          } else if (!wrap && s1 < (int32_t)l0 && wabs + s0 >= 0 &&
+                     (page_off + s0 >= 0) == (page_off + s1 >= 0)) {
+            const uint16_t* from = (page_off + s0 >= 0 ? pcur : pprev) + (page_off + s0 - x0);
 #pragma unroll
-        for (uint32_t k = 0; k < kWinPer; k++)
-          if (st[k] >> 31) {
-            st[k] = *(volatile uint32_t*)&S->stage[st[k] & 0xFFFFu];
-            *(volatile uint32_t*)&S->stage[tid + kCtaThreads * k] = st[k];
+            for (uint32_t i = 0; i < kWinPer; i++)
+              if ((mine >> i) & 1) st[i] = from[i];
+          } else {
+#pragma unroll
+            for (uint32_t i = 0; i < kWinPer; i++) {
+              if (!((mine >> i) & 1)) continue;
+              const int32_t sr = ms - (int32_t)md + (int32_t)r;
+              r = r + 1 == md ? 0u : r + 1;
+              const int32_t q = page_off + sr;
+              if (sr >= (int32_t)l0) st[i] = 0x80000000u | (uint32_t)sr;
+              else if (wabs + sr >= 0) st[i] = (q >= 0 ? pcur : pprev)[q];
+              else st[i] = zero_window ? 0u : (uint32_t)((int64_t)(kMarkerBase + kWindow) + wabs + sr);
+            }
           }
+        }
+        if (!bits) break;
+        bits &= bits - 1;
+        ms = (int32_t)(e0 + nx);
+        const uint32_t d = S->stage[ms];
+        ml = d >> 16;
+        md = (d & 0xFFFFu) + 1;
+      }
+      uint32_t left = 0;
+#pragma unroll
+      for (uint32_t i = 0; i < kWinPer; i++) left |= (cover >> i) & 1 ? st[i] : 0u;
+      const bool any_ref = __syncthreads_or((int)(left >> 31));
+      if (hi - 1 - e0 < kWinPer) {  // the last position's match may go on in the next window
+        S->c.carry_ms = ms - (int32_t)kWin;
+        S->c.carry_len = ms + (int32_t)ml > (int32_t)hi ? ml : 0u;
+        S->c.carry_dist = md;
       }
       if (tid < kWin / 32) S->bm[tid] = 0;
       if (tid == 0) S->c.any_match = 0;
-      if (!zero_window) {
-        uint32_t mk = 0;
+      if (any_ref) {
+        if (cover) {
+          reinterpret_cast<uint4*>(S->stage)[2 * tid] = make_uint4(st[0], st[1], st[2], st[3]);
+          reinterpret_cast<uint4*>(S->stage)[2 * tid + 1] = make_uint4(st[4], st[5], st[6], st[7]);
+        }
+        // references: a position takes its source's value, or the source's own
+        // reference (always further back), until none is left
+        for (;;) {
+          left = 0;
 #pragma unroll
-        for (uint32_t k = 0; k < kWinPer; k++)
-          if (st[k] >= kMarkerBase) mk = tid + kCtaThreads * k + 1;
-        mk = __reduce_max_sync(0xFFFFFFFFu, mk);
-        if (mk && (tid & 31) == 0) atomicMax(&S->c.mark_max, mk);
+          for (uint32_t i = 0; i < kWinPer; i++) left |= (cover >> i) & 1 ? st[i] : 0u;
+          if (!__syncthreads_or((int)(left >> 31))) break;
+          if (left >> 31) {
+#pragma unroll
+            for (uint32_t i = 0; i < kWinPer; i++)
+              if ((cover >> i) & 1 && st[i] >> 31) {
+                st[i] = *(volatile uint32_t*)&S->stage[st[i] & 0xFFFFu];
+                *(volatile uint32_t*)&S->stage[e0 + i] = st[i];
+              }
+          }
+        }
       }
     }
-    // out to the page, two entries per store
-#pragma unroll
-    for (uint32_t k = 0; k < kWinPer / 2; k++) {
-      const uint32_t e = 2 * (tid + kCtaThreads * k);
-      if (e + 1 < l0 || e >= hi) continue;
-      const uint2 v = *reinterpret_cast<const uint2*>(&S->stage[e]);
-      if (e >= l0 && e + 1 < hi) {
-        *reinterpret_cast<uint32_t*>(page + e) = v.x | v.y << 16;
-      } else if (e >= l0) {
-        page[e] = (uint16_t)v.x;
+    // out to the page, eight entries per store
+    {
+      const uint4 v = make_uint4(__byte_perm(st[0], st[1], 0x5410), __byte_perm(st[2], st[3], 0x5410),
+                                 __byte_perm(st[4], st[5], 0x5410), __byte_perm(st[6], st[7], 0x5410));
+      const bool full = e0 >= l0 && e0 + kWinPer <= hi;
+      if (full) {
+        *reinterpret_cast<uint4*>(page + e0) = v;
       } else {
-        page[e + 1] = (uint16_t)v.y;
+#pragma unroll
+        for (uint32_t i = 0; i < kWinPer; i++)
+          if (e0 + i >= l0 && e0 + i < hi) page[e0 + i] = (uint16_t)st[i];
+      }
+      if (matches && !zero_window) {
+        uint32_t mk = 0;
+        if ((v.x | v.y | v.z | v.w) & 0x80008000u) {
+#pragma unroll
+          for (uint32_t i = 0; i < kWinPer; i++)
+            if (e0 + i >= l0 && e0 + i < hi && (st[i] & 0x8000u)) mk = e0 + i + 1;
+        }
+        if (__any_sync(0xFFFFFFFFu, mk != 0)) {
+          mk = __reduce_max_sync(0xFFFFFFFFu, mk);
+          if ((tid & 31) == 0) atomicMax(&S->c.mark_max, mk);
+        }
       }
     }
     __syncthreads();
@@ -483,12 +677,14 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
       S->c.mark_max = 0;
     }
     lo = wbase + hi;
-    if (bend <= wend && lo < rel_end) {
+    if (bend <= wend) {  // the batch is used up
       b0 += kTokPer * kCtaThreads;
+      if (b0 >= n) break;
       bpos = bend;
       load_batch();
     }
   }
+  if (tid == 0) S->c.o = base + lo;
   return kOk;
 }
 
@@ -523,29 +719,25 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
     const uint64_t span = end - pos;
     const uint32_t pend = p0 + (uint32_t)min(span, (uint64_t)r * kCtaThreads);
     const uint32_t lanes = (pend - p0 + r - 1) / r;
-    // stage the input words (zeros past the stream's end)
-    const uint32_t nw = (pend >> 5) + 6;
-    for (uint32_t j = tid; j < nw; j += kCtaThreads)
-      S->in[in_at(j)] = w0 + j < trunc ? in32[w0 + j] : 0u;
+    const uint32_t* base = in32 + w0;
     if (tid < 2) S->c.min_need[tid] = S->c.min_term[tid] = kNone;
-    __syncthreads();
     // 1. from the guessed starts
     const bool active = tid < lanes;
-    const uint32_t e = min(p0 + (tid + 1) * r, pend);
-    uint32_t start = p0 + tid * r;
-    RangeOut ro{};
+    const uint32_t first = p0 + tid * r, e = min(first + r, pend);
+    Range ra{};
+    ra.start = first;
     if (active) {
-      walk_range<LB, false>(S, start, e, tid > 0, ro, nullptr);
-      S->end[tid] = ro.end;
+      walk_range<LB>(S, base, first, r, e, tid > 0, false, ra);
+      S->end[tid] = ra.end;
     }
     // 2. from the end of the range before, until nothing moves
     uint32_t last = kNone;  // range that holds the end of the block (kNone: not in this round)
     for (uint32_t it = 0;; it ^= 1) {
       __syncthreads();
-      const uint32_t s1 = active && tid ? S->end[tid - 1] : start;
-      const bool need = active && s1 != start;
+      const uint32_t s1 = active && tid ? S->end[tid - 1] : ra.start;
+      const bool need = active && (s1 != ra.start || ra.guessed_on);
       const uint32_t mn = __reduce_min_sync(0xFFFFFFFFu, need ? tid : kNone);
-      const uint32_t mt = __reduce_min_sync(0xFFFFFFFFu, active && ro.term ? tid : kNone);
+      const uint32_t mt = __reduce_min_sync(0xFFFFFFFFu, active && ra.term ? tid : kNone);
       if ((tid & 31) == 0) {
         if (mn != kNone) atomicMin(&S->c.min_need[it], mn);
         if (mt != kNone) atomicMin(&S->c.min_term[it], mt);
@@ -556,25 +748,22 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
       if (first_need == kNone || last < first_need) break;
       if (tid == 0) S->c.min_need[it ^ 1] = S->c.min_term[it ^ 1] = kNone;
       if (need) {
-        start = s1;
-        const uint32_t old = ro.end;
-        walk_range<LB, false>(S, start, e, false, ro, nullptr);
-        if (ro.term) ro.end = old;  // unknown past the stop: keep the guess
-        S->end[tid] = ro.end;
+        ra.start = s1;
+        walk_range<LB>(S, base, first, r, e, false, true, ra);
+        S->end[tid] = ra.end;
       }
     }
     // 3. places in the token list; ranges beyond its capacity wait for the next round
     const uint32_t used = last != kNone ? last + 1 : lanes;
     const bool in_use = tid < used;
-    uint32_t slots = in_use ? ro.slots : 0u, outs = in_use ? ro.outs : 0u, ts, to;
-    const uint32_t my_slots = slots;
-    cta_scan2(S, 0, slots, outs, ts, to);
+    uint32_t ts;
+    const uint32_t my_slots = in_use ? ra.slots : 0u;
+    const uint32_t slot0 = cta_scan(S, 0, my_slots, ts);
     if (ts > kTokCap) {
-      const uint32_t fit = (uint32_t)__syncthreads_count(in_use && slots + my_slots <= kTokCap);
+      const uint32_t fit = (uint32_t)__syncthreads_count(in_use && slot0 + my_slots <= kTokCap);
       if (tid == fit) {
-        S->c.round_slots = slots;
-        S->c.round_out = outs;
-        S->c.round_pos = start;  // = the end of range fit - 1
+        S->c.round_slots = slot0;
+        S->c.round_pos = ra.start;  // = the end of range fit - 1
       }
       if (tid == 0) {
         S->c.round_lanes = fit;
@@ -584,13 +773,12 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
       rcap = max(kRangeMin, min(rcap, (uint32_t)((uint64_t)r * kTokCap / ts * 9 / 10)) & ~31u);
     } else if (tid == used - 1) {
       S->c.round_slots = ts;
-      S->c.round_out = to;
       S->c.round_lanes = used;
-      S->c.round_kind = ro.term;
-      S->c.round_pos = ro.term ? ro.term_pos : ro.end;
+      S->c.round_kind = ra.term;
+      S->c.round_pos = ra.term ? ra.term_pos : ra.end;
     }
     __syncthreads();
-    const uint32_t n_lanes = S->c.round_lanes, n_slots = S->c.round_slots, n_out = S->c.round_out;
+    const uint32_t n_lanes = S->c.round_lanes, n_slots = S->c.round_slots;
     const uint32_t kind = S->c.round_kind;
     const uint64_t new_pos = w0 * 32 + S->c.round_pos;
     if (kind == kTermBad) {
@@ -598,14 +786,11 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
       if (tid == 0) S->c.status = kBadDeflate;
       break;
     }
-    if (tid < n_lanes) {
-      RangeOut rw;
-      walk_range<LB, true>(S, start, e, false, rw, S->tok + slots);
-    }
+    if (tid < n_lanes) write_tokens<LB>(S, base, ra.start, my_slots, S->tok + slot0);
     __syncthreads();
     // 4. expansion
-    if (n_out) {
-      const int32_t st = expand_tokens<LB>(S, pool, n_slots, n_out, zero_window);
+    if (n_slots) {
+      const int32_t st = expand_tokens<LB>(S, pool, n_slots, zero_window);
       if (st != kOk) {
         __syncthreads();
         if (tid == 0) S->c.status = st;
@@ -616,7 +801,6 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
     __syncthreads();
     if (tid == 0) {
       S->c.pos = new_pos;
-      S->c.o += n_out;
       if (kind == kTermNone && passed && new_pos != target) S->c.passed = 1;
     }
     __syncthreads();

@@ -175,7 +175,7 @@ struct gzgpu_ctx {
   int dev = 0, sms = 148;
   cudaStream_t st = nullptr;
   size_t chunk_bytes = 0;
-  int lut_bits = 10;
+  int lut_bits = 11;
   bool autotune = false;
   bool ring = false;  // history layout of the inflate kernel (false = pages)
   int ctas_per_sm = 3;  // page kernel CTAs per SM (3 or 4)
@@ -221,7 +221,12 @@ struct gzgpu_ctx {
     return kOk;
   }
 
-  cudaError_t launch_decode(uint32_t* d_work_count) {
+  // d_work_count: the work list's length on the device; n_work: the same on
+  // the host.  With fewer chunks than resident CTAs, one CTA per chunk: the
+  // hardware spreads a small grid over the SMs, while in a full grid the
+  // chunks would go to whichever CTAs come first, several to an SM.
+  cudaError_t launch_decode(uint32_t* d_work_count, uint32_t n_work) {
+    const int blocks = (int)std::min<uint32_t>((uint32_t)decode_blocks, std::max(n_work, 1u));
     PagePool pool{pages.as<uint16_t>(), owner.as<uint32_t>(), seq.as<uint32_t>(),
                   counters.as<uint32_t>() + 2, (uint32_t)(pages.cap / (kPageEntries * 2))};
     pool.cap = (uint32_t)std::min<uint64_t>(pool.cap, std::min(owner.cap, seq.cap) / 4);
@@ -238,15 +243,15 @@ struct gzgpu_ctx {
       case 11:
         return launch_inflate<11>(ring, ctas_per_sm, job_sync, cur_in, descs.as<ChunkDesc>(), results.as<ChunkResult>(),
                                   work.as<uint32_t>(), d_work_count, counters.as<uint32_t>() + 3,
-                                  pool, decode_blocks, st);
+                                  pool, blocks, st);
       case 12:
         return launch_inflate<12>(ring, ctas_per_sm, job_sync, cur_in, descs.as<ChunkDesc>(), results.as<ChunkResult>(),
                                   work.as<uint32_t>(), d_work_count, counters.as<uint32_t>() + 3,
-                                  pool, decode_blocks, st);
+                                  pool, blocks, st);
       default:
         return launch_inflate<10>(ring, ctas_per_sm, job_sync, cur_in, descs.as<ChunkDesc>(), results.as<ChunkResult>(),
                                   work.as<uint32_t>(), d_work_count, counters.as<uint32_t>() + 3,
-                                  pool, decode_blocks, st);
+                                  pool, blocks, st);
     }
   }
 
@@ -334,7 +339,7 @@ int gzgpu_ctx::job_tuned(const std::vector<StreamSpec>& S, std::vector<StreamOut
   uint64_t total_in = 0;
   for (const StreamSpec& s : S) total_in += s.len;
   // jobs of a kind not tuned yet start from the defaults
-  const TuneCfg dflt{pick_chunk_bytes(total_in), 10, 3};
+  const TuneCfg dflt{pick_chunk_bytes(total_in), 11, 3};
   apply(dflt);
   int rc = run(S, R);
   if (rc != kOk || tune_cache.count(last_key)) return rc;
@@ -361,7 +366,7 @@ int gzgpu_ctx::job_tuned(const std::vector<StreamSpec>& S, std::vector<StreamOut
     double ms = trial(t);
     if (ms < best_ms) best_ms = ms, best = t;
   }
-  for (int lb : {11, 12}) {
+  for (int lb : {10, 12}) {
     TuneCfg t = best;
     t.lut_bits = lb;
     double ms = trial(t);
@@ -429,7 +434,7 @@ int gzgpu_ctx::regrow(std::vector<ChunkDesc>& hd, std::vector<ChunkResult>& hr, 
     cudaMemcpyAsync(counters.as<uint32_t>() + 1, &nw, 4, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(counters.as<uint32_t>() + 2, &used, 4, cudaMemcpyHostToDevice, st);
     cudaEventRecord(ev[8], st);
-    if ((rc = check(launch_decode(counters.as<uint32_t>() + 1)))) return rc;
+    if ((rc = check(launch_decode(counters.as<uint32_t>() + 1, nw)))) return rc;
     cudaEventRecord(ev[9], st);
     cudaMemcpyAsync(hd.data() + b, descs.as<ChunkDesc>() + b, sizeof(ChunkDesc) * (e - b),
                     cudaMemcpyDeviceToHost, st);
@@ -725,13 +730,16 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
                               std::max<uint64_t>(cbits, 1ull << 21), st))))
     return rc;
   stats.kernel_launches += lpt ? 2 : 1;
+  uint32_t n_decode = 0;  // chunks with a start
   {
     // the decoder variant without sync-start handling when there are none
-    uint32_t h_sync = 1;
-    if ((rc = check(cudaMemcpyAsync(&h_sync, n_sync, 4, cudaMemcpyDeviceToHost, st))) ||
+    // and how many chunks there are to decode: counters[1 .. 4]
+    uint32_t h_cnt[4] = {0, 0, 0, 1};
+    if ((rc = check(cudaMemcpyAsync(h_cnt, counters.as<uint32_t>() + 1, 16, cudaMemcpyDeviceToHost, st))) ||
         (rc = check(cudaStreamSynchronize(st))))
       return rc;
-    job_sync = h_sync != 0;
+    job_sync = h_cnt[3] != 0;
+    n_decode = h_cnt[0];
   }
   cudaEventRecord(ev[4], st);
   // ---- 4. decode ----------------------------------------------------------
@@ -754,7 +762,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
       cudaMemsetAsync(counters.as<uint32_t>() + 8, 0, 4, st);
     }
     cudaEventRecord(ev[8], st);
-    if ((rc = check(launch_decode(counters.as<uint32_t>() + 1)))) return rc;
+    if ((rc = check(launch_decode(counters.as<uint32_t>() + 1, n_decode)))) return rc;
     cudaEventRecord(ev[9], st);
     hd.resize(n_grid);
     hr.resize(n_grid);
@@ -1021,7 +1029,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
     cudaMemcpyAsync(work.p, wl.data(), 4 * nr, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(counters.as<uint32_t>() + 1, &nr, 4, cudaMemcpyHostToDevice, st);
     cudaEventRecord(ev[8], st);
-    if ((rc = check(launch_decode(counters.as<uint32_t>() + 1)))) return rc;
+    if ((rc = check(launch_decode(counters.as<uint32_t>() + 1, nr)))) return rc;
     cudaEventRecord(ev[9], st);
     hd.insert(hd.end(), repairs.begin(), repairs.end());
     hr.resize(hd.size());
@@ -1306,7 +1314,7 @@ int gzgpu_create(gzgpu_ctx** out, const gzgpu_config* cfg) {
   if (cfg) {
     c->dev = cfg->device;
     c->chunk_bytes = cfg->chunk_bytes;
-    if (cfg->lut_bits == 11 || cfg->lut_bits == 12) c->lut_bits = cfg->lut_bits;
+    if (cfg->lut_bits >= 10 && cfg->lut_bits <= 12) c->lut_bits = cfg->lut_bits;
     c->autotune = cfg->autotune != 0;
     c->ring = cfg->ring_history != 0;
     if (cfg->ctas_per_sm == 3 || cfg->ctas_per_sm == 4) c->ctas_per_sm = cfg->ctas_per_sm;
@@ -1958,7 +1966,7 @@ int gzgpu_debug_decode(gzgpu_ctx* c, const uint8_t* in, size_t in_len, const uin
   c->cur_in = c->in.as<uint8_t>();
   c->job_sync = false;
   for (size_t i = 0; i < n; i++) c->job_sync |= (d[i].flags & kChunkSync) != 0;
-  if ((rc = c->check(c->launch_decode(c->counters.as<uint32_t>() + 1)))) return rc;
+  if ((rc = c->check(c->launch_decode(c->counters.as<uint32_t>() + 1, (uint32_t)n)))) return rc;
   std::vector<ChunkResult> r(n);
   uint32_t used = 0;
   if (n) cudaMemcpyAsync(r.data(), c->results.p, sizeof(ChunkResult) * n, cudaMemcpyDeviceToHost, c->st);

@@ -52,7 +52,7 @@ typedef struct gzgpu_ctx gzgpu_ctx;
 typedef struct {
   int device;         /* CUDA device ordinal */
   size_t chunk_bytes; /* compressed bytes per speculative chunk; 0 = tuned default */
-  int lut_bits;       /* litlen LUT index bits: 10, 11 or 12; 0 = tuned default */
+  int lut_bits;       /* litlen LUT index bits: 10, 11 or 12; 0 = tuned default (11) */
   int autotune;       /* 1 = choose chunk_bytes, lut_bits and ctas_per_sm per job: the
                          first job of each kind (compressed-size bucket, stream-count
                          bucket, share of streams whose first block is fixed-Huffman)
