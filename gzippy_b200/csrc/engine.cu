@@ -190,7 +190,7 @@ struct gzgpu_ctx {
   gzgpu_stats stats{};
   bool crc_ready = false;
 
-  DevBuf in, out, s_off, s_len, info, units, cands, counters, descs, results, spec, work, cost;
+  DevBuf in, out, s_off, s_len, info, units, cands, counters, descs, results, spec, work, cost, find;
   DevBuf pages, owner, seq, placed, placed_of, list, cblocks, mend, mraw, mtrail, mlen, mcrc,
       mstatus;
   // seek-index builds: the decoder's block log, the checkpoint interval and
@@ -206,7 +206,7 @@ struct gzgpu_ctx {
     return {&in,     &out,   &s_off,   &s_len,  &info,   &units,   &cands,  &counters, &descs,
             &results, &spec, &work,    &pages,  &owner,  &seq,     &placed, &placed_of, &list,
             &cblocks, &mend,  &mraw,   &mtrail, &mlen,    &mcrc,   &mstatus, &blk_log,
-            &cost};
+            &cost,  &find};
   }
   const uint8_t* cur_in = nullptr;  // input buffer of the running job
   uint8_t* user_out = nullptr;       // caller device output (device-resident API)
@@ -462,10 +462,14 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
     total_in += S[s].len;
   }
   std::vector<ScanUnit> units;
-  const uint64_t kUnit = 1 << 20;
+  // one CTA per unit: small enough that every SM has several (1 MiB units left
+  // all but 23 CTAs idle on a 23 MB stream: 113 us), 8 KiB (one load per
+  // thread) at least
+  const uint64_t unit =
+      std::min<uint64_t>(1u << 20, std::max<uint64_t>(8192, (total_in / (16 * (uint64_t)sms) + 4096) & ~4095ull));
   for (uint32_t s = 0; s < ns; s++)
-    for (uint64_t b = 0; b < S[s].len; b += kUnit)
-      units.push_back(ScanUnit{s, 0, b, std::min(S[s].len, b + kUnit)});
+    for (uint64_t b = 0; b < S[s].len; b += unit)
+      units.push_back(ScanUnit{s, 0, b, std::min(S[s].len, b + unit)});
   if ((rc = check(s_off.ensure(8 * ns))) || (rc = check(s_len.ensure(8 * ns))) ||
       (rc = check(info.ensure(sizeof(StreamInfo) * ns))) ||
       (rc = check(units.empty() ? cudaSuccess : this->units.ensure(sizeof(ScanUnit) * units.size()))) ||
@@ -637,10 +641,12 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   cudaEventRecord(ev[3], st);
   // ---- 3. finder + link ---------------------------------------------------
   uint32_t* n_sync = counters.as<uint32_t>() + 4;  // sync starts found (zeroed with the scan)
-  if ((rc = check(launch_finder(cur_in, descs.as<ChunkDesc>(), spec.as<uint32_t>(),
-                                (uint32_t)hspec.size(), n_sync, st))))
+  if (!hspec.empty() && (rc = check(find.ensure(finder_scratch_bytes((uint32_t)hspec.size())))))
     return rc;
-  stats.kernel_launches += 2;
+  if ((rc = check(launch_finder(cur_in, descs.as<ChunkDesc>(), spec.as<uint32_t>(),
+                                (uint32_t)hspec.size(), cbits, find.p, n_sync, fine_split, sms, st))))
+    return rc;
+  if (!hspec.empty()) stats.kernel_launches += 4;
   // ---- 3a. cut high-ratio partitions finer ---------------------------------
   // A chunk's decode time follows its output; the finder estimated each
   // dynamic start's output per input byte from its code lengths.  Partitions
@@ -704,10 +710,11 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
         return rc;
       cudaMemcpyAsync(descs.p, hd.data(), sizeof(ChunkDesc) * n_grid, cudaMemcpyHostToDevice, st);
       cudaMemcpyAsync(spec.p, hspec2.data(), 4 * hspec2.size(), cudaMemcpyHostToDevice, st);
-      if ((rc = check(launch_finder(cur_in, descs.as<ChunkDesc>(), spec.as<uint32_t>(),
-                                    (uint32_t)hspec2.size(), n_sync, st))))
+      if ((rc = check(find.ensure(finder_scratch_bytes((uint32_t)hspec2.size())))) ||
+          (rc = check(launch_finder(cur_in, descs.as<ChunkDesc>(), spec.as<uint32_t>(),
+                                    (uint32_t)hspec2.size(), cbits, find.p, n_sync, true, sms, st))))
         return rc;
-      stats.kernel_launches += 2;
+      stats.kernel_launches += 4;
     }
     // sync starts inside dynamic blocks for every partition still empty
     std::vector<uint32_t> hsync;
@@ -1857,8 +1864,12 @@ int gzgpu_debug_find(gzgpu_ctx* c, const uint8_t* in, size_t in_len, const uint6
   if (n) {
     cudaMemcpyAsync(c->descs.p, d.data(), sizeof(ChunkDesc) * n, cudaMemcpyHostToDevice, c->st);
     cudaMemcpyAsync(c->spec.p, sp.data(), 4 * n, cudaMemcpyHostToDevice, c->st);
-    if ((rc = c->check(launch_finder(c->in.as<uint8_t>(), c->descs.as<ChunkDesc>(),
-                                     c->spec.as<uint32_t>(), (uint32_t)n, nullptr, c->st))))
+    uint64_t most = 0;
+    for (size_t i = 0; i < n; i++) most = std::max(most, to[i] > from[i] ? to[i] - from[i] : 0);
+    if ((rc = c->check(c->find.ensure(finder_scratch_bytes((uint32_t)n)))) ||
+        (rc = c->check(launch_finder(c->in.as<uint8_t>(), c->descs.as<ChunkDesc>(),
+                                     c->spec.as<uint32_t>(), (uint32_t)n, most, c->find.p, nullptr,
+                                     false, c->sms, c->st))))
       return rc;
     cudaMemcpyAsync(d.data(), c->descs.p, sizeof(ChunkDesc) * n, cudaMemcpyDeviceToHost, c->st);
   }

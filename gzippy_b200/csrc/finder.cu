@@ -11,15 +11,6 @@
 
 namespace gzgpu {
 
-// One CTA per speculative chunk.  Its warps take the 1024-bit windows of
-// [guess_bit, limit_bit) round-robin, each window searched for its first
-// candidate (by start bit, so windows partition the candidates); a warp stops
-// as soon as a lower window has a hit, so the work is about the distance to
-// the first candidate, split over the CTA's warps.  Stored candidates must
-// also pass start_ok (a stored or dynamic block right after them).
-constexpr int kFinderWarps = 2;
-constexpr uint64_t kFinderWindow = 1024 * kFindGroup;  // bits a warp takes at a time
-
 // Stored block starts, searched first for every speculative chunk: the first
 // one (by byte offset, hence by start bit) in [guess_bit, limit_bit) whose
 // successor passes stored_successor_ok becomes the chunk's start, and the
@@ -30,30 +21,37 @@ constexpr uint64_t kFinderWindow = 1024 * kFindGroup;  // bits a warp takes at a
 // no predecessor hands over to, and the host chain walk repairs past it.
 // The pass runs before the sync search because the raw bytes of stored
 // blocks (text, runs) walk as fixed-Huffman codes and would give false sync
-// starts.  One CTA of kStoredThreads per chunk, scanning that many byte
-// offsets a round.
+// starts.  One CTA of kStoredThreads per chunk; a thread screens 16 aligned
+// byte offsets a round with word operations (a round covers 4 KiB, so a 24 KiB
+// partition is six load latencies; offset by offset, 1 KiB a round, took
+// 41 us for the 1,365 partitions of a 23 MB stream).
 constexpr int kStoredThreads = 256;
 
 __global__ void __launch_bounds__(kStoredThreads)
     stored_kernel(const uint8_t* __restrict__ in, ChunkDesc* descs,
                   const uint32_t* __restrict__ spec, uint32_t n_spec) {
   __shared__ unsigned long long s_first;
-  unsigned long long* s_off = &s_first;
   if (blockIdx.x >= n_spec) return;
   ChunkDesc& d = descs[spec[blockIdx.x]];
   if (d.flags & kChunkValid) return;
   const uint64_t from = d.guess_bit, to = d.limit_bit, nbytes = d.in_end;
-  if (threadIdx.x == 0) *s_off = ~0ull;
+  if (threadIdx.x == 0) s_first = ~0ull;
   __syncthreads();
+  const uint64_t begin = max((from + 3 + 7) / 8, (uint64_t)2);
   const uint64_t until = nbytes >= 5 ? min((to + 7) / 8, nbytes - 4) : 0;
-  const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
-  // each thread screens 4 consecutive byte offsets a round for LEN == ~NLEN
-  for (uint64_t base = max((from + 3 + 7) / 8, (uint64_t)2); base < until; base += 4 * blockDim.x) {
-    const uint64_t ob = base + 4 * (uint64_t)threadIdx.x;
+  for (uint64_t base = begin & ~15ull; base < until; base += 16 * kStoredThreads) {
+    const uint64_t ob = base + 16 * (uint64_t)threadIdx.x;
     uint32_t m = 0;
     if (ob < until) {
-      m = stored_filter4(bits64_at(in32, ob * 8));
-      if (ob + 4 > until) m &= (1u << (until - ob)) - 1;
+      const uint4 v = *reinterpret_cast<const uint4*>(in + ob);
+      const uint32_t w[5] = {v.x, v.y, v.z, v.w, *reinterpret_cast<const uint32_t*>(in + ob + 16)};
+#pragma unroll
+      for (int k = 0; k < 16; k++) {
+        const uint32_t sz = __funnelshift_r(w[k >> 2], w[(k >> 2) + 1 < 5 ? (k >> 2) + 1 : 4], 8 * (k & 3));
+        m |= (((sz ^ (sz >> 16)) & 0xFFFFu) == 0xFFFFu ? 1u : 0u) << k;
+      }
+      if (ob < begin) m &= 0xFFFFFFFFu << (begin - ob);
+      if (ob + 16 > until) m &= (1u << (until - ob)) - 1;
     }
     while (m) {
       const uint64_t off = ob + (uint64_t)(__ffs(m) - 1);
@@ -61,18 +59,18 @@ __global__ void __launch_bounds__(kStoredThreads)
       uint64_t lo = 0, hi = 0;
       if (stored_candidate(in, nbytes, off, from, to, to, lo, hi) &&
           stored_successor_ok(in, nbytes, off + 4 + (in[off] | (in[off + 1] << 8)))) {
-        atomicMin(s_off, (unsigned long long)off);
+        atomicMin(&s_first, (unsigned long long)off);
         break;
       }
     }
     __syncthreads();
-    const bool found = *s_off != ~0ull;
+    const bool found = s_first != ~0ull;
     __syncthreads();  // every thread has read it before the next round writes
     if (found) break;
   }
-  if (threadIdx.x == 0 && *s_off != ~0ull) {
+  if (threadIdx.x == 0 && s_first != ~0ull) {
     uint64_t lo = 0, hi = 0;
-    stored_candidate(in, nbytes, *s_off, from, to, to, lo, hi);
+    stored_candidate(in, nbytes, s_first, from, to, to, lo, hi);
     d.lo_bit = lo;
     d.start_bit = hi;
     d.flags |= kChunkValid;
@@ -81,8 +79,7 @@ __global__ void __launch_bounds__(kStoredThreads)
 }
 
 // The precode leaf count of 4 code-length codes (12 bits) for every value,
-// built at compile time and read through the L1 cache: a CTA needs no
-// shared copy, so more small CTAs fit on an SM.
+// built at compile time; each CTA copies it to shared memory.
 struct LeafLut {
   uint16_t v[4096];
   constexpr LeafLut() : v() {
@@ -98,110 +95,227 @@ struct LeafLut {
 };
 __device__ const LeafLut d_leaf_lut = LeafLut();
 
-__global__ void __launch_bounds__(32 * kFinderWarps)
-    finder_kernel(const uint8_t* __restrict__ in, ChunkDesc* descs,
-                  const uint32_t* __restrict__ spec, uint32_t n_spec) {
-  __shared__ unsigned long long best_win;
-  __shared__ uint64_t hit_lo[kFinderWarps], hit_hi[kFinderWarps], hit_win[kFinderWarps];
-  __shared__ FinderLists lists[kFinderWarps];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (blockIdx.x >= n_spec) return;
-  ChunkDesc& d = descs[spec[blockIdx.x]];
-  if (d.flags & kChunkValid) return;  // a stored or sync start was found first
-  const uint16_t* leaf_lut = d_leaf_lut.v;
-  const uint64_t from = d.guess_bit, to = d.limit_bit, nbytes = d.in_end;
-  if (threadIdx.x == 0) best_win = ~0ull;
-  if (lane == 0) hit_win[warp] = ~0ull;
+// Dynamic headers.  The ranges still without a start are searched in segments
+// of kFindSeg bits, one warp per segment, segment 0 of every range first, then
+// segment 1, and so on: a range's later segments are skipped once an earlier
+// one has a hit, while a small job's segments all run at once.  (One CTA per
+// range, walking it from its start, took 370 us for the 30 ranges of a 1 MB
+// stream and 630 us for 1,365 ranges, mostly latency.)  A segment's words go
+// to shared memory; its bit offsets are screened in passes of 4096: the
+// 13-bit filter for 32 offsets per lane at once, the survivors (1 in 9) to a
+// list, the precode leaf count for 32 of them at a time; what is left
+// (about 1 in 200 of the list) gets the full header test, one per lane.
+constexpr int kFindWarps = 8;
+constexpr uint32_t kFindSeg = 8192;                // bits per segment
+constexpr uint32_t kFindPass = 4096;               // bits per screening pass
+constexpr uint32_t kFindList = kFindPass / 3 + 2;  // most survivors: three bits apart (BFINAL 0, BTYPE 10)
+constexpr uint32_t kFindFull = 64;                 // full tests held
+
+struct FindWarp {
+  uint32_t w[kFindSeg / 32 + 6];
+  uint16_t list[kFindList];
+  uint16_t full[kFindFull];
+  uint32_t n_full;
+};
+
+__global__ void __launch_bounds__(32 * kFindWarps)
+    find_kernel(const uint8_t* __restrict__ in, const ChunkDesc* __restrict__ descs,
+                const uint32_t* __restrict__ spec, uint32_t n_spec, uint32_t n_seg,
+                unsigned long long* best, uint32_t* next_item) {
+  __shared__ uint16_t leaf[4096];
+  __shared__ FindWarp fw[kFindWarps];
+  const int lane = threadIdx.x & 31;
+  FindWarp& W = fw[threadIdx.x >> 5];
+  for (uint32_t i = threadIdx.x; i < 4096 / 8; i += 32 * kFindWarps)
+    reinterpret_cast<uint4*>(leaf)[i] = reinterpret_cast<const uint4*>(d_leaf_lut.v)[i];
   __syncthreads();
-  const uint64_t n_win = to > from ? (to - from + kFinderWindow - 1) / kFinderWindow : 0;
-  for (uint64_t k = warp; k < n_win; k += kFinderWarps) {
-    if (k > *(volatile unsigned long long*)&best_win) break;
-    const uint64_t w0 = from + k * kFinderWindow;
-    const uint64_t w1 = min(w0 + kFinderWindow, to);
-    uint64_t lo = 0, hi = 0, s0 = w0;
-    bool hit = false;
-    // stored candidates: the stored-start pass before this kernel took the
-    // first that could start this range, so only dynamic ones are left
-    while (s0 < w1 &&
-           warp_find_first(in, nbytes, s0, w1, to, lane, lo, hi, leaf_lut, &lists[warp], true)) {
-      if (start_ok(in, nbytes, hi)) {
-        hit = true;
-        break;
+  const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
+  const uint64_t n_items = (uint64_t)n_spec * n_seg;
+  for (;;) {
+    uint32_t item = 0;
+    if (lane == 0) item = atomicAdd(next_item, 1u);
+    item = __shfl_sync(0xFFFFFFFFu, item, 0);
+    if (item >= n_items) break;
+    const uint32_t k = item % n_spec, sg = item / n_spec;
+    const ChunkDesc& d = descs[spec[k]];
+    if (d.flags & kChunkValid) continue;  // a stored or sync start was found first
+    const uint64_t nbytes = d.in_end, nbits = nbytes * 8;
+    const uint64_t from = d.guess_bit, to = min(d.limit_bit, nbits);
+    // segments are cut at word boundaries of the input
+    const uint64_t s0 = (from & ~31ull) + (uint64_t)sg * kFindSeg;
+    if (s0 >= to) continue;
+    if (*(volatile unsigned long long*)&best[k] < s0) continue;
+    const uint32_t len = (uint32_t)min((uint64_t)kFindSeg, to - s0);
+    const uint32_t first = from > s0 ? (uint32_t)(from - s0) : 0u;
+    // the segment's words, and the 81 bits after it (a header up to its precode)
+    __syncwarp();
+    const uint64_t wi = s0 >> 5;
+#pragma unroll
+    for (uint32_t j = 0; j < kFindSeg / 32 + 6; j += 32)
+      if (j + lane < kFindSeg / 32 + 6 && 32 * (j + lane) < len + 160) W.w[j + lane] = in32[wi + j + lane];
+    if (lane == 0) W.n_full = 0;
+    __syncwarp();
+    uint32_t hit = kFindSeg;  // lowest passing offset
+    for (uint32_t p0 = 0; p0 < len && hit == kFindSeg; p0 += kFindPass) {
+      uint32_t m[kFindPass / 1024], c = 0;
+#pragma unroll
+      for (uint32_t q = 0; q < kFindPass / 1024; q++) {
+        const uint32_t p = p0 + 1024 * q + 32 * lane;
+        uint32_t v = 0;
+        if (p < len) {
+          v = dyn_filter32((uint64_t)W.w[(p >> 5) + 1] << 32 | W.w[p >> 5]);
+          if (p + 32 > len) v &= (1u << (len - p)) - 1;
+          if (p < first) v &= p + 32 > first ? 0xFFFFFFFFu << (first - p) : 0u;
+        }
+        m[q] = v;
+        c += __popc(v);
       }
-      s0 = lo + 1;  // a stored match without a plausible successor
-    }
-    if (hit) {
-      if (lane == 0) {
-        hit_lo[warp] = lo;
-        hit_hi[warp] = hi;
-        hit_win[warp] = k;
-        atomicMin(&best_win, (unsigned long long)k);
+      uint32_t at = c;
+#pragma unroll
+      for (int b = 1; b < 32; b <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, at, b);
+        if (lane >= b) at += v;
       }
-      break;
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint64_t bw = ~0ull;
-    int bwarp = -1;
-    for (int i = 0; i < kFinderWarps; i++)
-      if (hit_win[i] < bw) {
-        bw = hit_win[i];
-        bwarp = i;
+      const uint32_t tot = __shfl_sync(0xFFFFFFFFu, at, 31);
+      at -= c;
+#pragma unroll
+      for (uint32_t q = 0; q < kFindPass / 1024; q++)
+        while (m[q]) {
+          W.list[at++] = (uint16_t)(p0 + 1024 * q + 32 * lane + __ffs(m[q]) - 1);
+          m[q] &= m[q] - 1;
+        }
+      __syncwarp();
+      for (uint32_t j0 = 0; j0 < tot; j0 += 32) {
+        const bool act = j0 + lane < tot;
+        const uint32_t p = act ? W.list[j0 + lane] : 0u;
+        // HCLEN and the precode: bits 13 .. 76 of the header
+        const uint32_t a = (p + 13) >> 5, sh = (p + 13) & 31;
+        const uint32_t w1 = W.w[a + 1];
+        const uint32_t lo = __funnelshift_r(W.w[a], w1, sh), hi = __funnelshift_r(w1, W.w[a + 2], sh);
+        const uint32_t n = 3 * ((lo & 15) + 4);  // precode bits
+        uint64_t pb = ((uint64_t)hi << 32 | lo) >> 4;
+        pb &= (1ull << n) - 1;
+        const uint32_t x0 = (uint32_t)pb, x1 = (uint32_t)(pb >> 24);
+        const uint32_t sum = leaf[x0 & 0xFFF] + leaf[(x0 >> 12) & 0xFFF] + leaf[x1 & 0xFFF] +
+                             leaf[(x1 >> 12) & 0xFFF] + leaf[(uint32_t)(pb >> 48)];
+        const bool ok = act && (sum == 128 || sum == 64) && s0 + p + 17 + n <= nbits;
+        const uint32_t b = __ballot_sync(0xFFFFFFFFu, ok);
+        if (!b) continue;
+        uint32_t n0 = W.n_full;
+        __syncwarp();
+        if (n0 + __popc(b) > kFindFull) {
+          // (rare) the held ones first
+          for (uint32_t j = lane; j < n0; j += 32) {
+            const uint32_t f = W.full[j];
+            if (f < hit && dyn_candidate_full(in, nbytes, s0 + f)) hit = f;
+          }
+          __syncwarp();
+          n0 = 0;
+        }
+        if (ok) W.full[n0 + __popc(b & ((1u << lane) - 1))] = (uint16_t)p;
+        if (lane == 0) W.n_full = n0 + __popc(b);
+        __syncwarp();
       }
-    if (bwarp >= 0) {
-      d.lo_bit = hit_lo[bwarp];
-      d.start_bit = hit_hi[bwarp];
-      d.flags |= kChunkValid;
-      // BTYPE at the start: 2 = dynamic (estimate from its code lengths), 0 = stored
-      const uint32_t bt = (uint32_t)(peek_bits(in, nbytes, d.start_bit, 3) >> 1);
-      d.est_ratio = bt == 2 ? dyn_header_ratio(in, nbytes, d.start_bit) : 1.f;
-    } else {
-      d.flags &= ~kChunkValid;
+      const uint32_t n0 = W.n_full;
+      for (uint32_t j = lane; j < n0; j += 32) {
+        const uint32_t f = W.full[j];
+        if (f < hit && dyn_candidate_full(in, nbytes, s0 + f)) hit = f;
+      }
+      hit = __reduce_min_sync(0xFFFFFFFFu, hit);
+      if (lane == 0) W.n_full = 0;
+      __syncwarp();
     }
+    if (hit < kFindSeg && lane == 0) atomicMin(&best[k], (unsigned long long)(s0 + hit));
   }
 }
 
-// Sync starts in fixed-Huffman data (finder_core.cuh fixed_walk), searched
-// for every speculative chunk before the block finder, which then skips the
-// chunks that have one.  One CTA of kSyncOffsets threads per chunk; the walk
-// must end inside the chunk's range and the input.
+// the dynamic starts found, into the chunk table; ratio: with the output
+// estimate of their headers
+__global__ void assign_kernel(const uint8_t* __restrict__ in, ChunkDesc* descs,
+                              const uint32_t* __restrict__ spec, uint32_t n_spec,
+                              const unsigned long long* __restrict__ best, int ratio) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n_spec) return;
+  ChunkDesc& d = descs[spec[k]];
+  if ((d.flags & kChunkValid) || best[k] == ~0ull) return;
+  d.lo_bit = d.start_bit = best[k];
+  d.flags |= kChunkValid;
+  d.est_ratio = ratio ? dyn_header_ratio(in, d.in_end, d.start_bit) : 0.f;
+}
+
+// Sync starts in fixed-Huffman data (finder_core.cuh), searched for every
+// speculative chunk before the block finder, which then skips the chunks that
+// have one.  One CTA of kSyncOffsets threads per chunk, each walking the fixed
+// code's symbols from one start bit; the walk must end inside the chunk's range
+// and the input.  Walks go on in steps of kSyncStep bits and stop as soon as
+// fewer than two are left (other data fails within a few hundred symbols);
+// 1,365 ranges of text took 100 us when every walk ran to its end and one
+// thread compared the ends.
+constexpr uint32_t kSyncStep = 512;
+
 __global__ void __launch_bounds__(kSyncOffsets)
     sync_kernel(const uint8_t* __restrict__ in, ChunkDesc* descs, const uint32_t* __restrict__ spec,
                 uint32_t n_spec, uint32_t* n_sync) {
-  __shared__ uint32_t sync_words[kSyncWords];
-  __shared__ uint64_t sync_end[kSyncOffsets];
+  constexpr uint32_t kWords = sync_words(kSyncOffsets, kSyncSpan);
+  __shared__ uint32_t sw[kWords];
+  __shared__ uint8_t lut[512], dlut[32];
+  __shared__ uint32_t ends[kSyncOffsets];
+  __shared__ unsigned long long top;
   if (blockIdx.x >= n_spec) return;
   ChunkDesc& d = descs[spec[blockIdx.x]];
   if (d.flags & kChunkValid) return;
   const uint64_t from = d.guess_bit, to = d.limit_bit, nbytes = d.in_end;
   const uint64_t target = from + kSyncOffsets + kSyncSpan;
   if (target + 64 > to || target + 128 > nbytes * 8) return;
-  const uint64_t wbase = from >> 5;
-  const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
-  for (uint32_t i = threadIdx.x; i < kSyncWords; i += blockDim.x) sync_words[i] = in32[wbase + i];
+  const uint32_t tid = threadIdx.x;
+  const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in) + (from >> 5);
+  for (uint32_t i = tid; i < kWords; i += kSyncOffsets) sw[i] = in32[i];
+  for (uint32_t i = tid; i < 512; i += kSyncOffsets) lut[i] = (uint8_t)fixed_entry(i);
+  if (tid < 32) {
+    const uint32_t dc = __brev(tid) >> 27;
+    dlut[tid] = dc >= 30 ? 0xFF : (uint8_t)(5 + f_dist_extra[dc]);
+  }
+  if (tid == 0) top = 0;
   __syncthreads();
-  if (threadIdx.x < kSyncOffsets)
-    sync_end[threadIdx.x] = fixed_walk(sync_words, wbase, from + threadIdx.x, target);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint64_t best = kSyncFail;
-    uint32_t best_n = 1;
-    for (uint32_t i = 0; i < kSyncOffsets; i++) {
-      const uint64_t v = sync_end[i];
-      if (v == kSyncFail) continue;
-      uint32_t c = 0;
-      for (uint32_t j = 0; j < kSyncOffsets; j++) c += sync_end[j] == v;
-      if (c > best_n || (c == best_n && best != kSyncFail && v < best)) {
-        best = v;
-        best_n = c;
+  const uint32_t rel = (uint32_t)(from & 31);  // positions below count from the word of `from`
+  const uint32_t goal = rel + kSyncOffsets + (uint32_t)kSyncSpan;
+  uint32_t p = rel + tid;
+  bool ok = true;
+  for (uint32_t step = rel + kSyncOffsets + kSyncStep;; step += kSyncStep) {
+    const uint32_t e = min(step, goal);
+    while (ok && p < e) {
+      const uint32_t i = p >> 5;
+      const uint32_t x = __funnelshift_r(sw[i], sw[i + 1], p & 31);
+      const uint32_t ent = lut[x & 511];
+      p += ent & 31;
+      if (ent < 32) continue;  // a literal
+      const uint32_t j = p >> 5;
+      const uint32_t y = __funnelshift_r(sw[j], sw[j + 1], p & 31);
+      if (ent >> 5 == 1) {  // a length: the distance code
+        const uint32_t n = dlut[y & 31];
+        ok = n != 0xFF;
+        p += n;
+      } else {  // EOB: another fixed block must follow
+        ok = ent >> 5 == 2 && ((y >> 1) & 3) == 1;
+        p += 3;
       }
     }
-    if (best != kSyncFail) {
-      d.lo_bit = d.start_bit = best;
-      d.flags |= kChunkValid | kChunkSync;
-      if (n_sync) atomicAdd(n_sync, 1u);
-    }
+    if (__syncthreads_count(ok) < 2) return;
+    if (e == goal) break;
+  }
+  ends[tid] = ok ? p : 0u;
+  __syncthreads();
+  if (ok) {
+    uint32_t c = 0;
+    for (uint32_t i = 0; i < kSyncOffsets; i++) c += ends[i] == p;
+    // most walks first, then the lower position
+    if (c >= 2) atomicMax(&top, (unsigned long long)c << 32 | (0xFFFFFFFFu - p));
+  }
+  __syncthreads();
+  if (tid == 0 && top) {
+    d.lo_bit = d.start_bit = (from & ~31ull) + (0xFFFFFFFFu - (uint32_t)top);
+    d.flags |= kChunkValid | kChunkSync;
+    if (n_sync) atomicAdd(n_sync, 1u);
   }
 }
 
@@ -211,45 +325,17 @@ __global__ void __launch_bounds__(kSyncOffsets)
 // A speculative start may be a phantom whose garbage code table never fails;
 // such a chunk gives up `slack` bits past its stop and the chain walk
 // re-decodes the gap from the confirmed boundary instead.
-// Decode cost of a linked chunk.  The decoder's time follows its compressed
-// bits (one step per 32 bits) plus its copy work, which follows the output:
-// measured per 64 KiB chunk of the 1 GiB mixed stream, about 12.5 ms at 1
-// output byte per input byte (near-incompressible literals), 16 ms at 2.9
-// (text) and 29 ms at 13.6 (byte runs), and 0.6 ms for stored data.  So the
-// cost is the compressed bytes times (1 + 0.2 x the output-per-input estimate
-// of the dynamic header a chunk starts in), and a twentieth of that for a
-// stored start: the decode cost per compressed byte of the data a chunk
-// start begins in.
-__device__ float cost_factor(const uint8_t* __restrict__ in, const ChunkDesc& d) {
-  float r = d.est_ratio;
-  if (!(r > 0.f)) {
-    // member starts and sync starts carry no finder estimate: take it from
-    // the header of the block they start in
-    const uint64_t hdr = (d.flags & kChunkSync) ? d.table_bit : d.start_bit;
-    const uint32_t bt = hdr ? (uint32_t)(peek_bits(in, d.in_end, hdr, 3) >> 1) : 1u;
-    if (bt == 0) return 0.05f;
-    if (bt == 2) r = dyn_header_ratio(in, d.in_end, hdr);
-    if (!(r > 0.f)) r = 2.f;  // fixed-Huffman data: about 2 bytes per input byte
-  } else if (r == 1.f && (peek_bits(in, d.in_end, d.start_bit, 3) >> 1) == 0) {
-    return 0.05f;  // a stored start
-  }
-  return 1.f + 0.2f * r;
-}
-
-// A chunk's cost is its compressed bytes times the larger of the factors of
-// its own start and of its successor's, which shows the data at its far end:
-// a chunk that starts in stored data and runs into dense text or byte runs
-// is as costly as that data.
-__device__ float chunk_cost(const uint8_t* __restrict__ in, const ChunkDesc* descs,
-                            const ChunkDesc& d, uint64_t stop, uint32_t next) {
+// Decode cost of a linked chunk: its compressed bytes.  Text, byte runs and
+// noisy literals take the decoder about the same time per compressed byte
+// (within a factor of two); stored data is a copy, a twentieth of that.
+__device__ float chunk_cost(const uint8_t* __restrict__ in, const ChunkDesc& d, uint64_t stop) {
   const uint64_t nbits = d.in_end * 8;
   uint64_t end = stop != kNoStop ? stop : nbits;
   if (end > nbits) end = nbits;
   const float span = end > d.start_bit ? (float)(end - d.start_bit) * 0.125f : 0.f;
-  float f = cost_factor(in, d);
-  if (next != kNoChunk && !(descs[next].flags & kChunkMemberFirst))
-    f = fmaxf(f, cost_factor(in, descs[next]));
-  return f * span;
+  const bool stored =
+      !(d.flags & kChunkSync) && (peek_bits(in, d.in_end, d.start_bit, 3) >> 1) == 0;
+  return stored ? 0.05f * span : span;
 }
 
 __global__ void link_kernel(const uint8_t* __restrict__ in, ChunkDesc* descs, uint32_t n,
@@ -286,7 +372,7 @@ __global__ void link_kernel(const uint8_t* __restrict__ in, ChunkDesc* descs, ui
   if ((d.flags & kChunkSync) && stop != kNoStop && stop > d.start_bit)
     s = min(slack, max(stop - d.start_bit, (uint64_t)kSyncMinSlack));
   d.abort_bit = (stop != kNoStop && !(d.flags & kChunkMemberFirst)) ? stop + s : kNoStop;
-  if (cost) cost[i] = chunk_cost(in, descs, d, stop, next);
+  if (cost) cost[i] = chunk_cost(in, d, stop);
   else work[atomicAdd(n_work, 1u)] = i;
 }
 
@@ -322,8 +408,11 @@ __global__ void __launch_bounds__(1024)
     if (descs[i].flags & kChunkValid) work[atomicAdd(&base[bucket(i)], 1u)] = i;
 }
 
-cudaError_t launch_finder(const uint8_t* in, ChunkDesc* descs, const uint32_t* spec,
-                          uint32_t n_spec, uint32_t* n_sync, cudaStream_t stream) {
+size_t finder_scratch_bytes(uint32_t n_spec) { return 8 * (size_t)n_spec + 8; }
+
+cudaError_t launch_finder(const uint8_t* in, ChunkDesc* descs, const uint32_t* spec, uint32_t n_spec,
+                          uint64_t max_bits, void* scratch, uint32_t* n_sync, bool ratio, int sms,
+                          cudaStream_t stream) {
   if (n_spec == 0) return cudaSuccess;
   // Stored starts first (a byte scan), then the fixed-code sync search: it
   // costs a fraction of a full scan, which a fixed-Huffman partition (no
@@ -331,7 +420,17 @@ cudaError_t launch_finder(const uint8_t* in, ChunkDesc* descs, const uint32_t* s
   // symbols on other data.
   stored_kernel<<<n_spec, kStoredThreads, 0, stream>>>(in, descs, spec, n_spec);
   sync_kernel<<<n_spec, kSyncOffsets, 0, stream>>>(in, descs, spec, n_spec, n_sync);
-  finder_kernel<<<n_spec, 32 * kFinderWarps, 0, stream>>>(in, descs, spec, n_spec);
+  // best start per range, and the work counter after it
+  unsigned long long* best = reinterpret_cast<unsigned long long*>(scratch);
+  uint32_t* next_item = reinterpret_cast<uint32_t*>(best + n_spec);
+  cudaError_t e = cudaMemsetAsync(best, 0xFF, 8 * (size_t)n_spec, stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(next_item, 0, 8, stream);
+  if (e != cudaSuccess) return e;
+  const uint32_t n_seg = (uint32_t)((max_bits + 31) / kFindSeg + 1);
+  const uint64_t ctas = ((uint64_t)n_spec * n_seg + kFindWarps - 1) / kFindWarps;
+  const uint32_t grid = (uint32_t)(ctas < (uint64_t)sms * 4 ? ctas : (uint64_t)sms * 4);
+  find_kernel<<<grid, 32 * kFindWarps, 0, stream>>>(in, descs, spec, n_spec, n_seg, best, next_item);
+  assign_kernel<<<(n_spec + 127) / 128, 128, 0, stream>>>(in, descs, spec, n_spec, best, ratio);
   return cudaGetLastError();
 }
 

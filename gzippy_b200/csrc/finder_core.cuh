@@ -76,94 +76,93 @@ static __device__ __forceinline__ uint32_t precode_leaves4(uint32_t v) {
   return s;
 }
 
+// Place of each code-length symbol in the header's order.
+static __device__ __forceinline__ constexpr int precode_place(int sym) {
+  constexpr int at[19] = {3, 17, 15, 13, 11, 9, 7, 5, 4, 6, 8, 10, 12, 14, 16, 18, 0, 1, 2};
+  return at[sym];
+}
+
 // Rest of the dynamic-header predicate once the 13-bit filter and the
 // precode leaf count have passed: Kraft-exact precode, code lengths decode,
-// EOB present, Kraft-exact litlen and dist sets.
+// EOB present, Kraft-exact litlen and dist sets.  One thread per candidate,
+// all state in registers (the canonical precode as 7 limits and the symbols
+// in code order, 5 bits each): a candidate costs its serial chain of code
+// lengths, so it must not wait for local memory on the way.
 static __device__ __noinline__ bool dyn_candidate_full(const uint8_t* in, uint64_t nbytes,
                                                        uint64_t bit) {
+  const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
   const uint64_t nbits = nbytes * 8;
-  uint32_t h = (uint32_t)peek_bits(in, nbytes, bit, 17);
-  int hlit = (h >> 3) & 31, hdist = (h >> 8) & 31, pc = ((h >> 13) & 15) + 4;
-  uint64_t pbits = peek_bits(in, nbytes, bit + 17, 3 * pc);
-  uint32_t leaves15 = 0, gt1 = 0;
-  uint8_t cl[19];
+  const uint32_t h = (uint32_t)peek_bits(in, nbytes, bit, 17);
+  const int hl = 257 + (int)((h >> 3) & 31), total = hl + 1 + (int)((h >> 8) & 31);
+  const int pc = (int)((h >> 13) & 15) + 4;
+  const uint64_t pbits = peek_bits(in, nbytes, bit + 17, 3 * pc);
+  // codes per length, eight bits each; length 0 is not counted
+  uint64_t cnt = 0;
 #pragma unroll
-  for (int i = 0; i < 19; i++) cl[i] = 0;
-  for (int i = 0; i < pc; i++) {
-    uint32_t L = (uint32_t)(pbits >> (3 * i)) & 7;
-    cl[f_cl_order[i]] = (uint8_t)L;
-    if (L) {
-      leaves15 += 1u << (15 - L);
-      gt1 += L > 1;
-    }
-  }
-  if (!kraft_exact(leaves15, gt1)) return false;
-  // canonical precode tables
-  uint16_t cnt[8], first[8], offs[8];
-  uint8_t sorted[19];
-#pragma unroll
-  for (int L = 0; L < 8; L++) cnt[L] = 0;
-  for (int s = 0; s < 19; s++) cnt[cl[s]]++;
-  cnt[0] = 0;
+  for (int i = 0; i < 19; i++) cnt += 1ull << (8 * ((pbits >> (3 * i)) & 7));
+  cnt &= ~0xFFull;
+  uint32_t lim[8];  // left-aligned end of the codes of up to l bits
+  uint64_t base = 0, next = 0;
   {
-    uint32_t code = 0, off = 0;
-    for (int L = 1; L < 8; L++) {
-      if (L > 1) code = (code + cnt[L - 1]) << 1;
-      first[L] = (uint16_t)code;
-      offs[L] = (uint16_t)off;
-      off += cnt[L];
+    uint32_t code = 0, off = 0, c = 0, leaves = 0, gt1 = 0;
+#pragma unroll
+    for (int l = 1; l < 8; l++) {
+      code = (code + c) << 1;
+      c = (uint32_t)(cnt >> (8 * l)) & 0xFF;
+      lim[l] = (code + c) << (7 - l);
+      base |= (uint64_t)((off - code) & 0xFF) << (8 * l);
+      next |= (uint64_t)off << (8 * l);
+      off += c;
+      leaves += c << (15 - l);
+      if (l > 1) gt1 += c;
     }
-    uint16_t nx[8];
-    for (int L = 0; L < 8; L++) nx[L] = offs[L];
-    for (int s = 0; s < 19; s++)
-      if (cl[s]) sorted[nx[cl[s]]++] = (uint8_t)s;
+    if (!kraft_exact(leaves, gt1)) return false;
+  }
+  uint64_t s_lo = 0, s_hi = 0;  // symbols in code order: 12, then 7
+#pragma unroll
+  for (int sym = 0; sym < 19; sym++) {
+    const uint32_t L = (uint32_t)(pbits >> (3 * precode_place(sym))) & 7;
+    if (!L) continue;
+    const uint32_t at = (uint32_t)(next >> (8 * L)) & 0xFF;
+    next += 1ull << (8 * L);
+    if (at < 12) s_lo |= (uint64_t)sym << (5 * at);
+    else s_hi |= (uint64_t)sym << (5 * (at - 12));
   }
   // decode the litlen + dist code lengths, accumulating Kraft sums
-  const int hl = 257 + hlit, total = hl + 1 + hdist;
   uint64_t pos = bit + 17 + 3 * pc;
+  uint64_t wi = pos >> 5;
+  uint64_t buf = in32[wi] >> (pos & 31);
+  int have = 32 - (int)(pos & 31);
+  wi++;
   uint32_t lit_leaves = 0, lit_gt1 = 0, dist_leaves = 0, dist_gt1 = 0;
   int i = 0;
   uint32_t prev = 0, eob_len = 0;
   while (i < total) {
     if (pos >= nbits) return false;
-    uint32_t w = (uint32_t)peek_bits(in, nbytes, pos, 14);
-    // MSB-first 7-bit code
-    uint32_t rev = __brev(w) >> 25;
-    int sym = -1;
-    for (int L = 1; L < 8; L++) {
-      uint32_t c = rev >> (7 - L);
-      uint32_t idx = c - first[L];
-      if (idx < cnt[L]) {
-        sym = sorted[offs[L] + idx];
-        pos += L;
-        break;
-      }
+    if (have < 14) {
+      buf |= (uint64_t)in32[wi++] << have;
+      have += 32;
     }
-    if (sym < 0) return false;
-    uint32_t v;
-    int rep;
-    if (sym < 16) {
-      v = sym;
-      rep = 1;
-    } else if (sym == 16) {
-      if (i == 0) return false;
-      v = prev;
-      rep = 3 + (int)peek_bits(in, nbytes, pos, 2);
-      pos += 2;
-    } else if (sym == 17) {
-      v = 0;
-      rep = 3 + (int)peek_bits(in, nbytes, pos, 3);
-      pos += 3;
-    } else {
-      v = 0;
-      rep = 11 + (int)peek_bits(in, nbytes, pos, 7);
-      pos += 7;
-    }
-    if (i + rep > total) return false;
-    if (pos > nbits) return false;
+    const uint32_t rev = __brev((uint32_t)buf) >> 25;  // MSB-first 7-bit code
+    if (rev >= lim[7]) return false;
+    uint32_t L = 1;
+#pragma unroll
+    for (int l = 1; l < 7; l++) L += rev >= lim[l] ? 1u : 0u;
+    const uint32_t idx = ((rev >> (7 - L)) + (uint32_t)(base >> (8 * L))) & 0x1F;
+    const uint32_t sym = (uint32_t)(idx < 12 ? s_lo >> (5 * idx) : s_hi >> (5 * (idx - 12))) & 31;
+    // a repeat's bits: 2, 3 or 7
+    const uint32_t xb = sym < 16 ? 0u : (sym == 16 ? 2u : (sym == 17 ? 3u : 7u));
+    const uint32_t x = (uint32_t)(buf >> L) & ((1u << xb) - 1);
+    if (sym == 16 && i == 0) return false;
+    const uint32_t v = sym < 16 ? sym : (sym == 16 ? prev : 0u);
+    const int rep = sym < 16 ? 1 : (int)x + (sym == 18 ? 11 : 3);
+    buf >>= L + xb;
+    have -= (int)(L + xb);
+    pos += L + xb;
+    if (i + rep > total || pos > nbits) return false;
     if (v) {
-      int n_lit = i < hl ? min(rep, hl - i) : 0;
-      int n_dist = rep - n_lit;
+      const int n_lit = i < hl ? min(rep, hl - i) : 0;
+      const int n_dist = rep - n_lit;
       lit_leaves += (uint32_t)n_lit << (15 - v);
       dist_leaves += (uint32_t)n_dist << (15 - v);
       if (v > 1) {
@@ -182,11 +181,10 @@ static __device__ __noinline__ bool dyn_candidate_full(const uint8_t* in, uint64
 }
 
 // The cheap part of the dynamic-header predicate at `bit`: the 13-bit header
-// filter and the precode leaf count via `leaf_lut` (the 4096-entry leaf-count
-// table, or null to count arithmetically).  dyn_candidate_fast adds
+// filter and the precode leaf count; dyn_candidate_fast adds
 // dyn_candidate_full.
-static __device__ __forceinline__ bool dyn_leaf_ok(const uint8_t* in, uint64_t nbytes, uint64_t bit,
-                                                   const uint16_t* leaf_lut) {
+static __device__ __forceinline__ bool dyn_candidate_fast(const uint8_t* in, uint64_t nbytes,
+                                                          uint64_t bit) {
   if (bit + 17 > nbytes * 8) return false;
   uint64_t x;
   uint32_t xh;
@@ -198,22 +196,11 @@ static __device__ __forceinline__ bool dyn_leaf_ok(const uint8_t* in, uint64_t n
   // precode bits [17, 17 + 3*pc) of the 96-bit window
   uint64_t pb = (x >> 17) | ((uint64_t)xh << 47);
   pb &= (1ull << (3 * pc)) - 1;
-  uint32_t leaves;
-  if (leaf_lut) {
-    leaves = leaf_lut[pb & 0xFFF] + leaf_lut[(pb >> 12) & 0xFFF] + leaf_lut[(pb >> 24) & 0xFFF] +
-             leaf_lut[(pb >> 36) & 0xFFF] + leaf_lut[pb >> 48];
-  } else {
-    leaves = precode_leaves4((uint32_t)(pb & 0xFFF)) + precode_leaves4((uint32_t)((pb >> 12) & 0xFFF)) +
-             precode_leaves4((uint32_t)((pb >> 24) & 0xFFF)) +
-             precode_leaves4((uint32_t)((pb >> 36) & 0xFFF)) + precode_leaves4((uint32_t)(pb >> 48));
-  }
-  return leaves == 128 || leaves == 64;
-}
-
-static __device__ __forceinline__ bool dyn_candidate_fast(const uint8_t* in, uint64_t nbytes,
-                                                          uint64_t bit,
-                                                          const uint16_t* leaf_lut) {
-  return dyn_leaf_ok(in, nbytes, bit, leaf_lut) && dyn_candidate_full(in, nbytes, bit);
+  const uint32_t leaves =
+      precode_leaves4((uint32_t)(pb & 0xFFF)) + precode_leaves4((uint32_t)((pb >> 12) & 0xFFF)) +
+      precode_leaves4((uint32_t)((pb >> 24) & 0xFFF)) +
+      precode_leaves4((uint32_t)((pb >> 36) & 0xFFF)) + precode_leaves4((uint32_t)(pb >> 48));
+  return (leaves == 128 || leaves == 64) && dyn_candidate_full(in, nbytes, bit);
 }
 
 // The block after a true non-final stored block starts at byte `n` (its
@@ -239,17 +226,6 @@ static __device__ __forceinline__ bool stored_successor_ok(const uint8_t* in, ui
   const uint32_t h = (uint32_t)peek_bits(in, nbytes, bit, 13);
   if (((h >> 3) & 31) > 29 || ((h >> 8) & 31) > 29) return false;
   return dyn_candidate_full(in, nbytes, bit);
-}
-
-// A candidate found at seek bit `hi` stays a chunk start unless it is a stored
-// block whose successor fails stored_successor_ok (the finder kernel then
-// searches on from its first bit + 1; the decoder's in-kernel retry takes
-// the reference's candidates as they are).
-static __device__ __forceinline__ bool start_ok(const uint8_t* in, uint64_t nbytes, uint64_t hi) {
-  if (((peek_bits(in, nbytes, hi, 3) >> 1) & 3) != 0) return true;
-  const uint64_t off = (hi + 3) >> 3;
-  const uint32_t len = in[off] | (in[off + 1] << 8);
-  return stored_successor_ok(in, nbytes, off + 4 + len);
 }
 
 // Stored candidate test at byte offset `off` (find_uncompressed_blocks):
@@ -315,139 +291,10 @@ static __device__ __forceinline__ uint32_t stored_filter4(uint64_t B) {
 // and runs the full tests only on the offsets that pass (about 1 in 9 bits);
 // a ballot picks the lowest hit.  The first stored hit in byte order is the
 // smallest stored candidate, so the dynamic scan only needs to reach it.
-// Per-warp candidate lists of the grouped scan (finder kernel): positions of
-// one 1024-bit window that pass the 13-bit filter, then positions of a group
-// of windows that also pass the precode leaf count.
-constexpr uint32_t kFindGroup = 4;    // 1024-bit windows screened before the full tests
-constexpr uint32_t kFindFull = 64;    // leaf-count survivors held per group
-struct FinderLists {
-  uint16_t c1[1024];
-  uint32_t c2[kFindFull];
-  uint32_t n2;
-};
-
+// Used by the inflate kernel's retry; the finder kernel screens ahead of it.
 static __device__ bool warp_find_first(const uint8_t* __restrict__ in, uint64_t nbytes,
                                        uint64_t from, uint64_t to, uint64_t hi_to, int lane,
-                                       uint64_t& out_lo, uint64_t& out_hi,
-                                       const uint16_t* leaf_lut = nullptr,
-                                       FinderLists* L = nullptr, bool dyn_only = false);
-
-// The same search with the dynamic tests spread over the warp: a group of
-// kFindGroup windows is screened (13-bit filter per lane, then the leaf
-// count for every survivor, 32 at a time), and the full tests of the group's
-// survivors run one per lane, the lowest passing position winning.  Used by
-// the finder kernel, whose warps have the lists in shared memory.  With
-// `dyn_only` the stored candidates are not searched (the finder kernel runs
-// after the stored-start pass, which took every stored candidate that could
-// start its range).
-static __device__ bool warp_find_first_grouped(const uint8_t* __restrict__ in, uint64_t nbytes,
-                                               uint64_t from, uint64_t to, uint64_t hi_to,
-                                               int lane, uint64_t& out_lo, uint64_t& out_hi,
-                                               const uint16_t* leaf_lut, FinderLists* L,
-                                               bool dyn_only) {
-  const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
-  if (to > nbytes * 8) to = nbytes * 8;
-  if (hi_to > nbytes * 8) hi_to = nbytes * 8;
-  bool have = false;
-  uint64_t best_lo = 0, best_hi = 0;
-  const uint64_t until = nbytes >= 5 ? min((hi_to + 7) / 8, nbytes - 4) : 0;
-  uint64_t next_off = max((from + 3 + 7) / 8, (uint64_t)2);
-  for (uint64_t g0 = from; g0 < to; g0 += 1024 * kFindGroup) {
-    const uint64_t g1 = min(g0 + 1024 * kFindGroup, to);
-    const uint64_t off_end = min(until, (g1 + 10) / 8 + 1);
-    while (!dyn_only && !have && next_off < off_end) {
-      const uint64_t ob = next_off + 4 * (uint64_t)lane;
-      uint32_t m = 0;
-      if (ob < off_end) {
-        m = stored_filter4(bits64_at(in32, ob * 8));
-        if (ob + 4 > off_end) m &= (1u << (off_end - ob)) - 1;
-      }
-      uint64_t lo = 0, hi = 0;
-      bool hit = false;
-      while (m) {
-        const int k = __ffs(m) - 1;
-        m &= m - 1;
-        if (stored_candidate(in, nbytes, ob + k, from, to, hi_to, lo, hi)) {
-          hit = true;
-          break;
-        }
-      }
-      const uint32_t b = __ballot_sync(0xFFFFFFFFu, hit);
-      if (b) {
-        const int src = __ffs(b) - 1;
-        best_lo = __shfl_sync(0xFFFFFFFFu, lo, src);
-        best_hi = __shfl_sync(0xFFFFFFFFu, hi, src);
-        have = true;
-      }
-      next_off = min(next_off + 128, off_end);
-    }
-    const uint64_t lim = have ? min(g1, best_lo + 1) : g1;
-    if (lane == 0) L->n2 = 0;
-    __syncwarp();
-    for (uint64_t w0 = g0; w0 < lim; w0 += 1024) {
-      const uint64_t pl = w0 + 32 * (uint64_t)lane;
-      uint32_t m = 0;
-      if (pl < lim) {
-        m = dyn_filter32(bits64_at(in32, pl));
-        if (pl + 32 > lim) m &= (1u << (lim - pl)) - 1;
-      }
-      const uint32_t c = __popc(m);
-      uint32_t incl = c;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-        if (lane >= d) incl += v;
-      }
-      const uint32_t tot = __shfl_sync(0xFFFFFFFFu, incl, 31);
-      uint32_t k = incl - c;
-      while (m) {
-        const int i = __ffs(m) - 1;
-        m &= m - 1;
-        L->c1[k++] = (uint16_t)(32 * lane + i);
-      }
-      __syncwarp();
-      for (uint32_t j = lane; j < tot; j += 32) {
-        const uint64_t p = w0 + L->c1[j];
-        if (dyn_leaf_ok(in, nbytes, p, leaf_lut)) {
-          const uint32_t idx = atomicAdd(&L->n2, 1u);
-          if (idx < kFindFull) L->c2[idx] = (uint32_t)(p - g0);
-        }
-      }
-      __syncwarp();
-    }
-    const uint32_t n2 = L->n2;
-    if (n2 > kFindFull) {
-      // (rare: more survivors than the list holds) the lane-by-lane search
-      // from this group on gives the same answer
-      __syncwarp();
-      return warp_find_first(in, nbytes, g0, to, hi_to, lane, out_lo, out_hi, leaf_lut, nullptr);
-    }
-    uint64_t best = kNoStop;
-    for (uint32_t j = lane; j < n2; j += 32) {
-      const uint64_t p = g0 + L->c2[j];
-      if (p < best && dyn_candidate_full(in, nbytes, p)) best = p;
-    }
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) best = min(best, __shfl_xor_sync(0xFFFFFFFFu, best, d));
-    __syncwarp();
-    if (best != kNoStop) {
-      out_lo = out_hi = best;
-      return true;
-    }
-    if (have && best_lo < g1) break;
-  }
-  out_lo = best_lo;
-  out_hi = best_hi;
-  return have;
-}
-
-static __device__ bool warp_find_first(const uint8_t* __restrict__ in, uint64_t nbytes,
-                                       uint64_t from, uint64_t to, uint64_t hi_to, int lane,
-                                       uint64_t& out_lo, uint64_t& out_hi,
-                                       const uint16_t* leaf_lut, FinderLists* L, bool dyn_only) {
-  if (L)
-    return warp_find_first_grouped(in, nbytes, from, to, hi_to, lane, out_lo, out_hi, leaf_lut, L,
-                                   dyn_only);
+                                       uint64_t& out_lo, uint64_t& out_hi) {
   const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
   if (to > nbytes * 8) to = nbytes * 8;
   if (hi_to > nbytes * 8) hi_to = nbytes * 8;
@@ -497,7 +344,7 @@ static __device__ bool warp_find_first(const uint8_t* __restrict__ in, uint64_t 
     while (m) {
       const int i = __ffs(m) - 1;
       m &= m - 1;
-      if (dyn_candidate_fast(in, nbytes, pl + i, leaf_lut)) {
+      if (dyn_candidate_fast(in, nbytes, pl + i)) {
         hit = i;
         break;
       }
@@ -536,51 +383,26 @@ static __constant__ uint8_t f_len_extra[29] = {0, 0, 0, 0, 0, 0, 0, 0, 1, 1, 1, 
 static __constant__ uint8_t f_dist_extra[30] = {0, 0, 0, 0, 1, 1, 2, 2, 3, 3, 4, 4, 5, 5, 6,
                                                 6, 7, 7, 8, 8, 9, 9, 10, 10, 11, 11, 12, 12, 13, 13};
 
-// k <= 25 bits at absolute bit p from staged words sw (sw[0] = input word wbase)
-static __device__ __forceinline__ uint32_t staged_bits(const uint32_t* sw, uint64_t wbase,
-                                                       uint64_t p, int k) {
-  const uint32_t i = (uint32_t)((p >> 5) - wbase), sh = (uint32_t)(p & 31);
-  const uint64_t v = (((uint64_t)sw[i + 1] << 32) | sw[i]) >> sh;
-  return (uint32_t)v & ((1u << k) - 1);
+// Walk entry of the 9 bits at a symbol start, fixed code: [4:0] bits of the
+// code and a length's extra bits, [6:5] 0 literal, 1 length, 2 EOB, 3 invalid.
+static __device__ __forceinline__ uint32_t fixed_entry(uint32_t x) {
+  const uint32_t c7 = __brev(x & 127u) >> 25, c8 = __brev(x & 255u) >> 24;
+  uint32_t sym, n;
+  if (c7 <= 0x17) sym = 256 + c7, n = 7;
+  else if (c8 <= 0xBF) sym = c8 - 0x30, n = 8;
+  else if (c8 <= 0xC7) sym = 280 + (c8 - 0xC0), n = 8;
+  else sym = 0, n = 9;  // 144 .. 255
+  if (sym < 256) return n;
+  if (sym == 256) return 2u << 5 | n;
+  if (sym > 285) return 3u << 5;
+  return 1u << 5 | (n + f_len_extra[sym - 257]);
 }
 
-// first symbol boundary >= target of the fixed-code walk from p, or kSyncFail
-static __device__ uint64_t fixed_walk(const uint32_t* sw, uint64_t wbase, uint64_t p,
-                                      uint64_t target) {
-  while (p < target) {
-    const uint32_t x = staged_bits(sw, wbase, p, 9);
-    const uint32_t c7 = __brev(x & 127u) >> 25, c8 = __brev(x & 255u) >> 24;
-    uint32_t sym;
-    if (c7 <= 0x17) {
-      sym = 256 + c7;
-      p += 7;
-    } else if (c8 <= 0xBF) {
-      sym = c8 - 0x30;
-      p += 8;
-    } else if (c8 <= 0xC7) {
-      sym = 280 + (c8 - 0xC0);
-      p += 8;
-    } else {
-      sym = 144 + ((__brev(x) >> 23) - 0x190);
-      p += 9;
-    }
-    if (sym < 256) continue;
-    if (sym == 256) {
-      if ((staged_bits(sw, wbase, p, 3) >> 1) != 1) return kSyncFail;
-      p += 3;
-      continue;
-    }
-    if (sym > 285) return kSyncFail;
-    p += f_len_extra[sym - 257];
-    const uint32_t dc = __brev(staged_bits(sw, wbase, p, 5)) >> 27;
-    if (dc >= 30) return kSyncFail;
-    p += 5 + f_dist_extra[dc];
-  }
-  return p;
+// words a walk of `span` bits from a start inside `starts` bits stages
+static __host__ __device__ constexpr uint32_t sync_words(uint64_t starts, uint64_t span) {
+  return (uint32_t)((starts + span + 96 + 64) / 32) + 2;
 }
 
-// words a sync search from `from` stages: [from >> 5, (target + 96) >> 5] + 1
-constexpr uint32_t kSyncWords = (uint32_t)((kSyncOffsets + kSyncSpan + 96 + 64) / 32) + 2;
 
 // ---------------------------------------------------------------------------
 // Expected output bytes per compressed byte of the dynamic block whose header
