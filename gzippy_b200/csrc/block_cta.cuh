@@ -11,7 +11,7 @@
 //      to one that met the end of the block agree).  By induction from the
 //      first range, whose start is exact, the joined ranges are the serial
 //      decode.  Each pass confirms at least one more range.  A walk leaves
-//      the first boundary past each quarter of its range, and the lookups from
+//      the first boundary past the half of its range, and the lookups from
 //      there to its end; a later walk that meets one of them is done.
 //   3. a block scan of the ranges' lookup counts gives each its place in the
 //      round's token list (a literal: one slot; a match: length, then
@@ -35,20 +35,20 @@
 
 namespace gzgpu {
 
-constexpr uint32_t kRangeMax = 512;   // bits per thread and round, at most
-constexpr uint32_t kRangeMin = 64;    // and at least (more than the longest symbol's 48)
-constexpr uint32_t kTokCap = 12288;   // token slots per round
+constexpr uint32_t kRangeMax = 640;   // bits per thread and round, at most
+constexpr uint32_t kRangeMin = 256;   // and at least (more than the longest symbol's 48)
+constexpr uint32_t kTokCap = 20480;   // token slots per round
 constexpr uint32_t kWin = 2048;       // output positions expanded at a time (divides a page)
 constexpr uint32_t kWinPer = kWin / kCtaThreads;
 constexpr uint32_t kTokPer = 4;       // token slots per thread and batch
 constexpr uint32_t kCtaDistBits = 9;  // distance LUT index bits
-constexpr uint32_t kSegs = 4;           // a range is walked in quarters
+constexpr uint32_t kSegs = 2;           // a range is walked in halves
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 
 // Table entry: [4:0] bits of the code and its extra bits, bit 5 = length code,
 // [23:8] token value without the extra bits, [30:27] code length; bit 31 =
 // not a literal, length or distance: end of block, or, by value, invalid, or
-// not in the LUT ([4:0] = 0).  The shift amounts sit where the shifts read them, so the
+// not in the LUT ([4:0] = 0; bit 5 = the distance LUT's).  The shift amounts sit where the shifts read them, so the
 // chain from one lookup to the next is mask, load, shift.
 enum : uint32_t { kEntLen = 0x20, kEntStop = 0x80000000u };
 enum : uint32_t { kStopEob = 0, kStopBad = 1, kStopLong = 2 };
@@ -65,7 +65,7 @@ __device__ __forceinline__ uint32_t tok_lit_entry(uint32_t sym, uint32_t L) {
 }
 __device__ __forceinline__ uint32_t tok_dist_entry(uint32_t sym, uint32_t L) {
   if (sym < 30) return L << 27 | (uint32_t)(c_dist_base[sym] - 1) << 8 | (L + c_dist_extra[sym]);
-  return kEntStop | kStopBad << 8;
+  return kEntStop | kEntLen | kStopBad << 8;
 }
 
 // the chunk's state, written by thread 0 (or warp 0) and read by all after a barrier
@@ -116,7 +116,7 @@ struct alignas(16) CtaSmem {
   uint32_t lit_ent[288], dist_ent[32];  // entries in canonical order
   CodeIndex lit, dist;
   uint32_t end[kCtaThreads];
-  // per quarter of each range (but the last): [9:0] first boundary at or past
+  // per part of each range but the last: [9:0] first boundary at or past
   // its end, relative to the range's first bit, [31:10] lookups from there
   uint32_t cp[kSegs - 1][kCtaThreads];
   uint32_t scan[2][kCtaThreads / 32];
@@ -147,15 +147,18 @@ __device__ __forceinline__ uint32_t cta_scan(CtaSmem<LB>* S, uint32_t par, uint3
   return pa + x - a;
 }
 
-// The entry of a code longer than the LUT, or kStopBad.
+// The entry of a code longer than the LUT's bits (9 for distances, 10 or more
+// for literals and lengths), or kStopBad.  Inlined where it is used: a call in
+// the walks' loops, taken or not, cost 30 cycles an iteration.
 template <int LB>
-__device__ __noinline__ uint32_t long_entry(const CtaSmem<LB>* S, uint32_t x, bool dist) {
+__device__ __forceinline__ uint32_t long_entry(const CtaSmem<LB>* S, uint32_t x, bool dist) {
+  static_assert(LB >= 10 && kCtaDistBits == 9, "codes looked up here have 10 bits at least");
   const CodeIndex& I = dist ? S->dist : S->lit;
   const uint32_t rev = __brev(x) >> 17;  // 15 code bits, first bit = MSB
-  uint32_t L = 1;
+  uint32_t L = 10;
 #pragma unroll
-  for (int l = 1; l <= 15; l++) L += rev >= I.lim[l] ? 1u : 0u;
-  if (L > 15) return kEntStop | kStopBad << 8;
+  for (int l = 10; l <= 15; l++) L += rev >= I.lim[l] ? 1u : 0u;
+  if (L > 15) return kEntStop | (dist ? kEntLen : 0u) | kStopBad << 8;
   const uint32_t i = (rev >> (15 - L)) + I.base[L];
   return dist ? S->dist_ent[i] : S->lit_ent[i];
 }
@@ -207,17 +210,16 @@ struct RangeBits {
     q = (pos & ~31u) + 2;  // 32 - (pos & 31) bits in place
     refill_if_due();
   }
-  __device__ __forceinline__ void take(uint32_t ent) {  // ent[4:0] bits
+  __device__ __forceinline__ void shift(uint32_t ent) {  // by ent[4:0] bits
     lo = __funnelshift_r(lo, hi, ent);
     hi = __funnelshift_r(hi, 0, ent);
     p += ent & 31;
-    refill_if_due();
   }
 };
 
 // what ended a range's walk before its end
 enum : uint32_t { kTermNone = 0, kTermEob = 1, kTermBad = 2 };
-constexpr uint32_t kNoCp = 0x3FFu;  // a quarter without a recorded boundary
+constexpr uint32_t kNoCp = 0x3FFu;  // a part without a recorded boundary
 
 // One thread's range of a round: where it starts and ends, and the lookups
 // between (a literal is one, a match two).
@@ -227,54 +229,82 @@ struct Range {
   bool guessed_on;          // walked on from a guess past a stop: starts nowhere
 };
 
-// Walk the range [first, first + r) (cut at e) from r.start on, positions
-// relative to `base`.  One table lookup per iteration: a literal or a length
-// code, or the distance code of the length just read, so threads at literals
-// and threads inside matches run the same instructions.  guess: the start may
-// be no symbol boundary; go on past a stop (from the next bit) to find a
-// likely end for the range.  Otherwise a stop ends the walk.  again: an earlier
-// walk of this round left its boundaries, and meeting one ends this walk: from
-// there on they agree.
+// The two tables as one: the byte offset of the current one (0: literals and
+// lengths) and its index mask.  A stop entry keeps the table it came from.
+template <int LB>
+struct TableAt {
+  uint32_t off = 0, mask = ((1u << LB) - 1) << 2;
+  __device__ __forceinline__ uint32_t look(const char* lut, const RangeBits& b) const {
+    return *reinterpret_cast<const uint32_t*>(lut + ((b.lo & mask) | off));
+  }
+  __device__ __forceinline__ void after(uint32_t ent) {
+    off = ent & kEntLen ? 4u << LB : 0u;
+    mask = off ? ((1u << kCtaDistBits) - 1) << 2 : ((1u << LB) - 1) << 2;
+  }
+};
+
+// Walk the range [first, first + len) (cut at e) from r.start on, positions
+// relative to `base`.  A lookup is a literal or a length code, or the distance
+// code of the length just read, so threads at literals and threads inside
+// matches run the same instructions.  Four lookups per loop: a lookup that is
+// not due (past the end, or too few bits before the next refill) takes nothing,
+// which is cheaper than branching around it (warp alone: 143 cycles a lookup
+// one by one, 100 so; 24 warps: 216 and 165).  guess: the start may be no
+// symbol boundary; go on past a stop (from the next bit) to find a likely end
+// for the range.  Otherwise a stop ends the walk.  again: an earlier walk of
+// this round left its boundaries, and meeting one ends this walk: from there
+// on they agree.
 template <int LB>
 __device__ __forceinline__ void walk_range(CtaSmem<LB>* S, const uint32_t* base, uint32_t first,
                                            uint32_t len, uint32_t e, bool guess, bool again,
                                            Range& r) {
-  constexpr uint32_t LM = ((1u << LB) - 1) << 2, DM = ((1u << kCtaDistBits) - 1) << 2;
   const uint32_t tid = threadIdx.x;
   const char* lut = reinterpret_cast<const char*>(S->lut);
   RangeBits b;
   b.seek(base, r.start);
+  TableAt<LB> t;
   uint32_t slots = 0, valid_from = 0, seg = 0;
-  uint32_t mask = LM, off = 0;
   r.term = kTermNone;
   r.guessed_on = false;
   bool met = false;
   for (;; seg++) {
     uint32_t es = seg == kSegs - 1 ? e : min(e, first + (seg + 1) * (len / kSegs));
     if (b.p < es) do {
-      uint32_t ent = *reinterpret_cast<const uint32_t*>(lut + ((b.lo & mask) | off));
-      if (__builtin_expect((int32_t)ent < 0, 0)) {
-        if (((ent >> 8) & 3) == kStopLong) ent = long_entry<LB>(S, b.lo >> 2, off != 0);
-        if ((int32_t)ent < 0) {
-          if (guess) {
-            r.guessed_on = true;
-            valid_from = seg;  // boundaries before the stop lead to it
-            ent = 1;           // one bit on
-          } else {
-            const bool eob = ((ent >> 8) & 3) == kStopEob;
-            r.term = eob ? kTermEob : kTermBad;
-            r.term_pos = b.p + (eob ? (ent >> 27) & 15 : 0u);
-            slots--;
-            ent = 0;
-            es = 0;  // ends the walk
-          }
-        }
+      uint32_t stop = 0;
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const bool due = b.p < (t.off ? kNone : es) && (u % 2 == 0 || b.p < b.q);
+        const uint32_t ent = due ? t.look(lut, b) : 0u;
+        b.shift(ent);
+        slots += (int32_t)ent > 0 ? 1u : 0u;
+        if (due) t.after(ent);
+        stop |= ent;
+        if (u % 2) b.refill_if_due();
       }
-      b.take(ent);
-      slots++;
-      mask = ent & kEntLen ? DM : LM;
-      off = ent & kEntLen ? 4u << LB : 0u;
-    } while (b.p < (off ? kNone : es));
+      if (__builtin_expect((int32_t)stop < 0, 0)) {
+        // at p: a code beyond the LUT, or a stop
+        const bool dist = t.off != 0;
+        uint32_t ent = t.look(lut, b);
+        if (((ent >> 8) & 3) == kStopLong) ent = long_entry<LB>(S, b.lo >> 2, dist);
+        if ((int32_t)ent >= 0) {
+          slots++;
+        } else if (guess) {
+          r.guessed_on = true;
+          valid_from = seg;  // boundaries before the stop lead to it
+          slots++;
+          ent = 1;           // one bit on
+        } else {
+          const bool eob = ((ent >> 8) & 3) == kStopEob;
+          r.term = eob ? kTermEob : kTermBad;
+          r.term_pos = b.p + (eob ? (ent >> 27) & 15 : 0u);
+          ent = 0;
+          es = 0;  // ends the walk
+        }
+        b.shift(ent);
+        b.refill_if_due();
+        t.after(ent);
+      }
+    } while (b.p < (t.off ? kNone : es));
     if (r.term || seg == kSegs - 1) break;
     const uint32_t at = b.p - first;
     if (again) {
@@ -287,7 +317,7 @@ __device__ __forceinline__ void walk_range(CtaSmem<LB>* S, const uint32_t* base,
     }
     S->cp[seg][tid] = at | slots << 10;
   }
-  // seg quarters were passed; their lookups become those left to the end
+  // seg parts were passed; their lookups become those left to the end
   for (uint32_t k = 0; k < kSegs - 1; k++) {
     if (r.term || (guess && k < valid_from)) S->cp[k][tid] = kNoCp;
     else if (k < seg) S->cp[k][tid] = (S->cp[k][tid] & 0x3FFu) | (slots - (S->cp[k][tid] >> 10)) << 10;
@@ -296,24 +326,39 @@ __device__ __forceinline__ void walk_range(CtaSmem<LB>* S, const uint32_t* base,
   if (!r.term && !met) r.end = b.p;
 }
 
-// The tokens of the symbols that start in [start, e), n of them, to tok.
+// The tokens of the n lookups from start on to tok.
 template <int LB>
 __device__ __forceinline__ void write_tokens(const CtaSmem<LB>* S, const uint32_t* base,
                                              uint32_t start, uint32_t n, uint16_t* tok) {
-  constexpr uint32_t LM = ((1u << LB) - 1) << 2, DM = ((1u << kCtaDistBits) - 1) << 2;
   const char* lut = reinterpret_cast<const char*>(S->lut);
   RangeBits b;
   b.seek(base, start);
-  uint32_t mask = LM, off = 0;
-  for (uint32_t i = 0; i < n; i++) {
-    uint32_t ent = *reinterpret_cast<const uint32_t*>(lut + ((b.lo & mask) | off));
-    if (__builtin_expect((int32_t)ent < 0, 0)) ent = long_entry<LB>(S, b.lo >> 2, off != 0);
-    // value + extra bits: the code's bits cut off the front of what it takes
-    const uint32_t x = (b.lo >> 2) & ~(0xFFFFFFFFu << (ent & 31));
-    tok[i] = (uint16_t)((ent >> 8) + (x >> (ent >> 27)));
-    b.take(ent);
-    mask = ent & kEntLen ? DM : LM;
-    off = ent & kEntLen ? 4u << LB : 0u;
+  TableAt<LB> t;
+  uint16_t* const end = tok + n;
+  while (tok < end) {
+    uint32_t stop = 0;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const bool due = tok < end && (u % 2 == 0 || b.p < b.q);
+      const uint32_t ent = due ? t.look(lut, b) : 0u;
+      if ((int32_t)ent > 0) {
+        // value + extra bits: the code's bits cut off the front of what it takes
+        const uint32_t x = (b.lo >> 2) & ~(0xFFFFFFFFu << (ent & 31));
+        *tok++ = (uint16_t)((ent >> 8) + (x >> (ent >> 27)));
+      }
+      b.shift(ent);
+      if (due) t.after(ent);
+      stop |= ent;
+      if (u % 2) b.refill_if_due();
+    }
+    if (__builtin_expect((int32_t)stop < 0, 0)) {
+      const uint32_t ent = long_entry<LB>(S, b.lo >> 2, t.off != 0);
+      const uint32_t x = (b.lo >> 2) & ~(0xFFFFFFFFu << (ent & 31));
+      *tok++ = (uint16_t)((ent >> 8) + (x >> (ent >> 27)));
+      b.shift(ent);
+      b.refill_if_due();
+      t.after(ent);
+    }
   }
 }
 
@@ -371,12 +416,12 @@ __device__ __noinline__ bool index_code(const uint8_t* lens, int n, CodeIndex* I
 // LUT entry i: the entry of the code at the head of i's low TB bits
 template <int TB>
 __device__ __forceinline__ uint32_t lut_value(uint32_t i, const uint32_t* lim, const CodeIndex* I,
-                                              const uint32_t* ent) {
+                                              const uint32_t* ent, uint32_t longer) {
   const uint32_t rev = __brev(i) >> 17;
   uint32_t L = 1;
 #pragma unroll
   for (int l = 1; l <= TB; l++) L += rev >= lim[l] ? 1u : 0u;
-  if (L > TB) return kEntStop | kStopLong << 8;
+  if (L > TB) return longer;
   return ent[(rev >> (15 - L)) + I->base[L]];
 }
 
@@ -400,11 +445,12 @@ __device__ __forceinline__ bool cta_build_tables(CtaSmem<LB>* S) {
 #pragma unroll
   for (int l = 1; l <= LB; l++) lim[l] = S->lit.lim[l];
   for (uint32_t i = threadIdx.x; i < (1u << LB); i += kCtaThreads)
-    S->lut[i] = lut_value<LB>(i, lim, &S->lit, S->lit_ent);
+    S->lut[i] = lut_value<LB>(i, lim, &S->lit, S->lit_ent, kEntStop | kStopLong << 8);
 #pragma unroll
   for (int l = 1; l <= (int)kCtaDistBits; l++) lim[l] = S->dist.lim[l];
   for (uint32_t i = threadIdx.x; i < (1u << kCtaDistBits); i += kCtaThreads)
-    S->lut[(1u << LB) + i] = lut_value<(int)kCtaDistBits>(i, lim, &S->dist, S->dist_ent);
+    S->lut[(1u << LB) + i] = lut_value<(int)kCtaDistBits>(i, lim, &S->dist, S->dist_ent,
+                                                          kEntStop | kEntLen | kStopLong << 8);
   __syncthreads();
   return true;
 }
