@@ -18,6 +18,9 @@
 //      distance), written by one decode of each range.
 //   4. the tokens are expanded in windows of kWin output positions (see
 //      expand_tokens), which leave as coalesced stores to the pages.
+// Threads leave the data-dependent loops at different times; a warp barrier
+// joins its lanes before every barrier of the CTA, which all lanes of a warp
+// have to reach together.
 // What bounds a block is its serial chain of code lookups; the ranges cut
 // that chain into up to 256 pieces.  Ranges of 512 bits end in step after a
 // wrong start for 98 % of text, 88 % of byte runs and 59 % of noisy ramps
@@ -37,7 +40,7 @@ namespace gzgpu {
 
 constexpr uint32_t kRangeMax = 640;   // bits per thread and round, at most
 constexpr uint32_t kRangeMin = 256;   // and at least (more than the longest symbol's 48)
-constexpr uint32_t kTokCap = 20480;   // token slots per round
+constexpr uint32_t kTokCap = 18432;   // token slots per round
 constexpr uint32_t kWin = 2048;       // output positions expanded at a time (divides a page)
 constexpr uint32_t kWinPer = kWin / kCtaThreads;
 constexpr uint32_t kTokPer = 4;       // token slots per thread and batch
@@ -88,7 +91,7 @@ struct CtaCtl {
   uint32_t round_slots, round_lanes, round_kind, round_pos;
   int32_t carry_ms;         // match reaching into the next window: start (relative to it)
   uint32_t carry_len, carry_dist;
-  uint32_t any_match, bad_dist, mark_max;
+  uint32_t any_match[2], bad_dist[2], mark_max;
 };
 
 // A code beside its LUT: codes are canonical, so the length of the code at the
@@ -109,8 +112,9 @@ struct alignas(16) CtaSmem {
   union {
     HeaderScratch h;  // block header
     struct {          // expansion
-      alignas(16) uint32_t stage[kWin];
-      uint32_t bm[kWin / 32];  // match starts
+      // two windows, by turns
+      alignas(16) uint32_t stage[2][kWin];
+      uint32_t bm[2][kWin / 32];  // match starts
     };
   };
   uint32_t lit_ent[288], dist_ent[32];  // entries in canonical order
@@ -491,7 +495,10 @@ __device__ __forceinline__ bool cta_page(CtaSmem<LB>* S, const PagePool& pool, u
 // the chunk), or a position of this window, followed by pointer jumping
 // through the stage.  Neighbours mostly share a match, so a match is looked at
 // once per thread, its sources are loaded from one address, and the window
-// leaves in 16-byte stores; a window without matches goes out as it is.
+// leaves in 16-byte stores; a window without matches goes out as it is.  The
+// stage has two turns, so a window needs three barriers: its tokens are placed
+// (which also makes the window before it readable as history), its records are
+// read, its references are in place.
 // Returns kOk, kBadDeflate (a distance beyond the window) or kPoolExhausted.
 template <int LB>
 __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool& pool, uint32_t n,
@@ -504,10 +511,11 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
   uint32_t b0 = 0;             // first slot of the batch
   uint32_t bpos = rel0, bend;  // positions of the batch
   uint32_t pos[kTokPer], len[kTokPer], val[kTokPer], par = 0;
-  for (uint32_t i = tid; i < kWin / 32; i += kCtaThreads) S->bm[i] = 0;
+  if (tid < kWin / 16) (&S->bm[0][0])[tid] = 0;
   if (tid == 0) {
-    S->c.any_match = 0;
-    S->c.carry_len = 0;
+    S->c.any_match[0] = S->c.any_match[1] = 0;
+    S->c.bad_dist[0] = S->c.bad_dist[1] = 0;
+    S->c.carry_len = S->c.mark_max = 0;
   }
   __syncthreads();
   auto load_batch = [&]() {
@@ -540,7 +548,9 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
     bend = bpos + ta;
   };
   load_batch();
-  for (;;) {
+  for (uint32_t turn = 0;; turn ^= 1) {
+    uint32_t* const stage = S->stage[turn];
+    uint32_t* const bm = S->bm[turn];
     const uint32_t wbase = lo & ~(kWin - 1), wend = wbase + kWin;
     if (!cta_page(S, pool, base + wbase)) return kPoolExhausted;
     for (;;) {
@@ -551,12 +561,12 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
         const uint32_t q = pos[k] - wbase;
         if (val[k] & kTokMatch) {
           const uint32_t d1 = S->tok[b0 + kTokPer * tid + k + 1];  // distance - 1
-          S->stage[q] = len[k] << 16 | d1;
-          atomicOr(&S->bm[q >> 5], 1u << (q & 31));
-          S->c.any_match = 1;
-          if ((uint64_t)d1 + 1 > base + pos[k] + kWindow) S->c.bad_dist = 1;
+          stage[q] = len[k] << 16 | d1;
+          atomicOr(&bm[q >> 5], 1u << (q & 31));
+          S->c.any_match[turn] = 1;
+          if ((uint64_t)d1 + 1 > base + pos[k] + kWindow) S->c.bad_dist[turn] = 1;
         } else {
-          S->stage[q] = val[k];
+          stage[q] = val[k];
         }
       }
       if (bend >= wend || b0 + kTokPer * kCtaThreads >= n) break;
@@ -564,17 +574,19 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
       bpos = bend;
       load_batch();
     }
+    __syncwarp();
     __syncthreads();
+    if (S->c.bad_dist[turn]) return kBadDeflate;
     const uint32_t hi = min(wend, bend) - wbase, l0 = lo - wbase;
     uint16_t* page = pool.data + (size_t)S->c.page_cur * kPageEntries +
                      ((uint32_t)(base + wbase) & (kPageEntries - 1));
-    const bool matches = S->c.any_match != 0 || S->c.carry_len != 0;
+    const bool matches = S->c.any_match[turn] != 0 || S->c.carry_len != 0;
     // this thread's positions: e0 .. e0 + 7
     const uint32_t e0 = kWinPer * tid;
     uint32_t st[kWinPer];  // a position's value, or (bit 31) a reference into the window
     {
-      const uint4 a = reinterpret_cast<const uint4*>(S->stage)[2 * tid];
-      const uint4 b = reinterpret_cast<const uint4*>(S->stage)[2 * tid + 1];
+      const uint4 a = reinterpret_cast<const uint4*>(stage)[2 * tid];
+      const uint4 b = reinterpret_cast<const uint4*>(stage)[2 * tid + 1];
       st[0] = a.x, st[1] = a.y, st[2] = a.z, st[3] = a.w;
       st[4] = b.x, st[5] = b.y, st[6] = b.z, st[7] = b.w;
     }
@@ -589,11 +601,11 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
       // the last match start before e0: in this warp, else in the nine words
       // before the warp's (a match is at most 258 long), else the match that
       // reaches in from the window before
-      uint32_t bits = (S->bm[tid >> 2] >> (8 * (tid & 3))) & 0xFFu;
+      uint32_t bits = (bm[tid >> 2] >> (8 * (tid & 3))) & 0xFFu;
       const int32_t own = (int32_t)e0 + 31 - __clz(bits | 1u);
       const uint32_t have = __ballot_sync(0xFFFFFFFFu, bits != 0);
       const int32_t wi = (int32_t)(tid >> 5) * 8 - 1 - lane;
-      const uint32_t pw = lane < 9 && wi >= 0 ? S->bm[wi] : 0u;
+      const uint32_t pw = lane < 9 && wi >= 0 ? bm[wi] : 0u;
       const uint32_t havep = __ballot_sync(0xFFFFFFFFu, pw != 0);
       const int32_t far = __shfl_sync(0xFFFFFFFFu, 32 * wi + 31 - __clz(pw | 1u), __ffs(havep | 0x80000000u) - 1);
       const uint32_t below = have & ((1u << lane) - 1);
@@ -602,7 +614,7 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
       int32_t ms = at >= 0 ? at : c_ms;
       uint32_t ml = c_len, md = c_dist;
       if (at >= 0) {
-        const uint32_t d = S->stage[at];
+        const uint32_t d = stage[at];
         ml = d >> 16;
         md = (d & 0xFFFFu) + 1;
       }
@@ -653,42 +665,42 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
         if (!bits) break;
         bits &= bits - 1;
         ms = (int32_t)(e0 + nx);
-        const uint32_t d = S->stage[ms];
+        const uint32_t d = stage[ms];
         ml = d >> 16;
         md = (d & 0xFFFFu) + 1;
       }
       uint32_t left = 0;
 #pragma unroll
       for (uint32_t i = 0; i < kWinPer; i++) left |= (cover >> i) & 1 ? st[i] : 0u;
+      __syncwarp();
       const bool any_ref = __syncthreads_or((int)(left >> 31));
       if (hi - 1 - e0 < kWinPer) {  // the last position's match may go on in the next window
         S->c.carry_ms = ms - (int32_t)kWin;
         S->c.carry_len = ms + (int32_t)ml > (int32_t)hi ? ml : 0u;
         S->c.carry_dist = md;
       }
-      if (tid < kWin / 32) S->bm[tid] = 0;
-      if (tid == 0) S->c.any_match = 0;
+      if (tid < kWin / 32) bm[tid] = 0;
+      if (tid == 0) S->c.any_match[turn] = 0;
       if (any_ref) {
         if (cover) {
-          reinterpret_cast<uint4*>(S->stage)[2 * tid] = make_uint4(st[0], st[1], st[2], st[3]);
-          reinterpret_cast<uint4*>(S->stage)[2 * tid + 1] = make_uint4(st[4], st[5], st[6], st[7]);
+          reinterpret_cast<uint4*>(stage)[2 * tid] = make_uint4(st[0], st[1], st[2], st[3]);
+          reinterpret_cast<uint4*>(stage)[2 * tid + 1] = make_uint4(st[4], st[5], st[6], st[7]);
         }
-        // references: a position takes its source's value, or the source's own
-        // reference (always further back), until none is left
-        for (;;) {
+        __syncthreads();
+        // A reference takes its source's value, or the source's own reference,
+        // always further back: every thread follows its own to their ends,
+        // and what it learns on the way shortens the others' paths.
+        while (left >> 31) {
           left = 0;
 #pragma unroll
-          for (uint32_t i = 0; i < kWinPer; i++) left |= (cover >> i) & 1 ? st[i] : 0u;
-          if (!__syncthreads_or((int)(left >> 31))) break;
-          if (left >> 31) {
-#pragma unroll
-            for (uint32_t i = 0; i < kWinPer; i++)
-              if ((cover >> i) & 1 && st[i] >> 31) {
-                st[i] = *(volatile uint32_t*)&S->stage[st[i] & 0xFFFFu];
-                *(volatile uint32_t*)&S->stage[e0 + i] = st[i];
-              }
-          }
+          for (uint32_t i = 0; i < kWinPer; i++)
+            if ((cover >> i) & 1 && st[i] >> 31) {
+              st[i] = *(volatile uint32_t*)&stage[st[i] & 0xFFFFu];
+              *(volatile uint32_t*)&stage[e0 + i] = st[i];
+              left |= st[i];
+            }
         }
+        __syncwarp();
       }
     }
     // out to the page, eight entries per store
@@ -712,15 +724,9 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
         }
         if (__any_sync(0xFFFFFFFFu, mk != 0)) {
           mk = __reduce_max_sync(0xFFFFFFFFu, mk);
-          if ((tid & 31) == 0) atomicMax(&S->c.mark_max, mk);
+          if ((tid & 31) == 0) atomicMax(&S->c.mark_max, wbase + mk);
         }
       }
-    }
-    __syncthreads();
-    if (S->c.bad_dist) return kBadDeflate;
-    if (matches && !zero_window && tid == 0 && S->c.mark_max) {
-      S->c.marker_end = base + wbase + S->c.mark_max;
-      S->c.mark_max = 0;
     }
     lo = wbase + hi;
     if (bend <= wend) {  // the batch is used up
@@ -730,7 +736,11 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
       load_batch();
     }
   }
-  if (tid == 0) S->c.o = base + lo;
+  __syncthreads();
+  if (tid == 0) {
+    S->c.o = base + lo;
+    if (S->c.mark_max) S->c.marker_end = base + S->c.mark_max;
+  }
   return kOk;
 }
 
@@ -776,6 +786,7 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
       walk_range<LB>(S, base, first, r, e, tid > 0, false, ra);
       S->end[tid] = ra.end;
     }
+    __syncwarp();
     // 2. from the end of the range before, until nothing moves
     uint32_t last = kNone;  // range that holds the end of the block (kNone: not in this round)
     for (uint32_t it = 0;; it ^= 1) {
@@ -798,6 +809,7 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
         walk_range<LB>(S, base, first, r, e, false, true, ra);
         S->end[tid] = ra.end;
       }
+      __syncwarp();
     }
     // 3. places in the token list; ranges beyond its capacity wait for the next round
     const uint32_t used = last != kNone ? last + 1 : lanes;
@@ -833,6 +845,7 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
       break;
     }
     if (tid < n_lanes) write_tokens<LB>(S, base, ra.start, my_slots, S->tok + slot0);
+    __syncwarp();
     __syncthreads();
     // 4. expansion
     if (n_slots) {
@@ -1182,7 +1195,6 @@ __device__ __forceinline__ void cta_begin(CtaCtl& c, const ChunkDesc& d, uint32_
   c.page_cur = c.page_prev = kNoPage;
   c.page_seq = 0;
   c.n_pages = 0;
-  c.bad_dist = c.mark_max = 0;
   c.bfinal = c.btype = 0;
   cta_set_limit(c);
 }
