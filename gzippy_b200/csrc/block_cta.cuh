@@ -91,7 +91,7 @@ struct CtaCtl {
   uint32_t round_slots, round_lanes, round_kind, round_pos;
   int32_t carry_ms;         // match reaching into the next window: start (relative to it)
   uint32_t carry_len, carry_dist;
-  uint32_t any_match[2], bad_dist[2], mark_max;
+  uint32_t mark_max;
 };
 
 // A code beside its LUT: codes are canonical, so the length of the code at the
@@ -499,7 +499,8 @@ __device__ __forceinline__ bool cta_page(CtaSmem<LB>* S, const PagePool& pool, u
 // stage has two turns, so a window needs three barriers: its tokens are placed
 // (which also makes the window before it readable as history), its records are
 // read, its references are in place.
-// Returns kOk, kBadDeflate (a distance beyond the window) or kPoolExhausted.
+// Returns kOk or kPoolExhausted.  (No distance reaches beyond the window before
+// the chunk: a code names 32768 at most.)
 template <int LB>
 __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool& pool, uint32_t n,
                                                  bool zero_window) {
@@ -510,33 +511,31 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
   uint32_t lo = rel0;          // next position to write
   uint32_t b0 = 0;             // first slot of the batch
   uint32_t bpos = rel0, bend;  // positions of the batch
-  uint32_t pos[kTokPer], len[kTokPer], val[kTokPer], par = 0;
+  uint32_t pos[kTokPer], len[kTokPer], rec[kTokPer], par = 0;
   if (tid < kWin / 16) (&S->bm[0][0])[tid] = 0;
   if (tid == 0) {
-    S->c.any_match[0] = S->c.any_match[1] = 0;
-    S->c.bad_dist[0] = S->c.bad_dist[1] = 0;
     S->c.carry_len = S->c.mark_max = 0;
   }
   __syncthreads();
+  // rec: what the slot puts at its position, a literal or a match's record
+  // (length and distance - 1)
   auto load_batch = [&]() {
     const uint32_t i = b0 + kTokPer * tid;
-    uint32_t sum = 0;
-    uint32_t prev = 0;
+    uint32_t sum = 0, prev = 0, next = 0;
+    uint2 t = make_uint2(0, 0);
     if (i < n) {
-      const uint2 t = *reinterpret_cast<const uint2*>(S->tok + i);
+      t = *reinterpret_cast<const uint2*>(S->tok + i);
       prev = i ? S->tok[i - 1] : 0u;
-      val[0] = t.x & 0xFFFFu;
-      val[1] = t.x >> 16;
-      val[2] = t.y & 0xFFFFu;
-      val[3] = t.y >> 16;
-    } else {
-      val[0] = val[1] = val[2] = val[3] = 0;
+      next = S->tok[i + kTokPer];
     }
+    const uint32_t val[kTokPer + 1] = {t.x & 0xFFFFu, t.x >> 16, t.y & 0xFFFFu, t.y >> 16, next};
 #pragma unroll
     for (uint32_t k = 0; k < kTokPer; k++) {
-      const uint32_t t = val[k];
-      len[k] = i + k >= n ? 0u : (t & kTokMatch ? t & 0x1FFu : (prev & kTokMatch ? 0u : 1u));
-      prev = t;
+      const bool match = val[k] & kTokMatch;
+      len[k] = match ? val[k] & 0x1FFu : (prev & kTokMatch ? 0u : 1u);
+      if (i + k >= n) len[k] = 0;
+      rec[k] = match ? len[k] << 16 | val[k + 1] : val[k];
+      prev = val[k];
       pos[k] = sum;
       sum += len[k];
     }
@@ -553,20 +552,20 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
     uint32_t* const bm = S->bm[turn];
     const uint32_t wbase = lo & ~(kWin - 1), wend = wbase + kWin;
     if (!cta_page(S, pool, base + wbase)) return kPoolExhausted;
+    // (the thread that wrote it in the window before sees it in time, which is
+    // enough for the vote)
+    uint32_t any_match = S->c.carry_len;
     for (;;) {
       // the batch's tokens that start in this window
 #pragma unroll
       for (uint32_t k = 0; k < kTokPer; k++) {
-        if (!len[k] || pos[k] < lo || pos[k] >= wend) continue;
         const uint32_t q = pos[k] - wbase;
-        if (val[k] & kTokMatch) {
-          const uint32_t d1 = S->tok[b0 + kTokPer * tid + k + 1];  // distance - 1
-          stage[q] = len[k] << 16 | d1;
-          atomicOr(&bm[q >> 5], 1u << (q & 31));
-          S->c.any_match[turn] = 1;
-          if ((uint64_t)d1 + 1 > base + pos[k] + kWindow) S->c.bad_dist[turn] = 1;
-        } else {
-          stage[q] = val[k];
+        if (len[k] && pos[k] >= lo && q < kWin) {
+          stage[q] = rec[k];
+          if (len[k] > 1) {
+            atomicOr(&bm[q >> 5], 1u << (q & 31));
+            any_match = 1;
+          }
         }
       }
       if (bend >= wend || b0 + kTokPer * kCtaThreads >= n) break;
@@ -575,12 +574,10 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
       load_batch();
     }
     __syncwarp();
-    __syncthreads();
-    if (S->c.bad_dist[turn]) return kBadDeflate;
+    const bool matches = __syncthreads_or((int)any_match);
     const uint32_t hi = min(wend, bend) - wbase, l0 = lo - wbase;
     uint16_t* page = pool.data + (size_t)S->c.page_cur * kPageEntries +
                      ((uint32_t)(base + wbase) & (kPageEntries - 1));
-    const bool matches = S->c.any_match[turn] != 0 || S->c.carry_len != 0;
     // this thread's positions: e0 .. e0 + 7
     const uint32_t e0 = kWinPer * tid;
     uint32_t st[kWinPer];  // a position's value, or (bit 31) a reference into the window
@@ -634,7 +631,15 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
           const uint32_t mine = ((1u << x1) - 1) & ~((1u << x0) - 1);
           cover |= mine;
           const bool wrap = r + cnt > md;
-          if (!wrap && (s0 >= (int32_t)l0 || wabs + s1 < 0)) {
+          if (wrap && ms - (int32_t)md >= (int32_t)l0) {
+            // round and round one stretch of this window
+#pragma unroll
+            for (uint32_t i = 0; i < kWinPer; i++)
+              if ((mine >> i) & 1) {
+                st[i] = 0x80000000u | (uint32_t)(ms - (int32_t)md + (int32_t)r);
+                r = r + 1 == md ? 0u : r + 1;
+              }
+          } else if (!wrap && (s0 >= (int32_t)l0 || wabs + s1 < 0)) {
             // references into the window, or markers (zeros) before the chunk
             const bool ref = s0 >= (int32_t)l0;
             const uint32_t v0 = ref ? 0x80000000u | (uint32_t)s0
@@ -680,7 +685,6 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
         S->c.carry_dist = md;
       }
       if (tid < kWin / 32) bm[tid] = 0;
-      if (tid == 0) S->c.any_match[turn] = 0;
       if (any_ref) {
         if (cover) {
           reinterpret_cast<uint4*>(stage)[2 * tid] = make_uint4(st[0], st[1], st[2], st[3]);
