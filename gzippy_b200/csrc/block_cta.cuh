@@ -46,6 +46,10 @@ constexpr uint32_t kWinPer = kWin / kCtaThreads;
 constexpr uint32_t kTokPer = 4;       // token slots per thread and batch
 constexpr uint32_t kCtaDistBits = 9;  // distance LUT index bits
 constexpr uint32_t kSegs = 2;           // a range is walked in halves
+// a block header's code lengths: bits (316 codes of 7 bits, or fewer symbols)
+// and symbols at most
+constexpr uint32_t kHdrBits = 2240;
+constexpr uint32_t kHdrSyms = 320;
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 
 // Table entry: [4:0] bits of the code and its extra bits, bit 5 = length code,
@@ -75,6 +79,7 @@ __device__ __forceinline__ uint32_t tok_dist_entry(uint32_t sym, uint32_t L) {
 struct CtaCtl {
   uint64_t pos, o;          // next input bit, entries written
   uint64_t stop_lo, abort_bit, slack, limit_words, trunc_words, in_end, table_bit;
+  uint64_t hdr_pos;         // first bit after a dynamic header's precode
   uint64_t blk_hdr;         // header bit of the block being decoded (0 = unknown)
   uint64_t marker_end, sync_target, passed_bit;
   uint64_t cand_lo, cand_hi;
@@ -85,6 +90,7 @@ struct CtaCtl {
   uint32_t nlen, ndist, final_block, synced, passed, resume, in_sync_block;
   uint32_t spec, again;     // speculative start; try the next candidate
   uint32_t fixed_tables;    // the tables in place are the fixed code's
+  uint32_t hdr_move, hdr_end;  // move pos past the header; its length after hdr_pos
   uint32_t build_ok[2];
   uint32_t page_cur, page_prev, page_seq, n_pages;
   uint32_t min_need[2], min_term[2];
@@ -108,9 +114,18 @@ struct alignas(16) CtaSmem {
   // literal/length LUT, then the distance LUT (at a power of two, so that its
   // offset joins an index by OR)
   uint32_t lut[(1 << LB) + (1 << kCtaDistBits)];
-  uint16_t tok[kTokCap + 8];
   union {
-    HeaderScratch h;  // block header
+    uint16_t tok[kTokCap + 8];
+    uint16_t hop[4][kHdrBits];  // block header: position 1, 2, 4 and 8 symbols on
+  };
+  union {
+    struct {  // block header
+      uint8_t lens[320];        // literal/length codes at 0, distance codes at 288
+      uint8_t pre_lens[32];
+      uint32_t pre_lut[128];
+      uint16_t group[kHdrSyms / 8];  // position of every eighth symbol
+      uint8_t val[kHdrSyms];         // a symbol's length, 0xFF: that of the one before
+    };
     struct {          // expansion
       // two windows, by turns
       alignas(16) uint32_t stage[2][kWin];
@@ -429,7 +444,114 @@ __device__ __forceinline__ uint32_t lut_value(uint32_t i, const uint32_t* lim, c
   return ent[(rev >> (15 - L)) + I->base[L]];
 }
 
-// Both code tables from h.lens (whole CTA).  Warp 0 sorts the
+// The code lengths of a dynamic block's header into S->lens (whole CTA): the
+// precode's lengths are in S->pre_lens and indexed (S->lit), S->c.pos is the
+// first bit after them.  A symbol's place depends on all before it, 200 and
+// more of them one after another (150 cycles each when a warp read them so, a
+// fifth of the decode of a 16 KB block).  Here every bit position is decoded as
+// if a symbol started there; two, four and eight symbols on follow by doubling,
+// so one thread takes eight symbols a step, and the symbols on that chain are
+// then expanded in parallel.  Returns kOk or an error status; S->c.pos moves
+// past the header.
+template <int LB>
+__device__ __forceinline__ int32_t cta_read_lens(const uint8_t* __restrict__ in, CtaSmem<LB>* S,
+                                                 bool move) {
+  const uint32_t tid = threadIdx.x;
+  const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
+  const uint64_t pos = S->c.hdr_pos, w0 = pos >> 5, trunc = S->c.trunc_words;
+  const uint32_t nlen = S->c.nlen, total = nlen + S->c.ndist;
+  if (tid < 128) {
+    const uint32_t rev = __brev(tid) >> 17;
+    uint32_t L = 1;
+#pragma unroll
+    for (int l = 1; l <= 7; l++) L += rev >= S->lit.lim[l] ? 1u : 0u;
+    S->pre_lut[tid] = L > 7 ? 0u : S->lit_ent[(rev >> (15 - L)) + S->lit.base[L]];
+  }
+  for (uint32_t i = tid; i < 320; i += kCtaThreads) S->lens[i] = 0;
+  __syncthreads();
+  // [4:0] symbol, [12:8] bits taken (0: no such code), [23:16] lengths covered
+  auto at = [&](uint32_t i) {
+    const uint32_t p = (uint32_t)(pos & 31) + i, j = p >> 5;
+    const uint32_t a = w0 + j < trunc ? in32[w0 + j] : 0u, b = w0 + j + 1 < trunc ? in32[w0 + j + 1] : 0u;
+    const uint32_t x = __funnelshift_r(a, b, p & 31);
+    const uint32_t e = S->pre_lut[x & 127], L = e & 15, sym = e >> 16;
+    if (L == 0) return 0u;
+    const uint32_t xb = sym < 16 ? 0u : (sym == 16 ? 2u : (sym == 17 ? 3u : 7u));
+    const uint32_t rep = sym < 16 ? 1u : ((x >> L) & ((1u << xb) - 1)) + (sym == 18 ? 11u : 3u);
+    return sym | (L + xb) << 8 | rep << 16;
+  };
+  for (uint32_t i = tid; i < kHdrBits; i += kCtaThreads) {
+    const uint32_t n = (at(i) >> 8) & 31;
+    S->hop[0][i] = n && i + n < kHdrBits ? (uint16_t)(i + n) : (uint16_t)0xFFFF;
+  }
+  __syncthreads();
+  for (int k = 0; k < 3; k++) {
+    for (uint32_t i = tid; i < kHdrBits; i += kCtaThreads) {
+      const uint32_t h = S->hop[k][i];
+      S->hop[k + 1][i] = h == 0xFFFF ? (uint16_t)0xFFFF : S->hop[k][h];
+    }
+    __syncthreads();
+  }
+  if (tid == 0) {
+    uint32_t p = 0;
+    for (uint32_t g = 0; g < kHdrSyms / 8; g++) {
+      S->group[g] = (uint16_t)p;
+      if (p != 0xFFFF) p = S->hop[3][p];
+    }
+  }
+  __syncthreads();
+  // symbols 2 tid and 2 tid + 1
+  uint32_t e[2] = {0, 0}, p[2] = {0xFFFF, 0xFFFF};
+  if (tid < kHdrSyms / 2) {
+    p[0] = S->group[tid >> 2];
+    if ((tid & 1) && p[0] != 0xFFFF) p[0] = S->hop[1][p[0]];
+    if ((tid & 2) && p[0] != 0xFFFF) p[0] = S->hop[2][p[0]];
+    if (p[0] != 0xFFFF) {
+      e[0] = at(p[0]);
+      p[1] = S->hop[0][p[0]];
+      if (p[1] != 0xFFFF) e[1] = at(p[1]);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const uint32_t sym = e[k] & 31;
+      S->val[2 * tid + k] = sym < 16 ? (uint8_t)sym : (sym == 16 ? (uint8_t)0xFF : (uint8_t)0);
+    }
+  }
+  uint32_t sum;
+  uint32_t o = cta_scan(S, 0, (e[0] >> 16) + (e[1] >> 16), sum);
+  if (tid == 0) S->c.hdr_end = kNone;
+  __syncthreads();
+  bool bad = false;
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const uint32_t n = e[k] >> 16;
+    if (tid < kHdrSyms / 2 && o < total) {
+      uint32_t s = 2 * tid + k;
+      if (!n || o + n > total || (s == 0 && (e[k] & 31) == 16)) {
+        bad = true;
+      } else {
+        if (o + n == total) S->c.hdr_end = p[k] + ((e[k] >> 8) & 31);
+        while (s && S->val[s] == 0xFF) s--;
+        const uint8_t v = S->val[s];
+        if (v)
+          for (uint32_t j = o; j < o + n; j++) S->lens[j < nlen ? j : 288 + j - nlen] = v;
+      }
+    }
+    o += n;
+  }
+  __syncwarp();
+  bad = __syncthreads_or(bad) || S->c.hdr_end == kNone || S->lens[256] == 0;
+  // past the readable input (the reader ran 96 bits ahead): cut off, or over the abort bit
+  const uint64_t end = pos + (S->c.hdr_end == kNone ? 0u : S->c.hdr_end);
+  __syncthreads();
+  if (end + 96 > S->c.limit_words * 32) return end + 96 > trunc * 32 ? kTruncated : kOvershoot;
+  if (bad) return kBadDeflate;
+  if (tid == 0 && move) S->c.pos = end;
+  __syncthreads();
+  return kOk;
+}
+
+// Both code tables from S->lens (whole CTA).  Warp 0 sorts the
 // literal/length code, warp 1 the distance code, all threads fill the LUT.
 // Distance lengths sit at lens + 288.
 template <int LB>
@@ -438,9 +560,9 @@ __device__ __forceinline__ bool cta_build_tables(CtaSmem<LB>* S) {
   if (warp < 2) {
     bool ok;
     if (warp == 0)
-      ok = index_code(S->h.lens, (int)S->c.nlen, &S->lit, S->lit_ent, lane, tok_lit_entry);
+      ok = index_code(S->lens, (int)S->c.nlen, &S->lit, S->lit_ent, lane, tok_lit_entry);
     else
-      ok = index_code(S->h.lens + 288, (int)S->c.ndist, &S->dist, S->dist_ent, lane, tok_dist_entry);
+      ok = index_code(S->lens + 288, (int)S->c.ndist, &S->dist, S->dist_ent, lane, tok_dist_entry);
     if (lane == 0) S->c.build_ok[warp] = ok;
   }
   __syncthreads();
@@ -920,7 +1042,7 @@ enum : int32_t {
   kActTable,        // a sync start: read the header at table_bit, then go on at pos
   kActFixed,        // a sync start in a fixed block
   kActStored,       // copy stored_len bytes at pos
-  kActBlock,        // code lengths are read: build the tables, decode the block
+  kActBlock,        // read the code lengths (dynamic), build the tables, decode the block
 };
 
 // start bit a predecessor must reach to hand over to chunk k
@@ -1036,7 +1158,8 @@ __device__ __forceinline__ void cta_targets(CtaCtl& c, const ChunkDesc* descs, b
     c.passed_bit = ((const volatile ChunkDesc*)(descs + c.next))->start_bit;
 }
 
-// One warp: the boundary's decision and the header it leads to.
+// One warp: the boundary's decision and the start of the header it leads to
+// (a dynamic block's up to its precode).
 template <int LB>
 __device__ __noinline__ void cta_header(const uint8_t* __restrict__ in, const ChunkDesc* descs,
                                         CtaSmem<LB>* S, const PagePool& pool, bool sync, int lane) {
@@ -1046,59 +1169,76 @@ __device__ __noinline__ void cta_header(const uint8_t* __restrict__ in, const Ch
   act = __shfl_sync(0xFFFFFFFFu, act, 0);
   __syncwarp();
   int32_t status = kOk;
-  if (act == kActHeader || act == kActTable) {
-    BitReader br;
-    br.in32 = reinterpret_cast<const uint32_t*>(in);
-    br.limit_words = c.limit_words;
-    const uint64_t start = act == kActTable ? c.table_bit : c.pos;
-    br.load_windows((start >> 5) & ~31ull, lane);
-    br.seek(start, lane);
-    br.refill(lane);
-    const uint32_t hdr = (uint32_t)br.bb & 7;
-    br.consume(3);
-    const uint32_t btype = hdr >> 1;
-    uint64_t pos = c.pos;
-    int nlen = 0, ndist = 0;
-    uint32_t stored = 0;
-    if (btype == 3 || (btype == 0 && act == kActTable)) {
+  bool fixed = act == kActFixed;
+  const bool table = act == kActTable;
+  if (act == kActHeader || table) {
+    // 128 bits from the header on (zeros past the input)
+    const uint64_t start = table ? c.table_bit : c.pos, w0 = start >> 5;
+    const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
+    const uint32_t w = lane < 5 && w0 + lane < c.trunc_words ? in32[w0 + lane] : 0u;
+    const uint32_t wn = __shfl_down_sync(0xFFFFFFFFu, w, 1);
+    const uint32_t b = __funnelshift_r(w, wn, (uint32_t)(start & 31));
+    const uint64_t lo = (uint64_t)__shfl_sync(0xFFFFFFFFu, b, 1) << 32 | __shfl_sync(0xFFFFFFFFu, b, 0);
+    const uint64_t hi = (uint64_t)__shfl_sync(0xFFFFFFFFu, b, 3) << 32 | __shfl_sync(0xFFFFFFFFu, b, 2);
+    const uint32_t btype = (uint32_t)(lo >> 1) & 3;
+    uint64_t pos = start + 3;
+    uint32_t stored = 0, nlen = 0, ndist = 0;
+    if (btype == 3 || (btype == 0 && table)) {
       status = kBadDeflate;
     } else if (btype == 0) {
       // stored block: byte-align, LEN/NLEN
-      br.consume(br.bc & 7);
-      br.refill(lane);
-      stored = (uint32_t)br.bb & 0xFFFF;
-      const uint32_t nln = (uint32_t)(br.bb >> 16) & 0xFFFF;
-      br.consume(32);
-      const uint64_t byte = br.pos() >> 3;
-      pos = byte * 8;
+      pos = (pos + 7) & ~7ull;
+      const uint32_t sz = (uint32_t)(lo >> (pos - start));
+      stored = sz & 0xFFFF;
+      pos += 32;
+      const uint64_t byte = pos >> 3;
       if (byte > c.in_end) status = kTruncated;
-      else if (stored != (~nln & 0xFFFFu)) status = kBadDeflate;
+      else if (stored != (~(sz >> 16) & 0xFFFFu)) status = kBadDeflate;
       else if (byte + stored > c.in_end) status = kTruncated;
-    } else if (btype == 2 || !c.fixed_tables) {
-      status = read_lens(br, btype, &S->h, c.trunc_words, lane, nlen, ndist);
-      if (act == kActHeader) pos = br.pos();
-    } else if (act == kActHeader) {
-      pos = br.pos();
+      act = kActStored;
+    } else if (btype == 1) {
+      fixed = true;
+    } else {
+      const uint32_t h = (uint32_t)(lo >> 3);
+      nlen = 257 + (h & 31);
+      ndist = 1 + ((h >> 5) & 31);
+      const uint32_t ncl = 4 + ((h >> 10) & 15);
+      if (nlen > 286 || ndist > 30) status = kBadDeflate;
+      // code-length code lengths: 3 bits each from bit 17 on
+      const uint64_t pb = lo >> 17 | hi << 47;
+      if (lane < 19)
+        S->pre_lens[c_cl_order[lane]] =
+            (uint32_t)lane < ncl ? (uint8_t)((pb >> (3 * lane)) & 7) : (uint8_t)0;
+      __syncwarp();
+      if (status == kOk && !index_code(S->pre_lens, 19, &S->lit, S->lit_ent, lane, pre_entry))
+        status = kBadDeflate;
+      pos = start + 17 + 3 * ncl;
+      act = kActBlock;
     }
     __syncwarp();
     if (lane == 0) {
-      c.bfinal = hdr & 1;
+      c.bfinal = (uint32_t)lo & 1;
       c.btype = btype;
-      c.pos = pos;
-      c.nlen = (uint32_t)nlen;
-      c.ndist = (uint32_t)ndist;
+      c.hdr_pos = pos;
+      c.hdr_move = !table;
+      if (!table) c.pos = pos;
+      c.nlen = nlen;
+      c.ndist = ndist;
       c.stored_len = stored;
+      if (btype == 2) c.fixed_tables = 0;  // the precode took their place
     }
-    act = btype == 0 ? kActStored : kActBlock;
-  } else if (act == kActFixed) {
-    BitReader br{};
-    int nlen = 0, ndist = 0;
-    if (!c.fixed_tables) read_lens(br, 1, &S->h, 0, lane, nlen, ndist);
-    if (lane == 0) {
-      c.nlen = (uint32_t)nlen;
-      c.ndist = (uint32_t)ndist;
-    }
+  }
+  if (fixed) {
     act = kActBlock;
+    if (!c.fixed_tables) {
+      // fixed Huffman (RFC 1951 3.2.6): litlen 0..287, then 32 distance codes
+      for (int s = lane; s < 320; s += 32)
+        S->lens[s] = s < 144 ? 8 : (s < 256 ? 9 : (s < 280 ? 7 : (s < 288 ? 8 : 5)));
+      if (lane == 0) {
+        c.nlen = 288;
+        c.ndist = 32;
+      }
+    }
   }
   __syncwarp();
   if (lane == 0) {
@@ -1128,16 +1268,14 @@ __device__ __forceinline__ void cta_decode_chunk(const uint8_t* __restrict__ in,
       cta_stored<LB>(in, S, pool);
     } else {
       if (act == kActBlock && !(c.btype == 1 && c.fixed_tables)) {
-        const bool ok = cta_build_tables<LB>(S);
+        int32_t st = c.btype == 2 ? cta_read_lens<LB>(in, S, c.hdr_move != 0) : kOk;
+        if (st == kOk && !cta_build_tables<LB>(S)) st = kBadDeflate;
         if (tid == 0) {
-          c.fixed_tables = c.btype == 1;
-          if (!ok) c.status = kBadDeflate;
+          c.fixed_tables = st == kOk && c.btype == 1;
+          if (st != kOk) c.status = st;
         }
         __syncthreads();
-        if (!ok) {
-          if (tid == 0) c.fixed_tables = 0;
-          break;
-        }
+        if (st != kOk) break;
       }
       cta_block<LB>(in, S, pool, zero_window);
     }
