@@ -39,10 +39,7 @@
 namespace gzgpu {
 
 constexpr uint32_t kRangeMax = 640;   // bits per thread and round, at most
-constexpr uint32_t kRangeMin = 256;   // and at least (more than the longest symbol's 48)
-constexpr uint32_t kTokCap = 18432;   // token slots per round
-constexpr uint32_t kWin = 2048;       // output positions expanded at a time (divides a page)
-constexpr uint32_t kWinPer = kWin / kCtaThreads;
+constexpr uint32_t kWinPer = 8;         // output positions expanded at a time, per thread
 constexpr uint32_t kTokPer = 4;       // token slots per thread and batch
 constexpr uint32_t kCtaDistBits = 9;  // distance LUT index bits
 constexpr uint32_t kSegs = 2;           // a range is walked in halves
@@ -109,8 +106,11 @@ struct CodeIndex {
   uint16_t count[16], first[16], offs[16], next[16];
 };
 
-template <int LB>
+template <int LB, int NT>
 struct alignas(16) CtaSmem {
+  static constexpr uint32_t kWin = NT * kWinPer;
+  static constexpr uint32_t kTokCap = NT == 256 ? 18432 : 40960;  // token slots per round
+  static constexpr uint32_t kRangeMin = NT == 256 ? 256 : 128;    // bits per thread, at least
   // literal/length LUT, then the distance LUT (at a power of two, so that its
   // offset joins an index by OR)
   uint32_t lut[(1 << LB) + (1 << kCtaDistBits)];
@@ -134,18 +134,18 @@ struct alignas(16) CtaSmem {
   };
   uint32_t lit_ent[288], dist_ent[32];  // entries in canonical order
   CodeIndex lit, dist;
-  uint32_t end[kCtaThreads];
+  uint32_t end[NT];
   // per part of each range but the last: [9:0] first boundary at or past
   // its end, relative to the range's first bit, [31:10] lookups from there
-  uint32_t cp[kSegs - 1][kCtaThreads];
-  uint32_t scan[2][kCtaThreads / 32];
+  uint32_t cp[kSegs - 1][NT];
+  uint32_t scan[2][NT / 32];
   CtaCtl c;
 };
 
 // exclusive prefix sum of a over the CTA, total in ta.  One barrier; `par`
 // alternates between calls (0, 1, 0, ...).
-template <int LB>
-__device__ __forceinline__ uint32_t cta_scan(CtaSmem<LB>* S, uint32_t par, uint32_t a, uint32_t& ta) {
+template <int LB, int NT>
+__device__ __forceinline__ uint32_t cta_scan(CtaSmem<LB, NT>* S, uint32_t par, uint32_t a, uint32_t& ta) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t x = a;
 #pragma unroll
@@ -157,11 +157,23 @@ __device__ __forceinline__ uint32_t cta_scan(CtaSmem<LB>* S, uint32_t par, uint3
   __syncthreads();
   uint32_t pa = 0;
   ta = 0;
+  if constexpr (NT <= 256) {
 #pragma unroll
-  for (int w = 0; w < (int)kCtaThreads / 32; w++) {
-    const uint32_t u = S->scan[par][w];
-    if (w < warp) pa += u;
-    ta += u;
+    for (int w = 0; w < NT / 32; w++) {
+      const uint32_t u = S->scan[par][w];
+      if (w < warp) pa += u;
+      ta += u;
+    }
+  } else {  // the warps' totals by the same scan
+    const uint32_t own = lane < NT / 32 ? S->scan[par][lane] : 0u;
+    uint32_t y = own;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, y, d);
+      if (lane >= d) y += u;
+    }
+    pa = __shfl_sync(0xFFFFFFFFu, y - own, warp);
+    ta = __shfl_sync(0xFFFFFFFFu, y, 31);
   }
   return pa + x - a;
 }
@@ -169,8 +181,8 @@ __device__ __forceinline__ uint32_t cta_scan(CtaSmem<LB>* S, uint32_t par, uint3
 // The entry of a code longer than the LUT's bits (9 for distances, 10 or more
 // for literals and lengths), or kStopBad.  Inlined where it is used: a call in
 // the walks' loops, taken or not, cost 30 cycles an iteration.
-template <int LB>
-__device__ __forceinline__ uint32_t long_entry(const CtaSmem<LB>* S, uint32_t x, bool dist) {
+template <int LB, int NT>
+__device__ __forceinline__ uint32_t long_entry(const CtaSmem<LB, NT>* S, uint32_t x, bool dist) {
   static_assert(LB >= 10 && kCtaDistBits == 9, "codes looked up here have 10 bits at least");
   const CodeIndex& I = dist ? S->dist : S->lit;
   const uint32_t rev = __brev(x) >> 17;  // 15 code bits, first bit = MSB
@@ -273,8 +285,8 @@ struct TableAt {
 // for the range.  Otherwise a stop ends the walk.  again: an earlier walk of
 // this round left its boundaries, and meeting one ends this walk: from there
 // on they agree.
-template <int LB>
-__device__ __forceinline__ void walk_range(CtaSmem<LB>* S, const uint32_t* base, uint32_t first,
+template <int LB, int NT>
+__device__ __forceinline__ void walk_range(CtaSmem<LB, NT>* S, const uint32_t* base, uint32_t first,
                                            uint32_t len, uint32_t e, bool guess, bool again,
                                            Range& r) {
   const uint32_t tid = threadIdx.x;
@@ -304,7 +316,7 @@ __device__ __forceinline__ void walk_range(CtaSmem<LB>* S, const uint32_t* base,
         // at p: a code beyond the LUT, or a stop
         const bool dist = t.off != 0;
         uint32_t ent = t.look(lut, b);
-        if (((ent >> 8) & 3) == kStopLong) ent = long_entry<LB>(S, b.lo >> 2, dist);
+        if (((ent >> 8) & 3) == kStopLong) ent = long_entry<LB, NT>(S, b.lo >> 2, dist);
         if ((int32_t)ent >= 0) {
           slots++;
         } else if (guess) {
@@ -346,8 +358,8 @@ __device__ __forceinline__ void walk_range(CtaSmem<LB>* S, const uint32_t* base,
 }
 
 // The tokens of the n lookups from start on to tok.
-template <int LB>
-__device__ __forceinline__ void write_tokens(const CtaSmem<LB>* S, const uint32_t* base,
+template <int LB, int NT>
+__device__ __forceinline__ void write_tokens(const CtaSmem<LB, NT>* S, const uint32_t* base,
                                              uint32_t start, uint32_t n, uint16_t* tok) {
   const char* lut = reinterpret_cast<const char*>(S->lut);
   RangeBits b;
@@ -371,7 +383,7 @@ __device__ __forceinline__ void write_tokens(const CtaSmem<LB>* S, const uint32_
       if (u % 2) b.refill_if_due();
     }
     if (__builtin_expect((int32_t)stop < 0, 0)) {
-      const uint32_t ent = long_entry<LB>(S, b.lo >> 2, t.off != 0);
+      const uint32_t ent = long_entry<LB, NT>(S, b.lo >> 2, t.off != 0);
       const uint32_t x = (b.lo >> 2) & ~(0xFFFFFFFFu << (ent & 31));
       *tok++ = (uint16_t)((ent >> 8) + (x >> (ent >> 27)));
       b.shift(ent);
@@ -453,8 +465,8 @@ __device__ __forceinline__ uint32_t lut_value(uint32_t i, const uint32_t* lim, c
 // so one thread takes eight symbols a step, and the symbols on that chain are
 // then expanded in parallel.  Returns kOk or an error status; S->c.pos moves
 // past the header.
-template <int LB>
-__device__ __forceinline__ int32_t cta_read_lens(const uint8_t* __restrict__ in, CtaSmem<LB>* S,
+template <int LB, int NT>
+__device__ __forceinline__ int32_t cta_read_lens(const uint8_t* __restrict__ in, CtaSmem<LB, NT>* S,
                                                  bool move) {
   const uint32_t tid = threadIdx.x;
   const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
@@ -467,7 +479,7 @@ __device__ __forceinline__ int32_t cta_read_lens(const uint8_t* __restrict__ in,
     for (int l = 1; l <= 7; l++) L += rev >= S->lit.lim[l] ? 1u : 0u;
     S->pre_lut[tid] = L > 7 ? 0u : S->lit_ent[(rev >> (15 - L)) + S->lit.base[L]];
   }
-  for (uint32_t i = tid; i < 320; i += kCtaThreads) S->lens[i] = 0;
+  for (uint32_t i = tid; i < 320; i += NT) S->lens[i] = 0;
   __syncthreads();
   // [4:0] symbol, [12:8] bits taken (0: no such code), [23:16] lengths covered
   auto at = [&](uint32_t i) {
@@ -480,13 +492,13 @@ __device__ __forceinline__ int32_t cta_read_lens(const uint8_t* __restrict__ in,
     const uint32_t rep = sym < 16 ? 1u : ((x >> L) & ((1u << xb) - 1)) + (sym == 18 ? 11u : 3u);
     return sym | (L + xb) << 8 | rep << 16;
   };
-  for (uint32_t i = tid; i < kHdrBits; i += kCtaThreads) {
+  for (uint32_t i = tid; i < kHdrBits; i += NT) {
     const uint32_t n = (at(i) >> 8) & 31;
     S->hop[0][i] = n && i + n < kHdrBits ? (uint16_t)(i + n) : (uint16_t)0xFFFF;
   }
   __syncthreads();
   for (int k = 0; k < 3; k++) {
-    for (uint32_t i = tid; i < kHdrBits; i += kCtaThreads) {
+    for (uint32_t i = tid; i < kHdrBits; i += NT) {
       const uint32_t h = S->hop[k][i];
       S->hop[k + 1][i] = h == 0xFFFF ? (uint16_t)0xFFFF : S->hop[k][h];
     }
@@ -554,8 +566,8 @@ __device__ __forceinline__ int32_t cta_read_lens(const uint8_t* __restrict__ in,
 // Both code tables from S->lens (whole CTA).  Warp 0 sorts the
 // literal/length code, warp 1 the distance code, all threads fill the LUT.
 // Distance lengths sit at lens + 288.
-template <int LB>
-__device__ __forceinline__ bool cta_build_tables(CtaSmem<LB>* S) {
+template <int LB, int NT>
+__device__ __forceinline__ bool cta_build_tables(CtaSmem<LB, NT>* S) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (warp < 2) {
     bool ok;
@@ -570,11 +582,11 @@ __device__ __forceinline__ bool cta_build_tables(CtaSmem<LB>* S) {
   uint32_t lim[LB + 1];
 #pragma unroll
   for (int l = 1; l <= LB; l++) lim[l] = S->lit.lim[l];
-  for (uint32_t i = threadIdx.x; i < (1u << LB); i += kCtaThreads)
+  for (uint32_t i = threadIdx.x; i < (1u << LB); i += NT)
     S->lut[i] = lut_value<LB>(i, lim, &S->lit, S->lit_ent, kEntStop | kStopLong << 8);
 #pragma unroll
   for (int l = 1; l <= (int)kCtaDistBits; l++) lim[l] = S->dist.lim[l];
-  for (uint32_t i = threadIdx.x; i < (1u << kCtaDistBits); i += kCtaThreads)
+  for (uint32_t i = threadIdx.x; i < (1u << kCtaDistBits); i += NT)
     S->lut[(1u << LB) + i] = lut_value<(int)kCtaDistBits>(i, lim, &S->dist, S->dist_ent,
                                                           kEntStop | kEntLen | kStopLong << 8);
   __syncthreads();
@@ -584,8 +596,8 @@ __device__ __forceinline__ bool cta_build_tables(CtaSmem<LB>* S) {
 // Make the page of the window at chunk position w0 current (thread 0
 // allocates, then a barrier).  Windows are visited in order and never cross a
 // page.  False when the pool is exhausted.
-template <int LB>
-__device__ __forceinline__ bool cta_page(CtaSmem<LB>* S, const PagePool& pool, uint64_t w0) {
+template <int LB, int NT>
+__device__ __forceinline__ bool cta_page(CtaSmem<LB, NT>* S, const PagePool& pool, uint64_t w0) {
   const uint32_t s = (uint32_t)(w0 >> 16);
   if (S->c.page_cur != kNoPage && S->c.page_seq == s) return true;
   __syncthreads();
@@ -623,9 +635,10 @@ __device__ __forceinline__ bool cta_page(CtaSmem<LB>* S, const PagePool& pool, u
 // read, its references are in place.
 // Returns kOk or kPoolExhausted.  (No distance reaches beyond the window before
 // the chunk: a code names 32768 at most.)
-template <int LB>
-__device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool& pool, uint32_t n,
+template <int LB, int NT>
+__device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB, NT>* S, const PagePool& pool, uint32_t n,
                                                  bool zero_window) {
+  constexpr uint32_t kWin = CtaSmem<LB, NT>::kWin;
   const uint32_t tid = threadIdx.x;
   const uint64_t o = S->c.o;
   const uint64_t base = o & ~(uint64_t)(kWin - 1);  // positions below are relative to this
@@ -690,8 +703,8 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
           }
         }
       }
-      if (bend >= wend || b0 + kTokPer * kCtaThreads >= n) break;
-      b0 += kTokPer * kCtaThreads;
+      if (bend >= wend || b0 + kTokPer * NT >= n) break;
+      b0 += kTokPer * NT;
       bpos = bend;
       load_batch();
     }
@@ -856,7 +869,7 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
     }
     lo = wbase + hi;
     if (bend <= wend) {  // the batch is used up
-      b0 += kTokPer * kCtaThreads;
+      b0 += kTokPer * NT;
       if (b0 >= n) break;
       bpos = bend;
       load_batch();
@@ -873,10 +886,11 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB>* S, const PagePool&
 // The body of one Huffman-coded block, tables in place.  On return (after a
 // barrier) S->c holds the new position and entry count, status, synced (at
 // the successor's sync start) or passed (went by the successor's start).
-template <int LB>
-__device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSmem<LB>* S,
+template <int LB, int NT>
+__device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSmem<LB, NT>* S,
                                           const PagePool& pool, bool zero_window) {
   const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
+  constexpr uint32_t kTokCap = CtaSmem<LB, NT>::kTokCap, kRangeMin = CtaSmem<LB, NT>::kRangeMin;
   const uint32_t tid = threadIdx.x;
   uint32_t rcap = kRangeMax;
   for (;;) {
@@ -895,11 +909,11 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
     uint64_t end = (limit - 3) * 32;  // symbols start below this
     if (target != kNoStop && target > pos && target < end) end = target;
     const uint64_t likely = S->c.stop_lo > pos && S->c.stop_lo < end ? S->c.stop_lo : end;
-    const uint64_t want = ((likely - pos) / kCtaThreads + 32) & ~31ull;
+    const uint64_t want = ((likely - pos) / NT + 32) & ~31ull;
     const uint32_t r = (uint32_t)max((uint64_t)kRangeMin, min(want, (uint64_t)rcap));
     const uint32_t p0 = (uint32_t)(pos & 31);
     const uint64_t span = end - pos;
-    const uint32_t pend = p0 + (uint32_t)min(span, (uint64_t)r * kCtaThreads);
+    const uint32_t pend = p0 + (uint32_t)min(span, (uint64_t)r * NT);
     const uint32_t lanes = (pend - p0 + r - 1) / r;
     const uint32_t* base = in32 + w0;
     if (tid < 2) S->c.min_need[tid] = S->c.min_term[tid] = kNone;
@@ -909,7 +923,7 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
     Range ra{};
     ra.start = first;
     if (active) {
-      walk_range<LB>(S, base, first, r, e, tid > 0, false, ra);
+      walk_range<LB, NT>(S, base, first, r, e, tid > 0, false, ra);
       S->end[tid] = ra.end;
     }
     __syncwarp();
@@ -932,7 +946,7 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
       if (tid == 0) S->c.min_need[it ^ 1] = S->c.min_term[it ^ 1] = kNone;
       if (need) {
         ra.start = s1;
-        walk_range<LB>(S, base, first, r, e, false, true, ra);
+        walk_range<LB, NT>(S, base, first, r, e, false, true, ra);
         S->end[tid] = ra.end;
       }
       __syncwarp();
@@ -970,12 +984,12 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
       if (tid == 0) S->c.status = kBadDeflate;
       break;
     }
-    if (tid < n_lanes) write_tokens<LB>(S, base, ra.start, my_slots, S->tok + slot0);
+    if (tid < n_lanes) write_tokens<LB, NT>(S, base, ra.start, my_slots, S->tok + slot0);
     __syncwarp();
     __syncthreads();
     // 4. expansion
     if (n_slots) {
-      const int32_t st = expand_tokens<LB>(S, pool, n_slots, zero_window);
+      const int32_t st = expand_tokens<LB, NT>(S, pool, n_slots, zero_window);
       if (st != kOk) {
         __syncthreads();
         if (tid == 0) S->c.status = st;
@@ -995,8 +1009,8 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
 }
 
 // A stored block's bytes to the chunk's pages, four entries per thread.
-template <int LB>
-__device__ __forceinline__ void cta_stored(const uint8_t* __restrict__ in, CtaSmem<LB>* S,
+template <int LB, int NT>
+__device__ __forceinline__ void cta_stored(const uint8_t* __restrict__ in, CtaSmem<LB, NT>* S,
                                            const PagePool& pool) {
   const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
   uint64_t byte = S->c.pos >> 3, o = S->c.o;
@@ -1011,7 +1025,7 @@ __device__ __forceinline__ void cta_stored(const uint8_t* __restrict__ in, CtaSm
     const uint32_t n = min(left, kPageEntries - q);
     uint16_t* dst = pool.data + (size_t)S->c.page_cur * kPageEntries;
     // groups of 4 entries aligned to 4; the first and last may be partial
-    for (uint32_t g = (q & ~3u) + 4 * threadIdx.x; g < q + n; g += 4 * kCtaThreads) {
+    for (uint32_t g = (q & ~3u) + 4 * threadIdx.x; g < q + n; g += 4 * NT) {
       if (g >= q && g + 4 <= q + n) {
         const uint64_t a = byte + (g - q);
         const uint32_t v = __funnelshift_r(in32[a >> 2], in32[(a >> 2) + 1], 8 * ((uint32_t)a & 3));
@@ -1160,9 +1174,9 @@ __device__ __forceinline__ void cta_targets(CtaCtl& c, const ChunkDesc* descs, b
 
 // One warp: the boundary's decision and the start of the header it leads to
 // (a dynamic block's up to its precode).
-template <int LB>
+template <int LB, int NT>
 __device__ __noinline__ void cta_header(const uint8_t* __restrict__ in, const ChunkDesc* descs,
-                                        CtaSmem<LB>* S, const PagePool& pool, bool sync, int lane) {
+                                        CtaSmem<LB, NT>* S, const PagePool& pool, bool sync, int lane) {
   CtaCtl& c = S->c;
   int32_t act = kActDone;
   if (lane == 0) act = cta_boundary(c, descs, pool);
@@ -1252,24 +1266,24 @@ __device__ __noinline__ void cta_header(const uint8_t* __restrict__ in, const Ch
 }
 
 // Decode one chunk; its state is in S->c (prepared by cta_begin).
-template <int LB>
+template <int LB, int NT>
 __device__ __forceinline__ void cta_decode_chunk(const uint8_t* __restrict__ in, const ChunkDesc* descs,
-                                                 ChunkResult* res, CtaSmem<LB>* S,
+                                                 ChunkResult* res, CtaSmem<LB, NT>* S,
                                                  const PagePool& pool, bool sync) {
   const int tid = threadIdx.x;
   CtaCtl& c = S->c;
   const bool zero_window = (c.flags & kChunkMemberFirst) != 0;
   for (;;) {
-    if (tid < 32) cta_header<LB>(in, descs, S, pool, sync, tid);
+    if (tid < 32) cta_header<LB, NT>(in, descs, S, pool, sync, tid);
     __syncthreads();
     const int32_t act = c.act;
     if (act == kActDone) break;
     if (act == kActStored) {
-      cta_stored<LB>(in, S, pool);
+      cta_stored<LB, NT>(in, S, pool);
     } else {
       if (act == kActBlock && !(c.btype == 1 && c.fixed_tables)) {
-        int32_t st = c.btype == 2 ? cta_read_lens<LB>(in, S, c.hdr_move != 0) : kOk;
-        if (st == kOk && !cta_build_tables<LB>(S)) st = kBadDeflate;
+        int32_t st = c.btype == 2 ? cta_read_lens<LB, NT>(in, S, c.hdr_move != 0) : kOk;
+        if (st == kOk && !cta_build_tables<LB, NT>(S)) st = kBadDeflate;
         if (tid == 0) {
           c.fixed_tables = st == kOk && c.btype == 1;
           if (st != kOk) c.status = st;
@@ -1277,7 +1291,7 @@ __device__ __forceinline__ void cta_decode_chunk(const uint8_t* __restrict__ in,
         __syncthreads();
         if (st != kOk) break;
       }
-      cta_block<LB>(in, S, pool, zero_window);
+      cta_block<LB, NT>(in, S, pool, zero_window);
     }
     if (c.status != kOk || c.synced) break;
     const bool passed = c.passed != 0, fin = c.bfinal != 0;

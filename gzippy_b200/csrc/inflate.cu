@@ -474,13 +474,13 @@ __global__ void __launch_bounds__(32 * kRingWarps)
 // Pages layout: a persistent grid of CTAs takes chunks from the queue.  A
 // failed speculative start moves on to the next candidate of its partition.
 // sync: the job has sync starts, so successors are watched mid-block.
-template <int LB, int MINB>
-__global__ void __launch_bounds__(kCtaThreads, MINB)
+template <int LB, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB)
     inflate_pages_kernel(const uint8_t* __restrict__ in, ChunkDesc* descs, ChunkResult* results,
                        const uint32_t* __restrict__ work, const uint32_t* __restrict__ n_work_ptr,
                        uint32_t* work_counter, PagePool pool, int sync) {
   extern __shared__ __align__(16) uint8_t smem[];
-  CtaSmem<LB>* S = reinterpret_cast<CtaSmem<LB>*>(smem);
+  CtaSmem<LB, NT>* S = reinterpret_cast<CtaSmem<LB, NT>*>(smem);
   const int tid = threadIdx.x;
   const uint32_t n_work = *n_work_ptr;
   if (tid == 0) S->c.fixed_tables = 0;
@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(kCtaThreads, MINB)
     const uint32_t cid = S->c.cid;
     if (cid == kNone) break;
     for (;;) {
-      cta_decode_chunk<LB>(in, descs, &results[cid], S, pool, sync != 0);
+      cta_decode_chunk<LB, NT>(in, descs, &results[cid], S, pool, sync != 0);
       if (tid < 32) {
         // the partition's next candidate, if this start failed
         ChunkDesc& d = descs[cid];
@@ -536,37 +536,47 @@ __global__ void __launch_bounds__(kCtaThreads, MINB)
 }
 
 template <int LB>
-size_t inflate_smem_bytes(bool ring) {
-  return ring ? sizeof(RingSmem<LB>) * kRingWarps : sizeof(CtaSmem<LB>);
+static size_t ring_smem_bytes() {
+  return sizeof(RingSmem<LB>) * kRingWarps;
 }
 
-// page kernel instance for `ctas` CTAs per SM (registers sized for it)
+// page kernel instance: its function, threads and shared memory
+struct PagesFn {
+  const void* fn;
+  int threads;
+  size_t smem;
+};
 template <int LB>
-static const void* pages_kernel_fn(int ctas) {
-  return ctas >= 4 ? (const void*)inflate_pages_kernel<LB, 4> : (const void*)inflate_pages_kernel<LB, 3>;
+static PagesFn pages_fn(int ctas, bool wide) {
+  if (wide)
+    return {(const void*)inflate_pages_kernel<LB, kWideThreads, 1>, kWideThreads,
+            sizeof(CtaSmem<LB, kWideThreads>)};
+  return {ctas >= 4 ? (const void*)inflate_pages_kernel<LB, kCtaThreads, 4>
+                    : (const void*)inflate_pages_kernel<LB, kCtaThreads, 3>,
+          kCtaThreads, sizeof(CtaSmem<LB, kCtaThreads>)};
 }
 
 template <int LB>
-cudaError_t launch_inflate(bool ring, int ctas, bool sync, const uint8_t* in, ChunkDesc* descs,
-                           ChunkResult* results, const uint32_t* work, const uint32_t* n_work,
-                           uint32_t* work_counter, const PagePool& pool, int blocks,
-                           cudaStream_t stream) {
-  size_t smem = inflate_smem_bytes<LB>(ring);
+cudaError_t launch_inflate(bool ring, int ctas, bool wide, bool sync, const uint8_t* in,
+                           ChunkDesc* descs, ChunkResult* results, const uint32_t* work,
+                           const uint32_t* n_work, uint32_t* work_counter, const PagePool& pool,
+                           int blocks, cudaStream_t stream) {
   cudaError_t e;
   if (ring) {
+    const size_t smem = ring_smem_bytes<LB>();
     e = cudaFuncSetAttribute(inflate_ring_kernel<LB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
     if (e != cudaSuccess) return e;
     inflate_ring_kernel<LB><<<blocks, 32 * kRingWarps, smem, stream>>>(in, descs, results, work,
                                                                        n_work, work_counter, pool);
   } else {
-    const void* fn = pages_kernel_fn<LB>(ctas);
+    const PagesFn f = pages_fn<LB>(ctas, wide);
     int with_sync = sync;
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = cudaFuncSetAttribute(f.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem);
     if (e != cudaSuccess) return e;
     void* args[] = {(void*)&in,     (void*)&descs,        (void*)&results, (void*)&work,
                     (void*)&n_work, (void*)&work_counter, (void*)&pool,    (void*)&with_sync};
-    e = cudaLaunchKernel(fn, dim3(blocks), dim3(kCtaThreads), args, smem, stream);
+    e = cudaLaunchKernel(f.fn, dim3(blocks), dim3(f.threads), args, f.smem, stream);
     if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
@@ -575,26 +585,25 @@ cudaError_t launch_inflate(bool ring, int ctas, bool sync, const uint8_t* in, Ch
 template <int LB>
 int inflate_blocks_per_sm(bool ring, int ctas) {
   int n = 0;
-  size_t smem = inflate_smem_bytes<LB>(ring);
   if (ring) {
+    const size_t smem = ring_smem_bytes<LB>();
     cudaFuncSetAttribute(inflate_ring_kernel<LB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)smem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, inflate_ring_kernel<LB>, 32 * kRingWarps, smem);
   } else {
-    const void* fn = pages_kernel_fn<LB>(ctas);
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kCtaThreads, smem);
+    const PagesFn f = pages_fn<LB>(ctas, false);
+    cudaFuncSetAttribute(f.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f.fn, f.threads, f.smem);
     if (n > ctas) n = ctas;
   }
   return n;
 }
 
-#define GZGPU_INST(LB)                                                                       \
-  template size_t inflate_smem_bytes<LB>(bool);                                              \
-  template int inflate_blocks_per_sm<LB>(bool, int);                                         \
-  template cudaError_t launch_inflate<LB>(bool, int, bool, const uint8_t*, ChunkDesc*, ChunkResult*, \
-                                          const uint32_t*, const uint32_t*, uint32_t*,       \
-                                          const PagePool&, int, cudaStream_t);
+#define GZGPU_INST(LB)                                                                         \
+  template int inflate_blocks_per_sm<LB>(bool, int);                                           \
+  template cudaError_t launch_inflate<LB>(bool, int, bool, bool, const uint8_t*, ChunkDesc*,   \
+                                          ChunkResult*, const uint32_t*, const uint32_t*,      \
+                                          uint32_t*, const PagePool&, int, cudaStream_t);
 GZGPU_INST(10)
 GZGPU_INST(11)
 GZGPU_INST(12)
@@ -772,20 +781,22 @@ static __device__ uint64_t na_header(const uint8_t* in, uint64_t p, uint64_t n) 
   return o <= n ? o - p : 0;
 }
 
+using NoAllocSmem = CtaSmem<11, kWideThreads>;
+
 // The CRC of a member's entries: one slice of `per` entries per thread,
 // combined in order by thread 0 (all but the last non-empty slice have the
 // same length, hence one shift).
-__global__ void __launch_bounds__(kCtaThreads)
+__global__ void __launch_bounds__(kWideThreads)
     noalloc_kernel(const uint8_t* __restrict__ in, uint64_t n, uint8_t* __restrict__ out,
                    uint64_t out_cap, NoAllocScratch* scratch) {
   extern __shared__ __align__(16) uint8_t smem[];
-  CtaSmem<10>* S = reinterpret_cast<CtaSmem<10>*>(smem);
+  NoAllocSmem* S = reinterpret_cast<NoAllocSmem*>(smem);
   __shared__ uint32_t crc_tab[256];
-  __shared__ uint32_t slice_crc[kCtaThreads];
+  __shared__ uint32_t slice_crc[kWideThreads];
   __shared__ uint64_t m_pos;
   __shared__ int32_t m_act;  // < 0: decode the member at m_pos; else the final status
   const int tid = threadIdx.x;
-  for (uint32_t i = tid; i < 256; i += kCtaThreads) {
+  for (uint32_t i = tid; i < 256; i += kWideThreads) {
     uint32_t c = i;
     for (int k = 0; k < 8; k++) c = (c >> 1) ^ (0xEDB88320u & (0u - (c & 1u)));
     crc_tab[i] = c;
@@ -830,7 +841,7 @@ __global__ void __launch_bounds__(kCtaThreads)
       break;
     }
     const PagePool pool{scratch->pages, scratch->owner, scratch->seq, &scratch->page_next, kNoAllocPages};
-    cta_decode_chunk<10>(in, nullptr, &scratch->res, S, pool, false);
+    cta_decode_chunk<11, kWideThreads>(in, nullptr, &scratch->res, S, pool, false);
     const int32_t st = S->c.status;
     const uint64_t out_len = S->c.o, trailer = (S->c.pos + 7) / 8;
     if (st != kOk) {
@@ -851,8 +862,8 @@ __global__ void __launch_bounds__(kCtaThreads)
     // written, so that *out_len reports the exact size needed.
     if (!too_small && total + out_len > out_cap) too_small = true;
     if (!too_small)
-      for (uint64_t q = tid; q < out_len; q += kCtaThreads) out[total + q] = (uint8_t)scratch->pages[q];
-    const uint64_t per = (out_len + kCtaThreads - 1) / kCtaThreads;
+      for (uint64_t q = tid; q < out_len; q += kWideThreads) out[total + q] = (uint8_t)scratch->pages[q];
+    const uint64_t per = (out_len + kWideThreads - 1) / kWideThreads;
     const uint64_t b0 = min((uint64_t)tid * per, out_len), b1 = min(b0 + per, out_len);
     uint32_t c = 0xFFFFFFFFu;
     for (uint64_t q = b0; q < b1; q++) c = (c >> 8) ^ crc_tab[(c ^ (uint32_t)scratch->pages[q]) & 0xFF];
@@ -861,7 +872,7 @@ __global__ void __launch_bounds__(kCtaThreads)
     if (tid == 0) {
       uint32_t crc = 0;
       const uint32_t xp = na_x_pow_8n(per);
-      for (uint32_t l = 0; l < kCtaThreads && l * per < out_len; l++) {
+      for (uint32_t l = 0; l < kWideThreads && l * per < out_len; l++) {
         const uint64_t ll = min(per, out_len - l * per);
         crc = na_mulmod(ll == per ? xp : na_x_pow_8n(ll), crc) ^ slice_crc[l];
       }
@@ -927,9 +938,9 @@ extern "C" int gzgpu_decompress_device_noalloc(const void* d_in, size_t in_len, 
   uint8_t* k_out = reinterpret_cast<uint8_t*>(d_out);
   void* args[] = {(void*)&k_in, (void*)&k_n, (void*)&k_out, (void*)&k_cap, (void*)&S};
   if (cudaFuncSetAttribute((const void*)noalloc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sizeof(CtaSmem<10>)) != cudaSuccess ||
-      cudaLaunchKernel((const void*)noalloc_kernel, dim3(1), dim3(kCtaThreads), args,
-                       sizeof(CtaSmem<10>), st) != cudaSuccess)
+                           (int)sizeof(NoAllocSmem)) != cudaSuccess ||
+      cudaLaunchKernel((const void*)noalloc_kernel, dim3(1), dim3(kWideThreads), args,
+                       sizeof(NoAllocSmem), st) != cudaSuccess)
     return GZGPU_DEVICE_ERROR;
   struct {
     int32_t status;

@@ -7,21 +7,21 @@
 namespace gzgpu {
 
 constexpr int kRingWarps = 1;      // ring kernel: warps per CTA (64 KB ring each)
-constexpr uint32_t kCtaThreads = 256;  // page kernel: threads per CTA (one chunk each)
+constexpr int kCtaThreads = 256;    // page kernel: threads per CTA (one chunk each)
+constexpr int kWideThreads = 1024;  // the same in jobs of few chunks (one CTA per SM)
 constexpr int kDistBits = 8;       // distance LUT index bits (ring kernel, sync-start search)
 
-template <int LB>
-size_t inflate_smem_bytes(bool ring);
 // page kernel: `ctas` (3 or 4) CTAs per SM; registers are sized for that many
 // (80 or 64 per thread)
 template <int LB>
 int inflate_blocks_per_sm(bool ring, int ctas);
+// wide: CTAs of kWideThreads; sync: the job has sync starts (successors are
+// watched mid-block)
 template <int LB>
-// sync: the job has sync starts (successors are watched mid-block)
-cudaError_t launch_inflate(bool ring, int ctas, bool sync, const uint8_t* in, ChunkDesc* descs,
-                           ChunkResult* results, const uint32_t* work, const uint32_t* n_work,
-                           uint32_t* work_counter, const PagePool& pool, int blocks,
-                           cudaStream_t stream);
+cudaError_t launch_inflate(bool ring, int ctas, bool wide, bool sync, const uint8_t* in,
+                           ChunkDesc* descs, ChunkResult* results, const uint32_t* work,
+                           const uint32_t* n_work, uint32_t* work_counter, const PagePool& pool,
+                           int blocks, cudaStream_t stream);
 // sync starts inside dynamic blocks for the listed pieces left without a start
 cudaError_t launch_dyn_sync(const uint8_t* in, ChunkDesc* descs, const uint32_t* pieces, uint32_t n,
                             uint32_t* n_sync, cudaStream_t stream);
