@@ -39,6 +39,10 @@
 namespace gzgpu {
 
 constexpr uint32_t kRangeMax = 640;   // bits per thread and round, at most
+// and at least: shorter ranges fall into step in too few of them (passes over
+// 3.4 times the ranges of text at 256 bits, 7 at 128), and must be longer than
+// a symbol (48)
+constexpr uint32_t kRangeMin = 256;
 constexpr uint32_t kWinPer = 8;         // output positions expanded at a time, per thread
 constexpr uint32_t kTokPer = 4;       // token slots per thread and batch
 constexpr uint32_t kCtaDistBits = 9;  // distance LUT index bits
@@ -90,7 +94,6 @@ struct CtaCtl {
   uint32_t hdr_move, hdr_end;  // move pos past the header; its length after hdr_pos
   uint32_t build_ok[2];
   uint32_t page_cur, page_prev, page_seq, n_pages;
-  uint32_t min_need[2], min_term[2];
   uint32_t round_slots, round_lanes, round_kind, round_pos;
   int32_t carry_ms;         // match reaching into the next window: start (relative to it)
   uint32_t carry_len, carry_dist;
@@ -110,13 +113,13 @@ template <int LB, int NT>
 struct alignas(16) CtaSmem {
   static constexpr uint32_t kWin = NT * kWinPer;
   static constexpr uint32_t kTokCap = NT == 256 ? 18432 : 40960;  // token slots per round
-  static constexpr uint32_t kRangeMin = NT == 256 ? 256 : 128;    // bits per thread, at least
   // literal/length LUT, then the distance LUT (at a power of two, so that its
   // offset joins an index by OR)
   uint32_t lut[(1 << LB) + (1 << kCtaDistBits)];
   union {
     uint16_t tok[kTokCap + 8];
     uint16_t hop[4][kHdrBits];  // block header: position 1, 2, 4 and 8 symbols on
+    uint16_t list[NT];          // join: the ranges to walk again
   };
   union {
     struct {  // block header
@@ -134,7 +137,10 @@ struct alignas(16) CtaSmem {
   };
   uint32_t lit_ent[288], dist_ent[32];  // entries in canonical order
   CodeIndex lit, dist;
-  uint32_t end[NT];
+  // the round's ranges: where each starts and ends, [15:0] its lookups (a
+  // literal is one, a match two), [17:16] what ended it early and at which bit
+  uint32_t start[NT], end[NT], info[NT], term_pos[NT];
+  uint32_t need[NT / 32], term[NT / 32];
   // per part of each range but the last: [9:0] first boundary at or past
   // its end, relative to the range's first bit, [31:10] lookups from there
   uint32_t cp[kSegs - 1][NT];
@@ -252,13 +258,7 @@ struct RangeBits {
 enum : uint32_t { kTermNone = 0, kTermEob = 1, kTermBad = 2 };
 constexpr uint32_t kNoCp = 0x3FFu;  // a part without a recorded boundary
 
-// One thread's range of a round: where it starts and ends, and the lookups
-// between (a literal is one, a match two).
-struct Range {
-  uint32_t start, end, slots;
-  uint32_t term, term_pos;  // met the end of the block or an invalid code there
-  bool guessed_on;          // walked on from a guess past a stop: starts nowhere
-};
+enum : uint32_t { kInfoTerm = 1u << 16, kInfoOn = 1u << 18 };  // On: went on past a stop, starts nowhere
 
 // The two tables as one: the byte offset of the current one (0: literals and
 // lengths) and its index mask.  A stop entry keeps the table it came from.
@@ -274,8 +274,8 @@ struct TableAt {
   }
 };
 
-// Walk the range [first, first + len) (cut at e) from r.start on, positions
-// relative to `base`.  A lookup is a literal or a length code, or the distance
+// Walk range `id`, [first, first + len) cut at e, from its start on (S->start),
+// positions relative to `base`.  A lookup is a literal or a length code, or the distance
 // code of the length just read, so threads at literals and threads inside
 // matches run the same instructions.  Four lookups per loop: a lookup that is
 // not due (past the end, or too few bits before the next refill) takes nothing,
@@ -287,17 +287,15 @@ struct TableAt {
 // on they agree.
 template <int LB, int NT>
 __device__ __forceinline__ void walk_range(CtaSmem<LB, NT>* S, const uint32_t* base, uint32_t first,
-                                           uint32_t len, uint32_t e, bool guess, bool again,
-                                           Range& r) {
-  const uint32_t tid = threadIdx.x;
+                                           uint32_t len, uint32_t e, uint32_t id, bool guess,
+                                           bool again) {
   const char* lut = reinterpret_cast<const char*>(S->lut);
   RangeBits b;
-  b.seek(base, r.start);
+  b.seek(base, S->start[id]);
   TableAt<LB> t;
   uint32_t slots = 0, valid_from = 0, seg = 0;
-  r.term = kTermNone;
-  r.guessed_on = false;
-  bool met = false;
+  uint32_t term = kTermNone;
+  bool met = false, on = false;
   for (;; seg++) {
     uint32_t es = seg == kSegs - 1 ? e : min(e, first + (seg + 1) * (len / kSegs));
     if (b.p < es) do {
@@ -320,14 +318,14 @@ __device__ __forceinline__ void walk_range(CtaSmem<LB, NT>* S, const uint32_t* b
         if ((int32_t)ent >= 0) {
           slots++;
         } else if (guess) {
-          r.guessed_on = true;
+          on = true;
           valid_from = seg;  // boundaries before the stop lead to it
           slots++;
           ent = 1;           // one bit on
         } else {
           const bool eob = ((ent >> 8) & 3) == kStopEob;
-          r.term = eob ? kTermEob : kTermBad;
-          r.term_pos = b.p + (eob ? (ent >> 27) & 15 : 0u);
+          term = eob ? kTermEob : kTermBad;
+          S->term_pos[id] = b.p + (eob ? (ent >> 27) & 15 : 0u);
           ent = 0;
           es = 0;  // ends the walk
         }
@@ -336,25 +334,25 @@ __device__ __forceinline__ void walk_range(CtaSmem<LB, NT>* S, const uint32_t* b
         t.after(ent);
       }
     } while (b.p < (t.off ? kNone : es));
-    if (r.term || seg == kSegs - 1) break;
+    if (term || seg == kSegs - 1) break;
     const uint32_t at = b.p - first;
     if (again) {
-      const uint32_t old = S->cp[seg][tid];
+      const uint32_t old = S->cp[seg][id];
       if ((old & 0x3FFu) == at) {
         slots += old >> 10;
         met = true;
         break;
       }
     }
-    S->cp[seg][tid] = at | slots << 10;
+    S->cp[seg][id] = at | slots << 10;
   }
   // seg parts were passed; their lookups become those left to the end
   for (uint32_t k = 0; k < kSegs - 1; k++) {
-    if (r.term || (guess && k < valid_from)) S->cp[k][tid] = kNoCp;
-    else if (k < seg) S->cp[k][tid] = (S->cp[k][tid] & 0x3FFu) | (slots - (S->cp[k][tid] >> 10)) << 10;
+    if (term || (guess && k < valid_from)) S->cp[k][id] = kNoCp;
+    else if (k < seg) S->cp[k][id] = (S->cp[k][id] & 0x3FFu) | (slots - (S->cp[k][id] >> 10)) << 10;
   }
-  r.slots = slots;
-  if (!r.term && !met) r.end = b.p;
+  S->info[id] = slots | term * kInfoTerm | (on ? kInfoOn : 0u);
+  if (!term && !met) S->end[id] = b.p;
 }
 
 // The tokens of the n lookups from start on to tok.
@@ -890,8 +888,9 @@ template <int LB, int NT>
 __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSmem<LB, NT>* S,
                                           const PagePool& pool, bool zero_window) {
   const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
-  constexpr uint32_t kTokCap = CtaSmem<LB, NT>::kTokCap, kRangeMin = CtaSmem<LB, NT>::kRangeMin;
+  constexpr uint32_t kTokCap = CtaSmem<LB, NT>::kTokCap;
   const uint32_t tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
   uint32_t rcap = kRangeMax;
   for (;;) {
     // every thread computes the round's geometry from the shared state
@@ -916,38 +915,50 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
     const uint32_t pend = p0 + (uint32_t)min(span, (uint64_t)r * NT);
     const uint32_t lanes = (pend - p0 + r - 1) / r;
     const uint32_t* base = in32 + w0;
-    if (tid < 2) S->c.min_need[tid] = S->c.min_term[tid] = kNone;
-    // 1. from the guessed starts
+    // 1. from the guessed starts (a range cut off by a stop keeps the end it had: its own start)
     const bool active = tid < lanes;
-    const uint32_t first = p0 + tid * r, e = min(first + r, pend);
-    Range ra{};
-    ra.start = first;
     if (active) {
-      walk_range<LB, NT>(S, base, first, r, e, tid > 0, false, ra);
-      S->end[tid] = ra.end;
+      S->start[tid] = S->end[tid] = p0 + tid * r;
+      walk_range<LB, NT>(S, base, p0 + tid * r, r, min(p0 + tid * r + r, pend), tid, tid > 0, false);
     }
     __syncwarp();
-    // 2. from the end of the range before, until nothing moves
+    // 2. from the end of the range before, until nothing moves.  The ranges to
+    // walk again go to the first threads, so that few of them are few warps.
     uint32_t last = kNone;  // range that holds the end of the block (kNone: not in this round)
-    for (uint32_t it = 0;; it ^= 1) {
+    for (;;) {
       __syncthreads();
-      const uint32_t s1 = active && tid ? S->end[tid - 1] : ra.start;
-      const bool need = active && (s1 != ra.start || ra.guessed_on);
-      const uint32_t mn = __reduce_min_sync(0xFFFFFFFFu, need ? tid : kNone);
-      const uint32_t mt = __reduce_min_sync(0xFFFFFFFFu, active && ra.term ? tid : kNone);
-      if ((tid & 31) == 0) {
-        if (mn != kNone) atomicMin(&S->c.min_need[it], mn);
-        if (mt != kNone) atomicMin(&S->c.min_term[it], mt);
+      const uint32_t st = active ? S->start[tid] : 0u, inf = active ? S->info[tid] : 0u;
+      const uint32_t s1 = active && tid ? S->end[tid - 1] : st;
+      const bool need = active && (s1 != st || (inf & kInfoOn));
+      const uint32_t nb = __ballot_sync(0xFFFFFFFFu, need);
+      const uint32_t tb = __ballot_sync(0xFFFFFFFFu, (inf / kInfoTerm) & 3);
+      if (lane == 0) {
+        S->need[warp] = nb;
+        S->term[warp] = tb;
       }
+      if (need) S->start[tid] = s1;
       __syncthreads();
-      const uint32_t first_need = S->c.min_need[it];
-      last = S->c.min_term[it];
-      if (first_need == kNone || last < first_need) break;
-      if (tid == 0) S->c.min_need[it ^ 1] = S->c.min_term[it ^ 1] = kNone;
-      if (need) {
-        ra.start = s1;
-        walk_range<LB, NT>(S, base, first, r, e, false, true, ra);
-        S->end[tid] = ra.end;
+      const uint32_t mn = lane < NT / 32 ? S->need[lane] : 0u;
+      const uint32_t mt = lane < NT / 32 ? S->term[lane] : 0u;
+      const uint32_t bn = __ballot_sync(0xFFFFFFFFu, mn != 0), bt = __ballot_sync(0xFFFFFFFFu, mt != 0);
+      const int wn = __ffs(bn | 0x80000000u) - 1, wt = __ffs(bt | 0x80000000u) - 1;
+      const uint32_t first_need = 32u * wn + __ffs(__shfl_sync(0xFFFFFFFFu, mn, wn)) - 1;
+      const uint32_t first_term = 32u * wt + __ffs(__shfl_sync(0xFFFFFFFFu, mt, wt)) - 1;
+      last = bt ? first_term : kNone;
+      if (!bn || last < first_need) break;
+      uint32_t upto = __popc(mn);
+#pragma unroll
+      for (int d = 1; d < NT / 32; d <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, upto, d);
+        if (lane >= d) upto += u;
+      }
+      const uint32_t before = __shfl_sync(0xFFFFFFFFu, upto - __popc(mn), warp);
+      const uint32_t n_need = __shfl_sync(0xFFFFFFFFu, upto, NT / 32 - 1);
+      if (need) S->list[before + __popc(nb & ((1u << lane) - 1))] = (uint16_t)tid;
+      __syncthreads();
+      if (tid < n_need) {
+        const uint32_t id = S->list[tid], f = p0 + id * r;
+        walk_range<LB, NT>(S, base, f, r, min(f + r, pend), id, false, true);
       }
       __syncwarp();
     }
@@ -955,13 +966,14 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
     const uint32_t used = last != kNone ? last + 1 : lanes;
     const bool in_use = tid < used;
     uint32_t ts;
-    const uint32_t my_slots = in_use ? ra.slots : 0u;
+    const uint32_t my_info = in_use ? S->info[tid] : 0u, my_start = in_use ? S->start[tid] : 0u;
+    const uint32_t my_slots = my_info & 0xFFFFu, my_term = (my_info / kInfoTerm) & 3;
     const uint32_t slot0 = cta_scan(S, 0, my_slots, ts);
     if (ts > kTokCap) {
       const uint32_t fit = (uint32_t)__syncthreads_count(in_use && slot0 + my_slots <= kTokCap);
       if (tid == fit) {
         S->c.round_slots = slot0;
-        S->c.round_pos = ra.start;  // = the end of range fit - 1
+        S->c.round_pos = my_start;  // = the end of range fit - 1
       }
       if (tid == 0) {
         S->c.round_lanes = fit;
@@ -972,8 +984,8 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
     } else if (tid == used - 1) {
       S->c.round_slots = ts;
       S->c.round_lanes = used;
-      S->c.round_kind = ra.term;
-      S->c.round_pos = ra.term ? ra.term_pos : ra.end;
+      S->c.round_kind = my_term;
+      S->c.round_pos = my_term ? S->term_pos[tid] : S->end[tid];
     }
     __syncthreads();
     const uint32_t n_lanes = S->c.round_lanes, n_slots = S->c.round_slots;
@@ -984,7 +996,7 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
       if (tid == 0) S->c.status = kBadDeflate;
       break;
     }
-    if (tid < n_lanes) write_tokens<LB, NT>(S, base, ra.start, my_slots, S->tok + slot0);
+    if (tid < n_lanes) write_tokens<LB, NT>(S, base, my_start, my_slots, S->tok + slot0);
     __syncwarp();
     __syncthreads();
     // 4. expansion
