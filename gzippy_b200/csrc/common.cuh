@@ -130,14 +130,17 @@ struct PlacedChunk {
   uint64_t out_off;      // final output offset of entry 0
   uint64_t member_off;   // final output offset where the chunk's member begins
   uint32_t chunk;        // chunk id
-  uint32_t pad;
+  uint32_t last_page;    // page of its last entry,
+  uint32_t prev_page;    // the one before,
+  uint32_t last_seq;     // and the last page's index within the chunk
 };
 
-// CRC block: a run of final output bytes inside one member
+// CRC block: final output bytes [begin, last) of one member, in the block that
+// ends at `end` (on a 16-byte boundary, at or past last)
 struct CrcBlock {
-  uint64_t off;
-  uint32_t len;
-  uint32_t member;
+  uint64_t begin, last, end;
+  uint64_t after;        // bytes from end to the end of the member's last block
+  uint32_t member, pad;
 };
 
 }  // namespace gzgpu

@@ -8,7 +8,7 @@
 //   4. persistent inflate over the work list   (inflate.cu)
 //   5. chain walk                              (host: accept / repair, as the
 //      reference's consumer_loop, chunk_fetcher.rs:855; repairs re-enter 4)
-//   6. tails, window chain, bodies, CRC        (resolve.cu)
+//   6. bytes and markers, CRC                  (resolve.cu)
 // The plain path (gzgpu_decompress) runs one stream per job; the batched
 // path runs all of a batch's streams in one job, so every stage is one launch
 // for the whole batch.
@@ -191,8 +191,7 @@ struct gzgpu_ctx {
   bool crc_ready = false;
 
   DevBuf in, out, s_off, s_len, info, units, cands, counters, descs, results, spec, work, cost, find;
-  DevBuf pages, owner, seq, placed, placed_of, list, cblocks, mend, mraw, mtrail, mlen, mcrc,
-      mstatus;
+  DevBuf pages, owner, seq, placed, placed_of, cblocks, mend, mraw, mtrail, mlen, mstatus;
   // seek-index builds: the decoder's block log, the checkpoint interval and
   // the serialized index of the last job (gzgpu_build_index)
   DevBuf blk_log;
@@ -204,8 +203,8 @@ struct gzgpu_ctx {
   HostPinned h_stage;
   std::vector<DevBuf*> all_bufs() {
     return {&in,     &out,   &s_off,   &s_len,  &info,   &units,   &cands,  &counters, &descs,
-            &results, &spec, &work,    &pages,  &owner,  &seq,     &placed, &placed_of, &list,
-            &cblocks, &mend,  &mraw,   &mtrail, &mlen,    &mcrc,   &mstatus, &blk_log,
+            &results, &spec, &work,    &pages,  &owner,  &seq,     &placed, &placed_of,
+            &cblocks, &mend,  &mraw,   &mtrail, &mlen,    &mstatus, &blk_log,
             &cost,  &find};
   }
   const uint8_t* cur_in = nullptr;  // input buffer of the running job
@@ -1093,7 +1092,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   const uint32_t n_all = (uint32_t)hd.size();
   std::vector<PlacedChunk> placed;
   std::vector<uint32_t> placed_of(n_all, 0xFFFFFFFFu);
-  std::vector<uint32_t> tlist;  // placed chunks whose tails hold markers
+  uint64_t n_tail_markers = 0;  // placed chunks whose last 32 KiB hold markers
   std::vector<CrcBlock> cblk;
   std::vector<uint64_t> mtrail, mlenv, mendv;
   uint64_t out_total = 0;
@@ -1110,15 +1109,20 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
       for (uint32_t k = mp.order_begin; k < mp.order_end; k++) {
         uint32_t cid = w.order[k];
         placed_of[cid] = (uint32_t)placed.size();
-        placed.push_back(PlacedChunk{out_total + so, moff, cid, 0});
         const ChunkResult& r = hr[cid];
+        placed.push_back(PlacedChunk{out_total + so, moff, cid, r.last_page, r.prev_page,
+                                     r.out_len ? (uint32_t)((r.out_len - 1) / kPageEntries) : 0u});
         uint64_t t0 = r.out_len > kWindow ? r.out_len - kWindow : 0;
-        if (r.marker_end > t0) tlist.push_back((uint32_t)placed.size() - 1);
+        n_tail_markers += r.marker_end > t0;
         so += r.out_len;
       }
-      for (uint64_t b = 0; mp.trailer != kNoTrailer && b < mp.out_len; b += kCrcBlock)
-        cblk.push_back(CrcBlock{moff + b, (uint32_t)std::min<uint64_t>(kCrcBlock, mp.out_len - b),
-                                (uint32_t)mtrail.size()});
+      const uint64_t m1 = moff + mp.out_len, mcrc_end = (m1 + 15) & ~15ull;
+      for (uint64_t e = mcrc_end; mp.trailer != kNoTrailer && e > moff;) {
+        const uint64_t b = e > moff + kCrcBlock ? e - kCrcBlock : moff;
+        if (b < m1) cblk.push_back(CrcBlock{b, std::min(e, m1), e, mcrc_end - e, (uint32_t)mtrail.size(), 0});
+        if (b == moff) break;
+        e = b;
+      }
       mtrail.push_back(mp.trailer);
       mlenv.push_back(mp.out_len);
       mendv.push_back(moff + mp.out_len);
@@ -1127,7 +1131,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
     out_total += so;
   }
   stats.n_accepted = placed.size();
-  stats.n_tail_marker_chunks = tlist.size();
+  stats.n_tail_marker_chunks = n_tail_markers;
   stats.n_members = mtrail.size();
   stats.out_bytes = out_total;
   cudaEventRecord(ev[6], st);
@@ -1141,18 +1145,16 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   cur_out = (user_out && out_total <= user_cap) ? user_out : nullptr;
   if ((rc = check(cur_out ? cudaSuccess : out.ensure(out_total + 64))) ||
       (rc = check(this->placed.ensure(sizeof(PlacedChunk) * (placed.size() + 1)))) ||
-      (rc = check(this->placed_of.ensure(4 * (n_all + 1)))) || (rc = check(list.ensure(4 * (tlist.size() + 1)))) ||
+      (rc = check(this->placed_of.ensure(4 * (n_all + 1)))) ||
       (rc = check(cblocks.ensure(sizeof(CrcBlock) * (cblk.size() + 1)))) ||
       (rc = check(mend.ensure(8 * (mendv.size() + 1)))) || (rc = check(mraw.ensure(4 * (mtrail.size() + 1)))) ||
       (rc = check(this->mtrail.ensure(8 * (mtrail.size() + 1)))) || (rc = check(mlen.ensure(8 * (mlenv.size() + 1)))) ||
-      (rc = check(mcrc.ensure(4 * (mtrail.size() + 1)))) ||
       (rc = check(mstatus.ensure(4 * (mtrail.size() + 1)))))
     return rc;
   if (!placed.empty())
     cudaMemcpyAsync(this->placed.p, placed.data(), sizeof(PlacedChunk) * placed.size(),
                     cudaMemcpyHostToDevice, st);
   if (n_all) cudaMemcpyAsync(this->placed_of.p, placed_of.data(), 4 * n_all, cudaMemcpyHostToDevice, st);
-  if (!tlist.empty()) cudaMemcpyAsync(list.p, tlist.data(), 4 * tlist.size(), cudaMemcpyHostToDevice, st);
   if (!cblk.empty())
     cudaMemcpyAsync(cblocks.p, cblk.data(), sizeof(CrcBlock) * cblk.size(), cudaMemcpyHostToDevice, st);
   if (!mtrail.empty()) {
@@ -1169,24 +1171,16 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
     if ((rc = check(resolve_init(st)))) return rc;
     crc_ready = true;
   }
-  const uint32_t np = (uint32_t)placed.size();
-  if ((rc = check(launch_tail_literals(this->placed.as<PlacedChunk>(), np, results.as<ChunkResult>(),
-                                       pool, cur_out, st))) ||
-      (rc = check(launch_tail_markers(this->placed.as<PlacedChunk>(), list.as<uint32_t>(),
-                                      (uint32_t)tlist.size(), results.as<ChunkResult>(), pool,
-                                      cur_out, sms, st))) ||
-      (rc = check(launch_body(this->placed.as<PlacedChunk>(), this->placed_of.as<uint32_t>(),
-                              n_pages_used, results.as<ChunkResult>(), pool, cur_out, sms,
-                              st))))
+  if ((rc = check(launch_resolve(this->placed.as<PlacedChunk>(), this->placed_of.as<uint32_t>(),
+                                 n_pages_used, results.as<ChunkResult>(), pool, cur_out, sms, st))))
     return rc;
   cudaEventRecord(ev[11], st);
   if ((rc = check(launch_crc(cblocks.as<CrcBlock>(), (uint32_t)cblk.size(), cur_out,
                              mend.as<uint64_t>(), mraw.as<uint32_t>(),
                              this->mtrail.as<uint64_t>(), mlen.as<uint64_t>(),
-                             (uint32_t)mtrail.size(), cur_in, mcrc.as<uint32_t>(),
-                             mstatus.as<int32_t>(), sms, st))))
+                             (uint32_t)mtrail.size(), cur_in, mstatus.as<int32_t>(), sms, st))))
     return rc;
-  stats.kernel_launches += 5;
+  stats.kernel_launches += 3;
   std::vector<int32_t> mst(mtrail.size());
   if (!mst.empty())
     cudaMemcpyAsync(mst.data(), mstatus.p, 4 * mst.size(), cudaMemcpyDeviceToHost, st);

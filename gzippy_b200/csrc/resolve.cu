@@ -6,19 +6,21 @@
 // output (replace_markers.rs:7-23), i.e. final[out_off - 32768 + v - 32768],
 // read as 0 before the member's first byte (the zero window).
 //
-//   tail_literals : bytes of every chunk's last 32 KiB ("tail") -> output
-//   tail_markers  : markers in tails, chunk after chunk in output order: a
-//                   tail's markers only reach the tails of earlier chunks,
-//                   so this walk is the window chain (window_map.rs:80-103,
-//                   chunk_fetcher.rs publish_subchunk_windows :2295)
-//   body          : all other entries, fully parallel over pages, reading
-//                   windows the chain made final (resolve_and_narrow_markers
-//                   _in_place_crc, chunk_data.rs:1745)
-//   crc_blocks    : CRC32 of blocks of final output (up to 32 KiB of one
-//                   member each), each block's CRC moved to its member's end
-//                   and XORed into the member's register (crc32.rs
-//                   combine_crc32 :127 combines the same quantities)
-//   member_check  : each member's CRC32 and ISIZE against its trailer
+//   resolve      : every entry's byte.  A marker names a byte of the 32 KiB
+//                  before its chunk, which lies near the end of one of the few
+//                  chunks before it; that entry is a literal or again a marker,
+//                  naming a byte before its own chunk.  Each marker follows its
+//                  references through the chunks' entries until it reaches a
+//                  literal (or a position before the member: 0), so all chunks
+//                  resolve in parallel and the window chain (window_map.rs:
+//                  80-103, chunk_fetcher.rs publish_subchunk_windows :2295,
+//                  resolve_and_narrow_markers_in_place_crc, chunk_data.rs:1745)
+//                  needs no order
+//   crc_blocks   : CRC32 of blocks of final output (up to 64 KiB of one
+//                  member each), each block's CRC moved to its member's end
+//                  and XORed into the member's register (crc32.rs
+//                  combine_crc32 :127 combines the same quantities)
+//   member_check : each member's CRC32 and ISIZE against its trailer
 #include <cstdint>
 
 #include "common.cuh"
@@ -26,183 +28,112 @@
 
 namespace gzgpu {
 
-// page of entry q of a chunk's last 32 KiB: the page of its last entry or
-// the one before (a page holds 64 Ki entries)
-__device__ __forceinline__ const uint16_t* chunk_entry_page(const ChunkResult& r, uint64_t q,
-                                                            const PagePool& pool) {
-  uint64_t last_seq = (r.out_len - 1) / kPageEntries;
-  uint32_t page = (q / kPageEntries == last_seq) ? r.last_page : r.prev_page;
-  return pool.data + (size_t)page * kPageEntries;
+// entry q of placed chunk c, one of its last 32 Ki: its last page or the one before
+__device__ __forceinline__ const uint16_t* tail_entry(const PlacedChunk& c, uint64_t q,
+                                                      const PagePool& pool) {
+  const uint32_t page = (uint32_t)(q >> 16) == c.last_seq ? c.last_page : c.prev_page;
+  return pool.data + (size_t)page * kPageEntries + (q & (kPageEntries - 1));
 }
 
-// One warp writes the bytes of a span of 32 groups of 4 entries: lane L
-// holds the bytes of entries 4L .. 4L + 3 of the span in `w` (byte j of w =
-// entry 4L + j) and in `valid` which of them to write; `d0` is the output
-// address of the span's entry 0.  Each lane stores the aligned 32-bit word
-// that starts inside its group (its last bytes, then the next lane's first,
-// by a funnel shift), so a warp writes 128 contiguous bytes per store; bytes
-// of partly valid words and the two words the span shares with its
-// neighbours go out one by one.
-__device__ __forceinline__ void warp_store_bytes(uint8_t* __restrict__ out, uint64_t d0, uint32_t w,
-                                                 uint32_t valid, int lane) {
-  const uint32_t s = (uint32_t)(d0 & 3);
-  const uint64_t dl = d0 + 4 * (uint64_t)lane;
-  if (s == 0) {
-    if (valid == 0xFu) {
-      *reinterpret_cast<uint32_t*>(out + dl) = w;
-    } else {
-      for (int j = 0; j < 4; j++)
-        if ((valid >> j) & 1) out[dl + j] = (uint8_t)(w >> (8 * j));
-    }
-    return;
-  }
-  const uint32_t u = 4 - s;  // bytes of this group before the next aligned word
-  const uint32_t wn = __shfl_down_sync(0xFFFFFFFFu, w, 1);
-  const uint32_t vn = __shfl_down_sync(0xFFFFFFFFu, valid, 1);
-  if (lane < 31) {
-    const uint32_t vw = (valid >> u) | ((vn << s) & 0xFu);
-    const uint32_t ww = __funnelshift_r(w, wn, 8 * u);
-    if (vw == 0xFu) {
-      *reinterpret_cast<uint32_t*>(out + dl + u) = ww;
-    } else {
-      for (int j = 0; j < 4; j++)
-        if ((vw >> j) & 1) out[dl + u + j] = (uint8_t)(ww >> (8 * j));
-    }
-  } else {
-    for (uint32_t j = u; j < 4; j++)
-      if ((valid >> j) & 1) out[dl + j] = (uint8_t)(w >> (8 * j));
-  }
-  if (lane == 0)
-    for (uint32_t j = 0; j < u; j++)
-      if ((valid >> j) & 1) out[dl + j] = (uint8_t)(w >> (8 * j));
-}
-
-// the 4 entries of a group (page-relative index e, a multiple of 4)
-__device__ __forceinline__ void load_group(const uint16_t* page, uint32_t e, uint32_t v[4]) {
-  const uint2 x = *reinterpret_cast<const uint2*>(page + e);
-  v[0] = x.x & 0xFFFFu;
-  v[1] = x.x >> 16;
-  v[2] = x.y & 0xFFFFu;
-  v[3] = x.y >> 16;
-}
-
-// one CTA per chunk: the bytes of its last 32 KiB (markers written as 0,
-// which tail_markers_kernel replaces)
-__global__ void tail_literals_kernel(const PlacedChunk* __restrict__ placed, uint32_t n,
-                                     const ChunkResult* __restrict__ results, PagePool pool,
-                                     uint8_t* __restrict__ out) {
-  const uint32_t k = blockIdx.x;
-  if (k >= n) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const PlacedChunk pc = placed[k];
-  const ChunkResult r = results[pc.chunk];
-  const uint64_t len = r.out_len, t0 = len > kWindow ? len - kWindow : 0;
-  const uint64_t g0 = t0 & ~3ull;  // groups start at multiples of 4 (never across a page)
-  for (uint64_t base = g0 + 128 * (uint64_t)warp; base < len; base += 128 * (uint64_t)nwarps) {
-    const uint64_t q = base + 4 * (uint64_t)lane;
-    uint32_t w = 0, valid = 0;
-    if (q < len) {
-      uint32_t v[4];
-      load_group(chunk_entry_page(r, q, pool), (uint32_t)(q % kPageEntries), v);
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        if (q + j >= t0 && q + j < len) {
-          valid |= 1u << j;
-          w |= (v[j] < 256 ? v[j] : 0u) << (8 * j);
-        }
-    }
-    warp_store_bytes(out, pc.out_off + base, w, valid, lane);
+// The byte of marker v of a chunk that starts at `off`, placed[j] or a later
+// one of its member (`moff`: the member's first byte); from there back.
+__device__ uint32_t follow_marker(const PlacedChunk* __restrict__ placed, uint32_t j, uint64_t off,
+                                  uint64_t moff, uint32_t v, const PagePool& pool) {
+  for (;;) {
+    const int64_t src = (int64_t)off - (int64_t)kWindow + (int64_t)(v - kMarkerBase);
+    if (src < (int64_t)moff) return 0;  // before the member: the zero window
+    do {
+      j--;
+    } while ((int64_t)placed[j].out_off > src);
+    const PlacedChunk c = placed[j];
+    v = *tail_entry(c, (uint64_t)src - c.out_off, pool);
+    if (v < kMarkerBase) return v;
+    off = c.out_off;  // a marker of chunk j: its window is before chunk j
   }
 }
 
-// The markers of chunk tails.  A tail marker names a byte of the 32 KiB
-// before its chunk, which lies in the tails of earlier chunks of the member
-// (a chunk shorter than 32 KiB is all tail); that entry is a literal or
-// again a marker, naming a byte before its own chunk.  Each marker follows
-// its references through the chunks' entries until it reaches a literal (or
-// a position before the member: 0), so all tails resolve in parallel: one
-// CTA per chunk of the list (the chunks whose tails hold markers), placed
-// chunks in output order.
-__global__ void tail_markers_kernel(const PlacedChunk* __restrict__ placed,
-                                    const uint32_t* __restrict__ list, uint32_t n_list,
-                                    const ChunkResult* __restrict__ results, PagePool pool,
-                                    uint8_t* __restrict__ out) {
-  for (uint32_t i = blockIdx.x; i < n_list; i += gridDim.x) {
-    const uint32_t k = list[i];
-    const PlacedChunk pc = placed[k];
-    const ChunkResult r = results[pc.chunk];
-    const uint64_t len = r.out_len, t0 = len > kWindow ? len - kWindow : 0;
-    const uint64_t end = r.marker_end < len ? r.marker_end : len;
-    const int64_t moff = (int64_t)pc.member_off;
-    for (uint64_t q = t0 + threadIdx.x; q < end; q += blockDim.x) {
-      uint32_t v = chunk_entry_page(r, q, pool)[q % kPageEntries];
-      if (v < kMarkerBase) continue;  // a literal: written by tail_literals_kernel
-      uint32_t j = k;
-      int64_t off = (int64_t)pc.out_off;
-      uint32_t b = 0;
-      for (;;) {
-        const int64_t src = off - (int64_t)kWindow + (int64_t)(v - kMarkerBase);
-        if (src < moff) break;  // before the member: the zero window
-        // the chunk that holds src: one of the few before chunk j
-        do {
-          j--;
-        } while ((int64_t)placed[j].out_off > src);
-        const PlacedChunk pj = placed[j];
-        const ChunkResult rj = results[pj.chunk];
-        const uint64_t qj = (uint64_t)(src - (int64_t)pj.out_off);
-        v = chunk_entry_page(rj, qj, pool)[qj % kPageEntries];
-        if (v < kMarkerBase) {
-          b = v;
-          break;
-        }
-        off = (int64_t)pj.out_off;  // a marker of chunk j: its window is before chunk j
-      }
-      out[pc.out_off + q] = (uint8_t)b;
-    }
-  }
-}
+// One CTA per unit of kResolveUnit entries of a page (grid-stride): literal
+// bytes go to shared memory, markers to a list, which the threads then follow
+// one marker each (two dependent loads a reference is what the kernel waits
+// for, so no lane idles while a neighbour gathers), and the unit's bytes leave
+// in aligned 16-byte stores.  Units are small: many in flight, also when a job
+// has few chunks.
+constexpr uint32_t kResolveUnit = 4096;
+constexpr int kResolveThreads = 256;
+static_assert(kResolveUnit == 16 * kResolveThreads, "16 entries a thread");
 
-// one CTA per page: the entries before the chunk's tail, markers gathered
-// from the final window; 4 entries per lane, aligned 32-bit stores
-__global__ void body_kernel(const PlacedChunk* __restrict__ placed,
-                            const uint32_t* __restrict__ placed_of_chunk, uint32_t n_pages,
-                            const ChunkResult* __restrict__ results, PagePool pool,
-                            uint8_t* __restrict__ out) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  for (uint32_t p = blockIdx.x; p < n_pages; p += gridDim.x) {
-    const uint32_t cid = pool.owner[p];
+__global__ void __launch_bounds__(kResolveThreads)
+    resolve_kernel(const PlacedChunk* __restrict__ placed, const uint32_t* __restrict__ placed_of_chunk,
+                   uint32_t n_pages, const ChunkResult* __restrict__ results, PagePool pool,
+                   uint8_t* __restrict__ out) {
+  constexpr uint32_t kUnits = kPageEntries / kResolveUnit;
+  __shared__ alignas(16) uint8_t bytes[kResolveUnit + 16];
+  __shared__ uint32_t list[kResolveUnit];  // entry << 16 | marker
+  __shared__ uint32_t n_list;
+  const uint32_t tid = threadIdx.x;
+  const int lane = tid & 31;
+  for (uint32_t u = blockIdx.x; u < n_pages * kUnits; u += gridDim.x) {
+    const uint32_t p = u / kUnits, first = (u % kUnits) * kResolveUnit;
+    const uint32_t cid = pool.owner[p], sw = pool.seq[p];
     const uint32_t k = placed_of_chunk[cid];
     if (k == 0xFFFFFFFFu) continue;
-    const uint32_t sw = pool.seq[p];
-    if ((sw >> kGenShift) != results[cid].gen) continue;  // page of a failed attempt
-    const PlacedChunk pc = placed[k];
     const uint64_t len = results[cid].out_len;
-    const uint64_t t0 = len > kWindow ? len - kWindow : 0;
-    const uint64_t q0 = (uint64_t)(sw & kSeqMask) * kPageEntries;
-    if (q0 >= t0) continue;
-    const uint32_t n = (uint32_t)min((uint64_t)kPageEntries, t0 - q0);
-    const uint16_t* src = pool.data + (size_t)p * kPageEntries;
-    const int64_t wbase = (int64_t)pc.out_off - (int64_t)kWindow - (int64_t)kMarkerBase;
-    const int64_t moff = (int64_t)pc.member_off;
-    for (uint32_t base = 128 * warp; base < n; base += 128 * nwarps) {
-      const uint32_t e = base + 4 * lane;
-      uint32_t w = 0, valid = 0;
-      if (e < n) {
-        uint32_t v[4];
-        load_group(src, e, v);
+    const uint64_t q0 = (uint64_t)(sw & kSeqMask) * kPageEntries + first;
+    if (q0 >= len || (sw >> kGenShift) != results[cid].gen) continue;  // or a failed attempt's page
+    const uint32_t n = (uint32_t)min((uint64_t)kResolveUnit, len - q0);
+    const uint64_t off = placed[k].out_off, moff = placed[k].member_off;
+    const uint16_t* src = pool.data + (size_t)p * kPageEntries + first;
+    __syncthreads();  // the unit before has left
+    if (tid == 0) n_list = 0;
+    uint4 x[2];
 #pragma unroll
-        for (int j = 0; j < 4; j++)
-          if (e + j < n) {
-            valid |= 1u << j;
-            uint32_t b = v[j];
-            if (b >= 256) {
-              const int64_t sidx = wbase + b;
-              b = sidx >= moff ? out[sidx] : 0u;
-            }
-            w |= b << (8 * j);
-          }
+    for (uint32_t s = 0; s < 2; s++) {
+      const uint32_t e = 8 * (tid + kResolveThreads * s);
+      x[s] = e < n ? *reinterpret_cast<const uint4*>(src + e) : make_uint4(0, 0, 0, 0);
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t s = 0; s < 2; s++) {
+      const uint32_t e = 8 * (tid + kResolveThreads * s);
+      *reinterpret_cast<uint2*>(bytes + e) =
+          make_uint2(__byte_perm(x[s].x, x[s].y, 0x6420), __byte_perm(x[s].z, x[s].w, 0x6420));
+      const uint32_t h[4] = {x[s].x, x[s].y, x[s].z, x[s].w};
+      uint32_t m = 0;  // markers among the eight
+#pragma unroll
+      for (int i = 0; i < 4; i++) m |= ((h[i] >> 15 & 1) | (h[i] >> 30 & 2)) << (2 * i);
+      if (e + 8 > n) m &= e < n ? (1u << (n - e)) - 1 : 0u;
+      if (!__any_sync(0xFFFFFFFFu, m != 0)) continue;
+      uint32_t at = __popc(m);
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, at, d);
+        if (lane >= d) at += v;
       }
-      warp_store_bytes(out, pc.out_off + q0 + base, w, valid, lane);
+      uint32_t base = 0;
+      if (lane == 31) base = atomicAdd(&n_list, at);
+      at += __shfl_sync(0xFFFFFFFFu, base, 31) - __popc(m);
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+        if ((m >> i) & 1) list[at++] = (e + i) << 16 | ((h[i >> 1] >> (16 * (i & 1))) & 0xFFFFu);
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < n_list; i += kResolveThreads)
+      bytes[list[i] >> 16] = (uint8_t)follow_marker(placed, k, off, moff, list[i] & 0xFFFFu, pool);
+    __syncthreads();
+    // the unit's bytes, by aligned 16 of the output (one more than the unit's length needs)
+    const uint64_t d0 = off + q0;
+    for (uint32_t t = tid; t < kResolveUnit / 16 + 1; t += kResolveThreads) {
+      const int32_t o = 16 * (int32_t)t - (int32_t)(d0 & 15);  // its first byte in the unit
+      uint8_t* dst = out + ((d0 & ~15ull) + 16 * t);
+      if (o >= 0 && o + 16 <= (int32_t)n) {
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(bytes + (o & ~3));
+        const uint32_t sh = 8 * (o & 3);
+        *reinterpret_cast<uint4*>(dst) =
+            make_uint4(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], w[2], sh),
+                       __funnelshift_r(w[2], w[3], sh), __funnelshift_r(w[3], w[4], sh));
+      } else {
+        for (int32_t i = max(0, -o); i < 16 && o + i < (int32_t)n; i++) dst[i] = bytes[o + i];
+      }
     }
   }
 }
@@ -217,7 +148,7 @@ __global__ void body_kernel(const PlacedChunk* __restrict__ placed,
 // member's end with A^(bytes after the block) and XORed into the member's
 // register, so blocks fold in independently, in any order.
 // ---------------------------------------------------------------------------
-__device__ uint32_t d_crc_tab[4][256];  // slice-by-4 tables
+__device__ uint32_t d_crc_tab[256];
 __device__ uint32_t d_x2n[64];          // x^(2^k) mod P
 // d_crc_shift[j][k][v] = A^(kCrcSlice << j)(v << 8k): moves a register past
 // 2^j lane slices of zero bytes with 4 lookups
@@ -258,13 +189,7 @@ __global__ void crc_init_kernel() {
   uint32_t i = threadIdx.x;
   uint32_t c = i;
   for (int k = 0; k < 8; k++) c = (c >> 1) ^ (0xEDB88320u & (0u - (c & 1u)));
-  d_crc_tab[0][i] = c;
-  __syncthreads();
-  for (int t = 1; t < 4; t++) {
-    uint32_t p = d_crc_tab[t - 1][i];
-    d_crc_tab[t][i] = (p >> 8) ^ d_crc_tab[0][p & 0xFF];
-    __syncthreads();
-  }
+  d_crc_tab[i] = c;
   if (i == 0) {
     uint32_t v = 1u << 30;  // x^1
     for (int k = 0; k < 64; k++) {
@@ -295,46 +220,58 @@ __device__ __forceinline__ uint32_t crc_byte(const uint32_t* ltab, uint32_t lane
   return ltab[(((c ^ b) & 0xFFu) << 5) | lane] ^ (c >> 8);
 }
 
-// CRC32 of the final output, one warp per block of up to kCrcBlock bytes of
-// one member.  The block is cut into 32 lane slices of kCrcSlice bytes
-// counted back from its end, so every slice has the same length once the
-// bytes before the block count as zeros (they leave the register at 0).
-// Each lane folds its slice byte by byte with its own copy of the byte
-// table (no bank conflicts), reading aligned 16-byte words; the slices'
-// registers merge in a tree of fixed shifts, and the block's register,
-// moved past the rest of its member, is XORed into mem_raw.
+// CRC32 of the final output, one CTA per block of up to kCrcBlock bytes of one
+// member.  Blocks end on 16-byte boundaries of the output; the bytes before
+// the member's first and after its last count as zeros (the first leave the
+// register at 0, the others are taken back by member_check).  Every thread
+// folds a slice of kCrcSlice bytes byte by byte with its lane's copy of the
+// byte table (no bank conflicts), from aligned 16-byte loads; the slices'
+// registers merge in a tree of fixed shifts, and the block's register, moved
+// past the rest of its member, is XORed into mem_raw.  What a block waits for
+// is the serial chain of its bytes (a table read each), so slices are short:
+// with 1 KiB slices (a warp per 32 KiB) the pass took 50 us for a 4 KiB
+// stream and 75 us up to 64 MiB, now 9 and 21.
 __global__ void __launch_bounds__(kCrcThreads)
     crc_blocks_kernel(const CrcBlock* __restrict__ blocks, uint32_t n,
-                      const uint8_t* __restrict__ out, const uint64_t* __restrict__ mem_end,
-                      uint32_t* __restrict__ mem_raw) {
+                      const uint8_t* __restrict__ out, uint32_t* __restrict__ mem_raw) {
   extern __shared__ __align__(16) uint32_t sm[];
-  uint32_t* ltab = sm;              // [256][32] lane copies of the byte table
-  uint32_t* shf = sm + 256 * 32;    // [kCrcLevels][4][256] shift tables
-  for (uint32_t i = threadIdx.x; i < 256 * 32; i += kCrcThreads) ltab[i] = d_crc_tab[0][i >> 5];
-  for (uint32_t i = threadIdx.x; i < kCrcLevels * 4 * 256; i += kCrcThreads)
-    shf[i] = d_crc_shift[i >> 10][(i >> 8) & 3][i & 255];
+  uint32_t* ltab = sm;                                // [256][32] lane copies of the byte table
+  uint32_t* shf = sm + 256 * 32;                      // [kCrcLevels][4][256] shift tables
+  uint32_t* part = shf + kCrcLevels * 4 * 256;        // [2][warps]
+  constexpr int kWarps = kCrcThreads / 32;
+  for (uint32_t i = threadIdx.x; i < 256 * 32; i += kCrcThreads) ltab[i] = d_crc_tab[i >> 5];
+  for (uint32_t i = threadIdx.x; i < kCrcLevels * 256; i += kCrcThreads)
+    reinterpret_cast<uint4*>(shf)[i] = reinterpret_cast<const uint4*>(&d_crc_shift[0][0][0])[i];
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  for (uint32_t bi = (blockIdx.x * kCrcThreads + threadIdx.x) >> 5; bi < n;
-       bi += (gridDim.x * kCrcThreads) >> 5) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t turn = 0;
+  for (uint32_t bi = blockIdx.x; bi < n; bi += gridDim.x, turn++) {
     const CrcBlock blk = blocks[bi];
-    const uint8_t* p = out + blk.off;
-    const uint8_t* end = p + blk.len;
-    // lane slice [s0, s1), clipped to the block
-    const int64_t back = (int64_t)kCrcSlice * (32 - lane);
-    const uint8_t* s1 = end - (back - kCrcSlice);
-    const uint8_t* s0 = (int64_t)blk.len > back - kCrcSlice ? (back <= (int64_t)blk.len ? end - back : p) : s1;
+    // this thread's slice [s0, s0 + kCrcSlice) of the output
+    const int64_t s0 = (int64_t)blk.end - (int64_t)kCrcSlice * (kCrcThreads - (int)threadIdx.x);
     uint32_t c = 0;
-    const uint8_t* q = s0;
-    // bytes up to the first 16-byte boundary
-    while (q < s1 && (reinterpret_cast<uintptr_t>(q) & 15)) c = crc_byte(ltab, lane, c, *q++);
-    // aligned 16-byte words, the next one loaded while this one folds
-    if (q + 16 <= s1) {
-      uint4 w = *reinterpret_cast<const uint4*>(q);
-      for (;;) {
-        const bool more = q + 32 <= s1;
-        uint4 nx = more ? *reinterpret_cast<const uint4*>(q + 16) : make_uint4(0, 0, 0, 0);
-        const uint32_t wd[4] = {w.x, w.y, w.z, w.w};
+    if (s0 + (int64_t)kCrcSlice > (int64_t)blk.begin) {
+      uint4 v[kCrcSlice / 16];
+#pragma unroll
+      for (uint32_t i = 0; i < kCrcSlice / 16; i++) {
+        const int64_t a = s0 + 16 * (int64_t)i;
+        v[i] = a + 16 > (int64_t)blk.begin && a + 16 <= (int64_t)blk.last
+                   ? *reinterpret_cast<const uint4*>(out + a)
+                   : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (uint32_t i = 0; i < kCrcSlice / 16; i++) {
+        uint32_t wd[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+        const int64_t a = s0 + 16 * (int64_t)i;
+        if (a < (int64_t)blk.begin || a + 16 > (int64_t)blk.last) {
+          // the ends: bytes outside the member count as zeros
+#pragma unroll
+          for (int k = 0; k < 16; k++) {
+            const bool in = a + k >= (int64_t)blk.begin && a + k < (int64_t)blk.last;
+            const uint32_t byte = in ? out[a + k] : 0u;
+            wd[k >> 2] = (wd[k >> 2] & ~(0xFFu << (8 * (k & 3)))) | byte << (8 * (k & 3));
+          }
+        }
 #pragma unroll
         for (int k = 0; k < 4; k++) {
           c = crc_byte(ltab, lane, c, wd[k]);
@@ -342,45 +279,59 @@ __global__ void __launch_bounds__(kCrcThreads)
           c = crc_byte(ltab, lane, c, wd[k] >> 16);
           c = crc_byte(ltab, lane, c, wd[k] >> 24);
         }
-        q += 16;
-        if (!more) break;
-        w = nx;
       }
     }
-    while (q < s1) c = crc_byte(ltab, lane, c, *q++);
-    // slices merge: 2^j slices on each side at level j
+    __syncwarp();
+    // slices merge: 2^j slices on each side at level j, first in the warps
 #pragma unroll
     for (int j = 0; j < 5; j++) {
       const uint32_t r = __shfl_down_sync(0xFFFFFFFFu, c, 1 << j);
       if ((lane & ((2 << j) - 1)) == 0) c = crc_shift(shf, c, j) ^ r;
     }
-    // move the block's register past the rest of its member
-    const uint32_t xp = x_pow_8n_warp(mem_end[blk.member] - (blk.off + blk.len), lane);
-    if (lane == 0) atomicXor(mem_raw + blk.member, gf2_mulmod(xp, c));
+    // then the warps' registers, by one warp (another one each block)
+    if (lane == 0) part[(turn & 1) * kWarps + warp] = c;
+    __syncthreads();
+    if (warp == (int)(turn % kWarps)) {
+      c = lane < kWarps ? part[(turn & 1) * kWarps + lane] : 0u;
+#pragma unroll
+      for (int j = 0; (1 << j) < kWarps; j++) {
+        const uint32_t r = __shfl_down_sync(0xFFFFFFFFu, c, 1 << j);
+        if ((lane & ((2 << j) - 1)) == 0) c = crc_shift(shf, c, 5 + j) ^ r;
+      }
+      if (blk.after) {
+        const uint32_t xp = x_pow_8n_warp(blk.after, lane);
+        c = gf2_mulmod(xp, c);
+      }
+      if (lane == 0) atomicXor(mem_raw + blk.member, c);
+    }
   }
 }
 
-// one thread per member: its CRC from the accumulated blocks, checked with
-// the trailer's CRC32 and ISIZE
+// one warp per member: its CRC from the accumulated blocks, checked with the
+// trailer's CRC32 and ISIZE.  mem_end: the output offset past its last byte.
 __global__ void member_check_kernel(const uint64_t* __restrict__ mem_trailer,
-                                    const uint64_t* __restrict__ mem_len, uint32_t n_mem,
+                                    const uint64_t* __restrict__ mem_len,
+                                    const uint64_t* __restrict__ mem_end, uint32_t n_mem,
                                     const uint8_t* __restrict__ in,
-                                    const uint32_t* __restrict__ mem_raw,
-                                    uint32_t* __restrict__ mem_crc, int32_t* __restrict__ mem_status) {
-  const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
+                                    const uint32_t* __restrict__ mem_raw, int32_t* __restrict__ mem_status) {
+  const uint32_t m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
   if (m >= n_mem) return;
-  const uint64_t t = mem_trailer[m];
+  const uint64_t t = mem_trailer[m], len = mem_len[m];
   int32_t st = kOk;
-  uint32_t crc = 0;
   if (t != kNoTrailer) {
-    crc = ~(gf2_mulmod(x_pow_8n(mem_len[m]), 0xFFFFFFFFu) ^ mem_raw[m]);
+    // the register ran over `pad` zero bytes past the member; x^(2^32 - 1) = 1
+    // mod P, so x^(8 (2^32 - 1 - pad)) takes them back
+    const uint32_t pad = (uint32_t)(0 - mem_end[m]) & 15;
+    uint32_t raw = mem_raw[m];
+    if (pad) raw = gf2_mulmod(x_pow_8n_warp(0xFFFFFFFFull - pad, lane), raw);
+    const uint32_t crc = ~(gf2_mulmod(x_pow_8n_warp(len, lane), 0xFFFFFFFFu) ^ raw);
     const uint32_t ecrc = in[t] | (in[t + 1] << 8) | ((uint32_t)in[t + 2] << 16) | ((uint32_t)in[t + 3] << 24);
     const uint32_t eisz = in[t + 4] | (in[t + 5] << 8) | ((uint32_t)in[t + 6] << 16) | ((uint32_t)in[t + 7] << 24);
-    if ((uint32_t)mem_len[m] != eisz) st = kSizeMismatch;
+    if ((uint32_t)len != eisz) st = kSizeMismatch;
     else if (crc != ecrc) st = kCrcMismatch;
   }
-  mem_crc[m] = crc;
-  mem_status[m] = st;
+  if (lane == 0) mem_status[m] = st;
 }
 
 cudaError_t resolve_init(cudaStream_t stream) {
@@ -392,46 +343,28 @@ cudaError_t resolve_init(cudaStream_t stream) {
                               (int)kCrcSmem);
 }
 
-cudaError_t launch_tail_literals(const PlacedChunk* placed, uint32_t n, const ChunkResult* results,
-                                 const PagePool& pool, uint8_t* out, cudaStream_t stream) {
-  if (!n) return cudaSuccess;
-  tail_literals_kernel<<<n, 256, 0, stream>>>(placed, n, results, pool, out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_tail_markers(const PlacedChunk* placed, const uint32_t* list, uint32_t n_list,
-                                const ChunkResult* results, const PagePool& pool, uint8_t* out,
-                                int sms, cudaStream_t stream) {
-  if (!n_list) return cudaSuccess;
-  const uint32_t grid = n_list < (uint32_t)(sms * 8) ? n_list : (uint32_t)(sms * 8);
-  tail_markers_kernel<<<grid, 256, 0, stream>>>(placed, list, n_list, results, pool, out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_body(const PlacedChunk* placed, const uint32_t* placed_of_chunk,
-                        uint32_t n_pages, const ChunkResult* results, const PagePool& pool,
-                        uint8_t* out, int sms, cudaStream_t stream) {
+cudaError_t launch_resolve(const PlacedChunk* placed, const uint32_t* placed_of_chunk,
+                           uint32_t n_pages, const ChunkResult* results, const PagePool& pool,
+                           uint8_t* out, int sms, cudaStream_t stream) {
   if (!n_pages) return cudaSuccess;
-  uint32_t blocks = n_pages < (uint32_t)(sms * 8) ? n_pages : (uint32_t)(sms * 8);
-  body_kernel<<<blocks, 512, 0, stream>>>(placed, placed_of_chunk, n_pages, results, pool, out);
+  const uint64_t units = (uint64_t)n_pages * (kPageEntries / kResolveUnit);
+  const uint32_t grid = (uint32_t)min(units, (uint64_t)sms * 8);
+  resolve_kernel<<<grid, kResolveThreads, 0, stream>>>(placed, placed_of_chunk, n_pages, results, pool, out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_crc(const CrcBlock* blocks, uint32_t n_blocks, const uint8_t* out,
                        const uint64_t* mem_end, uint32_t* mem_raw, const uint64_t* mem_trailer,
                        const uint64_t* mem_len, uint32_t n_mem, const uint8_t* in,
-                       uint32_t* mem_crc, int32_t* mem_status, int sms, cudaStream_t stream) {
+                       int32_t* mem_status, int sms, cudaStream_t stream) {
   if (n_blocks) {
-    const uint32_t warps_per_cta = kCrcThreads / 32;
-    const uint32_t need = (n_blocks + warps_per_cta - 1) / warps_per_cta;
     const uint32_t cap = (uint32_t)sms * kCrcCtasPerSm;
-    const uint32_t grid = need < cap ? need : cap;
-    crc_blocks_kernel<<<grid, kCrcThreads, kCrcSmem, stream>>>(blocks, n_blocks, out, mem_end,
-                                                               mem_raw);
+    const uint32_t grid = n_blocks < cap ? n_blocks : cap;
+    crc_blocks_kernel<<<grid, kCrcThreads, kCrcSmem, stream>>>(blocks, n_blocks, out, mem_raw);
   }
   if (n_mem)
-    member_check_kernel<<<(n_mem + 255) / 256, 256, 0, stream>>>(mem_trailer, mem_len, n_mem, in,
-                                                                  mem_raw, mem_crc, mem_status);
+    member_check_kernel<<<(n_mem + 7) / 8, 256, 0, stream>>>(mem_trailer, mem_len, mem_end, n_mem, in,
+                                                            mem_raw, mem_status);
   return cudaGetLastError();
 }
 
