@@ -28,27 +28,39 @@
 
 namespace gzgpu {
 
-// entry q of placed chunk c, one of its last 32 Ki: its last page or the one before
-__device__ __forceinline__ const uint16_t* tail_entry(const PlacedChunk& c, uint64_t q,
-                                                      const PagePool& pool) {
-  const uint32_t page = (uint32_t)(q >> 16) == c.last_seq ? c.last_page : c.prev_page;
-  return pool.data + (size_t)page * kPageEntries + (q & (kPageEntries - 1));
+// A chunk before a unit's own: how many bytes before that one it starts, its
+// last page's index, and its last two pages.
+struct NearChunk {
+  uint32_t start, last_seq, last_page, prev_page;
+};
+constexpr uint32_t kNear = 8;  // kept at hand
+
+__device__ __forceinline__ NearChunk near_chunk(const PlacedChunk& c, uint64_t off) {
+  return NearChunk{(uint32_t)min(off - c.out_off, (uint64_t)0xFFFFFFFFu), c.last_seq, c.last_page, c.prev_page};
 }
 
-// The byte of marker v of a chunk that starts at `off`, placed[j] or a later
-// one of its member (`moff`: the member's first byte); from there back.
-__device__ uint32_t follow_marker(const PlacedChunk* __restrict__ placed, uint32_t j, uint64_t off,
-                                  uint64_t moff, uint32_t v, const PagePool& pool) {
+// The byte that marker v of placed chunk k names, `room` bytes after its
+// member's first.  Distances count back from the chunk's start: v names the
+// byte 65536 - v before it; an entry found there that is a marker of its own
+// chunk counts on from that chunk's start.  (A chunk further back than 32 bits
+// count lies past the reach of any window but one of chunks without bytes.)
+__device__ __forceinline__ uint32_t follow_marker(const PlacedChunk* __restrict__ placed,
+                                                  const NearChunk* near, uint32_t k, uint64_t off,
+                                                  uint64_t room, uint32_t v, const PagePool& pool) {
+  uint32_t at = 0, back = 0;  // the chunk the marker belongs to: where it starts, which it is
   for (;;) {
-    const int64_t src = (int64_t)off - (int64_t)kWindow + (int64_t)(v - kMarkerBase);
-    if (src < (int64_t)moff) return 0;  // before the member: the zero window
+    at += 2 * kMarkerBase - v;
+    if (at > room) return 0;  // before the member: the zero window
+    NearChunk c;
     do {
-      j--;
-    } while ((int64_t)placed[j].out_off > src);
-    const PlacedChunk c = placed[j];
-    v = *tail_entry(c, (uint64_t)src - c.out_off, pool);
+      c = back < kNear ? near[back] : near_chunk(placed[k - 1 - back], off);
+      back++;
+    } while (c.start < at);
+    const uint32_t q = c.start - at;  // the entry, one of its last 32 Ki
+    const uint32_t page = (q >> 16) == c.last_seq ? c.last_page : c.prev_page;
+    v = pool.data[(size_t)page * kPageEntries + (q & (kPageEntries - 1))];
     if (v < kMarkerBase) return v;
-    off = c.out_off;  // a marker of chunk j: its window is before chunk j
+    at = c.start;
   }
 }
 
@@ -70,10 +82,13 @@ __global__ void __launch_bounds__(kResolveThreads)
   __shared__ alignas(16) uint8_t bytes[kResolveUnit + 16];
   __shared__ uint32_t list[kResolveUnit];  // entry << 16 | marker
   __shared__ uint32_t n_list;
+  __shared__ NearChunk near[kNear];  // the chunks before the unit's, nearest first
   const uint32_t tid = threadIdx.x;
   const int lane = tid & 31;
   for (uint32_t u = blockIdx.x; u < n_pages * kUnits; u += gridDim.x) {
-    const uint32_t p = u / kUnits, first = (u % kUnits) * kResolveUnit;
+    // the first unit of every page, then the second, ...: markers thin out along
+    // a chunk, and a CTA must not get the same unit of every page
+    const uint32_t p = u % n_pages, first = (u / n_pages) * kResolveUnit;
     const uint32_t cid = pool.owner[p], sw = pool.seq[p];
     const uint32_t k = placed_of_chunk[cid];
     if (k == 0xFFFFFFFFu) continue;
@@ -85,6 +100,7 @@ __global__ void __launch_bounds__(kResolveThreads)
     const uint16_t* src = pool.data + (size_t)p * kPageEntries + first;
     __syncthreads();  // the unit before has left
     if (tid == 0) n_list = 0;
+    if (tid < kNear && tid < k) near[tid] = near_chunk(placed[k - 1 - tid], off);
     uint4 x[2];
 #pragma unroll
     for (uint32_t s = 0; s < 2; s++) {
@@ -118,7 +134,8 @@ __global__ void __launch_bounds__(kResolveThreads)
     }
     __syncthreads();
     for (uint32_t i = tid; i < n_list; i += kResolveThreads)
-      bytes[list[i] >> 16] = (uint8_t)follow_marker(placed, k, off, moff, list[i] & 0xFFFFu, pool);
+      bytes[list[i] >> 16] =
+          (uint8_t)follow_marker(placed, near, k, off, off - moff, list[i] & 0xFFFFu, pool);
     __syncthreads();
     // the unit's bytes, by aligned 16 of the output (one more than the unit's length needs)
     const uint64_t d0 = off + q0;
