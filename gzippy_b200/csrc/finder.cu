@@ -104,7 +104,7 @@ __device__ const LeafLut d_leaf_lut = LeafLut();
 // to shared memory; its bit offsets are screened in passes of 4096: the
 // 13-bit filter for 32 offsets per lane at once, the survivors (1 in 9) to a
 // list, the precode leaf count for 32 of them at a time; what is left
-// (about 1 in 200 of the list) gets the full header test, one per lane.
+// (about 1 in 100 of the list, in order) gets the full header test.
 constexpr int kFindWarps = 8;
 constexpr uint32_t kFindSeg = 8192;                // bits per segment
 constexpr uint32_t kFindPass = 4096;               // bits per screening pass
@@ -115,8 +115,142 @@ struct FindWarp {
   uint32_t w[kFindSeg / 32 + 6];
   uint16_t list[kFindList];
   uint16_t full[kFindFull];
+  uint8_t sorted[32];  // dyn_candidate_warp: the precode's symbols in code order
+  uint8_t lut[128];    // and its table, entry: symbol | length << 5
   uint32_t n_full;
 };
+
+// dyn_candidate_full (finder_core.cuh) by a whole warp, for one candidate.
+// Every lane decodes the code length that would start at its bit of the next
+// 32; a walk over shuffles picks the real ones (about nine), which are then
+// weighed together.  A true header is 200 and more lengths one after another,
+// 90,000 cycles and more for a thread by itself, 15,000 so; a false one ends
+// within two or three such steps.
+__device__ __noinline__ bool dyn_candidate_warp(const uint8_t* in, uint64_t nbytes, uint64_t bit,
+                                                FindWarp& W, int lane) {
+  constexpr uint32_t kAll = 0xFFFFFFFFu;
+  const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
+  const uint32_t below = (1u << lane) - 1;
+  const uint32_t h = (uint32_t)peek_bits(in, nbytes, bit, 17);
+  const uint32_t hl = 257 + ((h >> 3) & 31), total = hl + 1 + ((h >> 8) & 31);
+  const int pc = (int)((h >> 13) & 15) + 4;
+  const uint64_t pos0 = bit + 17 + 3 * pc;  // first bit of the code lengths
+  uint64_t wbase = pos0 >> 5;
+  uint32_t word = in32[wbase + lane], word2 = in32[wbase + 32 + lane];  // 2048 bits from there on
+  // the precode, canonical: lane s has symbol s
+  const uint64_t pbits = peek_bits(in, nbytes, bit + 17, 3 * pc);
+  const int place = lane < 16 ? (lane == 0 ? 3 : (lane < 8 ? 19 - 2 * lane : 2 * lane - 12)) : lane - 16;
+  const uint32_t my = lane < 19 ? (uint32_t)(pbits >> (3 * place)) & 7 : 0u;
+  uint32_t lim[8], base[8];
+  {
+    uint32_t code = 0, off = 0, c = 0, leaves = 0, at = 0;
+#pragma unroll
+    for (uint32_t l = 1; l < 8; l++) {
+      const uint32_t b = __ballot_sync(kAll, my == l);
+      code = (code + c) << 1;
+      c = __popc(b);
+      lim[l] = (code + c) << (7 - l);
+      base[l] = off - code;
+      if (my == l) at = off + __popc(b & below);
+      off += c;
+      leaves += c << (15 - l);
+    }
+    const uint32_t longer = __ballot_sync(kAll, my > 1);
+    if (!kraft_exact(leaves, longer)) return false;
+    if (my) W.sorted[at] = (uint8_t)lane;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const uint32_t rev = __brev(lane + 32 * k) >> 25;
+    uint32_t L = 1, b = base[1];
+#pragma unroll
+    for (int l = 1; l < 7; l++)
+      if (rev >= lim[l]) {
+        L = l + 1;
+        b = base[l + 1];
+      }
+    W.lut[lane + 32 * k] = rev >= lim[7] ? (uint8_t)0 : (uint8_t)(W.sorted[(rev >> (7 - L)) + b] | L << 5);
+  }
+  __syncwarp();
+  const uint64_t nbits = nbytes * 8;
+  const uint32_t room = pos0 < nbits ? (uint32_t)min(nbits - pos0, (uint64_t)1 << 20) : 0u;
+  uint32_t rel = (uint32_t)(pos0 & 31);  // position, from wbase on
+  uint32_t rel0 = rel;
+  uint32_t n = 0, prev = 0;              // lengths read, the last of them
+  uint32_t lit = 0, dist = 0, lit_gt1 = 0, dist_gt1 = 0, eob = 0;
+  while (n < total) {
+    if (rel >= 1024 + 960) {  // (rare: a header of over 2,000 bits)
+      word = word2;
+      wbase += 32;
+      word2 = in32[wbase + 32 + lane];
+      rel -= 1024;
+      rel0 -= 1024;  // only the difference counts
+    }
+    const uint32_t j = rel >> 5, t = (rel & 31) + lane;
+    const uint32_t wa = __shfl_sync(kAll, j < 32 ? word : word2, j & 31);
+    const uint32_t wb = __shfl_sync(kAll, j + 1 < 32 ? word : word2, (j + 1) & 31);
+    const uint32_t wc = __shfl_sync(kAll, j + 2 < 32 ? word : word2, (j + 2) & 31);
+    const uint32_t x = __funnelshift_r(t < 32 ? wa : wb, t < 32 ? wb : wc, t & 31);
+    const uint32_t e = W.lut[x & 127], L = e >> 5, sym = e & 31;
+    const uint32_t xb = sym < 16 ? 0u : (sym == 16 ? 2u : (sym == 17 ? 3u : 7u));
+    const uint32_t rep = sym < 16 ? 1u : ((x >> L) & ((1u << xb) - 1)) + (sym == 18 ? 11u : 3u);
+    // next length's bit (0x40: no such code), and the one after that
+    const uint32_t nx = L ? lane + L + xb : 0x40u;
+    const uint32_t nx2 = __shfl_sync(kAll, nx, nx & 31);
+    const uint32_t hop = nx | (nx < 32 ? nx2 : 0xFFu) << 8;
+    uint32_t chain = 0, p = 0;
+    for (;;) {
+      const uint32_t v = __shfl_sync(kAll, hop, p), a = v & 0xFF, b = v >> 8;
+      if (a == 0x40) break;  // not a code at p
+      chain |= 1u << p;
+      if (a >= 32) {
+        p = a;
+        break;
+      }
+      if (b == 0x40) {  // not a code at a
+        p = a;
+        break;
+      }
+      chain |= 1u << a;
+      p = b;
+      if (p >= 32) break;
+    }
+    const bool ends = p < 32;  // the chain runs into an invalid code at p
+    const bool on = (chain >> lane) & 1;
+    // a repeat of the one before (16) takes the value of the last other symbol
+    const uint32_t own = __ballot_sync(kAll, on && sym != 16);
+    const uint32_t before = own & (below | 1u << lane);
+    const uint32_t v0 = __shfl_sync(kAll, sym < 16 ? sym : 0u, 31 - __clz(before | 1u));
+    const uint32_t v = before ? v0 : prev;
+    const uint32_t r = on ? rep : 0u;
+    uint32_t at = r;  // lengths up to and with this one
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t u = __shfl_up_sync(kAll, at, d);
+      if (lane >= d) at += u;
+    }
+    const uint32_t i = n + at - r;                 // this one's place
+    const bool use = on && i < total;
+    // bad: a repeat with nothing before it, past the last length, past the input
+    const bool bad = use && ((sym == 16 && i == 0) || i + r > total || rel - rel0 + lane + L + xb > room);
+    const uint32_t n_lit = use && i < hl ? min(r, hl - i) : 0u, n_dist = use ? r - n_lit : 0u;
+    if (__any_sync(kAll, bad)) return false;
+    lit += __reduce_add_sync(kAll, v ? n_lit << (15 - v) : 0u);
+    dist += __reduce_add_sync(kAll, v ? n_dist << (15 - v) : 0u);
+    // Kraft sums only grow: an over-subscribed set fails the final test
+    if (lit > (1u << 15) || dist > (1u << 15)) return false;
+    lit_gt1 |= __ballot_sync(kAll, v > 1 && n_lit);
+    dist_gt1 |= __ballot_sync(kAll, v > 1 && n_dist);
+    eob |= __ballot_sync(kAll, use && v && i <= 256 && 256 < i + r);
+    const uint32_t last = 31 - __clz(chain | 1u);
+    n += __shfl_sync(kAll, at, 31);
+    prev = __shfl_sync(kAll, v, last);
+    if (ends && n < total) return false;
+    rel += p;
+  }
+  return eob && kraft_exact(lit, lit_gt1) && kraft_exact(dist, dist_gt1);
+}
 
 __global__ void __launch_bounds__(32 * kFindWarps)
     find_kernel(const uint8_t* __restrict__ in, const ChunkDesc* __restrict__ descs,
@@ -205,10 +339,8 @@ __global__ void __launch_bounds__(32 * kFindWarps)
         __syncwarp();
         if (n0 + __popc(b) > kFindFull) {
           // (rare) the held ones first
-          for (uint32_t j = lane; j < n0; j += 32) {
-            const uint32_t f = W.full[j];
-            if (f < hit && dyn_candidate_full(in, nbytes, s0 + f)) hit = f;
-          }
+          for (uint32_t j = 0; j < n0 && hit == kFindSeg; j++)
+            if (dyn_candidate_warp(in, nbytes, s0 + W.full[j], W, lane)) hit = W.full[j];
           __syncwarp();
           n0 = 0;
         }
@@ -217,11 +349,9 @@ __global__ void __launch_bounds__(32 * kFindWarps)
         __syncwarp();
       }
       const uint32_t n0 = W.n_full;
-      for (uint32_t j = lane; j < n0; j += 32) {
-        const uint32_t f = W.full[j];
-        if (f < hit && dyn_candidate_full(in, nbytes, s0 + f)) hit = f;
-      }
-      hit = __reduce_min_sync(0xFFFFFFFFu, hit);
+      for (uint32_t j = 0; j < n0 && hit == kFindSeg; j++)
+        if (dyn_candidate_warp(in, nbytes, s0 + W.full[j], W, lane)) hit = W.full[j];
+      __syncwarp();
       if (lane == 0) W.n_full = 0;
       __syncwarp();
     }
