@@ -97,6 +97,54 @@ struct HostPinned {
   }
 };
 
+// Allocator of page-locked host memory, for the tables a job exchanges with
+// the device: a copy from or to it needs no staging by the driver and no wait
+// on the host.  Its users keep their capacity from job to job.  Where no more
+// can be page-locked, plain memory does.
+template <typename T>
+struct PinnedAlloc {
+  using value_type = T;
+  static constexpr size_t kHead = 64;  // before the elements: whether they are page-locked
+  PinnedAlloc() = default;
+  template <typename U>
+  PinnedAlloc(const PinnedAlloc<U>&) {}
+  T* allocate(size_t n) {
+    void* p = nullptr;
+    bool locked = cudaMallocHost(&p, n * sizeof(T) + kHead) == cudaSuccess;
+    if (!locked) {
+      cudaGetLastError();
+      p = ::operator new(n * sizeof(T) + kHead);
+    }
+    *static_cast<bool*>(p) = locked;
+    return reinterpret_cast<T*>(static_cast<char*>(p) + kHead);
+  }
+  void deallocate(T* q, size_t) {
+    void* p = reinterpret_cast<char*>(q) - kHead;
+    if (*static_cast<bool*>(p)) cudaFreeHost(p);
+    else ::operator delete(p);
+  }
+  template <typename U>
+  bool operator==(const PinnedAlloc<U>&) const { return true; }
+  template <typename U>
+  bool operator!=(const PinnedAlloc<U>&) const { return false; }
+};
+template <typename T>
+using PinnedVec = std::vector<T, PinnedAlloc<T>>;
+
+// Byte ranges packed into one page-locked buffer, for one copy to the device.
+struct Pack {
+  PinnedVec<uint8_t>& buf;
+  explicit Pack(PinnedVec<uint8_t>& b) : buf(b) { buf.clear(); }
+  // n bytes of src (zeros when null); returns their offset, 16-byte aligned
+  size_t add(const void* src, size_t n) {
+    const size_t at = (buf.size() + 15) & ~(size_t)15;
+    if (at + n > buf.capacity()) buf.reserve(2 * (at + n) + 4096);
+    buf.resize(at + n);
+    if (src && n) memcpy(buf.data() + at, src, n);
+    return at;
+  }
+};
+
 struct StreamSpec {
   uint64_t off, len;  // byte range in the device input buffer
 };
@@ -183,15 +231,24 @@ struct gzgpu_ctx {
   bool high_priority = false;  // stream at the device's greatest priority
   bool lpt = true;             // decode work list longest-first (else in stream order)
   bool job_raw = false;        // the job's streams are raw DEFLATE (no gzip framing)
-  bool job_sync = true;     // the running job has sync starts (decoder variant)
   int decode_blocks = 0;
+  // Job tables in page-locked memory: uploads (by turns, so that one is filled
+  // while the other may still be on its way), results, and the chunk table,
+  // which also stays as the last job's (diagnostics)
+  PinnedVec<uint8_t> up[2], down;
+  PinnedVec<uint32_t> h_spec;
+  PinnedVec<ChunkDesc> hd, hd_cut;  // hd_cut: the table with its partitions cut finer
+  PinnedVec<ChunkResult> hr;
+  uint32_t n_pages_used = 0;  // pages taken from the pool by the job's decodes
   cudaEvent_t ev[12];
   cudaEvent_t stage_ev[2];  // last DMA of each pinned staging slot
   gzgpu_stats stats{};
   bool crc_ready = false;
 
-  DevBuf in, out, s_off, s_len, info, units, cands, counters, descs, results, spec, work, cost, find;
-  DevBuf pages, owner, seq, placed, placed_of, cblocks, mend, mraw, mtrail, mlen, mstatus;
+  // scan: streams and units to scan, the job's counters, stream headers and
+  // member candidates; plan: everything the resolve and CRC passes read
+  DevBuf in, out, scan, plan, counters, descs, results, spec, work, cost, find;
+  DevBuf pages, owner, seq, mstatus;
   // seek-index builds: the decoder's block log, the checkpoint interval and
   // the serialized index of the last job (gzgpu_build_index)
   DevBuf blk_log;
@@ -202,10 +259,8 @@ struct gzgpu_ctx {
   std::vector<uint8_t> index_bytes;
   HostPinned h_stage;
   std::vector<DevBuf*> all_bufs() {
-    return {&in,     &out,   &s_off,   &s_len,  &info,   &units,   &cands,  &counters, &descs,
-            &results, &spec, &work,    &pages,  &owner,  &seq,     &placed, &placed_of,
-            &cblocks, &mend,  &mraw,   &mtrail, &mlen,    &mstatus, &blk_log,
-            &cost,  &find};
+    return {&in,   &out,  &scan,  &plan,  &counters, &descs, &results, &spec,
+            &work, &cost, &find,  &pages, &owner,    &seq,   &mstatus, &blk_log};
   }
   const uint8_t* cur_in = nullptr;  // input buffer of the running job
   uint8_t* user_out = nullptr;       // caller device output (device-resident API)
@@ -240,23 +295,26 @@ struct gzgpu_ctx {
       pool.n_blocks = counters.as<uint32_t>() + 8;
       pool.blocks_cap = blk_cap;
     }
-    cudaError_t e = cudaMemsetAsync(counters.as<uint32_t>() + 3, 0, 4, st);
-    if (e != cudaSuccess) return e;
+    // the work counter: zero at the start of a job
+    if (stats.decode_passes) {
+      const cudaError_t e = cudaMemsetAsync(counters.as<uint32_t>() + 3, 0, 4, st);
+      if (e != cudaSuccess) return e;
+    }
     stats.kernel_launches++;
     stats.decode_passes++;
     switch (lut_bits) {
       case 11:
-        return launch_inflate<11>(ring, ctas_per_sm, wide, job_sync, cur_in, descs.as<ChunkDesc>(), results.as<ChunkResult>(),
+        return launch_inflate<11>(ring, ctas_per_sm, wide, cur_in, descs.as<ChunkDesc>(), results.as<ChunkResult>(),
                                   work.as<uint32_t>(), d_work_count, counters.as<uint32_t>() + 3,
-                                  pool, blocks, st);
+                                  counters.as<uint32_t>() + 4, pool, blocks, st);
       case 12:
-        return launch_inflate<12>(ring, ctas_per_sm, wide, job_sync, cur_in, descs.as<ChunkDesc>(), results.as<ChunkResult>(),
+        return launch_inflate<12>(ring, ctas_per_sm, wide, cur_in, descs.as<ChunkDesc>(), results.as<ChunkResult>(),
                                   work.as<uint32_t>(), d_work_count, counters.as<uint32_t>() + 3,
-                                  pool, blocks, st);
+                                  counters.as<uint32_t>() + 4, pool, blocks, st);
       default:
-        return launch_inflate<10>(ring, ctas_per_sm, wide, job_sync, cur_in, descs.as<ChunkDesc>(), results.as<ChunkResult>(),
+        return launch_inflate<10>(ring, ctas_per_sm, wide, cur_in, descs.as<ChunkDesc>(), results.as<ChunkResult>(),
                                   work.as<uint32_t>(), d_work_count, counters.as<uint32_t>() + 3,
-                                  pool, blocks, st);
+                                  counters.as<uint32_t>() + 4, pool, blocks, st);
     }
   }
 
@@ -278,8 +336,10 @@ struct gzgpu_ctx {
                                         std::min(owner.cap, seq.cap) / 4);
   }
   // decode again, in a grown page pool, the chunks of [b, e) that ran out of pages
-  int regrow(std::vector<ChunkDesc>& hd, std::vector<ChunkResult>& hr, uint32_t b, uint32_t e,
-             float& ms_kernel);
+  int regrow(uint32_t b, uint32_t e, float& ms_kernel);
+  // a decode pass's chunks [b, e) (their descriptors too: with_descs) and page
+  // count to the host
+  int fetch_results(uint32_t b, uint32_t e, bool with_descs);
   // run() under the autotuner when it is on
   int job(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R);
   int job_tuned(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R);
@@ -299,9 +359,6 @@ struct gzgpu_ctx {
     setup_decode_grid();
   }
 
-  // chunk tables of the last job (diagnostics)
-  std::vector<ChunkDesc> last_descs;
-  std::vector<ChunkResult> last_results;
 };
 
 // shortest partition of a high-ratio member (8 KiB of compressed input)
@@ -348,6 +405,8 @@ int gzgpu_ctx::job_tuned(const std::vector<StreamSpec>& S, std::vector<StreamOut
   apply(dflt);
   int rc = run(S, R);
   if (rc != kOk || tune_cache.count(last_key)) return rc;
+  // nothing to tune on
+  if (std::all_of(R.begin(), R.end(), [](const StreamOut& r) { return r.status == kNotGzip; })) return rc;
   // Coordinate search, one full decode per candidate (outputs are identical,
   // so any run's result stands): chunk size, then LUT bits, then warps/SM.
   const uint32_t key = last_key;
@@ -392,8 +451,28 @@ int gzgpu_ctx::job_tuned(const std::vector<StreamSpec>& S, std::vector<StreamOut
   return rc;
 }
 
-int gzgpu_ctx::regrow(std::vector<ChunkDesc>& hd, std::vector<ChunkResult>& hr, uint32_t b,
-                      uint32_t e, float& ms_kernel) {
+int gzgpu_ctx::fetch_results(uint32_t b, uint32_t e, bool with_descs) {
+  int rc;
+  if (down.size() < 64) down.resize(4096);
+  if (e > b) {
+    if (with_descs &&
+        (rc = check(cudaMemcpyAsync(hd.data() + b, descs.as<ChunkDesc>() + b, sizeof(ChunkDesc) * (e - b),
+                                    cudaMemcpyDeviceToHost, st))))
+      return rc;
+    if ((rc = check(cudaMemcpyAsync(hr.data() + b, results.as<ChunkResult>() + b,
+                                    sizeof(ChunkResult) * (e - b), cudaMemcpyDeviceToHost, st))))
+      return rc;
+  }
+  if ((rc = check(cudaMemcpyAsync(down.data(), counters.as<uint32_t>() + 2, 4, cudaMemcpyDeviceToHost, st))) ||
+      (rc = check(cudaStreamSynchronize(st))))
+    return rc;
+  uint32_t used;
+  memcpy(&used, down.data(), 4);
+  n_pages_used = std::min(used, pool_cap());
+  return kOk;
+}
+
+int gzgpu_ctx::regrow(uint32_t b, uint32_t e, float& ms_kernel) {
   int rc;
   for (;;) {
     std::vector<uint32_t> ids;
@@ -414,13 +493,8 @@ int gzgpu_ctx::regrow(std::vector<ChunkDesc>& hd, std::vector<ChunkResult>& hr, 
       if ((d.flags >> kGenBaseShift) + 2 * kMaxTries > kGenBaseMax) return kPoolExhausted;
     }
     if (ids.empty()) return kOk;
-    uint32_t used = 0;
-    if ((rc = check(cudaMemcpyAsync(&used, counters.as<uint32_t>() + 2, 4, cudaMemcpyDeviceToHost,
-                                    st))) ||
-        (rc = check(cudaStreamSynchronize(st))))
-      return rc;
     const uint64_t cap0 = pool_cap();
-    used = (uint32_t)std::min<uint64_t>(used, cap0);
+    const uint32_t used = n_pages_used;
     const uint64_t need = std::max<uint64_t>(used + extra + 64, cap0 + cap0 / 4);
     if (need >= kNoPage) return kPoolExhausted;
     if ((rc = check(pages.grow_keep(need * kPageEntries * 2, (uint64_t)used * kPageEntries * 2))) ||
@@ -441,11 +515,7 @@ int gzgpu_ctx::regrow(std::vector<ChunkDesc>& hd, std::vector<ChunkResult>& hr, 
     cudaEventRecord(ev[8], st);
     if ((rc = check(launch_decode(counters.as<uint32_t>() + 1, nw)))) return rc;
     cudaEventRecord(ev[9], st);
-    cudaMemcpyAsync(hd.data() + b, descs.as<ChunkDesc>() + b, sizeof(ChunkDesc) * (e - b),
-                    cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(hr.data() + b, results.as<ChunkResult>() + b, sizeof(ChunkResult) * (e - b),
-                    cudaMemcpyDeviceToHost, st);
-    if ((rc = check(cudaStreamSynchronize(st)))) return rc;
+    if ((rc = fetch_results(b, e, true))) return rc;
     float t = 0;
     cudaEventElapsedTime(&t, ev[8], ev[9]);
     ms_kernel += t;
@@ -475,40 +545,60 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   for (uint32_t s = 0; s < ns; s++)
     for (uint64_t b = 0; b < S[s].len; b += unit)
       units.push_back(ScanUnit{s, 0, b, std::min(S[s].len, b + unit)});
-  if ((rc = check(s_off.ensure(8 * ns))) || (rc = check(s_len.ensure(8 * ns))) ||
-      (rc = check(info.ensure(sizeof(StreamInfo) * ns))) ||
-      (rc = check(units.empty() ? cudaSuccess : this->units.ensure(sizeof(ScanUnit) * units.size()))) ||
-      (rc = check(counters.ensure(64))))
+  // one buffer: what goes up (offsets, lengths, units, a zero), then what comes
+  // down (the candidates' count, the streams' headers, the candidates)
+  const uint32_t cand_cap = (uint32_t)std::min<uint64_t>(total_in / 4096 + 4096, 1u << 22);
+  Pack pa(up[0]);
+  const size_t at_off = pa.add(h_off.data(), 8 * (size_t)ns), at_len = pa.add(h_len.data(), 8 * (size_t)ns);
+  const size_t at_units = pa.add(units.data(), sizeof(ScanUnit) * units.size());
+  const size_t at_count = pa.add(nullptr, 16), at_info = pa.buf.size();
+  const size_t at_cands = at_info + sizeof(StreamInfo) * (size_t)ns;
+  if ((rc = check(scan.ensure(at_cands + sizeof(MemberCand) * (size_t)cand_cap))) ||
+      (rc = check(counters.ensure(64))) || (rc = check(cudaMemsetAsync(counters.p, 0, 64, st))))
     return rc;
-  uint32_t cand_cap = (uint32_t)std::min<uint64_t>(total_in / 4096 + 4096, 1u << 22);
-  if ((rc = check(cands.ensure(sizeof(MemberCand) * cand_cap)))) return rc;
-  cudaMemcpyAsync(s_off.p, h_off.data(), 8 * ns, cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(s_len.p, h_len.data(), 8 * ns, cudaMemcpyHostToDevice, st);
-  if (!units.empty())
-    cudaMemcpyAsync(this->units.p, units.data(), sizeof(ScanUnit) * units.size(),
-                    cudaMemcpyHostToDevice, st);
-  cudaMemsetAsync(counters.p, 0, 64, st);
   std::vector<StreamInfo> hinfo(ns);
-  uint32_t n_cand = 0;
+  std::vector<MemberCand> hc;
   if (job_raw) {
     // raw DEFLATE: no header to check and no members to find; each stream
     // is one member whose data starts at its first bit
     for (StreamInfo& h : hinfo) h = StreamInfo{kOk, 0, 0, 4};
-  } else {
-    if ((rc = check(launch_stream_headers(cur_in, s_off.as<uint64_t>(), s_len.as<uint64_t>(),
-                                          ns, info.as<StreamInfo>(), st))))
+  } else if (!units.empty()) {
+    uint8_t* const d = scan.as<uint8_t>();
+    constexpr uint32_t kFirst = 256;  // candidates that come down with the rest
+    const size_t n_down = at_cands - at_count + sizeof(MemberCand) * std::min(cand_cap, kFirst);
+    if (down.size() < n_down) down.resize(n_down);
+    if ((rc = check(cudaMemcpyAsync(d, pa.buf.data(), pa.buf.size(), cudaMemcpyHostToDevice, st))) ||
+        (rc = check(launch_member_scan(cur_in, reinterpret_cast<ScanUnit*>(d + at_units),
+                                       (uint32_t)units.size(), reinterpret_cast<uint64_t*>(d + at_off),
+                                       reinterpret_cast<uint64_t*>(d + at_len),
+                                       reinterpret_cast<StreamInfo*>(d + at_info),
+                                       reinterpret_cast<MemberCand*>(d + at_cands),
+                                       reinterpret_cast<uint32_t*>(d + at_count), cand_cap, sms, st))) ||
+        (rc = check(cudaMemcpyAsync(down.data(), d + at_count, n_down, cudaMemcpyDeviceToHost, st))) ||
+        (rc = check(cudaStreamSynchronize(st))))
       return rc;
-    if ((rc = check(launch_member_scan(cur_in, this->units.as<ScanUnit>(),
-                                       (uint32_t)units.size(), s_off.as<uint64_t>(),
-                                       s_len.as<uint64_t>(), info.as<StreamInfo>(),
-                                       cands.as<MemberCand>(), counters.as<uint32_t>(), cand_cap,
-                                       sms, st))))
-      return rc;
-    stats.kernel_launches += 2;
-    cudaMemcpyAsync(hinfo.data(), info.p, sizeof(StreamInfo) * ns, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(&n_cand, counters.p, 4, cudaMemcpyDeviceToHost, st);
+    stats.kernel_launches++;
+    uint32_t n_cand;
+    memcpy(&n_cand, down.data(), 4);
+    n_cand = std::min(n_cand, cand_cap);
+    memcpy(hinfo.data(), down.data() + (at_info - at_count), sizeof(StreamInfo) * (size_t)ns);
+    hc.resize(n_cand);
+    if (n_cand) memcpy(hc.data(), down.data() + (at_cands - at_count), sizeof(MemberCand) * std::min(n_cand, kFirst));
+    if (n_cand > kFirst) {
+      const size_t n = sizeof(MemberCand) * (size_t)(n_cand - kFirst);
+      if (down.size() < n) down.resize(n);
+      if ((rc = check(cudaMemcpyAsync(down.data(), d + at_cands + sizeof(MemberCand) * kFirst, n,
+                                      cudaMemcpyDeviceToHost, st))) ||
+          (rc = check(cudaStreamSynchronize(st))))
+        return rc;
+      memcpy(hc.data() + kFirst, down.data(), n);
+    }
+    std::sort(hc.begin(), hc.end(), [](const MemberCand& a, const MemberCand& b) {
+      return a.stream != b.stream ? a.stream < b.stream : a.pos < b.pos;
+    });
   }
-  if ((rc = check(cudaStreamSynchronize(st)))) return rc;
+  for (uint32_t s = 0; s < ns; s++)
+    if (!S[s].len && !job_raw) hinfo[s] = StreamInfo{kNotGzip, 0, 0, 4};
   cudaEventRecord(ev[2], st);
   if (autotune) {
     // the kind of job: compressed size (log2), stream count (log4) and the
@@ -530,15 +620,6 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
       auto it = tune_cache.find(last_key);
       if (it != tune_cache.end()) apply(it->second);
     }
-  }
-  n_cand = std::min(n_cand, cand_cap);
-  std::vector<MemberCand> hc(n_cand);
-  if (n_cand) {
-    cudaMemcpyAsync(hc.data(), cands.p, sizeof(MemberCand) * n_cand, cudaMemcpyDeviceToHost, st);
-    if ((rc = check(cudaStreamSynchronize(st)))) return rc;
-    std::sort(hc.begin(), hc.end(), [](const MemberCand& a, const MemberCand& b) {
-      return a.stream != b.stream ? a.stream < b.stream : a.pos < b.pos;
-    });
   }
   // ---- 2. members + chunk grid (host) -----------------------------------
   struct Mem {
@@ -589,8 +670,10 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
     mems[s] = std::move(ms);
   }
   // grid
-  std::vector<ChunkDesc> hd;
-  std::vector<uint32_t> hspec;
+  hd.clear();
+  hr.clear();
+  PinnedVec<uint32_t>& hspec = h_spec;
+  hspec.clear();
   std::vector<uint32_t> c0(ns), c1(ns);
   std::vector<std::vector<uint32_t>> mc0(ns);  // first grid chunk of each planned member
   uint64_t cb = chunk_bytes ? chunk_bytes : pick_chunk_bytes(total_in);
@@ -598,6 +681,10 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   stats.lut_bits = lut_bits;
   stats.ctas_per_sm = ring ? 0 : ctas_per_sm;
   const uint64_t cbits = cb * 8;
+  size_t n_mems = 0;
+  for (const auto& m : mems) n_mems += m.size();
+  hd.reserve(n_mems + (size_t)(total_in / cb) + 64);  // (page-locked: growing is dear)
+  hspec.reserve((size_t)(total_in / cb) + 64);
   for (uint32_t s = 0; s < ns; s++) {
     c0[s] = (uint32_t)hd.size();
     for (const Mem& m : mems[s]) {
@@ -642,14 +729,13 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   if (n_grid) cudaMemcpyAsync(descs.p, hd.data(), sizeof(ChunkDesc) * n_grid, cudaMemcpyHostToDevice, st);
   if (!hspec.empty())
     cudaMemcpyAsync(spec.p, hspec.data(), 4 * hspec.size(), cudaMemcpyHostToDevice, st);
-  cudaMemsetAsync(counters.as<uint32_t>() + 1, 0, 4, st);
   cudaEventRecord(ev[3], st);
   // ---- 3. finder + link ---------------------------------------------------
   uint32_t* n_sync = counters.as<uint32_t>() + 4;  // sync starts found (zeroed with the scan)
-  if (!hspec.empty() && (rc = check(find.ensure(finder_scratch_bytes((uint32_t)hspec.size())))))
-    return rc;
+  if (!hspec.empty() && (rc = check(find.ensure(8 * hspec.size())))) return rc;
   if ((rc = check(launch_finder(cur_in, descs.as<ChunkDesc>(), spec.as<uint32_t>(),
-                                (uint32_t)hspec.size(), cbits, find.p, n_sync, fine_split, sms, st))))
+                                (uint32_t)hspec.size(), cbits, find.as<uint64_t>(),
+                                counters.as<uint32_t>() + 9, n_sync, fine_split, sms, st))))
     return rc;
   if (!hspec.empty()) stats.kernel_launches += 4;
   // ---- 3a. cut high-ratio partitions finer ---------------------------------
@@ -663,7 +749,8 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
         (rc = check(cudaStreamSynchronize(st))))
       return rc;
     const double target = 2.0 * (double)cb;
-    std::vector<ChunkDesc> hd2;
+    PinnedVec<ChunkDesc>& hd2 = hd_cut;
+    hd2.clear();
     std::vector<uint32_t> newpos(n_grid + 1), hspec2;
     hd2.reserve(n_grid + n_grid / 4);
     for (uint32_t i = 0; i < n_grid; i++) {
@@ -715,9 +802,10 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
         return rc;
       cudaMemcpyAsync(descs.p, hd.data(), sizeof(ChunkDesc) * n_grid, cudaMemcpyHostToDevice, st);
       cudaMemcpyAsync(spec.p, hspec2.data(), 4 * hspec2.size(), cudaMemcpyHostToDevice, st);
-      if ((rc = check(find.ensure(finder_scratch_bytes((uint32_t)hspec2.size())))) ||
+      if ((rc = check(find.ensure(8 * hspec2.size()))) ||
           (rc = check(launch_finder(cur_in, descs.as<ChunkDesc>(), spec.as<uint32_t>(),
-                                    (uint32_t)hspec2.size(), cbits, find.p, n_sync, true, sms, st))))
+                                    (uint32_t)hspec2.size(), cbits, find.as<uint64_t>(),
+                                    counters.as<uint32_t>() + 9, n_sync, true, sms, st))))
         return rc;
       stats.kernel_launches += 4;
     }
@@ -742,16 +830,15 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
                               std::max<uint64_t>(cbits, 1ull << 21), st))))
     return rc;
   stats.kernel_launches += lpt ? 2 : 1;
-  uint32_t n_decode = 0;  // chunks with a start
-  {
-    // the decoder variant without sync-start handling when there are none
-    // and how many chunks there are to decode: counters[1 .. 4]
-    uint32_t h_cnt[4] = {0, 0, 0, 1};
-    if ((rc = check(cudaMemcpyAsync(h_cnt, counters.as<uint32_t>() + 1, 16, cudaMemcpyDeviceToHost, st))) ||
+  // Chunks with a start, which decides how the decode is launched.  A grid
+  // small enough for wide CTAs needs no count.
+  uint32_t n_decode = n_grid;
+  if (n_grid > 2 * (uint32_t)sms) {
+    if (down.size() < 4096) down.resize(4096);
+    if ((rc = check(cudaMemcpyAsync(down.data(), counters.as<uint32_t>() + 1, 4, cudaMemcpyDeviceToHost, st))) ||
         (rc = check(cudaStreamSynchronize(st))))
       return rc;
-    job_sync = h_cnt[3] != 0;
-    n_decode = h_cnt[0];
+    memcpy(&n_decode, down.data(), 4);
   }
   cudaEventRecord(ev[4], st);
   // ---- 4. decode ----------------------------------------------------------
@@ -760,33 +847,26 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   // none): the chunks that run out of pages are decoded again in a grown
   // pool, the others keep theirs (regrow).
   uint64_t pages_needed = (est_out + n_grid * (uint64_t)kPageEntries) / kPageEntries + 64;
-  std::vector<ChunkResult> hr;
   float ms_dec_kernel = 0;
   {
     if ((rc = check(pages.ensure(pages_needed * kPageEntries * 2))) ||
         (rc = check(owner.ensure(4 * pages_needed))) || (rc = check(seq.ensure(4 * pages_needed))))
       return rc;
-    cudaMemsetAsync(counters.as<uint32_t>() + 2, 0, 4, st);
     if (job_index) {
       blk_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(blk_need, total_in / 64 + 65536),
                                              1u << 30);
       if ((rc = check(blk_log.ensure(sizeof(BlockRec) * (uint64_t)blk_cap)))) return rc;
-      cudaMemsetAsync(counters.as<uint32_t>() + 8, 0, 4, st);
     }
     cudaEventRecord(ev[8], st);
     if ((rc = check(launch_decode(counters.as<uint32_t>() + 1, n_decode)))) return rc;
     cudaEventRecord(ev[9], st);
     hd.resize(n_grid);
     hr.resize(n_grid);
-    if (n_grid) {
-      cudaMemcpyAsync(hd.data(), descs.p, sizeof(ChunkDesc) * n_grid, cudaMemcpyDeviceToHost, st);
-      cudaMemcpyAsync(hr.data(), results.p, sizeof(ChunkResult) * n_grid, cudaMemcpyDeviceToHost, st);
-    }
-    if ((rc = check(cudaStreamSynchronize(st)))) return rc;
+    if ((rc = fetch_results(0, n_grid, true))) return rc;
     float t = 0;
     cudaEventElapsedTime(&t, ev[8], ev[9]);
     ms_dec_kernel += t;
-    if ((rc = regrow(hd, hr, 0, n_grid, ms_dec_kernel))) return rc;
+    if ((rc = regrow(0, n_grid, ms_dec_kernel))) return rc;
   }
   cudaEventRecord(ev[5], st);
   // ---- 5. chain walk with repairs (host) ---------------------------------
@@ -1045,13 +1125,11 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
     cudaEventRecord(ev[9], st);
     hd.insert(hd.end(), repairs.begin(), repairs.end());
     hr.resize(hd.size());
-    cudaMemcpyAsync(hr.data() + base_id, results.as<ChunkResult>() + base_id,
-                    sizeof(ChunkResult) * nr, cudaMemcpyDeviceToHost, st);
-    if ((rc = check(cudaStreamSynchronize(st)))) return rc;
+    if ((rc = fetch_results(base_id, base_id + nr, false))) return rc;
     float t = 0;
     cudaEventElapsedTime(&t, ev[8], ev[9]);
     ms_dec_kernel += t;
-    if ((rc = regrow(hd, hr, base_id, base_id + nr, ms_dec_kernel))) return rc;
+    if ((rc = regrow(base_id, base_id + nr, ms_dec_kernel))) return rc;
     for (auto& sw : SW) {
       for (Walker& w : sw) {
         if (w.pending >= 0) {
@@ -1086,8 +1164,6 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   }
   stats.n_rejected = n_rejected;
   stats.n_repairs = n_repairs;
-  last_descs = hd;
-  last_results = hr;
   // ---- output placement ----------------------------------------------------
   const uint32_t n_all = (uint32_t)hd.size();
   std::vector<PlacedChunk> placed;
@@ -1136,56 +1212,55 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   stats.out_bytes = out_total;
   cudaEventRecord(ev[6], st);
   // ---- 6. resolve + CRC ----------------------------------------------------
-  uint32_t n_pages_used = 0;
-  cudaMemcpyAsync(&n_pages_used, counters.as<uint32_t>() + 2, 4, cudaMemcpyDeviceToHost, st);
-  if ((rc = check(cudaStreamSynchronize(st)))) return rc;
-  const uint32_t pcap = pool_cap();
-  n_pages_used = std::min(n_pages_used, pcap);
   stats.n_pages = n_pages_used;
   cur_out = (user_out && out_total <= user_cap) ? user_out : nullptr;
+  // everything the passes read, in one copy
+  Pack pc(up[1]);
+  const size_t at_placed = pc.add(placed.data(), sizeof(PlacedChunk) * placed.size());
+  const size_t at_pof = pc.add(placed_of.data(), 4 * placed_of.size());
+  const size_t at_cblk = pc.add(cblk.data(), sizeof(CrcBlock) * cblk.size());
+  const size_t at_mtrail = pc.add(mtrail.data(), 8 * mtrail.size());
+  const size_t at_mlen = pc.add(mlenv.data(), 8 * mlenv.size());
+  const size_t at_mend = pc.add(mendv.data(), 8 * mendv.size());
+  const size_t at_mraw = pc.add(nullptr, 4 * mtrail.size());
   if ((rc = check(cur_out ? cudaSuccess : out.ensure(out_total + 64))) ||
-      (rc = check(this->placed.ensure(sizeof(PlacedChunk) * (placed.size() + 1)))) ||
-      (rc = check(this->placed_of.ensure(4 * (n_all + 1)))) ||
-      (rc = check(cblocks.ensure(sizeof(CrcBlock) * (cblk.size() + 1)))) ||
-      (rc = check(mend.ensure(8 * (mendv.size() + 1)))) || (rc = check(mraw.ensure(4 * (mtrail.size() + 1)))) ||
-      (rc = check(this->mtrail.ensure(8 * (mtrail.size() + 1)))) || (rc = check(mlen.ensure(8 * (mlenv.size() + 1)))) ||
+      (rc = check(plan.ensure(pc.buf.size() + 16))) ||
       (rc = check(mstatus.ensure(4 * (mtrail.size() + 1)))))
     return rc;
-  if (!placed.empty())
-    cudaMemcpyAsync(this->placed.p, placed.data(), sizeof(PlacedChunk) * placed.size(),
-                    cudaMemcpyHostToDevice, st);
-  if (n_all) cudaMemcpyAsync(this->placed_of.p, placed_of.data(), 4 * n_all, cudaMemcpyHostToDevice, st);
-  if (!cblk.empty())
-    cudaMemcpyAsync(cblocks.p, cblk.data(), sizeof(CrcBlock) * cblk.size(), cudaMemcpyHostToDevice, st);
-  if (!mtrail.empty()) {
-    cudaMemcpyAsync(this->mtrail.p, mtrail.data(), 8 * mtrail.size(), cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(mlen.p, mlenv.data(), 8 * mlenv.size(), cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(mend.p, mendv.data(), 8 * mendv.size(), cudaMemcpyHostToDevice, st);
-    cudaMemsetAsync(mraw.p, 0, 4 * mtrail.size(), st);
-  }
+  if (!pc.buf.empty() &&
+      (rc = check(cudaMemcpyAsync(plan.p, pc.buf.data(), pc.buf.size(), cudaMemcpyHostToDevice, st))))
+    return rc;
+  uint8_t* const d_plan = plan.as<uint8_t>();
   if (!cur_out) cur_out = out.as<uint8_t>();
   PagePool pool{pages.as<uint16_t>(), owner.as<uint32_t>(), seq.as<uint32_t>(),
-                counters.as<uint32_t>() + 2, pcap};
+                counters.as<uint32_t>() + 2, pool_cap()};
   cudaEventRecord(ev[10], st);
   if (!crc_ready) {
     if ((rc = check(resolve_init(st)))) return rc;
     crc_ready = true;
   }
-  if ((rc = check(launch_resolve(this->placed.as<PlacedChunk>(), this->placed_of.as<uint32_t>(),
-                                 n_pages_used, results.as<ChunkResult>(), pool, cur_out, sms, st))))
+  if ((rc = check(launch_resolve(reinterpret_cast<PlacedChunk*>(d_plan + at_placed),
+                                 reinterpret_cast<uint32_t*>(d_plan + at_pof), n_pages_used,
+                                 results.as<ChunkResult>(), pool, cur_out, sms, st))))
     return rc;
   cudaEventRecord(ev[11], st);
-  if ((rc = check(launch_crc(cblocks.as<CrcBlock>(), (uint32_t)cblk.size(), cur_out,
-                             mend.as<uint64_t>(), mraw.as<uint32_t>(),
-                             this->mtrail.as<uint64_t>(), mlen.as<uint64_t>(),
-                             (uint32_t)mtrail.size(), cur_in, mstatus.as<int32_t>(), sms, st))))
+  if ((rc = check(launch_crc(reinterpret_cast<CrcBlock*>(d_plan + at_cblk), (uint32_t)cblk.size(), cur_out,
+                             reinterpret_cast<uint64_t*>(d_plan + at_mend),
+                             reinterpret_cast<uint32_t*>(d_plan + at_mraw),
+                             reinterpret_cast<uint64_t*>(d_plan + at_mtrail),
+                             reinterpret_cast<uint64_t*>(d_plan + at_mlen), (uint32_t)mtrail.size(),
+                             cur_in, mstatus.as<int32_t>(), sms, st))))
     return rc;
   stats.kernel_launches += 3;
   std::vector<int32_t> mst(mtrail.size());
-  if (!mst.empty())
-    cudaMemcpyAsync(mst.data(), mstatus.p, 4 * mst.size(), cudaMemcpyDeviceToHost, st);
+  if (!mst.empty()) {
+    if (down.size() < 4 * mst.size()) down.resize(4 * mst.size());
+    if ((rc = check(cudaMemcpyAsync(down.data(), mstatus.p, 4 * mst.size(), cudaMemcpyDeviceToHost, st))))
+      return rc;
+  }
   cudaEventRecord(ev[7], st);
   if ((rc = check(cudaStreamSynchronize(st)))) return rc;
+  if (!mst.empty()) memcpy(mst.data(), down.data(), 4 * mst.size());
   {
     size_t mi = 0;
     for (uint32_t s = 0; s < ns; s++) {
@@ -1628,10 +1703,7 @@ int gzgpu_decompress_device(gzgpu_ctx* c, const void* d_in, size_t in_len, void*
   reset_stats(c);
   if ((reinterpret_cast<uintptr_t>(d_in) | reinterpret_cast<uintptr_t>(d_out)) & 15)
     return GZGPU_INVALID_ARGUMENT;  // the kernels use 16-byte vector access
-  uint8_t magic[2] = {0, 0};
-  if (in_len >= 2 && c->check(cudaMemcpy(magic, d_in, 2, cudaMemcpyDeviceToHost)))
-    return GZGPU_DEVICE_ERROR;
-  if (in_len < 2 || magic[0] != 0x1f || magic[1] != 0x8b) return GZGPU_NOT_GZIP;
+  if (in_len < 2) return GZGPU_NOT_GZIP;  // (the scan looks at the magic)
   cudaEventRecord(c->ev[0], c->st);
   c->cur_in = reinterpret_cast<const uint8_t*>(d_in);
   c->user_out = reinterpret_cast<uint8_t*>(d_out);
@@ -1866,10 +1938,11 @@ int gzgpu_debug_find(gzgpu_ctx* c, const uint8_t* in, size_t in_len, const uint6
     cudaMemcpyAsync(c->spec.p, sp.data(), 4 * n, cudaMemcpyHostToDevice, c->st);
     uint64_t most = 0;
     for (size_t i = 0; i < n; i++) most = std::max(most, to[i] > from[i] ? to[i] - from[i] : 0);
-    if ((rc = c->check(c->find.ensure(finder_scratch_bytes((uint32_t)n)))) ||
+    if ((rc = c->check(c->find.ensure(8 * n))) || (rc = c->check(c->counters.ensure(64))) ||
+        (rc = c->check(cudaMemsetAsync(c->counters.p, 0, 64, c->st))) ||
         (rc = c->check(launch_finder(c->in.as<uint8_t>(), c->descs.as<ChunkDesc>(),
-                                     c->spec.as<uint32_t>(), (uint32_t)n, most, c->find.p, nullptr,
-                                     false, c->sms, c->st))))
+                                     c->spec.as<uint32_t>(), (uint32_t)n, most, c->find.as<uint64_t>(),
+                                     c->counters.as<uint32_t>() + 9, nullptr, false, c->sms, c->st))))
       return rc;
     cudaMemcpyAsync(d.data(), c->descs.p, sizeof(ChunkDesc) * n, cudaMemcpyDeviceToHost, c->st);
   }
@@ -1975,8 +2048,9 @@ int gzgpu_debug_decode(gzgpu_ctx* c, const uint8_t* in, size_t in_len, const uin
   }
   cudaMemcpyAsync(c->counters.as<uint32_t>() + 1, &nn, 4, cudaMemcpyHostToDevice, c->st);
   c->cur_in = c->in.as<uint8_t>();
-  c->job_sync = false;
-  for (size_t i = 0; i < n; i++) c->job_sync |= (d[i].flags & kChunkSync) != 0;
+  uint32_t n_sync = 0;
+  for (size_t i = 0; i < n; i++) n_sync += (d[i].flags & kChunkSync) != 0;
+  cudaMemcpyAsync(c->counters.as<uint32_t>() + 4, &n_sync, 4, cudaMemcpyHostToDevice, c->st);
   if ((rc = c->check(c->launch_decode(c->counters.as<uint32_t>() + 1, (uint32_t)n)))) return rc;
   std::vector<ChunkResult> r(n);
   uint32_t used = 0;
@@ -2018,10 +2092,10 @@ int gzgpu_debug_decode(gzgpu_ctx* c, const uint8_t* in, size_t in_len, const uin
 int gzgpu_debug_last_chunks(gzgpu_ctx* c, void* descs, void* results, size_t cap, size_t* n) {
   if (!c || !n) return GZGPU_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> g(c->mu);
-  *n = c->last_descs.size();
-  size_t k = std::min(cap, c->last_descs.size());
-  if (descs && k) memcpy(descs, c->last_descs.data(), k * sizeof(ChunkDesc));
-  if (results && k) memcpy(results, c->last_results.data(), k * sizeof(ChunkResult));
+  *n = c->hr.size();
+  size_t k = std::min(cap, c->hr.size());
+  if (descs && k) memcpy(descs, c->hd.data(), k * sizeof(ChunkDesc));
+  if (results && k) memcpy(results, c->hr.data(), k * sizeof(ChunkResult));
   return GZGPU_OK;
 }
 

@@ -29,9 +29,10 @@ constexpr int kStoredThreads = 256;
 
 __global__ void __launch_bounds__(kStoredThreads)
     stored_kernel(const uint8_t* __restrict__ in, ChunkDesc* descs,
-                  const uint32_t* __restrict__ spec, uint32_t n_spec) {
+                  const uint32_t* __restrict__ spec, uint32_t n_spec, unsigned long long* best) {
   __shared__ unsigned long long s_first;
   if (blockIdx.x >= n_spec) return;
+  if (threadIdx.x == 0) best[blockIdx.x] = ~0ull;  // for find_kernel
   ChunkDesc& d = descs[spec[blockIdx.x]];
   if (d.flags & kChunkValid) return;
   const uint64_t from = d.guess_bit, to = d.limit_bit, nbytes = d.in_end;
@@ -363,8 +364,10 @@ __global__ void __launch_bounds__(32 * kFindWarps)
 // estimate of their headers
 __global__ void assign_kernel(const uint8_t* __restrict__ in, ChunkDesc* descs,
                               const uint32_t* __restrict__ spec, uint32_t n_spec,
-                              const unsigned long long* __restrict__ best, int ratio) {
+                              const unsigned long long* __restrict__ best, int ratio,
+                              uint32_t* next_item) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k == 0) *next_item = 0;
   if (k >= n_spec) return;
   ChunkDesc& d = descs[spec[k]];
   if ((d.flags & kChunkValid) || best[k] == ~0ull) return;
@@ -538,29 +541,23 @@ __global__ void __launch_bounds__(1024)
     if (descs[i].flags & kChunkValid) work[atomicAdd(&base[bucket(i)], 1u)] = i;
 }
 
-size_t finder_scratch_bytes(uint32_t n_spec) { return 8 * (size_t)n_spec + 8; }
-
 cudaError_t launch_finder(const uint8_t* in, ChunkDesc* descs, const uint32_t* spec, uint32_t n_spec,
-                          uint64_t max_bits, void* scratch, uint32_t* n_sync, bool ratio, int sms,
-                          cudaStream_t stream) {
+                          uint64_t max_bits, uint64_t* best64, uint32_t* next_item, uint32_t* n_sync,
+                          bool ratio, int sms, cudaStream_t stream) {
   if (n_spec == 0) return cudaSuccess;
   // Stored starts first (a byte scan), then the fixed-code sync search: it
   // costs a fraction of a full scan, which a fixed-Huffman partition (no
   // block header to find) would need, and it fails within a few dozen
   // symbols on other data.
-  stored_kernel<<<n_spec, kStoredThreads, 0, stream>>>(in, descs, spec, n_spec);
+  unsigned long long* best = reinterpret_cast<unsigned long long*>(best64);
+  stored_kernel<<<n_spec, kStoredThreads, 0, stream>>>(in, descs, spec, n_spec, best);
   sync_kernel<<<n_spec, kSyncOffsets, 0, stream>>>(in, descs, spec, n_spec, n_sync);
-  // best start per range, and the work counter after it
-  unsigned long long* best = reinterpret_cast<unsigned long long*>(scratch);
-  uint32_t* next_item = reinterpret_cast<uint32_t*>(best + n_spec);
-  cudaError_t e = cudaMemsetAsync(best, 0xFF, 8 * (size_t)n_spec, stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(next_item, 0, 8, stream);
-  if (e != cudaSuccess) return e;
   const uint32_t n_seg = (uint32_t)((max_bits + 31) / kFindSeg + 1);
   const uint64_t ctas = ((uint64_t)n_spec * n_seg + kFindWarps - 1) / kFindWarps;
   const uint32_t grid = (uint32_t)(ctas < (uint64_t)sms * 4 ? ctas : (uint64_t)sms * 4);
   find_kernel<<<grid, 32 * kFindWarps, 0, stream>>>(in, descs, spec, n_spec, n_seg, best, next_item);
-  assign_kernel<<<(n_spec + 127) / 128, 128, 0, stream>>>(in, descs, spec, n_spec, best, ratio);
+  assign_kernel<<<(n_spec + 127) / 128, 128, 0, stream>>>(in, descs, spec, n_spec, best, ratio,
+                                                         next_item);
   return cudaGetLastError();
 }
 

@@ -473,16 +473,17 @@ __global__ void __launch_bounds__(32 * kRingWarps)
 
 // Pages layout: a persistent grid of CTAs takes chunks from the queue.  A
 // failed speculative start moves on to the next candidate of its partition.
-// sync: the job has sync starts, so successors are watched mid-block.
+// *n_sync != 0: the job has sync starts, so successors are watched mid-block.
 template <int LB, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
     inflate_pages_kernel(const uint8_t* __restrict__ in, ChunkDesc* descs, ChunkResult* results,
                        const uint32_t* __restrict__ work, const uint32_t* __restrict__ n_work_ptr,
-                       uint32_t* work_counter, PagePool pool, int sync) {
+                       uint32_t* work_counter, const uint32_t* __restrict__ n_sync, PagePool pool) {
   extern __shared__ __align__(16) uint8_t smem[];
   CtaSmem<LB, NT>* S = reinterpret_cast<CtaSmem<LB, NT>*>(smem);
   const int tid = threadIdx.x;
   const uint32_t n_work = *n_work_ptr;
+  const bool sync = *n_sync != 0;
   if (tid == 0) S->c.fixed_tables = 0;
   for (;;) {
     __syncthreads();
@@ -501,7 +502,7 @@ __global__ void __launch_bounds__(NT, MINB)
     const uint32_t cid = S->c.cid;
     if (cid == kNone) break;
     for (;;) {
-      cta_decode_chunk<LB, NT>(in, descs, &results[cid], S, pool, sync != 0);
+      cta_decode_chunk<LB, NT>(in, descs, &results[cid], S, pool, sync);
       if (tid < 32) {
         // the partition's next candidate, if this start failed
         ChunkDesc& d = descs[cid];
@@ -557,25 +558,19 @@ static PagesFn pages_fn(int ctas, bool wide) {
 }
 
 template <int LB>
-cudaError_t launch_inflate(bool ring, int ctas, bool wide, bool sync, const uint8_t* in,
-                           ChunkDesc* descs, ChunkResult* results, const uint32_t* work,
-                           const uint32_t* n_work, uint32_t* work_counter, const PagePool& pool,
+cudaError_t launch_inflate(bool ring, int ctas, bool wide, const uint8_t* in, ChunkDesc* descs,
+                           ChunkResult* results, const uint32_t* work, const uint32_t* n_work,
+                           uint32_t* work_counter, const uint32_t* n_sync, const PagePool& pool,
                            int blocks, cudaStream_t stream) {
   cudaError_t e;
   if (ring) {
     const size_t smem = ring_smem_bytes<LB>();
-    e = cudaFuncSetAttribute(inflate_ring_kernel<LB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-    if (e != cudaSuccess) return e;
     inflate_ring_kernel<LB><<<blocks, 32 * kRingWarps, smem, stream>>>(in, descs, results, work,
                                                                        n_work, work_counter, pool);
   } else {
     const PagesFn f = pages_fn<LB>(ctas, wide);
-    int with_sync = sync;
-    e = cudaFuncSetAttribute(f.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem);
-    if (e != cudaSuccess) return e;
     void* args[] = {(void*)&in,     (void*)&descs,        (void*)&results, (void*)&work,
-                    (void*)&n_work, (void*)&work_counter, (void*)&pool,    (void*)&with_sync};
+                    (void*)&n_work, (void*)&work_counter, (void*)&n_sync,  (void*)&pool};
     e = cudaLaunchKernel(f.fn, dim3(blocks), dim3(f.threads), args, f.smem, stream);
     if (e != cudaSuccess) return e;
   }
@@ -591,8 +586,9 @@ int inflate_blocks_per_sm(bool ring, int ctas) {
                          (int)smem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, inflate_ring_kernel<LB>, 32 * kRingWarps, smem);
   } else {
-    const PagesFn f = pages_fn<LB>(ctas, false);
+    const PagesFn f = pages_fn<LB>(ctas, false), w = pages_fn<LB>(ctas, true);
     cudaFuncSetAttribute(f.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem);
+    cudaFuncSetAttribute(w.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)w.smem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f.fn, f.threads, f.smem);
     if (n > ctas) n = ctas;
   }
@@ -601,9 +597,10 @@ int inflate_blocks_per_sm(bool ring, int ctas) {
 
 #define GZGPU_INST(LB)                                                                         \
   template int inflate_blocks_per_sm<LB>(bool, int);                                           \
-  template cudaError_t launch_inflate<LB>(bool, int, bool, bool, const uint8_t*, ChunkDesc*,   \
+  template cudaError_t launch_inflate<LB>(bool, int, bool, const uint8_t*, ChunkDesc*,         \
                                           ChunkResult*, const uint32_t*, const uint32_t*,      \
-                                          uint32_t*, const PagePool&, int, cudaStream_t);
+                                          uint32_t*, const uint32_t*, const PagePool&, int,    \
+                                          cudaStream_t);
 GZGPU_INST(10)
 GZGPU_INST(11)
 GZGPU_INST(12)

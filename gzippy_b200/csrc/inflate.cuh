@@ -12,15 +12,15 @@ constexpr int kWideThreads = 1024;  // the same in jobs of few chunks (one CTA p
 constexpr int kDistBits = 8;       // distance LUT index bits (ring kernel, sync-start search)
 
 // page kernel: `ctas` (3 or 4) CTAs per SM; registers are sized for that many
-// (80 or 64 per thread)
+// (80 or 64 per thread).  Also sets the kernels up for launch_inflate.
 template <int LB>
 int inflate_blocks_per_sm(bool ring, int ctas);
-// wide: CTAs of kWideThreads; sync: the job has sync starts (successors are
-// watched mid-block)
+// wide: CTAs of kWideThreads; *n_sync (device): sync starts in the job (then
+// successors are watched mid-block)
 template <int LB>
-cudaError_t launch_inflate(bool ring, int ctas, bool wide, bool sync, const uint8_t* in,
-                           ChunkDesc* descs, ChunkResult* results, const uint32_t* work,
-                           const uint32_t* n_work, uint32_t* work_counter, const PagePool& pool,
+cudaError_t launch_inflate(bool ring, int ctas, bool wide, const uint8_t* in, ChunkDesc* descs,
+                           ChunkResult* results, const uint32_t* work, const uint32_t* n_work,
+                           uint32_t* work_counter, const uint32_t* n_sync, const PagePool& pool,
                            int blocks, cudaStream_t stream);
 // sync starts inside dynamic blocks for the listed pieces left without a start
 cudaError_t launch_dyn_sync(const uint8_t* in, ChunkDesc* descs, const uint32_t* pieces, uint32_t n,

@@ -1,6 +1,6 @@
 // members.cu -- gzip member location on the device.
 //
-// stream_header_kernel: per stream, the magic check (non-gzip -> kNotGzip,
+// stream_info: per stream, the magic check (non-gzip -> kNotGzip,
 //   src/lib.rs:50-52) and the first member's header length (RFC 1952,
 //   gzip_format.rs read_header :47-133).
 // member_scan_kernel: every byte position of every stream is tested like
@@ -48,13 +48,7 @@ __device__ uint64_t parse_header(const uint8_t* in, uint64_t p, uint64_t end) {
   return o - p;
 }
 
-__global__ void stream_header_kernel(const uint8_t* __restrict__ in,
-                                     const uint64_t* __restrict__ s_off,
-                                     const uint64_t* __restrict__ s_len, uint32_t n,
-                                     StreamInfo* info) {
-  uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  uint64_t p = s_off[s], len = s_len[s];
+__device__ StreamInfo stream_info(const uint8_t* __restrict__ in, uint64_t p, uint64_t len) {
   StreamInfo si{};
   if (len < 2 || in[p] != 0x1f || in[p + 1] != 0x8b) {
     si.status = kNotGzip;
@@ -74,7 +68,7 @@ __global__ void stream_header_kernel(const uint8_t* __restrict__ in,
     const uint8_t* t = in + p + len - 4;
     si.last_isize = t[0] | (t[1] << 8) | ((uint32_t)t[2] << 16) | ((uint32_t)t[3] << 24);
   }
-  info[s] = si;
+  return si;
 }
 
 // bit 7 of each byte of the result is set exactly where w's byte is zero
@@ -83,19 +77,31 @@ __device__ __forceinline__ uint32_t zero_bytes(uint32_t w) {
   return ~(t | w | 0x7F7F7F7Fu);
 }
 
-// grid-stride over scan units (stream, byte range); each thread screens 16
-// aligned bytes at a time for the 0x1f of the magic with word operations
-// and tests only the positions that have one
+// grid-stride over scan units (stream, byte range); every CTA reads the
+// stream's first header for itself (a kernel for that alone would be one more
+// wait) and the first unit's writes it down; each thread screens 16 aligned
+// bytes at a time for the 0x1f of the magic with word operations and tests
+// only the positions that have one
 __global__ void member_scan_kernel(const uint8_t* __restrict__ in, const ScanUnit* __restrict__ units,
                                    uint32_t n_units, const uint64_t* __restrict__ s_off,
-                                   const uint64_t* __restrict__ s_len,
-                                   const StreamInfo* __restrict__ info, MemberCand* cands,
-                                   uint32_t* n_cands, uint32_t cap) {
+                                   const uint64_t* __restrict__ s_len, StreamInfo* info,
+                                   MemberCand* cands, uint32_t* n_cands, uint32_t cap) {
+  __shared__ StreamInfo s_info;
+  uint32_t known = 0xFFFFFFFFu;  // the stream s_info is of
   for (uint32_t u = blockIdx.x; u < n_units; u += gridDim.x) {
     const ScanUnit su = units[u];
-    const StreamInfo si = info[su.stream];
-    if (si.status != kOk) continue;
     const uint64_t base = s_off[su.stream], len = s_len[su.stream];
+    __syncwarp();
+    __syncthreads();  // the unit before has read s_info
+    if (threadIdx.x == 0) {
+      if (su.stream != known) s_info = stream_info(in, base, len);
+      if (su.begin == 0) info[su.stream] = s_info;
+    }
+    __syncwarp();
+    __syncthreads();
+    known = su.stream;
+    const StreamInfo si = s_info;
+    if (si.status != kOk) continue;
     const uint64_t lo = su.begin > (uint64_t)si.header_len + 1 ? su.begin : si.header_len + 1;
     for (uint64_t a = ((base + lo) & ~15ull) + 16 * (uint64_t)threadIdx.x; a < base + su.end;
          a += 16 * (uint64_t)blockDim.x) {
@@ -137,17 +143,10 @@ __global__ void member_scan_kernel(const uint8_t* __restrict__ in, const ScanUni
   }
 }
 
-cudaError_t launch_stream_headers(const uint8_t* in, const uint64_t* s_off, const uint64_t* s_len,
-                                  uint32_t n, StreamInfo* info, cudaStream_t stream) {
-  if (!n) return cudaSuccess;
-  stream_header_kernel<<<(n + 127) / 128, 128, 0, stream>>>(in, s_off, s_len, n, info);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_member_scan(const uint8_t* in, const ScanUnit* units, uint32_t n_units,
-                               const uint64_t* s_off, const uint64_t* s_len,
-                               const StreamInfo* info, MemberCand* cands, uint32_t* n_cands,
-                               uint32_t cap, int sms, cudaStream_t stream) {
+                               const uint64_t* s_off, const uint64_t* s_len, StreamInfo* info,
+                               MemberCand* cands, uint32_t* n_cands, uint32_t cap, int sms,
+                               cudaStream_t stream) {
   if (!n_units) return cudaSuccess;
   uint32_t grid = n_units < (uint32_t)(sms * 16) ? n_units : (uint32_t)(sms * 16);
   member_scan_kernel<<<grid, 512, 0, stream>>>(in, units, n_units, s_off, s_len, info, cands,

@@ -27,11 +27,11 @@ struct MemberCand {
   uint32_t pad;
 };
 
-cudaError_t launch_stream_headers(const uint8_t* in, const uint64_t* s_off, const uint64_t* s_len,
-                                  uint32_t n, StreamInfo* info, cudaStream_t stream);
+// the first member's header of every stream with a unit (info), and every
+// unit's member candidates (n_cands: zero before)
 cudaError_t launch_member_scan(const uint8_t* in, const ScanUnit* units, uint32_t n_units,
-                               const uint64_t* s_off, const uint64_t* s_len,
-                               const StreamInfo* info, MemberCand* cands, uint32_t* n_cands,
-                               uint32_t cap, int sms, cudaStream_t stream);
+                               const uint64_t* s_off, const uint64_t* s_len, StreamInfo* info,
+                               MemberCand* cands, uint32_t* n_cands, uint32_t cap, int sms,
+                               cudaStream_t stream);
 
 }  // namespace gzgpu
