@@ -49,6 +49,7 @@ enum : uint32_t {
                            // a block header (table_bit: that block's header; 0 = a
                            // non-final fixed-Huffman block)
   kChunkPiece = 16u,       // a piece of a partition cut by its output estimate
+  kChunkTail = 32u,        // a partition near its member's end, where the final block may start
 };
 // flags bits 24..31: the chunk's first decode attempt number (its pages carry
 // attempt numbers from there; raised when a chunk is decoded again after the

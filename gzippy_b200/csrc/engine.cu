@@ -366,6 +366,12 @@ constexpr uint64_t kMinPartitionBits = 8ull << 13;
 // shortest piece of a partition cut by the output estimate (4 KiB of input)
 constexpr uint64_t kMinPieceBits = 4ull << 13;
 
+// Partitions this close to their member's end are searched for the header of
+// the final block too.  A block of 16,383 symbols (zlib's) takes about 35 KB
+// at most; the search looks at twice the candidates there, so it is not made
+// for the others.
+constexpr uint64_t kTailBits = 48ull << 13;
+
 static uint64_t pick_chunk_bytes(uint64_t in_len) {
   // several chunks per decoding warp on large inputs, which the
   // longest-first order balances; smaller chunks for small inputs so the
@@ -712,7 +718,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
         x.limit_bit = std::min(g + mbits, bend);
         x.stop_lo = kNoStop;
         x.in_end = d.in_end;
-        x.flags = 0;
+        x.flags = bend - x.limit_bit < kTailBits ? kChunkTail : 0u;
         x.stream = s;
         hspec.push_back((uint32_t)hd.size());
         hd.push_back(x);

@@ -109,7 +109,10 @@ __device__ const LeafLut d_leaf_lut = LeafLut();
 constexpr int kFindWarps = 8;
 constexpr uint32_t kFindSeg = 8192;                // bits per segment
 constexpr uint32_t kFindPass = 4096;               // bits per screening pass
-constexpr uint32_t kFindList = kFindPass / 3 + 2;  // most survivors: three bits apart (BFINAL 0, BTYPE 10)
+// most survivors of a pass: three bits apart (BFINAL 0, BTYPE 10); near a
+// member's end, where BFINAL may be either, two, in passes half as long
+constexpr uint32_t kFindList = kFindPass / 3 + 2;
+static_assert(kFindPass / 4 + 2 <= kFindList, "");
 constexpr uint32_t kFindFull = 64;                 // full tests held
 
 struct FindWarp {
@@ -291,15 +294,18 @@ __global__ void __launch_bounds__(32 * kFindWarps)
     if (lane == 0) W.n_full = 0;
     __syncwarp();
     uint32_t hit = kFindSeg;  // lowest passing offset
-    for (uint32_t p0 = 0; p0 < len && hit == kFindSeg; p0 += kFindPass) {
+    const bool tail = d.flags & kChunkTail;
+    const uint32_t pass = tail ? kFindPass / 2 : kFindPass;
+    for (uint32_t p0 = 0; p0 < len && hit == kFindSeg; p0 += pass) {
+      const uint32_t p1 = min(len, p0 + pass);
       uint32_t m[kFindPass / 1024], c = 0;
 #pragma unroll
       for (uint32_t q = 0; q < kFindPass / 1024; q++) {
         const uint32_t p = p0 + 1024 * q + 32 * lane;
         uint32_t v = 0;
-        if (p < len) {
-          v = dyn_filter32((uint64_t)W.w[(p >> 5) + 1] << 32 | W.w[p >> 5]);
-          if (p + 32 > len) v &= (1u << (len - p)) - 1;
+        if (p < p1) {
+          v = dyn_filter32((uint64_t)W.w[(p >> 5) + 1] << 32 | W.w[p >> 5], tail);
+          if (p + 32 > p1) v &= (1u << (p1 - p)) - 1;
           if (p < first) v &= p + 32 > first ? 0xFFFFFFFFu << (first - p) : 0u;
         }
         m[q] = v;
@@ -469,8 +475,7 @@ __device__ float chunk_cost(const uint8_t* __restrict__ in, const ChunkDesc& d, 
   uint64_t bit = d.start_bit, copied = 0;
   if (bit >= end) return 0.f;
   const float span = (float)(end - bit) * 0.125f;
-  if (d.flags & kChunkSync) return span;
-  for (int k = 0; k < 8 && bit < end; k++) {
+  for (int k = 0; k < 8 && bit < end && !(d.flags & kChunkSync); k++) {
     if (peek_bits(in, d.in_end, bit, 3) >> 1) break;
     const uint64_t at = (bit + 10) >> 3;  // LEN
     if (at + 2 > d.in_end) break;

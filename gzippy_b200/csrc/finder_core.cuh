@@ -262,12 +262,12 @@ static __device__ __forceinline__ uint64_t bits64_at(const uint32_t* in32, uint6
 
 // Positions i < 32 (bit i of the result) where the 13-bit dynamic header
 // filter passes, for the 64 stream bits X starting at the first of them:
-// BFINAL = 0, BTYPE = 10, HLIT <= 29 (not bits 4..7 all set), HDIST <= 29
+// BFINAL = 0 (or either: any_final), BTYPE = 10, HLIT <= 29 (not bits 4..7 all set), HDIST <= 29
 // (not bits 9..12 all set).  All 32 positions at once, bit-parallel.
-static __device__ __forceinline__ uint32_t dyn_filter32(uint64_t X) {
+static __device__ __forceinline__ uint32_t dyn_filter32(uint64_t X, bool any_final = false) {
   const uint64_t hlit_big = (X >> 4) & (X >> 5) & (X >> 6) & (X >> 7);
   const uint64_t hdist_big = (X >> 9) & (X >> 10) & (X >> 11) & (X >> 12);
-  return (uint32_t)(~X & ~(X >> 1) & (X >> 2) & ~hlit_big & ~hdist_big);
+  return (uint32_t)((any_final ? ~0ull : ~X) & ~(X >> 1) & (X >> 2) & ~hlit_big & ~hdist_big);
 }
 
 // Byte offsets k < 4 (bit k) among off .. off + 3 where LEN == ~NLEN, from
