@@ -78,7 +78,8 @@ struct ChunkDesc {
   uint32_t flags;
   uint32_t stream;     // stream id
   uint32_t next;       // index of the next valid chunk of the stream (kNoChunk = none)
-  float est_ratio;     // finder's estimate of output bytes per input byte (0 = none)
+  float est_ratio;     // estimate of output bytes per input byte (0 = none): the
+                       // member's by its ISIZE, or the finder's by the block's code
 };
 constexpr uint32_t kNoChunk = 0xFFFFFFFFu;
 // phantom successors a speculative chunk decodes through; a chunk whose start

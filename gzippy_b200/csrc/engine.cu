@@ -696,8 +696,12 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
     for (const Mem& m : mems[s]) {
       const uint64_t b0 = (S[s].off + m.ds) * 8, bend = (S[s].off + m.end) * 8;
       mc0[s].push_back((uint32_t)hd.size());
+      const uint64_t clen = m.end > m.ds ? m.end - m.ds : 0;
+      // a first estimate for the decode order (the finder's own, per chunk, in its place)
+      const float ratio = fine_split || !clen ? 0.f : std::min((float)m.isize / (float)clen, 1032.f);
       ChunkDesc d{};
       d.start_bit = d.lo_bit = d.guess_bit = b0;
+      d.est_ratio = ratio;
       d.limit_bit = S[s].off + m.start;  // member-first: the member's header byte
       d.stop_lo = kNoStop;
       d.in_end = S[s].off + S[s].len;
@@ -707,7 +711,6 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
       // members that expand a lot (ISIZE over compressed size) get shorter
       // partitions, so chunks carry similar output (about 2 x chunk_bytes)
       uint64_t mbits = cbits;
-      const uint64_t clen = m.end > m.ds ? m.end - m.ds : 0;
       if (clen && (uint64_t)m.isize > 2 * clen) {
         mbits = (uint64_t)((double)cbits * 2.0 * (double)clen / (double)m.isize) & ~63ull;
         mbits = std::max<uint64_t>(mbits, std::min<uint64_t>(cbits, kMinPartitionBits));
@@ -720,6 +723,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
         x.in_end = d.in_end;
         x.flags = bend - x.limit_bit < kTailBits ? kChunkTail : 0u;
         x.stream = s;
+        x.est_ratio = ratio;
         hspec.push_back((uint32_t)hd.size());
         hd.push_back(x);
       }

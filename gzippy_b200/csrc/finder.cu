@@ -114,6 +114,8 @@ constexpr uint32_t kFindPass = 4096;               // bits per screening pass
 constexpr uint32_t kFindList = kFindPass / 3 + 2;
 static_assert(kFindPass / 4 + 2 <= kFindList, "");
 constexpr uint32_t kFindFull = 64;                 // full tests held
+// a hit: its bit, then its code's mean bytes per symbol in eighths (up to 258)
+constexpr int kMeanBits = 12;
 
 struct FindWarp {
   uint32_t w[kFindSeg / 32 + 6];
@@ -129,9 +131,11 @@ struct FindWarp {
 // 32; a walk over shuffles picks the real ones (about nine), which are then
 // weighed together.  A true header is 200 and more lengths one after another,
 // 90,000 cycles and more for a thread by itself, 15,000 so; a false one ends
-// within two or three such steps.
+// within two or three such steps.  mean: of a true one, the bytes a symbol
+// gives on average by its code (a code of length v stands for a probability of
+// 2^-v), in units of 2^-15.
 __device__ __noinline__ bool dyn_candidate_warp(const uint8_t* in, uint64_t nbytes, uint64_t bit,
-                                                FindWarp& W, int lane) {
+                                                FindWarp& W, int lane, uint32_t& mean) {
   constexpr uint32_t kAll = 0xFFFFFFFFu;
   const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
   const uint32_t below = (1u << lane) - 1;
@@ -182,6 +186,7 @@ __device__ __noinline__ bool dyn_candidate_warp(const uint8_t* in, uint64_t nbyt
   uint32_t rel = (uint32_t)(pos0 & 31);  // position, from wbase on
   uint32_t rel0 = rel;
   uint32_t n = 0, prev = 0;              // lengths read, the last of them
+  mean = 1u << 15;
   uint32_t lit = 0, dist = 0, lit_gt1 = 0, dist_gt1 = 0, eob = 0;
   while (n < total) {
     if (rel >= 1024 + 960) {  // (rare: a header of over 2,000 bits)
@@ -247,6 +252,13 @@ __device__ __noinline__ bool dyn_candidate_warp(const uint8_t* in, uint64_t nbyt
     lit_gt1 |= __ballot_sync(kAll, v > 1 && n_lit);
     dist_gt1 |= __ballot_sync(kAll, v > 1 && n_dist);
     eob |= __ballot_sync(kAll, use && v && i <= 256 && 256 < i + r);
+    {
+      // length symbols: more than a byte each (a repeat's by the first of them)
+      const uint32_t s = max(i, 257u);
+      const uint32_t c = v && i + n_lit > s ? i + n_lit - s : 0u;
+      const uint32_t more = c ? f_len_base[min(s - 257, 28u)] + (1u << f_len_extra[min(s - 257, 28u)]) / 2 - 1 : 0u;
+      mean += __reduce_add_sync(kAll, c * more << (15 - v));
+    }
     const uint32_t last = 31 - __clz(chain | 1u);
     n += __shfl_sync(kAll, at, 31);
     prev = __shfl_sync(kAll, v, last);
@@ -282,7 +294,7 @@ __global__ void __launch_bounds__(32 * kFindWarps)
     // segments are cut at word boundaries of the input
     const uint64_t s0 = (from & ~31ull) + (uint64_t)sg * kFindSeg;
     if (s0 >= to) continue;
-    if (*(volatile unsigned long long*)&best[k] < s0) continue;
+    if (*(volatile unsigned long long*)&best[k] >> kMeanBits < s0) continue;
     const uint32_t len = (uint32_t)min((uint64_t)kFindSeg, to - s0);
     const uint32_t first = from > s0 ? (uint32_t)(from - s0) : 0u;
     // the segment's words, and the 81 bits after it (a header up to its precode)
@@ -293,7 +305,7 @@ __global__ void __launch_bounds__(32 * kFindWarps)
       if (j + lane < kFindSeg / 32 + 6 && 32 * (j + lane) < len + 160) W.w[j + lane] = in32[wi + j + lane];
     if (lane == 0) W.n_full = 0;
     __syncwarp();
-    uint32_t hit = kFindSeg;  // lowest passing offset
+    uint32_t hit = kFindSeg, mean = 0;  // lowest passing offset, its code's bytes per symbol
     const bool tail = d.flags & kChunkTail;
     const uint32_t pass = tail ? kFindPass / 2 : kFindPass;
     for (uint32_t p0 = 0; p0 < len && hit == kFindSeg; p0 += pass) {
@@ -347,7 +359,7 @@ __global__ void __launch_bounds__(32 * kFindWarps)
         if (n0 + __popc(b) > kFindFull) {
           // (rare) the held ones first
           for (uint32_t j = 0; j < n0 && hit == kFindSeg; j++)
-            if (dyn_candidate_warp(in, nbytes, s0 + W.full[j], W, lane)) hit = W.full[j];
+            if (dyn_candidate_warp(in, nbytes, s0 + W.full[j], W, lane, mean)) hit = W.full[j];
           __syncwarp();
           n0 = 0;
         }
@@ -357,12 +369,13 @@ __global__ void __launch_bounds__(32 * kFindWarps)
       }
       const uint32_t n0 = W.n_full;
       for (uint32_t j = 0; j < n0 && hit == kFindSeg; j++)
-        if (dyn_candidate_warp(in, nbytes, s0 + W.full[j], W, lane)) hit = W.full[j];
+        if (dyn_candidate_warp(in, nbytes, s0 + W.full[j], W, lane, mean)) hit = W.full[j];
       __syncwarp();
       if (lane == 0) W.n_full = 0;
       __syncwarp();
     }
-    if (hit < kFindSeg && lane == 0) atomicMin(&best[k], (unsigned long long)(s0 + hit));
+    if (hit < kFindSeg && lane == 0)
+      atomicMin(&best[k], (unsigned long long)(s0 + hit) << kMeanBits | min(mean >> 12, (1u << kMeanBits) - 1));
   }
 }
 
@@ -377,9 +390,11 @@ __global__ void assign_kernel(const uint8_t* __restrict__ in, ChunkDesc* descs,
   if (k >= n_spec) return;
   ChunkDesc& d = descs[spec[k]];
   if ((d.flags & kChunkValid) || best[k] == ~0ull) return;
-  d.lo_bit = d.start_bit = best[k];
+  d.lo_bit = d.start_bit = best[k] >> kMeanBits;
   d.flags |= kChunkValid;
-  d.est_ratio = ratio ? dyn_header_ratio(in, d.in_end, d.start_bit) : 0.f;
+  // (without the codes' lengths: a symbol taken for two bytes)
+  d.est_ratio = ratio ? dyn_header_ratio(in, d.in_end, d.start_bit)
+                      : (float)(best[k] & ((1u << kMeanBits) - 1)) * (0.125f / 2);
 }
 
 // Sync starts in fixed-Huffman data (finder_core.cuh), searched for every
@@ -464,12 +479,15 @@ __global__ void __launch_bounds__(kSyncOffsets)
 // A speculative start may be a phantom whose garbage code table never fails;
 // such a chunk gives up `slack` bits past its stop and the chain walk
 // re-decodes the gap from the confirmed boundary instead.
-// Decode cost of a linked chunk: its compressed bytes.  Text, byte runs and
-// noisy literals take the decoder about the same time per compressed byte
-// (within a factor of two); stored data is a copy, a twentieth of that.  Only
-// the stored blocks themselves count so: chunks that begin with one and go on
-// with Huffman blocks were taken for short, started last, and kept the decode
-// of a mixed 128 MiB stream waiting (1.54 ms, now 1.29).
+// Decode cost of a linked chunk: its compressed bytes.  Text and noisy
+// literals take the decoder 8.6 us per KB; stored data is a copy, a twentieth
+// of that (only the stored blocks themselves count so: chunks that begin with
+// one and go on with Huffman blocks are not short); byte runs take two to five
+// times as long, so data estimated to give over twice its bytes counts half
+// its output.  128 MiB mixed stream: 1.54 ms by bytes alone, 1.29 with stored
+// blocks by themselves, 1.21 with the output; 600 files: 1.51 without the
+// output, 1.17 with it (a file's runs went last where false sync starts made
+// them look short).
 __device__ float chunk_cost(const uint8_t* __restrict__ in, const ChunkDesc& d, uint64_t stop) {
   const uint64_t end = min(stop, d.in_end * 8);
   uint64_t bit = d.start_bit, copied = 0;
@@ -483,7 +501,7 @@ __device__ float chunk_cost(const uint8_t* __restrict__ in, const ChunkDesc& d, 
     copied += len;
     bit = (at + 4 + len) * 8;
   }
-  return fmaxf(span - 0.95f * (float)copied, 0.05f * span);
+  return fmaxf(span - 0.95f * (float)copied, 0.05f * span) * fmaxf(1.f, 0.5f * d.est_ratio);
 }
 
 __global__ void link_kernel(const uint8_t* __restrict__ in, ChunkDesc* descs, uint32_t n,
