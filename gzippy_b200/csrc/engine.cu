@@ -1251,7 +1251,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   }
   if ((rc = check(launch_resolve(reinterpret_cast<PlacedChunk*>(d_plan + at_placed),
                                  reinterpret_cast<uint32_t*>(d_plan + at_pof), n_pages_used,
-                                 results.as<ChunkResult>(), pool, cur_out, sms, st))))
+                                 results.as<ChunkResult>(), pool, cur_out, st))))
     return rc;
   cudaEventRecord(ev[11], st);
   if ((rc = check(launch_crc(reinterpret_cast<CrcBlock*>(d_plan + at_cblk), (uint32_t)cblk.size(), cur_out,

@@ -10,7 +10,7 @@ cudaError_t resolve_init(cudaStream_t stream);
 // every placed chunk's bytes, markers resolved, from the pages [0, n_pages)
 cudaError_t launch_resolve(const PlacedChunk* placed, const uint32_t* placed_of_chunk,
                            uint32_t n_pages, const ChunkResult* results, const PagePool& pool,
-                           uint8_t* out, int sms, cudaStream_t stream);
+                           uint8_t* out, cudaStream_t stream);
 // CRC: one CTA per block of up to kCrcBlock bytes, a slice of kCrcSlice per thread
 constexpr int kCrcThreads = 512;
 constexpr uint32_t kCrcSlice = 128;
