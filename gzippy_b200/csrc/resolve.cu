@@ -230,12 +230,11 @@ __device__ __forceinline__ uint32_t crc_shift(const uint32_t* shf, uint32_t s, i
   return t[s & 0xFF] ^ t[256 + ((s >> 8) & 0xFF)] ^ t[512 + ((s >> 16) & 0xFF)] ^ t[768 + (s >> 24)];
 }
 
-// one byte into a CRC register, from the lane's own copy of the byte table
-// (word 32 * index + lane of the shared array: every lane of a warp reads
-// its own bank)
-__device__ __forceinline__ uint32_t crc_byte(const uint32_t* ltab, uint32_t lane, uint32_t c,
-                                             uint32_t b) {
-  return ltab[(((c ^ b) & 0xFFu) << 5) | lane] ^ (c >> 8);
+// the register moved past one byte (added to its low end before), from the
+// lane's own copy of the byte table (word 32 * index + lane of the shared
+// array: every lane of a warp reads its own bank)
+__device__ __forceinline__ uint32_t crc_step(const uint32_t* ltab, uint32_t lane, uint32_t c) {
+  return ltab[((c & 0xFFu) << 5) | lane] ^ (c >> 8);
 }
 
 // CRC32 of the final output, one CTA per block of up to kCrcBlock bytes of one
@@ -246,82 +245,86 @@ __device__ __forceinline__ uint32_t crc_byte(const uint32_t* ltab, uint32_t lane
 // byte table (no bank conflicts), from aligned 16-byte loads; the slices'
 // registers merge in a tree of fixed shifts, and the block's register, moved
 // past the rest of its member, is XORed into mem_raw.  What a block waits for
-// is the serial chain of its bytes (a table read each), so slices are short:
-// with 1 KiB slices (a warp per 32 KiB) the pass took 50 us for a 4 KiB
-// stream and 75 us up to 64 MiB, now 9 and 21.
+// is the serial chain of its bytes (a table read each), so slices are short
+// (with 1 KiB slices, a warp per 32 KiB, a 4 KiB stream took 50 us, now 9).
+// The warps merge their own slices and leave their registers; the blocks are
+// put together at the end, a warp each, so that no warp waits for another in
+// between (the move past a member's rest alone is 6,000 cycles of one warp:
+// 128 MiB took 113 us with it between the blocks, now 86).
 __global__ void __launch_bounds__(kCrcThreads)
     crc_blocks_kernel(const CrcBlock* __restrict__ blocks, uint32_t n,
                       const uint8_t* __restrict__ out, uint32_t* __restrict__ mem_raw) {
   extern __shared__ __align__(16) uint32_t sm[];
   uint32_t* ltab = sm;                                // [256][32] lane copies of the byte table
   uint32_t* shf = sm + 256 * 32;                      // [kCrcLevels][4][256] shift tables
-  uint32_t* part = shf + kCrcLevels * 4 * 256;        // [2][warps]
+  uint32_t* part = shf + kCrcLevels * 4 * 256;        // [kCrcTurns][warps]
   constexpr int kWarps = kCrcThreads / 32;
   for (uint32_t i = threadIdx.x; i < 256 * 32; i += kCrcThreads) ltab[i] = d_crc_tab[i >> 5];
   for (uint32_t i = threadIdx.x; i < kCrcLevels * 256; i += kCrcThreads)
     reinterpret_cast<uint4*>(shf)[i] = reinterpret_cast<const uint4*>(&d_crc_shift[0][0][0])[i];
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t turn = 0;
-  for (uint32_t bi = blockIdx.x; bi < n; bi += gridDim.x, turn++) {
-    const CrcBlock blk = blocks[bi];
-    // this thread's slice [s0, s0 + kCrcSlice) of the output
-    const int64_t s0 = (int64_t)blk.end - (int64_t)kCrcSlice * (kCrcThreads - (int)threadIdx.x);
-    uint32_t c = 0;
-    if (s0 + (int64_t)kCrcSlice > (int64_t)blk.begin) {
-      uint4 v[kCrcSlice / 16];
+  for (uint32_t b0 = blockIdx.x; b0 < n; b0 += kCrcTurns * gridDim.x) {
+    uint32_t turns = 0;
+    for (uint32_t bi = b0; bi < n && turns < kCrcTurns; bi += gridDim.x, turns++) {
+      const CrcBlock blk = blocks[bi];
+      // this thread's slice [s0, s0 + kCrcSlice) of the output
+      const int64_t s0 = (int64_t)blk.end - (int64_t)kCrcSlice * (kCrcThreads - (int)threadIdx.x);
+      uint32_t c = 0;
+      if (s0 + (int64_t)kCrcSlice > (int64_t)blk.begin) {
+        uint4 v[kCrcSlice / 16];
 #pragma unroll
-      for (uint32_t i = 0; i < kCrcSlice / 16; i++) {
-        const int64_t a = s0 + 16 * (int64_t)i;
-        v[i] = a + 16 > (int64_t)blk.begin && a + 16 <= (int64_t)blk.last
-                   ? *reinterpret_cast<const uint4*>(out + a)
-                   : make_uint4(0, 0, 0, 0);
-      }
+        for (uint32_t i = 0; i < kCrcSlice / 16; i++) {
+          const int64_t a = s0 + 16 * (int64_t)i;
+          v[i] = a + 16 > (int64_t)blk.begin && a + 16 <= (int64_t)blk.last
+                     ? *reinterpret_cast<const uint4*>(out + a)
+                     : make_uint4(0, 0, 0, 0);
+        }
 #pragma unroll
-      for (uint32_t i = 0; i < kCrcSlice / 16; i++) {
-        uint32_t wd[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
-        const int64_t a = s0 + 16 * (int64_t)i;
-        if (a < (int64_t)blk.begin || a + 16 > (int64_t)blk.last) {
-          // the ends: bytes outside the member count as zeros
+        for (uint32_t i = 0; i < kCrcSlice / 16; i++) {
+          uint32_t wd[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+          const int64_t a = s0 + 16 * (int64_t)i;
+          if (a < (int64_t)blk.begin || a + 16 > (int64_t)blk.last) {
+            // the ends: bytes outside the member count as zeros
 #pragma unroll
-          for (int k = 0; k < 16; k++) {
-            const bool in = a + k >= (int64_t)blk.begin && a + k < (int64_t)blk.last;
-            const uint32_t byte = in ? out[a + k] : 0u;
-            wd[k >> 2] = (wd[k >> 2] & ~(0xFFu << (8 * (k & 3)))) | byte << (8 * (k & 3));
+            for (int k = 0; k < 16; k++) {
+              const bool in = a + k >= (int64_t)blk.begin && a + k < (int64_t)blk.last;
+              const uint32_t byte = in ? out[a + k] : 0u;
+              wd[k >> 2] = (wd[k >> 2] & ~(0xFFu << (8 * (k & 3)))) | byte << (8 * (k & 3));
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            c ^= wd[k];
+#pragma unroll
+            for (int b = 0; b < 4; b++) c = crc_step(ltab, lane, c);
           }
         }
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          c = crc_byte(ltab, lane, c, wd[k]);
-          c = crc_byte(ltab, lane, c, wd[k] >> 8);
-          c = crc_byte(ltab, lane, c, wd[k] >> 16);
-          c = crc_byte(ltab, lane, c, wd[k] >> 24);
-        }
       }
+      __syncwarp();
+      // slices merge: 2^j slices on each side at level j, first in the warps
+#pragma unroll
+      for (int j = 0; j < 5; j++) {
+        const uint32_t r = __shfl_down_sync(0xFFFFFFFFu, c, 1 << j);
+        if ((lane & ((2 << j) - 1)) == 0) c = crc_shift(shf, c, j) ^ r;
+      }
+      if (lane == 0) part[turns * kWarps + warp] = c;
     }
     __syncwarp();
-    // slices merge: 2^j slices on each side at level j, first in the warps
-#pragma unroll
-    for (int j = 0; j < 5; j++) {
-      const uint32_t r = __shfl_down_sync(0xFFFFFFFFu, c, 1 << j);
-      if ((lane & ((2 << j) - 1)) == 0) c = crc_shift(shf, c, j) ^ r;
-    }
-    // then the warps' registers, by one warp (another one each block)
-    if (lane == 0) part[(turn & 1) * kWarps + warp] = c;
     __syncthreads();
-    if (warp == (int)(turn % kWarps)) {
-      c = lane < kWarps ? part[(turn & 1) * kWarps + lane] : 0u;
+    for (uint32_t t = warp; t < turns; t += kWarps) {
+      const CrcBlock blk = blocks[b0 + t * gridDim.x];
+      uint32_t c = lane < kWarps ? part[t * kWarps + lane] : 0u;
 #pragma unroll
       for (int j = 0; (1 << j) < kWarps; j++) {
         const uint32_t r = __shfl_down_sync(0xFFFFFFFFu, c, 1 << j);
         if ((lane & ((2 << j) - 1)) == 0) c = crc_shift(shf, c, 5 + j) ^ r;
       }
-      if (blk.after) {
-        const uint32_t xp = x_pow_8n_warp(blk.after, lane);
-        c = gf2_mulmod(xp, c);
-      }
+      if (blk.after) c = gf2_mulmod(x_pow_8n_warp(blk.after, lane), c);
       if (lane == 0) atomicXor(mem_raw + blk.member, c);
     }
+    __syncwarp();
+    __syncthreads();
   }
 }
 

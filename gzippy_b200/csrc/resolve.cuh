@@ -17,8 +17,10 @@ constexpr uint32_t kCrcSlice = 128;
 constexpr uint32_t kCrcBlock = kCrcSlice * kCrcThreads;
 constexpr int kCrcCtasPerSm = 2;
 constexpr int kCrcLevels = 9;  // log2(512 slices)
-// shared memory: 32 lane copies of the byte table, shift tables, the warps' registers (twice)
-constexpr size_t kCrcSmem = 256 * 32 * 4 + kCrcLevels * 4 * 256 * 4 + 2 * (kCrcThreads / 32) * 4;
+constexpr uint32_t kCrcTurns = 64;  // blocks of a CTA whose warps' registers are kept
+// shared memory: 32 lane copies of the byte table, shift tables, the warps' registers
+constexpr size_t kCrcSmem =
+    256 * 32 * 4 + kCrcLevels * 4 * 256 * 4 + kCrcTurns * (kCrcThreads / 32) * 4;
 
 // mem_end[m]: output offset just past member m; mem_raw[m]: its CRC register
 // accumulator (zeroed before the launch); then each member's status
