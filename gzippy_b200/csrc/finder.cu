@@ -24,13 +24,25 @@ namespace gzgpu {
 // starts.  One CTA of kStoredThreads per chunk; a thread screens 16 aligned
 // byte offsets a round with word operations (a round covers 4 KiB, so a 24 KiB
 // partition is six load latencies; offset by offset, 1 KiB a round, took
-// 41 us for the 1,365 partitions of a 23 MB stream).
+// 41 us for the 1,365 partitions of a 23 MB stream).  A dynamic header after a
+// candidate's block is read by the whole warp: by one thread it is 90,000
+// cycles, which the last CTAs waited for (3,286 partitions of a mixed stream:
+// 89 us, now 49).
 constexpr int kStoredThreads = 256;
+
+// A warp's scratch for dyn_candidate_warp
+struct HeaderTest {
+  uint8_t sorted[32];  // the precode's symbols in code order
+  uint8_t lut[128];    // and its table, entry: symbol | length << 5
+};
+__device__ __noinline__ bool dyn_candidate_warp(const uint8_t* in, uint64_t nbytes, uint64_t bit,
+                                                HeaderTest& W, int lane, uint32_t& mean);
 
 __global__ void __launch_bounds__(kStoredThreads)
     stored_kernel(const uint8_t* __restrict__ in, ChunkDesc* descs,
                   const uint32_t* __restrict__ spec, uint32_t n_spec, unsigned long long* best) {
   __shared__ unsigned long long s_first;
+  __shared__ HeaderTest ht[kStoredThreads / 32];
   if (blockIdx.x >= n_spec) return;
   if (threadIdx.x == 0) best[blockIdx.x] = ~0ull;  // for find_kernel
   ChunkDesc& d = descs[spec[blockIdx.x]];
@@ -40,34 +52,66 @@ __global__ void __launch_bounds__(kStoredThreads)
   __syncthreads();
   const uint64_t begin = max((from + 3 + 7) / 8, (uint64_t)2);
   const uint64_t until = nbytes >= 5 ? min((to + 7) / 8, nbytes - 4) : 0;
+  // (the next round's bytes are on their way while this one's are tested)
+  uint64_t ob = (begin & ~15ull) + 16 * (uint64_t)threadIdx.x;
+  uint4 v = make_uint4(0, 0, 0, 0);
+  uint32_t v4 = 0;
+  auto load = [&]() {
+    if (ob >= until) return;
+    v = *reinterpret_cast<const uint4*>(in + ob);
+    v4 = *reinterpret_cast<const uint32_t*>(in + ob + 16);
+  };
+  load();
   for (uint64_t base = begin & ~15ull; base < until; base += 16 * kStoredThreads) {
-    const uint64_t ob = base + 16 * (uint64_t)threadIdx.x;
+    const uint32_t w[5] = {v.x, v.y, v.z, v.w, v4};
+    const uint64_t at = ob;
+    ob += 16 * kStoredThreads;
+    load();
     uint32_t m = 0;
-    if (ob < until) {
-      const uint4 v = *reinterpret_cast<const uint4*>(in + ob);
-      const uint32_t w[5] = {v.x, v.y, v.z, v.w, *reinterpret_cast<const uint32_t*>(in + ob + 16)};
+    if (at < until) {
 #pragma unroll
       for (int k = 0; k < 16; k++) {
         const uint32_t sz = __funnelshift_r(w[k >> 2], w[(k >> 2) + 1 < 5 ? (k >> 2) + 1 : 4], 8 * (k & 3));
         m |= (((sz ^ (sz >> 16)) & 0xFFFFu) == 0xFFFFu ? 1u : 0u) << k;
       }
-      if (ob < begin) m &= 0xFFFFFFFFu << (begin - ob);
-      if (ob + 16 > until) m &= (1u << (until - ob)) - 1;
+      if (at < begin) m &= 0xFFFFFFFFu << (begin - at);
+      if (at + 16 > until) m &= (1u << (until - at)) - 1;
     }
-    while (m) {
-      const uint64_t off = ob + (uint64_t)(__ffs(m) - 1);
-      m &= m - 1;
-      uint64_t lo = 0, hi = 0;
-      if (stored_candidate(in, nbytes, off, from, to, to, lo, hi) &&
-          stored_successor_ok(in, nbytes, off + 4 + (in[off] | (in[off + 1] << 8)))) {
-        atomicMin(&s_first, (unsigned long long)off);
-        break;
+    bool found = false;
+    for (;;) {
+      // this lane's next candidate whose successor's header decides
+      uint64_t off = 0, hdr = 0;
+      while (m && !hdr) {
+        off = at + (uint64_t)(__ffs(m) - 1);
+        m &= m - 1;
+        uint64_t lo = 0, hi = 0;
+        if (!stored_candidate(in, nbytes, off, from, to, to, lo, hi)) continue;
+        const uint64_t next = off + 4 + (in[off] | (in[off + 1] << 8));
+        const int s = stored_successor(in, nbytes, next);
+        if (s == kSuccHeader) hdr = next * 8;
+        if (s == kSuccYes) {
+          atomicMin(&s_first, (unsigned long long)off);
+          found = true;
+          m = 0;
+        }
+      }
+      __syncwarp();
+      uint32_t b = __ballot_sync(0xFFFFFFFFu, hdr != 0);
+      if (!b) break;
+      for (; b; b &= b - 1) {
+        const int src = __ffs(b) - 1;
+        uint32_t mean;
+        const bool ok = dyn_candidate_warp(in, nbytes, __shfl_sync(0xFFFFFFFFu, hdr, src),
+                                           ht[threadIdx.x >> 5], threadIdx.x & 31, mean);
+        if (ok && (int)(threadIdx.x & 31) == src) {
+          atomicMin(&s_first, (unsigned long long)off);
+          found = true;
+          m = 0;
+        }
+        __syncwarp();
       }
     }
-    __syncthreads();
-    const bool found = s_first != ~0ull;
-    __syncthreads();  // every thread has read it before the next round writes
-    if (found) break;
+    if (__syncthreads_or(found)) break;
   }
   if (threadIdx.x == 0 && s_first != ~0ull) {
     uint64_t lo = 0, hi = 0;
@@ -121,8 +165,7 @@ struct FindWarp {
   uint32_t w[kFindSeg / 32 + 6];
   uint16_t list[kFindList];
   uint16_t full[kFindFull];
-  uint8_t sorted[32];  // dyn_candidate_warp: the precode's symbols in code order
-  uint8_t lut[128];    // and its table, entry: symbol | length << 5
+  HeaderTest ht;
   uint32_t n_full;
 };
 
@@ -135,7 +178,7 @@ struct FindWarp {
 // gives on average by its code (a code of length v stands for a probability of
 // 2^-v), in units of 2^-15.
 __device__ __noinline__ bool dyn_candidate_warp(const uint8_t* in, uint64_t nbytes, uint64_t bit,
-                                                FindWarp& W, int lane, uint32_t& mean) {
+                                                HeaderTest& W, int lane, uint32_t& mean) {
   constexpr uint32_t kAll = 0xFFFFFFFFu;
   const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
   const uint32_t below = (1u << lane) - 1;
@@ -351,7 +394,8 @@ __global__ void __launch_bounds__(32 * kFindWarps)
         const uint32_t x0 = (uint32_t)pb, x1 = (uint32_t)(pb >> 24);
         const uint32_t sum = leaf[x0 & 0xFFF] + leaf[(x0 >> 12) & 0xFFF] + leaf[x1 & 0xFFF] +
                              leaf[(x1 >> 12) & 0xFFF] + leaf[(uint32_t)(pb >> 48)];
-        const bool ok = act && (sum == 128 || sum == 64) && s0 + p + 17 + n <= nbits;
+        // a complete code, or a single code of one bit
+        const bool ok = act && (sum == 128 || (sum == 64 && !(pb & (pb - 1)))) && s0 + p + 17 + n <= nbits;
         const uint32_t b = __ballot_sync(0xFFFFFFFFu, ok);
         if (!b) continue;
         uint32_t n0 = W.n_full;
@@ -359,7 +403,7 @@ __global__ void __launch_bounds__(32 * kFindWarps)
         if (n0 + __popc(b) > kFindFull) {
           // (rare) the held ones first
           for (uint32_t j = 0; j < n0 && hit == kFindSeg; j++)
-            if (dyn_candidate_warp(in, nbytes, s0 + W.full[j], W, lane, mean)) hit = W.full[j];
+            if (dyn_candidate_warp(in, nbytes, s0 + W.full[j], W.ht, lane, mean)) hit = W.full[j];
           __syncwarp();
           n0 = 0;
         }
@@ -369,7 +413,7 @@ __global__ void __launch_bounds__(32 * kFindWarps)
       }
       const uint32_t n0 = W.n_full;
       for (uint32_t j = 0; j < n0 && hit == kFindSeg; j++)
-        if (dyn_candidate_warp(in, nbytes, s0 + W.full[j], W, lane, mean)) hit = W.full[j];
+        if (dyn_candidate_warp(in, nbytes, s0 + W.full[j], W.ht, lane, mean)) hit = W.full[j];
       __syncwarp();
       if (lane == 0) W.n_full = 0;
       __syncwarp();

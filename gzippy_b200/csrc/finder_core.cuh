@@ -210,22 +210,28 @@ static __device__ __forceinline__ bool dyn_candidate_fast(const uint8_t* in, uin
 // LEN/NLEN matches (about one per 64 KiB of random bytes) that would
 // otherwise start speculative chunks inside stored data.  A true stored
 // block followed by a fixed-Huffman block is given up as a start.
-static __device__ __forceinline__ bool stored_successor_ok(const uint8_t* in, uint64_t nbytes,
-                                                           uint64_t n) {
-  if (n >= nbytes) return false;
+// stored_successor: all but that predicate (kSuccHeader: it decides).
+enum : int { kSuccNo = 0, kSuccYes = 1, kSuccHeader = 2 };
+static __device__ __forceinline__ int stored_successor(const uint8_t* in, uint64_t nbytes, uint64_t n) {
+  if (n >= nbytes) return kSuccNo;
   const uint32_t bt = (in[n] >> 1) & 3;
   if (bt == 0) {
-    if (n + 5 > nbytes) return false;
+    if (n + 5 > nbytes) return kSuccNo;
     const uint32_t sz = in[n + 1] | (in[n + 2] << 8) | ((uint32_t)in[n + 3] << 16) |
                         ((uint32_t)in[n + 4] << 24);
-    return ((sz ^ (sz >> 16)) & 0xFFFF) == 0xFFFF;
+    return ((sz ^ (sz >> 16)) & 0xFFFF) == 0xFFFF ? kSuccYes : kSuccNo;
   }
-  if (bt != 2) return false;
+  if (bt != 2) return kSuccNo;
   const uint64_t bit = n * 8;
-  if (bit + 17 > nbytes * 8) return false;
+  if (bit + 17 > nbytes * 8) return kSuccNo;
   const uint32_t h = (uint32_t)peek_bits(in, nbytes, bit, 13);
-  if (((h >> 3) & 31) > 29 || ((h >> 8) & 31) > 29) return false;
-  return dyn_candidate_full(in, nbytes, bit);
+  if (((h >> 3) & 31) > 29 || ((h >> 8) & 31) > 29) return kSuccNo;
+  return kSuccHeader;
+}
+static __device__ __forceinline__ bool stored_successor_ok(const uint8_t* in, uint64_t nbytes,
+                                                           uint64_t n) {
+  const int s = stored_successor(in, nbytes, n);
+  return s == kSuccHeader ? dyn_candidate_full(in, nbytes, n * 8) : s == kSuccYes;
 }
 
 // Stored candidate test at byte offset `off` (find_uncompressed_blocks):
