@@ -373,15 +373,16 @@ constexpr uint64_t kMinPieceBits = 4ull << 13;
 constexpr uint64_t kTailBits = 48ull << 13;
 
 static uint64_t pick_chunk_bytes(uint64_t in_len) {
-  // several chunks per decoding warp on large inputs, which the
-  // longest-first order balances; smaller chunks for small inputs so the
-  // warps still fill.  Measured on the 1 GiB mixed stream, whole decode,
-  // one box: 48 KiB 43.5 ms, 40 KiB 44.1, 32 KiB 36.4-38.6, 24 KiB 35.3
-  // (the decode's tail shrinks faster than the finder and the per-chunk
-  // resolve work grow)
-  uint64_t c = 24 << 10;
-  if (in_len < (4ull << 20)) c = 16 << 10;
-  return c;
+  // Shorter chunks spread a small job over more SMs; longer ones need fewer
+  // header searches (a third of the decode's time at 24 KiB) and leave fewer
+  // markers.  Measured, whole call: 8.4 MB (342 chunks of 24 KiB) 0.64 ms at
+  // 24 KiB, 0.67 at 28; 22 MB of text 1.38 ms at 24, 1.33 at 28, 1.29 at 32;
+  // 81 MB of mixed data, where chunks differ more, 2.39 at 24, 2.31 at 28, 2.45
+  // at 32; 644 MB of it 15.3 ms at 24, 14.4 at 32, 13.4 at 48 and no less above.
+  // So from 16 MiB on about six chunks for each of 444 CTAs, 28 to 48 KiB each.
+  if (in_len < (4ull << 20)) return 16 << 10;
+  if (in_len < (16ull << 20)) return 24 << 10;
+  return std::min<uint64_t>(48 << 10, std::max<uint64_t>(28 << 10, in_len / 2800 & ~1023ull));
 }
 
 // Internal statuses that reach a caller as public codes: a page pool that
