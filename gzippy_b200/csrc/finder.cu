@@ -141,7 +141,7 @@ struct LeafLut {
 __device__ const LeafLut d_leaf_lut = LeafLut();
 
 // Dynamic headers.  The ranges still without a start are searched in segments
-// of kFindSeg bits, one warp per segment, segment 0 of every range first, then
+// of up to kFindSeg bits, one warp per segment, segment 0 of every range first, then
 // segment 1, and so on: a range's later segments are skipped once an earlier
 // one has a hit, while a small job's segments all run at once.  (One CTA per
 // range, walking it from its start, took 370 us for the 30 ranges of a 1 MB
@@ -151,7 +151,8 @@ __device__ const LeafLut d_leaf_lut = LeafLut();
 // list, the precode leaf count for 32 of them at a time; what is left
 // (about 1 in 100 of the list, in order) gets the full header test.
 constexpr int kFindWarps = 8;
-constexpr uint32_t kFindSeg = 8192;                // bits per segment
+constexpr uint32_t kFindSeg = 8192;                // bits per segment, at most
+constexpr uint32_t kFindSegMin = 1024;             // and at least
 constexpr uint32_t kFindPass = 4096;               // bits per screening pass
 // most survivors of a pass: three bits apart (BFINAL 0, BTYPE 10); near a
 // member's end, where BFINAL may be either, two, in passes half as long
@@ -313,7 +314,7 @@ __device__ __noinline__ bool dyn_candidate_warp(const uint8_t* in, uint64_t nbyt
 
 __global__ void __launch_bounds__(32 * kFindWarps)
     find_kernel(const uint8_t* __restrict__ in, const ChunkDesc* __restrict__ descs,
-                const uint32_t* __restrict__ spec, uint32_t n_spec, uint32_t n_seg,
+                const uint32_t* __restrict__ spec, uint32_t n_spec, uint32_t n_seg, uint32_t seg,
                 unsigned long long* best, uint32_t* next_item) {
   __shared__ uint16_t leaf[4096];
   __shared__ FindWarp fw[kFindWarps];
@@ -335,10 +336,10 @@ __global__ void __launch_bounds__(32 * kFindWarps)
     const uint64_t nbytes = d.in_end, nbits = nbytes * 8;
     const uint64_t from = d.guess_bit, to = min(d.limit_bit, nbits);
     // segments are cut at word boundaries of the input
-    const uint64_t s0 = (from & ~31ull) + (uint64_t)sg * kFindSeg;
+    const uint64_t s0 = (from & ~31ull) + (uint64_t)sg * seg;
     if (s0 >= to) continue;
     if (*(volatile unsigned long long*)&best[k] >> kMeanBits < s0) continue;
-    const uint32_t len = (uint32_t)min((uint64_t)kFindSeg, to - s0);
+    const uint32_t len = (uint32_t)min((uint64_t)seg, to - s0);
     const uint32_t first = from > s0 ? (uint32_t)(from - s0) : 0u;
     // the segment's words, and the 81 bits after it (a header up to its precode)
     __syncwarp();
@@ -629,10 +630,17 @@ cudaError_t launch_finder(const uint8_t* in, ChunkDesc* descs, const uint32_t* s
   unsigned long long* best = reinterpret_cast<unsigned long long*>(best64);
   stored_kernel<<<n_spec, kStoredThreads, 0, stream>>>(in, descs, spec, n_spec, best);
   sync_kernel<<<n_spec, kSyncOffsets, 0, stream>>>(in, descs, spec, n_spec, n_sync);
-  const uint32_t n_seg = (uint32_t)((max_bits + 31) / kFindSeg + 1);
+  // Shorter segments while a small search leaves warps without one: a segment's
+  // four or five false candidates are tested one after another.  31 ranges of a
+  // 1 MiB stream: 102 us in segments of 8192 bits, 42 of 1024.
+  const uint64_t warps = (uint64_t)sms * 3 * kFindWarps;  // resident
+  uint32_t seg = kFindSeg;
+  while (seg > kFindSegMin && n_spec * ((max_bits + 31) / (seg / 2) + 1) <= warps) seg /= 2;
+  const uint32_t n_seg = (uint32_t)((max_bits + 31) / seg + 1);
   const uint64_t ctas = ((uint64_t)n_spec * n_seg + kFindWarps - 1) / kFindWarps;
   const uint32_t grid = (uint32_t)(ctas < (uint64_t)sms * 4 ? ctas : (uint64_t)sms * 4);
-  find_kernel<<<grid, 32 * kFindWarps, 0, stream>>>(in, descs, spec, n_spec, n_seg, best, next_item);
+  find_kernel<<<grid, 32 * kFindWarps, 0, stream>>>(in, descs, spec, n_spec, n_seg, seg, best,
+                                                    next_item);
   assign_kernel<<<(n_spec + 127) / 128, 128, 0, stream>>>(in, descs, spec, n_spec, best, ratio,
                                                          next_item);
   return cudaGetLastError();

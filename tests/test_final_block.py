@@ -55,3 +55,14 @@ def test_patterns_inside_coded_data(ctx):
     co = zlib.compressobj(6, zlib.DEFLATED, -15, 8, zlib.Z_HUFFMAN_ONLY)
     comp = co.compress(plain) + co.flush()
     assert ctx.inflate_raw(comp) == plain
+
+
+@pytest.mark.parametrize("bits", [1000, 1024, 1056, 8191, 16384, 70000, 196608])
+def test_search_of_few_and_of_many_ranges(ctx, bits):
+    """A small search is cut into shorter segments, one warp each: the first
+    start of a range is the same in both."""
+    comp = W.gzip_member(W.content(W.MARKOV, 8, 400000), 6)
+    total = comp.size * 8
+    for lo in range(100, total - bits, max(bits, 100003)):
+        alone = ctx.debug_find(comp, [(lo, lo + bits)])
+        assert ctx.debug_find(comp, [(lo, lo + bits)] * 600) == alone * 600
