@@ -130,6 +130,11 @@ struct PinnedAlloc {
 };
 template <typename T>
 using PinnedVec = std::vector<T, PinnedAlloc<T>>;
+// room for n elements; twice that when it has to grow, since growing is dear
+template <typename T>
+void make_room(PinnedVec<T>& v, size_t n) {
+  if (n > v.capacity()) v.reserve(2 * n);
+}
 
 // Byte ranges packed into one page-locked buffer, for one copy to the device.
 struct Pack {
@@ -283,8 +288,9 @@ struct gzgpu_ctx {
     const int blocks = (int)std::min<uint32_t>((uint32_t)decode_blocks, std::max(n_work, 1u));
     // Up to two chunks per SM: CTAs of 1,024 threads, one chunk after the other.
     // A chunk's decode is then what the job waits for, and four times the
-    // threads shorten it (64 MiB of byte runs, 137 chunks: 1.27 -> 0.72 ms; 232
-    // chunks of small streams: 0.42 -> 0.32).  From 300 chunks on the SMs are
+    // threads shorten it (64 MiB of byte runs, 137 chunks, the last of two
+    // blocks: 1.27 -> 0.72 ms, 0.45 since it is two chunks; 232 chunks of small
+    // streams: 0.42 -> 0.32).  From 300 chunks on the SMs are
     // better filled by three CTAs of 256 (342 chunks: 0.25 ms, wide 0.37).
     const bool wide = n_work <= 2 * (uint32_t)sms;
     PagePool pool{pages.as<uint16_t>(), owner.as<uint32_t>(), seq.as<uint32_t>(),
@@ -690,8 +696,8 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   const uint64_t cbits = cb * 8;
   size_t n_mems = 0;
   for (const auto& m : mems) n_mems += m.size();
-  hd.reserve(n_mems + (size_t)(total_in / cb) + 64);  // (page-locked: growing is dear)
-  hspec.reserve((size_t)(total_in / cb) + 64);
+  make_room(hd, n_mems + (size_t)(total_in / cb) + 64);
+  make_room(hspec, (size_t)(total_in / cb) + 64);
   for (uint32_t s = 0; s < ns; s++) {
     c0[s] = (uint32_t)hd.size();
     for (const Mem& m : mems[s]) {
@@ -763,7 +769,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
     PinnedVec<ChunkDesc>& hd2 = hd_cut;
     hd2.clear();
     std::vector<uint32_t> newpos(n_grid + 1), hspec2;
-    hd2.reserve(n_grid + n_grid / 4);
+    make_room(hd2, n_grid + n_grid / 4);
     for (uint32_t i = 0; i < n_grid; i++) {
       newpos[i] = (uint32_t)hd2.size();
       hd2.push_back(hd[i]);
@@ -872,6 +878,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
     if ((rc = check(launch_decode(counters.as<uint32_t>() + 1, n_decode)))) return rc;
     cudaEventRecord(ev[9], st);
     hd.resize(n_grid);
+    make_room(hr, n_grid);
     hr.resize(n_grid);
     if ((rc = fetch_results(0, n_grid, true))) return rc;
     float t = 0;
