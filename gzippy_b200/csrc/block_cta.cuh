@@ -873,6 +873,9 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB, NT>* S, const PageP
       if (b0 >= n) break;
       bpos = bend;
       load_batch();
+      // only the distance of the match before is left: no position, so no window
+      // (at a page's end it would take a page that gets no entry)
+      if (bend == bpos) break;
     }
   }
   __syncthreads();
