@@ -24,45 +24,10 @@
 #include <cstdint>
 
 #include "common.cuh"
+#include "markers.cuh"
 #include "resolve.cuh"
 
 namespace gzgpu {
-
-// A chunk before a unit's own: how many bytes before that one it starts, its
-// last page's index, and its last two pages.
-struct NearChunk {
-  uint32_t start, last_seq, last_page, prev_page;
-};
-constexpr uint32_t kNear = 8;  // kept at hand
-
-__device__ __forceinline__ NearChunk near_chunk(const PlacedChunk& c, uint64_t off) {
-  return NearChunk{(uint32_t)min(off - c.out_off, (uint64_t)0xFFFFFFFFu), c.last_seq, c.last_page, c.prev_page};
-}
-
-// The byte that marker v of placed chunk k names, `room` bytes after its
-// member's first.  Distances count back from the chunk's start: v names the
-// byte 65536 - v before it; an entry found there that is a marker of its own
-// chunk counts on from that chunk's start.  (A chunk further back than 32 bits
-// count lies past the reach of any window but one of chunks without bytes.)
-__device__ __forceinline__ uint32_t follow_marker(const PlacedChunk* __restrict__ placed,
-                                                  const NearChunk* near, uint32_t k, uint64_t off,
-                                                  uint64_t room, uint32_t v, const PagePool& pool) {
-  uint32_t at = 0, back = 0;  // the chunk the marker belongs to: where it starts, which it is
-  for (;;) {
-    at += 2 * kMarkerBase - v;
-    if (at > room) return 0;  // before the member: the zero window
-    NearChunk c;
-    do {
-      c = back < kNear ? near[back] : near_chunk(placed[k - 1 - back], off);
-      back++;
-    } while (c.start < at);
-    const uint32_t q = c.start - at;  // the entry, one of its last 32 Ki
-    const uint32_t page = (q >> 16) == c.last_seq ? c.last_page : c.prev_page;
-    v = pool.data[(size_t)page * kPageEntries + (q & (kPageEntries - 1))];
-    if (v < kMarkerBase) return v;
-    at = c.start;
-  }
-}
 
 // One warp per unit of kResolveUnit entries of a page: literal bytes go to
 // shared memory, markers to a list, which the lanes then follow one marker each
@@ -108,7 +73,7 @@ __global__ void __launch_bounds__(kResolveThreads, 6)
     x[s] = e < n ? *reinterpret_cast<const uint4*>(src + e) : make_uint4(0, 0, 0, 0);
   }
   const uint64_t off = placed[k].out_off, moff = placed[k].member_off;
-  if (lane < kNear && lane < k) W.near[lane] = near_chunk(placed[k - 1 - lane], off);
+  if (lane < kNear && lane < k) W.near[lane] = near_chunk(placed[k - 1 - lane]);
   uint32_t n_list = 0;
 #pragma unroll
   for (uint32_t s = 0; s < 2; s++) {
@@ -137,7 +102,10 @@ __global__ void __launch_bounds__(kResolveThreads, 6)
   __syncwarp();
   for (uint32_t i = lane; i < n_list; i += 32) {
     const uint32_t item = W.list[i];
-    W.bytes[item >> 16] = (uint8_t)follow_marker(placed, W.near, k, off, off - moff, item & 0xFFFFu, pool);
+    W.bytes[item >> 16] = (uint8_t)follow_marker(
+        placed, W.near, k, off, moff, item & 0xFFFFu, [&](uint32_t page, uint32_t e) -> uint32_t {
+          return pool.data[(size_t)page * kPageEntries + e];
+        });
   }
   __syncwarp();
   // the unit's bytes: aligned 16 of the output, then what lies around them
