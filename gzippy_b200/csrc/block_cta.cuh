@@ -18,9 +18,8 @@
 //      distance), written by one decode of each range.
 //   4. the tokens are expanded in windows of kWin output positions (see
 //      expand_tokens), which leave as coalesced stores to the pages.
-// Threads leave the data-dependent loops at different times; a warp barrier
-// joins its lanes before every barrier of the CTA, which all lanes of a warp
-// have to reach together.
+// Threads leave the data-dependent loops at different times; every barrier of
+// the CTA joins each warp's lanes first (barrier.cuh).
 // What bounds a block is its serial chain of code lookups; the ranges cut
 // that chain into up to 256 pieces.  Ranges of 512 bits end in step after a
 // wrong start for 98 % of text, 88 % of byte runs and 59 % of noisy ramps
@@ -34,6 +33,7 @@
 #pragma once
 #include <cstdint>
 
+#include "barrier.cuh"
 #include "common.cuh"
 #include "huffman.cuh"
 #include "inflate.cuh"
@@ -162,7 +162,7 @@ __device__ __forceinline__ uint32_t cta_scan(CtaSmem<LB, NT>* S, uint32_t par, u
     if (lane >= d) x += u;
   }
   if (lane == 31) S->scan[par][warp] = x;
-  __syncthreads();
+  cta_sync();
   uint32_t pa = 0;
   ta = 0;
   if constexpr (NT <= 256) {
@@ -480,7 +480,7 @@ __device__ __forceinline__ int32_t cta_read_lens(const uint8_t* __restrict__ in,
     S->pre_lut[tid] = L > 7 ? 0u : S->lit_ent[(rev >> (15 - L)) + S->lit.base[L]];
   }
   for (uint32_t i = tid; i < 320; i += NT) S->lens[i] = 0;
-  __syncthreads();
+  cta_sync();
   // [4:0] symbol, [12:8] bits taken (0: no such code), [23:16] lengths covered
   auto at = [&](uint32_t i) {
     const uint32_t p = (uint32_t)(pos & 31) + i, j = p >> 5;
@@ -496,13 +496,13 @@ __device__ __forceinline__ int32_t cta_read_lens(const uint8_t* __restrict__ in,
     const uint32_t n = (at(i) >> 8) & 31;
     S->hop[0][i] = n && i + n < kHdrBits ? (uint16_t)(i + n) : (uint16_t)0xFFFF;
   }
-  __syncthreads();
+  cta_sync();
   for (int k = 0; k < 3; k++) {
     for (uint32_t i = tid; i < kHdrBits; i += NT) {
       const uint32_t h = S->hop[k][i];
       S->hop[k + 1][i] = h == 0xFFFF ? (uint16_t)0xFFFF : S->hop[k][h];
     }
-    __syncthreads();
+    cta_sync();
   }
   if (tid == 0) {
     uint32_t p = 0;
@@ -511,7 +511,7 @@ __device__ __forceinline__ int32_t cta_read_lens(const uint8_t* __restrict__ in,
       if (p != 0xFFFF) p = S->hop[3][p];
     }
   }
-  __syncthreads();
+  cta_sync();
   // symbols 2 tid and 2 tid + 1
   uint32_t e[2] = {0, 0}, p[2] = {0xFFFF, 0xFFFF};
   if (tid < kHdrSyms / 2) {
@@ -532,7 +532,7 @@ __device__ __forceinline__ int32_t cta_read_lens(const uint8_t* __restrict__ in,
   uint32_t sum;
   uint32_t o = cta_scan(S, 0, (e[0] >> 16) + (e[1] >> 16), sum);
   if (tid == 0) S->c.hdr_end = kNone;
-  __syncthreads();
+  cta_sync();
   bool bad = false;
 #pragma unroll
   for (int k = 0; k < 2; k++) {
@@ -551,15 +551,14 @@ __device__ __forceinline__ int32_t cta_read_lens(const uint8_t* __restrict__ in,
     }
     o += n;
   }
-  __syncwarp();
-  bad = __syncthreads_or(bad) || S->c.hdr_end == kNone || S->lens[256] == 0;
+  bad = cta_sync_or(bad) || S->c.hdr_end == kNone || S->lens[256] == 0;
   // past the readable input (the reader ran 96 bits ahead): cut off, or over the abort bit
   const uint64_t end = pos + (S->c.hdr_end == kNone ? 0u : S->c.hdr_end);
-  __syncthreads();
+  cta_sync();
   if (end + 96 > S->c.limit_words * 32) return end + 96 > trunc * 32 ? kTruncated : kOvershoot;
   if (bad) return kBadDeflate;
   if (tid == 0 && move) S->c.pos = end;
-  __syncthreads();
+  cta_sync();
   return kOk;
 }
 
@@ -577,7 +576,7 @@ __device__ __forceinline__ bool cta_build_tables(CtaSmem<LB, NT>* S) {
       ok = index_code(S->lens + 288, (int)S->c.ndist, &S->dist, S->dist_ent, lane, tok_dist_entry);
     if (lane == 0) S->c.build_ok[warp] = ok;
   }
-  __syncthreads();
+  cta_sync();
   if (!S->c.build_ok[0] || !S->c.build_ok[1]) return false;
   uint32_t lim[LB + 1];
 #pragma unroll
@@ -589,7 +588,7 @@ __device__ __forceinline__ bool cta_build_tables(CtaSmem<LB, NT>* S) {
   for (uint32_t i = threadIdx.x; i < (1u << kCtaDistBits); i += NT)
     S->lut[(1u << LB) + i] = lut_value<(int)kCtaDistBits>(i, lim, &S->dist, S->dist_ent,
                                                           kEntStop | kEntLen | kStopLong << 8);
-  __syncthreads();
+  cta_sync();
   return true;
 }
 
@@ -600,7 +599,7 @@ template <int LB, int NT>
 __device__ __forceinline__ bool cta_page(CtaSmem<LB, NT>* S, const PagePool& pool, uint64_t w0) {
   const uint32_t s = (uint32_t)(w0 >> 16);
   if (S->c.page_cur != kNoPage && S->c.page_seq == s) return true;
-  __syncthreads();
+  cta_sync();
   if (threadIdx.x == 0) {
     uint32_t p = atomicAdd(pool.next, 1u);
     if (p < pool.cap) {
@@ -614,7 +613,7 @@ __device__ __forceinline__ bool cta_page(CtaSmem<LB, NT>* S, const PagePool& poo
     S->c.page_seq = s;
     S->c.n_pages++;
   }
-  __syncthreads();
+  cta_sync();
   return S->c.page_cur != kNoPage;
 }
 
@@ -651,7 +650,7 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB, NT>* S, const PageP
   if (tid == 0) {
     S->c.carry_len = S->c.mark_max = 0;
   }
-  __syncthreads();
+  cta_sync();
   // rec: what the slot puts at its position, a literal or a match's record
   // (length and distance - 1)
   auto load_batch = [&]() {
@@ -708,8 +707,7 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB, NT>* S, const PageP
       bpos = bend;
       load_batch();
     }
-    __syncwarp();
-    const bool matches = __syncthreads_or((int)any_match);
+    const bool matches = cta_sync_or(any_match != 0);
     const uint32_t hi = min(wend, bend) - wbase, l0 = lo - wbase;
     uint16_t* page = pool.data + (size_t)S->c.page_cur * kPageEntries +
                      ((uint32_t)(base + wbase) & (kPageEntries - 1));
@@ -812,8 +810,7 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB, NT>* S, const PageP
       uint32_t left = 0;
 #pragma unroll
       for (uint32_t i = 0; i < kWinPer; i++) left |= (cover >> i) & 1 ? st[i] : 0u;
-      __syncwarp();
-      const bool any_ref = __syncthreads_or((int)(left >> 31));
+      const bool any_ref = cta_sync_or(left >> 31);
       if (hi - 1 - e0 < kWinPer) {  // the last position's match may go on in the next window
         S->c.carry_ms = ms - (int32_t)kWin;
         S->c.carry_len = ms + (int32_t)ml > (int32_t)hi ? ml : 0u;
@@ -825,7 +822,7 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB, NT>* S, const PageP
           reinterpret_cast<uint4*>(stage)[2 * tid] = make_uint4(st[0], st[1], st[2], st[3]);
           reinterpret_cast<uint4*>(stage)[2 * tid + 1] = make_uint4(st[4], st[5], st[6], st[7]);
         }
-        __syncthreads();
+        cta_sync();
         // A reference takes its source's value, or the source's own reference,
         // always further back: every thread follows its own to their ends,
         // and what it learns on the way shortens the others' paths.
@@ -878,7 +875,7 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB, NT>* S, const PageP
       if (bend == bpos) break;
     }
   }
-  __syncthreads();
+  cta_sync();
   if (tid == 0) {
     S->c.o = base + lo;
     if (S->c.mark_max) S->c.marker_end = base + S->c.mark_max;
@@ -903,7 +900,7 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
     const uint64_t target = S->c.sync_target;
     const uint64_t w0 = pos >> 5;
     if (target == pos || w0 + 4 > limit) {
-      __syncthreads();
+      cta_sync();
       if (tid == 0) {
         if (target == pos) S->c.synced = 1;
         else S->c.status = w0 + 4 > trunc ? kTruncated : kOvershoot;
@@ -931,7 +928,7 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
     // walk again go to the first threads, so that few of them are few warps.
     uint32_t last = kNone;  // range that holds the end of the block (kNone: not in this round)
     for (;;) {
-      __syncthreads();
+      cta_sync();
       const uint32_t st = active ? S->start[tid] : 0u, inf = active ? S->info[tid] : 0u;
       const uint32_t s1 = active && tid ? S->end[tid - 1] : st;
       const bool need = active && (s1 != st || (inf & kInfoOn));
@@ -942,7 +939,7 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
         S->term[warp] = tb;
       }
       if (need) S->start[tid] = s1;
-      __syncthreads();
+      cta_sync();
       const uint32_t mn = lane < NT / 32 ? S->need[lane] : 0u;
       const uint32_t mt = lane < NT / 32 ? S->term[lane] : 0u;
       const uint32_t bn = __ballot_sync(0xFFFFFFFFu, mn != 0), bt = __ballot_sync(0xFFFFFFFFu, mt != 0);
@@ -960,7 +957,7 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
       const uint32_t before = __shfl_sync(0xFFFFFFFFu, upto - __popc(mn), warp);
       const uint32_t n_need = __shfl_sync(0xFFFFFFFFu, upto, NT / 32 - 1);
       if (need) S->list[before + __popc(nb & ((1u << lane) - 1))] = (uint16_t)tid;
-      __syncthreads();
+      cta_sync();
       if (tid < n_need) {
         const uint32_t id = S->list[tid], f = p0 + id * r;
         walk_range<LB, NT>(S, base, f, r, min(f + r, pend), id, false, true);
@@ -975,7 +972,7 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
     const uint32_t my_slots = my_info & 0xFFFFu, my_term = (my_info / kInfoTerm) & 3;
     const uint32_t slot0 = cta_scan(S, 0, my_slots, ts);
     if (ts > kTokCap) {
-      const uint32_t fit = (uint32_t)__syncthreads_count(in_use && slot0 + my_slots <= kTokCap);
+      const uint32_t fit = (uint32_t)cta_sync_count(in_use && slot0 + my_slots <= kTokCap);
       if (tid == fit) {
         S->c.round_slots = slot0;
         S->c.round_pos = my_start;  // = the end of range fit - 1
@@ -992,37 +989,36 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
       S->c.round_kind = my_term;
       S->c.round_pos = my_term ? S->term_pos[tid] : S->end[tid];
     }
-    __syncthreads();
+    cta_sync();
     const uint32_t n_lanes = S->c.round_lanes, n_slots = S->c.round_slots;
     const uint32_t kind = S->c.round_kind;
     const uint64_t new_pos = w0 * 32 + S->c.round_pos;
     if (kind == kTermBad) {
-      __syncthreads();
+      cta_sync();
       if (tid == 0) S->c.status = kBadDeflate;
       break;
     }
     if (tid < n_lanes) write_tokens<LB, NT>(S, base, my_start, my_slots, S->tok + slot0);
-    __syncwarp();
-    __syncthreads();
+    cta_sync();
     // 4. expansion
     if (n_slots) {
       const int32_t st = expand_tokens<LB, NT>(S, pool, n_slots, zero_window);
       if (st != kOk) {
-        __syncthreads();
+        cta_sync();
         if (tid == 0) S->c.status = st;
         break;
       }
     }
     const bool passed = S->c.passed_bit < new_pos;
-    __syncthreads();
+    cta_sync();
     if (tid == 0) {
       S->c.pos = new_pos;
       if (kind == kTermNone && passed && new_pos != target) S->c.passed = 1;
     }
-    __syncthreads();
+    cta_sync();
     if (kind == kTermEob || S->c.passed) break;
   }
-  __syncthreads();
+  cta_sync();
 }
 
 // A stored block's bytes to the chunk's pages, four entries per thread.
@@ -1056,13 +1052,13 @@ __device__ __forceinline__ void cta_stored(const uint8_t* __restrict__ in, CtaSm
     o += n;
     left -= n;
   }
-  __syncthreads();
+  cta_sync();
   if (threadIdx.x == 0) {
     S->c.pos = byte * 8;
     S->c.o = o;
     if (!ok) S->c.status = kPoolExhausted;
   }
-  __syncthreads();
+  cta_sync();
 }
 
 // what the chunk does next
@@ -1292,7 +1288,7 @@ __device__ __forceinline__ void cta_decode_chunk(const uint8_t* __restrict__ in,
   const bool zero_window = (c.flags & kChunkMemberFirst) != 0;
   for (;;) {
     if (tid < 32) cta_header<LB, NT>(in, descs, S, pool, sync, tid);
-    __syncthreads();
+    cta_sync();
     const int32_t act = c.act;
     if (act == kActDone) break;
     if (act == kActStored) {
@@ -1305,14 +1301,14 @@ __device__ __forceinline__ void cta_decode_chunk(const uint8_t* __restrict__ in,
           c.fixed_tables = st == kOk && c.btype == 1;
           if (st != kOk) c.status = st;
         }
-        __syncthreads();
+        cta_sync();
         if (st != kOk) break;
       }
       cta_block<LB, NT>(in, S, pool, zero_window);
     }
     if (c.status != kOk || c.synced) break;
     const bool passed = c.passed != 0, fin = c.bfinal != 0;
-    __syncthreads();
+    cta_sync();
     if (tid == 0) {
       if (passed) {
         c.passed = 0;
@@ -1325,7 +1321,7 @@ __device__ __forceinline__ void cta_decode_chunk(const uint8_t* __restrict__ in,
     }
     if (!passed && fin) break;
   }
-  __syncthreads();
+  cta_sync();
   if (tid == 0) {
     if (c.status == kOk && c.pos > c.in_end * 8) c.status = kTruncated;
     res->end_bit = c.pos;
@@ -1342,7 +1338,7 @@ __device__ __forceinline__ void cta_decode_chunk(const uint8_t* __restrict__ in,
     res->sync_end = c.synced;
     res->end_hdr_bit = c.synced ? c.blk_hdr : 0;
   }
-  __syncthreads();
+  cta_sync();
 }
 
 // Thread 0: the state a chunk's decode begins with.

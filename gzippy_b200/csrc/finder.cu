@@ -5,6 +5,7 @@
 // warps of one CTA.
 #include <cstdint>
 
+#include "barrier.cuh"
 #include "common.cuh"
 #include "finder.cuh"
 #include "finder_core.cuh"
@@ -49,7 +50,7 @@ __global__ void __launch_bounds__(kStoredThreads)
   if (d.flags & kChunkValid) return;
   const uint64_t from = d.guess_bit, to = d.limit_bit, nbytes = d.in_end;
   if (threadIdx.x == 0) s_first = ~0ull;
-  __syncthreads();
+  cta_sync();
   const uint64_t begin = max((from + 3 + 7) / 8, (uint64_t)2);
   const uint64_t until = nbytes >= 5 ? min((to + 7) / 8, nbytes - 4) : 0;
   // (the next round's bytes are on their way while this one's are tested)
@@ -111,7 +112,7 @@ __global__ void __launch_bounds__(kStoredThreads)
         __syncwarp();
       }
     }
-    if (__syncthreads_or(found)) break;
+    if (cta_sync_or(found)) break;
   }
   if (threadIdx.x == 0 && s_first != ~0ull) {
     uint64_t lo = 0, hi = 0;
@@ -322,7 +323,7 @@ __global__ void __launch_bounds__(32 * kFindWarps)
   FindWarp& W = fw[threadIdx.x >> 5];
   for (uint32_t i = threadIdx.x; i < 4096 / 8; i += 32 * kFindWarps)
     reinterpret_cast<uint4*>(leaf)[i] = reinterpret_cast<const uint4*>(d_leaf_lut.v)[i];
-  __syncthreads();
+  cta_sync();
   const uint32_t* in32 = reinterpret_cast<const uint32_t*>(in);
   const uint64_t n_items = (uint64_t)n_spec * n_seg;
   for (;;) {
@@ -475,7 +476,7 @@ __global__ void __launch_bounds__(kSyncOffsets)
     dlut[tid] = dc >= 30 ? 0xFF : (uint8_t)(5 + f_dist_extra[dc]);
   }
   if (tid == 0) top = 0;
-  __syncthreads();
+  cta_sync();
   const uint32_t rel = (uint32_t)(from & 31);  // positions below count from the word of `from`
   const uint32_t goal = rel + kSyncOffsets + (uint32_t)kSyncSpan;
   uint32_t p = rel + tid;
@@ -499,18 +500,18 @@ __global__ void __launch_bounds__(kSyncOffsets)
         p += 3;
       }
     }
-    if (__syncthreads_count(ok) < 2) return;
+    if (cta_sync_count(ok) < 2) return;
     if (e == goal) break;
   }
   ends[tid] = ok ? p : 0u;
-  __syncthreads();
+  cta_sync();
   if (ok) {
     uint32_t c = 0;
     for (uint32_t i = 0; i < kSyncOffsets; i++) c += ends[i] == p;
     // most walks first, then the lower position
     if (c >= 2) atomicMax(&top, (unsigned long long)c << 32 | (0xFFFFFFFFu - p));
   }
-  __syncthreads();
+  cta_sync();
   if (tid == 0 && top) {
     d.lo_bit = d.start_bit = (from & ~31ull) + (0xFFFFFFFFu - (uint32_t)top);
     d.flags |= kChunkValid | kChunkSync;
@@ -598,7 +599,7 @@ __global__ void __launch_bounds__(1024)
                  uint32_t* work, uint32_t* n_work) {
   __shared__ uint32_t hist[kCostBuckets], base[kCostBuckets];
   if (threadIdx.x < kCostBuckets) hist[threadIdx.x] = 0;
-  __syncthreads();
+  cta_sync();
   auto bucket = [&](uint32_t i) {
     const float c = fmaxf(cost[i], 0.f) + 1.f;
     const int b = (int)(4.f * __log2f(c));
@@ -606,7 +607,7 @@ __global__ void __launch_bounds__(1024)
   };
   for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
     if (descs[i].flags & kChunkValid) atomicAdd(&hist[bucket(i)], 1u);
-  __syncthreads();
+  cta_sync();
   if (threadIdx.x == 0) {
     uint32_t a = 0;
     for (int b = 0; b < kCostBuckets; b++) {
@@ -615,7 +616,7 @@ __global__ void __launch_bounds__(1024)
     }
     *n_work = a;
   }
-  __syncthreads();
+  cta_sync();
   for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
     if (descs[i].flags & kChunkValid) work[atomicAdd(&base[bucket(i)], 1u)] = i;
 }

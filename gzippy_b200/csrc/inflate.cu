@@ -26,6 +26,7 @@
 // (chunk_fetcher.rs speculative_decode_find_boundary :2616-2740).
 #include <cstdint>
 
+#include "barrier.cuh"
 #include "block_cta.cuh"
 #include "common.cuh"
 #include "finder_core.cuh"
@@ -486,7 +487,7 @@ __global__ void __launch_bounds__(NT, MINB)
   const bool sync = *n_sync != 0;
   if (tid == 0) S->c.fixed_tables = 0;
   for (;;) {
-    __syncthreads();
+    cta_sync();
     if (tid == 0) {
       const uint32_t w = atomicAdd(work_counter, 1u);
       S->c.cid = w < n_work ? work[w] : kNone;
@@ -498,7 +499,7 @@ __global__ void __launch_bounds__(NT, MINB)
         cta_begin(S->c, d, S->c.cid, d.flags >> kGenBaseShift);
       }
     }
-    __syncthreads();
+    cta_sync();
     const uint32_t cid = S->c.cid;
     if (cid == kNone) break;
     for (;;) {
@@ -530,7 +531,7 @@ __global__ void __launch_bounds__(NT, MINB)
           }
         }
       }
-      __syncthreads();
+      cta_sync();
       if (!S->c.again) break;
     }
   }
@@ -654,7 +655,7 @@ __global__ void __launch_bounds__(kSyncOffsets)
     table = t;
     ok = 0;
   }
-  __syncthreads();
+  cta_sync();
   if (!table) return;
   const int lane = threadIdx.x & 31;
   const uint64_t trunc_words = (nbytes * 8 + 31) / 32 + 5;
@@ -668,7 +669,7 @@ __global__ void __launch_bounds__(kSyncOffsets)
     const int32_t st = read_tables<LB>(br, 2, &T, trunc_words, lane);
     if (lane == 0) ok = st == kOk;
   }
-  __syncthreads();
+  cta_sync();
   if (!ok) return;
   uint64_t p = from + threadIdx.x, e = kSyncFail;
   while (p < target) {
@@ -680,7 +681,7 @@ __global__ void __launch_bounds__(kSyncOffsets)
     if (p >= target) e = p;
   }
   ends[threadIdx.x] = e;
-  __syncthreads();
+  cta_sync();
   if (threadIdx.x == 0) {
     uint64_t best = kSyncFail;
     uint32_t best_n = 1;
@@ -803,7 +804,7 @@ __global__ void __launch_bounds__(kWideThreads)
   uint64_t total = 0, pos = 0;
   bool too_small = false;  // some member did not fit out_cap
   for (uint32_t member = 0;; member++) {
-    __syncthreads();
+    cta_sync();
     if (tid == 0) {
       m_act = -1;
       m_pos = 0;
@@ -832,7 +833,7 @@ __global__ void __launch_bounds__(kWideThreads)
         cta_begin(S->c, d, 0, 0);
       }
     }
-    __syncthreads();
+    cta_sync();
     if (m_act >= 0) {
       status = m_act;
       break;
@@ -865,7 +866,7 @@ __global__ void __launch_bounds__(kWideThreads)
     uint32_t c = 0xFFFFFFFFu;
     for (uint64_t q = b0; q < b1; q++) c = (c >> 8) ^ crc_tab[(c ^ (uint32_t)scratch->pages[q]) & 0xFF];
     slice_crc[tid] = ~c;
-    __syncthreads();
+    cta_sync();
     if (tid == 0) {
       uint32_t crc = 0;
       const uint32_t xp = na_x_pow_8n(per);
@@ -878,7 +879,7 @@ __global__ void __launch_bounds__(kWideThreads)
       const uint32_t eisz = t[4] | (t[5] << 8) | ((uint32_t)t[6] << 16) | ((uint32_t)t[7] << 24);
       m_act = (uint32_t)out_len != eisz ? kSizeMismatch : (crc != ecrc ? kCrcMismatch : kOk);
     }
-    __syncthreads();
+    cta_sync();
     status = m_act;
     total += out_len;
     pos = trailer + 8;

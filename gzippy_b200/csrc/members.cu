@@ -14,6 +14,7 @@
 //   start.
 #include <cstdint>
 
+#include "barrier.cuh"
 #include "common.cuh"
 #include "members.cuh"
 
@@ -91,14 +92,12 @@ __global__ void member_scan_kernel(const uint8_t* __restrict__ in, const ScanUni
   for (uint32_t u = blockIdx.x; u < n_units; u += gridDim.x) {
     const ScanUnit su = units[u];
     const uint64_t base = s_off[su.stream], len = s_len[su.stream];
-    __syncwarp();
-    __syncthreads();  // the unit before has read s_info
+    cta_sync();  // the unit before has read s_info
     if (threadIdx.x == 0) {
       if (su.stream != known) s_info = stream_info(in, base, len);
       if (su.begin == 0) info[su.stream] = s_info;
     }
-    __syncwarp();
-    __syncthreads();
+    cta_sync();
     known = su.stream;
     const StreamInfo si = s_info;
     if (si.status != kOk) continue;

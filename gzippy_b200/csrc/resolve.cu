@@ -23,6 +23,7 @@
 //   member_check : each member's CRC32 and ISIZE against its trailer
 #include <cstdint>
 
+#include "barrier.cuh"
 #include "common.cuh"
 #include "markers.cuh"
 #include "resolve.cuh"
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(kCrcThreads)
   for (uint32_t i = threadIdx.x; i < 256 * 32; i += kCrcThreads) ltab[i] = d_crc_tab[i >> 5];
   for (uint32_t i = threadIdx.x; i < kCrcLevels * 256; i += kCrcThreads)
     reinterpret_cast<uint4*>(shf)[i] = reinterpret_cast<const uint4*>(&d_crc_shift[0][0][0])[i];
-  __syncthreads();
+  cta_sync();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (uint32_t b0 = blockIdx.x; b0 < n; b0 += kCrcTurns * gridDim.x) {
     uint32_t turns = 0;
@@ -278,8 +279,7 @@ __global__ void __launch_bounds__(kCrcThreads)
       }
       if (lane == 0) part[turns * kWarps + warp] = c;
     }
-    __syncwarp();
-    __syncthreads();
+    cta_sync();
     for (uint32_t t = warp; t < turns; t += kWarps) {
       const CrcBlock blk = blocks[b0 + t * gridDim.x];
       uint32_t c = lane < kWarps ? part[t * kWarps + lane] : 0u;
@@ -291,8 +291,7 @@ __global__ void __launch_bounds__(kCrcThreads)
       if (blk.after) c = gf2_mulmod(x_pow_8n_warp(blk.after, lane), c);
       if (lane == 0) atomicXor(mem_raw + blk.member, c);
     }
-    __syncwarp();
-    __syncthreads();
+    cta_sync();
   }
 }
 
