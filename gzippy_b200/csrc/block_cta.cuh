@@ -93,7 +93,9 @@ struct CtaCtl {
   uint32_t nlen, ndist, final_block, synced, passed, resume, in_sync_block;
   uint32_t spec, again;     // speculative start; try the next candidate
   uint32_t fixed_tables;    // the tables in place are the fixed code's
-  uint32_t hdr_move, hdr_end;  // move pos past the header; its length after hdr_pos
+  // move pos past the header; its length after hdr_pos; where the symbol that
+  // ends its reading, the last or the first wrong one, begins after it
+  uint32_t hdr_move, hdr_end, hdr_last;
   uint32_t build_ok[2];
   uint32_t page_cur, page_prev, page_seq, n_pages;
   uint32_t round_slots, round_lanes, round_kind, round_pos;
@@ -531,7 +533,7 @@ __device__ __forceinline__ int32_t cta_read_lens(const uint8_t* __restrict__ in,
   }
   uint32_t sum;
   uint32_t o = cta_scan(S, 0, (e[0] >> 16) + (e[1] >> 16), sum);
-  if (tid == 0) S->c.hdr_end = kNone;
+  if (tid == 0) S->c.hdr_end = S->c.hdr_last = kNone;
   cta_sync();
   bool bad = false;
 #pragma unroll
@@ -541,8 +543,12 @@ __device__ __forceinline__ int32_t cta_read_lens(const uint8_t* __restrict__ in,
       uint32_t s = 2 * tid + k;
       if (!n || o + n > total || (s == 0 && (e[k] & 31) == 16)) {
         bad = true;
+        atomicMin(&S->c.hdr_last, p[k]);
       } else {
-        if (o + n == total) S->c.hdr_end = p[k] + ((e[k] >> 8) & 31);
+        if (o + n == total) {
+          S->c.hdr_end = p[k] + ((e[k] >> 8) & 31);
+          atomicMin(&S->c.hdr_last, p[k]);
+        }
         while (s && S->val[s] == 0xFF) s--;
         const uint8_t v = S->val[s];
         if (v)
@@ -552,10 +558,11 @@ __device__ __forceinline__ int32_t cta_read_lens(const uint8_t* __restrict__ in,
     o += n;
   }
   bad = cta_sync_or(bad) || S->c.hdr_end == kNone || S->lens[256] == 0;
-  // past the readable input (the reader ran 96 bits ahead): cut off, or over the abort bit
-  const uint64_t end = pos + (S->c.hdr_end == kNone ? 0u : S->c.hdr_end);
+  // Past the readable input (a serial reader ran 96 bits ahead of the symbol it
+  // stopped at): cut off, or over the abort bit, whatever the lengths say.
+  const uint64_t end = pos + S->c.hdr_end, ahead = pos + S->c.hdr_last + 96;
   cta_sync();
-  if (end + 96 > S->c.limit_words * 32) return end + 96 > trunc * 32 ? kTruncated : kOvershoot;
+  if (ahead >= S->c.limit_words * 32) return ahead >= trunc * 32 ? kTruncated : kOvershoot;
   if (bad) return kBadDeflate;
   if (tid == 0 && move) S->c.pos = end;
   cta_sync();

@@ -51,7 +51,7 @@ def test_device_over_4gib_of_one_repetition():
     cx = G.Context()
     try:
         d_in = torch.zeros(comp.size + 1024, dtype=torch.uint8, device="cuda")
-        d_in[: comp.size] = torch.from_numpy(comp).cuda()
+        d_in[: comp.size] = torch.from_numpy(comp.copy()).cuda()
         d_out = torch.empty(n + 64, dtype=torch.uint8, device="cuda")
         torch.cuda.synchronize()
         assert cx.decompress_device(d_in.data_ptr(), comp.size, d_out.data_ptr(), d_out.numel()) == n
