@@ -247,6 +247,7 @@ struct gzgpu_ctx {
   uint32_t n_pages_used = 0;  // pages taken from the pool by the job's decodes
   cudaEvent_t ev[12];
   cudaEvent_t stage_ev[2];  // last DMA of each pinned staging slot
+  cudaEvent_t caller_ev;    // the default stream's work when a device entry point was called
   gzgpu_stats stats{};
   bool crc_ready = false;
 
@@ -1437,6 +1438,7 @@ int gzgpu_create(gzgpu_ctx** out, const gzgpu_config* cfg) {
   }
   for (auto& e : c->ev) cudaEventCreate(&e);
   for (auto& e : c->stage_ev) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+  cudaEventCreateWithFlags(&c->caller_ev, cudaEventDisableTiming);
   for (DevBuf* b : c->all_bufs()) b->st = c->st;
   {
     // keep memory freed by buffer growth in the device's pool for reuse
@@ -1460,6 +1462,7 @@ void gzgpu_destroy(gzgpu_ctx* c) {
   c->h_stage.release();
   for (auto& e : c->ev) cudaEventDestroy(e);
   for (auto& e : c->stage_ev) cudaEventDestroy(e);
+  cudaEventDestroy(c->caller_ev);
   cudaStreamDestroy(c->st);
   delete c;
 }
@@ -1722,6 +1725,12 @@ int gzgpu_decompress_device(gzgpu_ctx* c, const void* d_in, size_t in_len, void*
   if ((reinterpret_cast<uintptr_t>(d_in) | reinterpret_cast<uintptr_t>(d_out)) & 15)
     return GZGPU_INVALID_ARGUMENT;  // the kernels use 16-byte vector access
   if (in_len < 2) return GZGPU_NOT_GZIP;  // (the scan looks at the magic)
+  // The context's stream does not wait for the default stream by itself; what
+  // the caller has put there (the copy that fills d_in, a use of d_out) comes
+  // before the decode.
+  if (c->check(cudaEventRecord(c->caller_ev, cudaStreamLegacy)) ||
+      c->check(cudaStreamWaitEvent(c->st, c->caller_ev, 0)))
+    return GZGPU_DEVICE_ERROR;
   cudaEventRecord(c->ev[0], c->st);
   c->cur_in = reinterpret_cast<const uint8_t*>(d_in);
   c->user_out = reinterpret_cast<uint8_t*>(d_out);

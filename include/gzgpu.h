@@ -156,8 +156,9 @@ int gzgpu_decompress_to_writer(gzgpu_ctx *ctx, const uint8_t *in, size_t in_len,
 /* Device-resident form of gzgpu_decompress (internal decompress_bytes,
  * src/decompress/mod.rs:317): d_in / d_out are device pointers of this
  * context's device, both 16-byte aligned (cudaMalloc memory is); d_in must
- * have GZGPU_INPUT_PAD readable bytes past in_len.  No host copies of
- * payload. */
+ * have GZGPU_INPUT_PAD readable bytes past in_len.  The decode comes after
+ * what the calling thread has put on the (legacy) default stream before, and
+ * is complete when the call returns.  No host copies of payload. */
 int gzgpu_decompress_device(gzgpu_ctx *ctx, const void *d_in, size_t in_len, void *d_out,
                             size_t out_cap, size_t *out_len);
 
