@@ -1187,6 +1187,8 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   const uint32_t n_all = (uint32_t)hd.size();
   std::vector<PlacedChunk> placed;
   std::vector<uint32_t> placed_of(n_all, 0xFFFFFFFFu);
+  std::vector<uint32_t> tails;  // placed chunks with a tail
+  bool bodies = false;          // some chunk has entries before its tail
   uint64_t n_tail_markers = 0;  // placed chunks whose last 32 KiB hold markers
   std::vector<CrcBlock> cblk;
   std::vector<uint64_t> mtrail, mlenv, mendv;
@@ -1205,9 +1207,13 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
         uint32_t cid = w.order[k];
         placed_of[cid] = (uint32_t)placed.size();
         const ChunkResult& r = hr[cid];
-        placed.push_back(PlacedChunk{out_total + so, moff, cid, r.last_page, r.prev_page,
-                                     r.out_len ? (uint32_t)((r.out_len - 1) / kPageEntries) : 0u});
         uint64_t t0 = r.out_len > kWindow ? r.out_len - kWindow : 0;
+        // no chunk looks back at a member's last, whose tail is as the rest
+        const uint64_t body_end = k + 1 == mp.order_end && t0 ? r.out_len : t0 & ~(uint64_t)(kTailUnit - 1);
+        if (body_end < r.out_len) tails.push_back((uint32_t)placed.size());
+        bodies |= body_end != 0;
+        placed.push_back(PlacedChunk{out_total + so, moff, cid, r.last_page, r.prev_page,
+                                     r.out_len ? (uint32_t)((r.out_len - 1) / kPageEntries) : 0u, body_end});
         n_tail_markers += r.marker_end > t0;
         so += r.out_len;
       }
@@ -1237,6 +1243,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   Pack pc(up[1]);
   const size_t at_placed = pc.add(placed.data(), sizeof(PlacedChunk) * placed.size());
   const size_t at_pof = pc.add(placed_of.data(), 4 * placed_of.size());
+  const size_t at_tails = pc.add(tails.data(), 4 * tails.size());
   const size_t at_cblk = pc.add(cblk.data(), sizeof(CrcBlock) * cblk.size());
   const size_t at_mtrail = pc.add(mtrail.data(), 8 * mtrail.size());
   const size_t at_mlen = pc.add(mlenv.data(), 8 * mlenv.size());
@@ -1259,8 +1266,9 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
     crc_ready = true;
   }
   if ((rc = check(launch_resolve(reinterpret_cast<PlacedChunk*>(d_plan + at_placed),
-                                 reinterpret_cast<uint32_t*>(d_plan + at_pof), n_pages_used,
-                                 results.as<ChunkResult>(), pool, cur_out, st))))
+                                 reinterpret_cast<uint32_t*>(d_plan + at_pof),
+                                 reinterpret_cast<uint32_t*>(d_plan + at_tails), (uint32_t)tails.size(), bodies,
+                                 out_total, n_pages_used, results.as<ChunkResult>(), pool, cur_out, st))))
     return rc;
   cudaEventRecord(ev[11], st);
   if ((rc = check(launch_crc(reinterpret_cast<CrcBlock*>(d_plan + at_cblk), (uint32_t)cblk.size(), cur_out,
@@ -1270,7 +1278,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
                              reinterpret_cast<uint64_t*>(d_plan + at_mlen), (uint32_t)mtrail.size(),
                              cur_in, mstatus.as<int32_t>(), sms, st))))
     return rc;
-  stats.kernel_launches += 3;
+  stats.kernel_launches += 3 + (bodies && !tails.empty() && out_total > kTwoPass);
   std::vector<int32_t> mst(mtrail.size());
   if (!mst.empty()) {
     if (down.size() < 4 * mst.size()) down.resize(4 * mst.size());

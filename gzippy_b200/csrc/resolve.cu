@@ -7,13 +7,14 @@
 // read as 0 before the member's first byte (the zero window).
 //
 //   resolve      : every entry's byte.  A marker names a byte of the 32 KiB
-//                  before its chunk, which lies near the end of one of the few
-//                  chunks before it; that entry is a literal or again a marker,
-//                  naming a byte before its own chunk.  Each marker follows its
-//                  references through the chunks' entries until it reaches a
-//                  literal (or a position before the member: 0), so all chunks
-//                  resolve in parallel and the window chain (window_map.rs:
-//                  80-103, chunk_fetcher.rs publish_subchunk_windows :2295,
+//                  before its chunk, which lies in the tail (the last 32 KiB) of
+//                  one of the few chunks before it; that entry is a literal or
+//                  again a marker, naming a byte before its own chunk.  Each
+//                  marker follows its references through the chunks' tails until
+//                  it reaches a literal (or a position before the member: 0), so
+//                  all chunks resolve in parallel and the window chain
+//                  (window_map.rs:80-103, chunk_fetcher.rs
+//                  publish_subchunk_windows :2295,
 //                  resolve_and_narrow_markers_in_place_crc, chunk_data.rs:1745)
 //                  needs no order
 //   crc_blocks   : CRC32 of blocks of final output (up to 64 KiB of one
@@ -35,12 +36,27 @@ namespace gzgpu {
 // (two dependent loads a reference), and the unit's bytes leave in aligned
 // 16-byte stores.  The pass is instructions (94 per 32 entries of text, of which
 // 40 % are markers of 1.4 references each) and scattered loads in between, so
-// what counts is warps that never wait for each other: with units of 4096 entries for a CTA of 256 threads, its three
-// barriers cost a third of the time (64 MiB of text: 0.35 ms, now 0.23).
+// what counts is warps that never wait for each other: with units of 4096
+// entries for a CTA of 256 threads, its three barriers cost a third of the time
+// (64 MiB of text: 0.35 ms, 0.23 by warps).
+//
+// Where data repeats for longer than a chunk, every entry is a marker and its
+// chain leads back over all chunks; following each to its end took 55 ms of 1 GiB
+// of zeros in 43 chunks.  What chains pass through are the chunks' tails, so the
+// tails (`tails`: their places) come first, and a walk of more than one
+// reference writes its byte over the marker it began at, where later walks end:
+// chunks in flight together take about the root of their number in references.
+// Above kTwoPass bytes the tails are a launch of their own, and a marker before
+// them (kFinal) one load of the final output: 1 GiB of zeros 6.0 ms in one
+// launch, 2.0 in two; 64 MiB of text 0.206 and 0.173.  A second launch costs a
+// small job more than that (1 MB of text: 24 us in one, 31 in two).  The second
+// may start while the first one's last CTAs run: it reads its entries and makes
+// its lists, then waits for the tails (5 us less than one after the other).
 constexpr uint32_t kResolveUnit = 512;
 constexpr int kResolveThreads = 256;
 constexpr uint32_t kResolveWarps = kResolveThreads / 32;
 static_assert(kResolveUnit == 16 * 32, "16 entries a lane");
+static_assert(kResolveUnit == kTailUnit, "the body ends at a unit's edge");
 
 struct ResolveWarp {
   alignas(16) uint8_t bytes[kResolveUnit + 16];
@@ -48,25 +64,46 @@ struct ResolveWarp {
   NearChunk near[kNear];        // the chunks before the unit's, nearest first
 };
 
+template <bool kFinal>
 __global__ void __launch_bounds__(kResolveThreads, 6)
     resolve_kernel(const PlacedChunk* __restrict__ placed, const uint32_t* __restrict__ placed_of_chunk,
-                   uint32_t n_pages, const ChunkResult* __restrict__ results, PagePool pool,
-                   uint8_t* __restrict__ out) {
+                   const uint32_t* __restrict__ tails, uint32_t n_tails, uint32_t n_pages,
+                   const ChunkResult* __restrict__ results, PagePool pool, uint8_t* out) {
   __shared__ ResolveWarp rw[kResolveWarps];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ResolveWarp& W = rw[warp];
-  // a CTA takes kResolveWarps units in a row; the first ones of every page,
-  // then the next, ...: markers thin out along a chunk
-  const uint32_t p = blockIdx.x % n_pages;
-  const uint32_t first = ((blockIdx.x / n_pages) * kResolveWarps + warp) * kResolveUnit;
-  const uint32_t cid = pool.owner[p], sw = pool.seq[p];
-  const uint32_t k = placed_of_chunk[cid];
-  if (k == 0xFFFFFFFFu) return;
-  const uint64_t len = results[cid].out_len;
-  const uint64_t q0 = (uint64_t)(sw & kSeqMask) * kPageEntries + first;
-  if (q0 >= len || (sw >> kGenShift) != results[cid].gen) return;  // or a failed attempt's page
+  const uint32_t tail_ctas = (n_tails * kTailUnits + kResolveWarps - 1) / kResolveWarps;
+  const bool tail = blockIdx.x < tail_ctas;
+  uint32_t k, page, first;  // the chunk, the page and the unit's first entry in it
+  uint64_t q0, len;         // the same in the chunk, and where to stop
+  if (!kFinal) cudaTriggerProgrammaticLaunchCompletion();
+  if (tail) {
+    const uint32_t id = blockIdx.x * kResolveWarps + warp;
+    if (id >= n_tails * kTailUnits) return;
+    k = tails[id / kTailUnits];
+    const PlacedChunk& pc = placed[k];
+    len = results[pc.chunk].out_len;
+    q0 = pc.body_end + (id % kTailUnits) * kResolveUnit;
+    page = (uint32_t)(q0 >> 16) == pc.last_seq ? pc.last_page : pc.prev_page;
+    first = (uint32_t)q0 & (kPageEntries - 1);
+  } else {
+    // kResolveWarps units in a row; the first ones of every page, then the
+    // next, ...: markers thin out along a chunk
+    const uint32_t id = blockIdx.x - tail_ctas;
+    page = id % n_pages;
+    first = ((id / n_pages) * kResolveWarps + warp) * kResolveUnit;
+    const uint32_t cid = pool.owner[page], sw = pool.seq[page];
+    k = placed_of_chunk[cid];
+    q0 = (uint64_t)(sw & kSeqMask) * kPageEntries + first;
+    // nothing of a chunk not accepted, or of a failed attempt's page
+    len = k != 0xFFFFFFFFu && (sw >> kGenShift) == results[cid].gen ? placed[k].body_end : 0u;
+  }
+  if (q0 >= len) {
+    if (kFinal) cudaGridDependencySynchronize();
+    return;
+  }
   const uint32_t n = (uint32_t)min((uint64_t)kResolveUnit, len - q0);
-  const uint16_t* src = pool.data + (size_t)p * kPageEntries + first;
+  uint16_t* const src = pool.data + (size_t)page * kPageEntries + first;
   uint4 x[2];
 #pragma unroll
   for (uint32_t s = 0; s < 2; s++) {
@@ -74,7 +111,7 @@ __global__ void __launch_bounds__(kResolveThreads, 6)
     x[s] = e < n ? *reinterpret_cast<const uint4*>(src + e) : make_uint4(0, 0, 0, 0);
   }
   const uint64_t off = placed[k].out_off, moff = placed[k].member_off;
-  if (lane < kNear && lane < k) W.near[lane] = near_chunk(placed[k - 1 - lane]);
+  if (!kFinal && lane < kNear && lane < k) W.near[lane] = near_chunk(placed[k - 1 - lane]);
   uint32_t n_list = 0;
 #pragma unroll
   for (uint32_t s = 0; s < 2; s++) {
@@ -101,12 +138,23 @@ __global__ void __launch_bounds__(kResolveThreads, 6)
       if ((m >> i) & 1) W.list[at++] = (e + i) << 16 | ((h[i >> 1] >> (16 * (i & 1))) & 0xFFFFu);
   }
   __syncwarp();
+  if (kFinal) cudaGridDependencySynchronize();  // the tails are in place
   for (uint32_t i = lane; i < n_list; i += 32) {
     const uint32_t item = W.list[i];
-    W.bytes[item >> 16] = (uint8_t)follow_marker(
-        placed, W.near, k, off, moff, item & 0xFFFFu, [&](uint32_t page, uint32_t e) -> uint32_t {
-          return pool.data[(size_t)page * kPageEntries + e];
-        });
+    const uint32_t v = item & 0xFFFFu;
+    uint32_t byte;
+    if constexpr (kFinal) {
+      const uint32_t dist = 2 * kMarkerBase - v;
+      byte = dist <= off - moff ? out[off - dist] : 0u;
+    } else {
+      uint32_t refs = 0;
+      byte = follow_marker(placed, W.near, k, off, moff, v, [&](uint32_t p, uint32_t e) -> uint32_t {
+        refs++;
+        return __ldcg(pool.data + (size_t)p * kPageEntries + e);
+      });
+      if (tail && refs > 1) src[item >> 16] = (uint16_t)byte;
+    }
+    W.bytes[item >> 16] = (uint8_t)byte;
   }
   __syncwarp();
   // the unit's bytes: aligned 16 of the output, then what lies around them
@@ -120,9 +168,9 @@ __global__ void __launch_bounds__(kResolveThreads, 6)
         make_uint4(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], w[2], sh),
                    __funnelshift_r(w[2], w[3], sh), __funnelshift_r(w[3], w[4], sh));
   }
-  const uint32_t tail = head + ((n - head) & ~15u) + (lane & 15);
+  const uint32_t rest = head + ((n - head) & ~15u) + (lane & 15);
   if (lane < head) dst[lane] = W.bytes[lane];
-  if (lane >= 16 && tail < n) dst[tail] = W.bytes[tail];
+  if (lane >= 16 && rest < n) dst[rest] = W.bytes[rest];
 }
 
 // ---------------------------------------------------------------------------
@@ -332,11 +380,30 @@ cudaError_t resolve_init(cudaStream_t stream) {
 }
 
 cudaError_t launch_resolve(const PlacedChunk* placed, const uint32_t* placed_of_chunk,
-                           uint32_t n_pages, const ChunkResult* results, const PagePool& pool,
-                           uint8_t* out, cudaStream_t stream) {
-  if (!n_pages) return cudaSuccess;
-  const uint32_t grid = n_pages * (kPageEntries / (kResolveUnit * kResolveWarps));
-  resolve_kernel<<<grid, kResolveThreads, 0, stream>>>(placed, placed_of_chunk, n_pages, results, pool, out);
+                           const uint32_t* tails, uint32_t n_tails, bool bodies, uint64_t out_len,
+                           uint32_t n_pages, const ChunkResult* results, const PagePool& pool, uint8_t* out,
+                           cudaStream_t stream) {
+  const uint32_t tail_ctas = (n_tails * kTailUnits + kResolveWarps - 1) / kResolveWarps;
+  const uint32_t body_ctas = bodies ? n_pages * (kPageEntries / (kResolveUnit * kResolveWarps)) : 0u;
+  if (tail_ctas && body_ctas && out_len > kTwoPass) {
+    resolve_kernel<false><<<tail_ctas, kResolveThreads, 0, stream>>>(placed, placed_of_chunk, tails, n_tails,
+                                                                     n_pages, results, pool, out);
+    cudaLaunchAttribute overlap{};
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(body_ctas);
+    cfg.blockDim = dim3(kResolveThreads);
+    cfg.stream = stream;
+    cfg.attrs = &overlap;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, resolve_kernel<true>, placed, placed_of_chunk, tails, 0u, n_pages,
+                                             results, pool, out);
+    if (e != cudaSuccess) return e;
+  } else if (tail_ctas + body_ctas) {
+    resolve_kernel<false><<<tail_ctas + body_ctas, kResolveThreads, 0, stream>>>(
+        placed, placed_of_chunk, tails, n_tails, n_pages, results, pool, out);
+  }
   return cudaGetLastError();
 }
 

@@ -54,7 +54,7 @@ def _fixed_block(slots, size, seed):
     return np.packbits(np.array(bits, np.uint8), bitorder="little").tobytes() + b"\x00\x00\xff\xff"
 
 
-def _copying_block(window, size, seed):
+def _copying_block(window, size, seed, any_type=False):
     """A dynamic block of `size` bytes, pieces of the 32 KiB before it between
     bytes of its own, then an empty stored block."""
     rng = np.random.default_rng(seed)
@@ -67,7 +67,7 @@ def _copying_block(window, size, seed):
     plain = b"".join(parts)[:size]
     c = zlib.compressobj(9, zlib.DEFLATED, -15, 9, zlib.Z_DEFAULT_STRATEGY, window)
     comp = c.compress(plain) + c.flush(zlib.Z_SYNC_FLUSH)
-    assert comp[0] & 7 == 4  # dynamic
+    assert any_type or comp[0] & 7 == 4  # dynamic
     return comp
 
 
@@ -118,5 +118,49 @@ def _check(slots, size, units, narrow):
         assert (used["out_len"] % 65536 == 0).sum() >= units // 2  # chunks that end on a page
         # no page without an entry
         assert np.array_equal(used["n_pages"], -(-used["out_len"].astype(np.int64) // 65536))
+    finally:
+        cx.close()
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_chunks_of_every_length(seed):
+    """Chunks shorter and longer than a window, a page and a resolve unit (512
+    entries), whose last 32 KiB are resolved apart from the rest, each copying from
+    what lies before it."""
+    import gzippy_b200 as G
+    rng = np.random.default_rng(seed)
+    sizes = [511, 512, 513, 3000, 32255, 32256, 32767, 32768, 32769, 33279, 33280, 33281, 65535, 65536, 65537,
+             98303, 98304, 98305, 131072, 200001]
+    d = zlib.decompressobj(-15)
+    comp, window, plain = [], rng.integers(0, 256, 32768, dtype=np.uint8).tobytes(), []
+    comp.append(b"".join(b"\x00" + n.to_bytes(2, "little") + (n ^ 0xFFFF).to_bytes(2, "little") + window
+                         for n in (32768,)))
+    plain.append(d.decompress(comp[0]))
+    for i in rng.permutation(np.tile(sizes, 12)):
+        comp.append(_copying_block(window, int(i), int(rng.integers(1 << 30)), any_type=True))
+        plain.append(d.decompress(comp[-1]))
+        window = (window + plain[-1])[-32768:]
+    comp.append(b"\x03\x00")
+    raw, plain = b"".join(comp), b"".join(plain)
+    for chunk_bytes in (1024, 4096, 0):
+        cx = G.Context(chunk_bytes=chunk_bytes)
+        try:
+            assert cx.inflate_raw(raw) == plain
+        finally:
+            cx.close()
+
+
+@pytest.mark.parametrize("period", [1, 2, 100, 5000, 32768])
+def test_repetition_over_many_chunks(period):
+    """Every chunk but the first is all markers, and chains lead back over all."""
+    import gzippy_b200 as G
+    rec = np.random.default_rng(period).integers(0, 256, period, dtype=np.uint8)
+    plain = np.tile(rec, (48 << 20) // period + 1).tobytes()
+    comp = zlib.compressobj(9 if period < 32768 else 6, zlib.DEFLATED, 31)
+    comp = comp.compress(plain) + comp.flush()
+    cx = G.Context(chunk_bytes=1024)
+    try:
+        assert cx.decompress(comp) == plain
+        assert cx.stats().n_accepted > (8 if period > 1 else 2)
     finally:
         cx.close()
