@@ -535,19 +535,18 @@ __device__ __forceinline__ int32_t cta_read_lens(const uint8_t* __restrict__ in,
   uint32_t o = cta_scan(S, 0, (e[0] >> 16) + (e[1] >> 16), sum);
   if (tid == 0) S->c.hdr_end = S->c.hdr_last = kNone;
   cta_sync();
-  bool bad = false;
+  uint32_t wrong = kNone;  // where this thread's first wrong symbol begins
 #pragma unroll
   for (int k = 0; k < 2; k++) {
     const uint32_t n = e[k] >> 16;
     if (tid < kHdrSyms / 2 && o < total) {
       uint32_t s = 2 * tid + k;
       if (!n || o + n > total || (s == 0 && (e[k] & 31) == 16)) {
-        bad = true;
-        atomicMin(&S->c.hdr_last, p[k]);
+        wrong = min(wrong, p[k]);
       } else {
         if (o + n == total) {
           S->c.hdr_end = p[k] + ((e[k] >> 8) & 31);
-          atomicMin(&S->c.hdr_last, p[k]);
+          S->c.hdr_last = p[k];
         }
         while (s && S->val[s] == 0xFF) s--;
         const uint8_t v = S->val[s];
@@ -557,7 +556,12 @@ __device__ __forceinline__ int32_t cta_read_lens(const uint8_t* __restrict__ in,
     }
     o += n;
   }
-  bad = cta_sync_or(bad) || S->c.hdr_end == kNone || S->lens[256] == 0;
+  bool bad = cta_sync_or(wrong != kNone);
+  if (bad) {
+    if (wrong != kNone) atomicMin(&S->c.hdr_last, wrong);
+    cta_sync();
+  }
+  bad = bad || S->c.hdr_end == kNone || S->lens[256] == 0;
   // Past the readable input (a serial reader ran 96 bits ahead of the symbol it
   // stopped at): cut off, or over the abort bit, whatever the lengths say.
   const uint64_t end = pos + S->c.hdr_end, ahead = pos + S->c.hdr_last + 96;

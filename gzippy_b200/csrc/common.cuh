@@ -136,7 +136,7 @@ struct PlacedChunk {
   uint32_t prev_page;    // the one before,
   uint32_t last_seq;     // and the last page's index within the chunk
   uint64_t body_end;     // entries before its tail (up to the resolve unit that holds the
-                         // first of its last 32 Ki); all of a longer last chunk of a member
+                         // first of its last 32 Ki); all of a member's last chunk
 };
 
 // CRC block: final output bytes [begin, last) of one member, in the block that

@@ -1187,8 +1187,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   const uint32_t n_all = (uint32_t)hd.size();
   std::vector<PlacedChunk> placed;
   std::vector<uint32_t> placed_of(n_all, 0xFFFFFFFFu);
-  std::vector<uint32_t> tails;  // placed chunks with a tail
-  bool bodies = false;          // some chunk has entries before its tail
+  std::vector<uint32_t> tails;  // placed chunks with a tail (in large jobs)
   uint64_t n_tail_markers = 0;  // placed chunks whose last 32 KiB hold markers
   std::vector<CrcBlock> cblk;
   std::vector<uint64_t> mtrail, mlenv, mendv;
@@ -1209,9 +1208,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
         const ChunkResult& r = hr[cid];
         uint64_t t0 = r.out_len > kWindow ? r.out_len - kWindow : 0;
         // no chunk looks back at a member's last, whose tail is as the rest
-        const uint64_t body_end = k + 1 == mp.order_end && t0 ? r.out_len : t0 & ~(uint64_t)(kTailUnit - 1);
-        if (body_end < r.out_len) tails.push_back((uint32_t)placed.size());
-        bodies |= body_end != 0;
+        const uint64_t body_end = k + 1 == mp.order_end ? r.out_len : t0 & ~(uint64_t)(kTailUnit - 1);
         placed.push_back(PlacedChunk{out_total + so, moff, cid, r.last_page, r.prev_page,
                                      r.out_len ? (uint32_t)((r.out_len - 1) / kPageEntries) : 0u, body_end});
         n_tail_markers += r.marker_end > t0;
@@ -1239,6 +1236,9 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   // ---- 6. resolve + CRC ----------------------------------------------------
   stats.n_pages = n_pages_used;
   cur_out = (user_out && out_total <= user_cap) ? user_out : nullptr;
+  if (out_total >= kTwoPass)
+    for (uint32_t k = 0; k < placed.size(); k++)
+      if (placed[k].body_end < hr[placed[k].chunk].out_len) tails.push_back(k);
   // everything the passes read, in one copy
   Pack pc(up[1]);
   const size_t at_placed = pc.add(placed.data(), sizeof(PlacedChunk) * placed.size());
@@ -1267,8 +1267,8 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   }
   if ((rc = check(launch_resolve(reinterpret_cast<PlacedChunk*>(d_plan + at_placed),
                                  reinterpret_cast<uint32_t*>(d_plan + at_pof),
-                                 reinterpret_cast<uint32_t*>(d_plan + at_tails), (uint32_t)tails.size(), bodies,
-                                 out_total, n_pages_used, results.as<ChunkResult>(), pool, cur_out, st))))
+                                 reinterpret_cast<uint32_t*>(d_plan + at_tails), (uint32_t)tails.size(),
+                                 n_pages_used, results.as<ChunkResult>(), pool, cur_out, st))))
     return rc;
   cudaEventRecord(ev[11], st);
   if ((rc = check(launch_crc(reinterpret_cast<CrcBlock*>(d_plan + at_cblk), (uint32_t)cblk.size(), cur_out,
@@ -1278,7 +1278,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
                              reinterpret_cast<uint64_t*>(d_plan + at_mlen), (uint32_t)mtrail.size(),
                              cur_in, mstatus.as<int32_t>(), sms, st))))
     return rc;
-  stats.kernel_launches += 3 + (bodies && !tails.empty() && out_total > kTwoPass);
+  stats.kernel_launches += 3 + !tails.empty();
   std::vector<int32_t> mst(mtrail.size());
   if (!mst.empty()) {
     if (down.size() < 4 * mst.size()) down.resize(4 * mst.size());

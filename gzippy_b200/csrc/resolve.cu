@@ -42,16 +42,18 @@ namespace gzgpu {
 //
 // Where data repeats for longer than a chunk, every entry is a marker and its
 // chain leads back over all chunks; following each to its end took 55 ms of 1 GiB
-// of zeros in 43 chunks.  What chains pass through are the chunks' tails, so the
-// tails (`tails`: their places) come first, and a walk of more than one
-// reference writes its byte over the marker it began at, where later walks end:
-// chunks in flight together take about the root of their number in references.
-// Above kTwoPass bytes the tails are a launch of their own, and a marker before
-// them (kFinal) one load of the final output: 1 GiB of zeros 6.0 ms in one
-// launch, 2.0 in two; 64 MiB of text 0.206 and 0.173.  A second launch costs a
-// small job more than that (1 MB of text: 24 us in one, 31 in two).  The second
-// may start while the first one's last CTAs run: it reads its entries and makes
-// its lists, then waits for the tails (5 us less than one after the other).
+// of zeros in 43 chunks.  All that chains pass through are the chunks' tails, so
+// a walk of more than one reference writes its byte over the marker it began at,
+// if that lies in its chunk's tail, and later walks end there.
+// Above kTwoPass bytes the tails (`tails`: their chunks' places) are a launch of
+// their own, in output order, so that chunks in flight together take about the
+// root of their number in references; a marker before them is then one load of
+// the final output.  1 GiB of zeros 2.0 ms, 64 MiB of text 0.202 -> 0.175.  A
+// second launch costs a smaller job more than that (12 MiB of noisy ramps: 21 us
+// in one, 29 in two).  It may start while the first one's last CTAs run: it reads
+// its entries and makes its lists, then waits for the tails (5 us less than one
+// after the other).
+enum ResolvePart { kResolveAll, kResolveTails, kResolveBodies };
 constexpr uint32_t kResolveUnit = 512;
 constexpr int kResolveThreads = 256;
 constexpr uint32_t kResolveWarps = kResolveThreads / 32;
@@ -64,7 +66,7 @@ struct ResolveWarp {
   NearChunk near[kNear];        // the chunks before the unit's, nearest first
 };
 
-template <bool kFinal>
+template <ResolvePart kPart>
 __global__ void __launch_bounds__(kResolveThreads, 6)
     resolve_kernel(const PlacedChunk* __restrict__ placed, const uint32_t* __restrict__ placed_of_chunk,
                    const uint32_t* __restrict__ tails, uint32_t n_tails, uint32_t n_pages,
@@ -72,12 +74,10 @@ __global__ void __launch_bounds__(kResolveThreads, 6)
   __shared__ ResolveWarp rw[kResolveWarps];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ResolveWarp& W = rw[warp];
-  const uint32_t tail_ctas = (n_tails * kTailUnits + kResolveWarps - 1) / kResolveWarps;
-  const bool tail = blockIdx.x < tail_ctas;
   uint32_t k, page, first;  // the chunk, the page and the unit's first entry in it
   uint64_t q0, len;         // the same in the chunk, and where to stop
-  if (!kFinal) cudaTriggerProgrammaticLaunchCompletion();
-  if (tail) {
+  if (kPart == kResolveTails) {
+    cudaTriggerProgrammaticLaunchCompletion();
     const uint32_t id = blockIdx.x * kResolveWarps + warp;
     if (id >= n_tails * kTailUnits) return;
     k = tails[id / kTailUnits];
@@ -89,17 +89,18 @@ __global__ void __launch_bounds__(kResolveThreads, 6)
   } else {
     // kResolveWarps units in a row; the first ones of every page, then the
     // next, ...: markers thin out along a chunk
-    const uint32_t id = blockIdx.x - tail_ctas;
-    page = id % n_pages;
-    first = ((id / n_pages) * kResolveWarps + warp) * kResolveUnit;
+    page = blockIdx.x % n_pages;
+    first = ((blockIdx.x / n_pages) * kResolveWarps + warp) * kResolveUnit;
     const uint32_t cid = pool.owner[page], sw = pool.seq[page];
     k = placed_of_chunk[cid];
     q0 = (uint64_t)(sw & kSeqMask) * kPageEntries + first;
     // nothing of a chunk not accepted, or of a failed attempt's page
-    len = k != 0xFFFFFFFFu && (sw >> kGenShift) == results[cid].gen ? placed[k].body_end : 0u;
+    len = 0;
+    if (k != 0xFFFFFFFFu && (sw >> kGenShift) == results[cid].gen)
+      len = kPart == kResolveAll ? results[cid].out_len : placed[k].body_end;
   }
   if (q0 >= len) {
-    if (kFinal) cudaGridDependencySynchronize();
+    if (kPart == kResolveBodies) cudaGridDependencySynchronize();
     return;
   }
   const uint32_t n = (uint32_t)min((uint64_t)kResolveUnit, len - q0);
@@ -111,7 +112,7 @@ __global__ void __launch_bounds__(kResolveThreads, 6)
     x[s] = e < n ? *reinterpret_cast<const uint4*>(src + e) : make_uint4(0, 0, 0, 0);
   }
   const uint64_t off = placed[k].out_off, moff = placed[k].member_off;
-  if (!kFinal && lane < kNear && lane < k) W.near[lane] = near_chunk(placed[k - 1 - lane]);
+  if (kPart != kResolveBodies && lane < kNear && lane < k) W.near[lane] = near_chunk(placed[k - 1 - lane]);
   uint32_t n_list = 0;
 #pragma unroll
   for (uint32_t s = 0; s < 2; s++) {
@@ -138,12 +139,12 @@ __global__ void __launch_bounds__(kResolveThreads, 6)
       if ((m >> i) & 1) W.list[at++] = (e + i) << 16 | ((h[i >> 1] >> (16 * (i & 1))) & 0xFFFFu);
   }
   __syncwarp();
-  if (kFinal) cudaGridDependencySynchronize();  // the tails are in place
+  if (kPart == kResolveBodies) cudaGridDependencySynchronize();  // the tails are in place
   for (uint32_t i = lane; i < n_list; i += 32) {
     const uint32_t item = W.list[i];
     const uint32_t v = item & 0xFFFFu;
     uint32_t byte;
-    if constexpr (kFinal) {
+    if constexpr (kPart == kResolveBodies) {
       const uint32_t dist = 2 * kMarkerBase - v;
       byte = dist <= off - moff ? out[off - dist] : 0u;
     } else {
@@ -152,7 +153,7 @@ __global__ void __launch_bounds__(kResolveThreads, 6)
         refs++;
         return __ldcg(pool.data + (size_t)p * kPageEntries + e);
       });
-      if (tail && refs > 1) src[item >> 16] = (uint16_t)byte;
+      if (refs > 1 && (kPart == kResolveTails || q0 + (item >> 16) + kWindow >= len)) src[item >> 16] = (uint16_t)byte;
     }
     W.bytes[item >> 16] = (uint8_t)byte;
   }
@@ -380,31 +381,32 @@ cudaError_t resolve_init(cudaStream_t stream) {
 }
 
 cudaError_t launch_resolve(const PlacedChunk* placed, const uint32_t* placed_of_chunk,
-                           const uint32_t* tails, uint32_t n_tails, bool bodies, uint64_t out_len,
-                           uint32_t n_pages, const ChunkResult* results, const PagePool& pool, uint8_t* out,
+                           const uint32_t* tails, uint32_t n_tails, uint32_t n_pages,
+                           const ChunkResult* results, const PagePool& pool, uint8_t* out,
                            cudaStream_t stream) {
-  const uint32_t tail_ctas = (n_tails * kTailUnits + kResolveWarps - 1) / kResolveWarps;
-  const uint32_t body_ctas = bodies ? n_pages * (kPageEntries / (kResolveUnit * kResolveWarps)) : 0u;
-  if (tail_ctas && body_ctas && out_len > kTwoPass) {
-    resolve_kernel<false><<<tail_ctas, kResolveThreads, 0, stream>>>(placed, placed_of_chunk, tails, n_tails,
-                                                                     n_pages, results, pool, out);
-    cudaLaunchAttribute overlap{};
-    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    overlap.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(body_ctas);
-    cfg.blockDim = dim3(kResolveThreads);
-    cfg.stream = stream;
-    cfg.attrs = &overlap;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, resolve_kernel<true>, placed, placed_of_chunk, tails, 0u, n_pages,
-                                             results, pool, out);
-    if (e != cudaSuccess) return e;
-  } else if (tail_ctas + body_ctas) {
-    resolve_kernel<false><<<tail_ctas + body_ctas, kResolveThreads, 0, stream>>>(
-        placed, placed_of_chunk, tails, n_tails, n_pages, results, pool, out);
+  const uint32_t body_ctas = n_pages * (kPageEntries / (kResolveUnit * kResolveWarps));
+  if (!body_ctas) return cudaSuccess;
+  if (!n_tails) {
+    resolve_kernel<kResolveAll><<<body_ctas, kResolveThreads, 0, stream>>>(placed, placed_of_chunk, tails, n_tails,
+                                                                           n_pages, results, pool, out);
+    return cudaGetLastError();
   }
-  return cudaGetLastError();
+  const uint32_t tail_ctas = (n_tails * kTailUnits + kResolveWarps - 1) / kResolveWarps;
+  resolve_kernel<kResolveTails><<<tail_ctas, kResolveThreads, 0, stream>>>(placed, placed_of_chunk, tails, n_tails,
+                                                                           n_pages, results, pool, out);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  cudaLaunchAttribute overlap{};
+  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(body_ctas);
+  cfg.blockDim = dim3(kResolveThreads);
+  cfg.stream = stream;
+  cfg.attrs = &overlap;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, resolve_kernel<kResolveBodies>, placed, placed_of_chunk, tails, n_tails, n_pages,
+                            results, pool, out);
 }
 
 cudaError_t launch_crc(const CrcBlock* blocks, uint32_t n_blocks, const uint8_t* out,

@@ -7,15 +7,15 @@
 namespace gzgpu {
 
 cudaError_t resolve_init(cudaStream_t stream);
-// every placed chunk's bytes (out_len of them), markers resolved: of the chunks in
-// `tails` those from body_end on, and (bodies: if there are any) all before their
-// body_end, from the pages [0, n_pages)
-constexpr uint64_t kTwoPass = 8u << 20;                   // output from which tails and bodies are two launches
+// every placed chunk's bytes, markers resolved, from the pages [0, n_pages).
+// tails (for kTwoPass bytes of output and more): the placed chunks whose entries
+// from body_end on are resolved before the others
+constexpr uint64_t kTwoPass = 16u << 20;
 constexpr uint32_t kTailUnit = 512;                       // body_end is a multiple of it, or all
 constexpr uint32_t kTailUnits = kWindow / kTailUnit + 1;  // a tail's, at most
 cudaError_t launch_resolve(const PlacedChunk* placed, const uint32_t* placed_of_chunk,
-                           const uint32_t* tails, uint32_t n_tails, bool bodies, uint64_t out_len,
-                           uint32_t n_pages, const ChunkResult* results, const PagePool& pool, uint8_t* out,
+                           const uint32_t* tails, uint32_t n_tails, uint32_t n_pages,
+                           const ChunkResult* results, const PagePool& pool, uint8_t* out,
                            cudaStream_t stream);
 // CRC: one CTA per block of up to kCrcBlock bytes, a slice of kCrcSlice per thread
 constexpr int kCrcThreads = 512;
