@@ -643,7 +643,8 @@ __device__ __forceinline__ bool cta_page(CtaSmem<LB, NT>* S, const PagePool& poo
 // stage has two turns, so a window needs three barriers: its tokens are placed
 // (which also makes the window before it readable as history), its records are
 // read, its references are in place.
-// Returns kOk or kPoolExhausted.  (No distance reaches beyond the window before
+// Returns kOk, or kPoolExhausted with S->c.o and round_slots as far as it got.
+// (No distance reaches beyond the window before
 // the chunk: a code names 32768 at most.)
 template <int LB, int NT>
 __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB, NT>* S, const PagePool& pool, uint32_t n,
@@ -696,7 +697,14 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB, NT>* S, const PageP
     uint32_t* const stage = S->stage[turn];
     uint32_t* const bm = S->bm[turn];
     const uint32_t wbase = lo & ~(kWin - 1), wend = wbase + kWin;
-    if (!cta_page(S, pool, base + wbase)) return kPoolExhausted;
+    if (!cta_page(S, pool, base + wbase)) {
+      // what the larger pool is sized by: the entries written, and the slots that gave them
+      if (tid == 0) {
+        S->c.o = base + lo;
+        S->c.round_slots = b0 + (uint32_t)((uint64_t)kTokPer * NT * (lo - bpos) / (bend - bpos));
+      }
+      return kPoolExhausted;
+    }
     // (the thread that wrote it in the window before sees it in time, which is
     // enough for the vote)
     uint32_t any_match = S->c.carry_len;
@@ -1016,7 +1024,10 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
       const int32_t st = expand_tokens<LB, NT>(S, pool, n_slots, zero_window);
       if (st != kOk) {
         cta_sync();
-        if (tid == 0) S->c.status = st;
+        if (tid == 0) {
+          S->c.status = st;
+          S->c.pos += (new_pos - pos) * min(S->c.round_slots, n_slots) / n_slots;
+        }
         break;
       }
     }
