@@ -97,39 +97,62 @@ struct HostPinned {
   }
 };
 
-// Allocator of page-locked host memory, for the tables a job exchanges with
-// the device: a copy from or to it needs no staging by the driver and no wait
-// on the host.  Its users keep their capacity from job to job.  Where no more
-// can be page-locked, plain memory does.
+// Page-locked host memory of a context.  Locking or unlocking pages can stall
+// every stream of the device, so a context locks at most two blocks in its life
+// (reserve_tables: with its first job, and with its first large one) and unlocks
+// none before its end.  What outgrows them goes on in plain memory.
+struct TableArena {
+  struct Block {
+    char* base;
+    size_t cap, used;
+  } blocks[2];
+  int n = 0;
+  void add(size_t bytes) {
+    Block& b = blocks[n];
+    b = Block{nullptr, bytes, 0};
+    if (cudaMallocHost(reinterpret_cast<void**>(&b.base), bytes) == cudaSuccess) n++;
+    else cudaGetLastError();  // the tables stay in plain memory
+  }
+  void* take(size_t bytes) {
+    bytes = (bytes + 63) & ~(size_t)63;
+    if (!n || bytes > blocks[n - 1].cap - blocks[n - 1].used) return nullptr;
+    Block& b = blocks[n - 1];
+    b.used += bytes;
+    return b.base + b.used - bytes;
+  }
+  bool holds(const void* p) const {
+    for (int i = 0; i < n; i++)
+      if (p >= blocks[i].base && p < blocks[i].base + blocks[i].cap) return true;
+    return false;
+  }
+  ~TableArena() {
+    for (int i = 0; i < n; i++) cudaFreeHost(blocks[i].base);
+  }
+};
+
+// Allocator of the tables a job exchanges with the device: a copy from or to
+// the arena needs no staging by the driver and no wait on the host.
 template <typename T>
-struct PinnedAlloc {
+struct TableAlloc {
   using value_type = T;
-  static constexpr size_t kHead = 64;  // before the elements: whether they are page-locked
-  PinnedAlloc() = default;
+  TableArena* arena;
+  explicit TableAlloc(TableArena* a) : arena(a) {}
   template <typename U>
-  PinnedAlloc(const PinnedAlloc<U>&) {}
+  TableAlloc(const TableAlloc<U>& o) : arena(o.arena) {}
   T* allocate(size_t n) {
-    void* p = nullptr;
-    bool locked = cudaMallocHost(&p, n * sizeof(T) + kHead) == cudaSuccess;
-    if (!locked) {
-      cudaGetLastError();
-      p = ::operator new(n * sizeof(T) + kHead);
-    }
-    *static_cast<bool*>(p) = locked;
-    return reinterpret_cast<T*>(static_cast<char*>(p) + kHead);
+    void* p = arena->take(n * sizeof(T));
+    return static_cast<T*>(p ? p : ::operator new(n * sizeof(T)));
   }
-  void deallocate(T* q, size_t) {
-    void* p = reinterpret_cast<char*>(q) - kHead;
-    if (*static_cast<bool*>(p)) cudaFreeHost(p);
-    else ::operator delete(p);
+  void deallocate(T* p, size_t) {
+    if (!arena->holds(p)) ::operator delete(p);
   }
   template <typename U>
-  bool operator==(const PinnedAlloc<U>&) const { return true; }
+  bool operator==(const TableAlloc<U>& o) const { return arena == o.arena; }
   template <typename U>
-  bool operator!=(const PinnedAlloc<U>&) const { return false; }
+  bool operator!=(const TableAlloc<U>& o) const { return arena != o.arena; }
 };
 template <typename T>
-using PinnedVec = std::vector<T, PinnedAlloc<T>>;
+using PinnedVec = std::vector<T, TableAlloc<T>>;
 // room for n elements; twice that when it has to grow, since growing is dear
 template <typename T>
 void make_room(PinnedVec<T>& v, size_t n) {
@@ -240,10 +263,35 @@ struct gzgpu_ctx {
   // Job tables in page-locked memory: uploads (by turns, so that one is filled
   // while the other may still be on its way), results, and the chunk table,
   // which also stays as the last job's (diagnostics)
-  PinnedVec<uint8_t> up[2], down;
-  PinnedVec<uint32_t> h_spec;
-  PinnedVec<ChunkDesc> hd, hd_cut;  // hd_cut: the table with its partitions cut finer
-  PinnedVec<ChunkResult> hr;
+  TableArena arena;
+  PinnedVec<uint8_t> up[2]{PinnedVec<uint8_t>(TableAlloc<uint8_t>(&arena)),
+                           PinnedVec<uint8_t>(TableAlloc<uint8_t>(&arena))};
+  PinnedVec<uint8_t> down{TableAlloc<uint8_t>(&arena)};
+  PinnedVec<uint32_t> h_spec{TableAlloc<uint32_t>(&arena)};
+  PinnedVec<ChunkDesc> hd{TableAlloc<ChunkDesc>(&arena)};
+  PinnedVec<ChunkDesc> hd_cut{TableAlloc<ChunkDesc>(&arena)};  // the table with its partitions cut finer
+  PinnedVec<ChunkResult> hr{TableAlloc<ChunkResult>(&arena)};
+  // Room for a job of total_in bytes: 1 MB (0.5 ms to lock), or from kLargeJob on
+  // 10 MB (5 ms), which is for 32,768 chunks, about 1.5 GiB.
+  static constexpr uint64_t kLargeJob = 64ull << 20;
+  int tables_for = 0;  // 1 small jobs, 2 large ones
+  void reserve_tables(uint64_t total_in) {
+    const int want = total_in > kLargeJob ? 2 : 1;
+    if (want <= tables_for) return;
+    tables_for = want;
+    const size_t n = want == 2 ? 32768 : 3072;
+    const size_t scan_up = (sizeof(ScanUnit) + 16) * (want == 2 ? 8192 : 2048), down_n = want == 2 ? 1 << 18 : 1 << 16;
+    const size_t plan_up = (sizeof(PlacedChunk) + sizeof(CrcBlock) + 40) * n;
+    arena.add(((1 + fine_split) * sizeof(ChunkDesc) + sizeof(ChunkResult) + 4) * n + scan_up + plan_up + down_n +
+              8 * 64);
+    hd.reserve(n);
+    if (fine_split) hd_cut.reserve(n);
+    hr.reserve(n);
+    h_spec.reserve(n);
+    up[0].reserve(scan_up);
+    up[1].reserve(plan_up);
+    down.reserve(down_n);
+  }
   uint32_t n_pages_used = 0;  // pages taken from the pool by the job's decodes
   cudaEvent_t ev[12];
   cudaEvent_t stage_ev[2];  // last DMA of each pinned staging slot
@@ -550,6 +598,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
     h_len[s] = S[s].len;
     total_in += S[s].len;
   }
+  reserve_tables(total_in);
   std::vector<ScanUnit> units;
   // one CTA per unit: small enough that every SM has several (1 MiB units left
   // all but 23 CTAs idle on a 23 MB stream: 113 us), 8 KiB (one load per
