@@ -329,6 +329,7 @@ struct gzgpu_ctx {
     return kOk;
   }
 
+  bool few_chunks(uint32_t n) const { return n <= 2 * (uint32_t)sms; }
   // d_work_count: the work list's length on the device; n_work: the same on
   // the host.  With fewer chunks than resident CTAs, one CTA per chunk: the
   // hardware spreads a small grid over the SMs, while in a full grid the
@@ -341,7 +342,7 @@ struct gzgpu_ctx {
     // blocks: 1.27 -> 0.72 ms, 0.45 since it is two chunks; 232 chunks of small
     // streams: 0.42 -> 0.32).  From 300 chunks on the SMs are
     // better filled by three CTAs of 256 (342 chunks: 0.25 ms, wide 0.37).
-    const bool wide = n_work <= 2 * (uint32_t)sms;
+    const bool wide = few_chunks(n_work);
     PagePool pool{pages.as<uint16_t>(), owner.as<uint32_t>(), seq.as<uint32_t>(),
                   counters.as<uint32_t>() + 2, (uint32_t)(pages.cap / (kPageEntries * 2))};
     pool.cap = (uint32_t)std::min<uint64_t>(pool.cap, std::min(owner.cap, seq.cap) / 4);
@@ -406,6 +407,7 @@ struct gzgpu_ctx {
   };
   std::map<uint32_t, TuneCfg> tune_cache;
   bool tuning = false;     // a trial run: parameters are forced, no cache lookup
+  bool job_wide = false;   // the job's chunks were decoded by CTAs of 1,024 threads
   uint32_t last_key = 0;   // key of the last job
   void apply(const TuneCfg& t) {
     chunk_bytes = t.chunk_bytes;
@@ -470,7 +472,8 @@ int gzgpu_ctx::job_tuned(const std::vector<StreamSpec>& S, std::vector<StreamOut
   // nothing to tune on
   if (std::all_of(R.begin(), R.end(), [](const StreamOut& r) { return r.status == kNotGzip; })) return rc;
   // Coordinate search, one full decode per candidate (outputs are identical,
-  // so any run's result stands): chunk size, then LUT bits, then warps/SM.
+  // so any run's result stands): chunk size, then LUT bits, then CTAs per SM
+  // (where that has an effect).
   const uint32_t key = last_key;
   uint32_t trials = 0;
   auto trial = [&](const TuneCfg& t) {
@@ -485,24 +488,26 @@ int gzgpu_ctx::job_tuned(const std::vector<StreamSpec>& S, std::vector<StreamOut
   };
   TuneCfg best = dflt;
   double best_ms = trial(best);
+  bool best_wide = job_wide;
+  auto consider = [&](const TuneCfg& t) {
+    const double ms = trial(t);
+    if (ms < best_ms) best_ms = ms, best = t, best_wide = job_wide;
+  };
   for (uint64_t cb : {16ull << 10, 32ull << 10, 64ull << 10, 128ull << 10}) {
     if (cb == best.chunk_bytes) continue;
     TuneCfg t = best;
     t.chunk_bytes = cb;
-    double ms = trial(t);
-    if (ms < best_ms) best_ms = ms, best = t;
+    consider(t);
   }
   for (int lb : {10, 12}) {
     TuneCfg t = best;
     t.lut_bits = lb;
-    double ms = trial(t);
-    if (ms < best_ms) best_ms = ms, best = t;
+    consider(t);
   }
-  {
+  if (!best_wide && !ring) {
     TuneCfg t = best;
     t.ctas_per_sm = 4;
-    double ms = trial(t);
-    if (ms < best_ms) best_ms = ms, best = t;
+    consider(t);
   }
   tune_cache[key] = best;
   // the final decode with the chosen parameters gives the call's stats
@@ -900,7 +905,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
   // Chunks with a start, which decides how the decode is launched.  A grid
   // small enough for wide CTAs needs no count.
   uint32_t n_decode = n_grid;
-  if (n_grid > 2 * (uint32_t)sms) {
+  if (!few_chunks(n_grid)) {
     if (down.size() < 4096) down.resize(4096);
     if ((rc = check(cudaMemcpyAsync(down.data(), counters.as<uint32_t>() + 1, 4, cudaMemcpyDeviceToHost, st))) ||
         (rc = check(cudaStreamSynchronize(st))))
@@ -924,6 +929,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
                                              1u << 30);
       if ((rc = check(blk_log.ensure(sizeof(BlockRec) * (uint64_t)blk_cap)))) return rc;
     }
+    job_wide = few_chunks(n_decode);
     cudaEventRecord(ev[8], st);
     if ((rc = check(launch_decode(counters.as<uint32_t>() + 1, n_decode)))) return rc;
     cudaEventRecord(ev[9], st);

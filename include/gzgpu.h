@@ -59,10 +59,11 @@ typedef struct {
                          is decoded once per candidate and the fastest is kept for
                          later jobs of that kind; overrides the three fields */
   int ring_history;   /* 1 = decode history in a shared-memory ring (one warp per chunk, 3
-                         per SM) instead of the output pages in HBM (one CTA of 256 threads
-                         per chunk, the default) */
+                         per SM) instead of the output pages in HBM (one CTA of 256 or
+                         1,024 threads per chunk, the default) */
   int ctas_per_sm;    /* page-history decoder: 3 (80 registers per thread; default) or
-                         4 (64 registers); 0 = default */
+                         4 (64 registers); 0 = default.  Jobs of up to two chunks per SM
+                         run CTAs of 1,024 threads instead, one per SM */
   int fine_split;     /* 1 = cut partitions whose first blocks promise a high output
                          ratio into pieces and give pieces without a block start a
                          sync start inside their dynamic block; 0 = off (default:
