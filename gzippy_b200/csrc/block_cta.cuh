@@ -1,7 +1,8 @@
 // block_cta.cuh -- one CTA decodes one chunk (page history).
 //
 // Block body.  A Huffman-coded block is decoded in rounds of up to
-// kCtaThreads bit ranges of `r` bits each, one range per thread:
+// NT (the CTA's threads, 256 or 1,024) bit ranges of `r` bits each, one range per
+// thread:
 //   1. every thread walks its range from a guessed start (its first bit),
 //      following symbol lengths only.  Prefix codes resynchronise: a walk that
 //      starts off a symbol boundary falls into step with the true one, so most
@@ -21,7 +22,7 @@
 // Threads leave the data-dependent loops at different times; every barrier of
 // the CTA joins each warp's lanes first (barrier.cuh).
 // What bounds a block is its serial chain of code lookups; the ranges cut
-// that chain into up to 256 pieces.  Ranges of 512 bits end in step after a
+// that chain into up to NT pieces.  Ranges of 512 bits end in step after a
 // wrong start for 98 % of text, 88 % of byte runs and 59 % of noisy ramps
 // (codes nearly all of one length), measured on zlib level 6 streams.
 // Inflate kernel, before (one warp per chunk, steps of 64 bits decoded by the
@@ -110,7 +111,7 @@ struct CtaCtl {
 // and symbol is (window >> (15 - length)) + base[length].
 struct CodeIndex {
   uint32_t lim[16], base[16];
-  uint16_t count[16], first[16], offs[16], next[16];
+  uint16_t count[16], offs[16];
 };
 
 template <int LB, int NT>
@@ -213,7 +214,6 @@ struct RangeBits {
   uint32_t p, q;  // position; refill when p >= q, which leaves 30 bits at least
 
   __device__ __forceinline__ void refill_if_due() {
-#ifdef __CUDA_ARCH__
     // 2 + the bits left (2 .. 32) is where the next word goes
     asm("{\n\t"
         ".reg .pred due;\n\t"
@@ -230,14 +230,6 @@ struct RangeBits {
         "@due add.u64 %5, %5, 4;\n\t"
         "}"
         : "+r"(lo), "+r"(hi), "+r"(w), "+r"(q), "+r"(p), "+l"(next));
-#else
-    if (p < q) return;
-    const uint32_t s = q + 32 - p;
-    lo |= __funnelshift_lc(0, w, s);
-    hi |= __funnelshift_lc(w, 0, s);
-    q += 32;
-    w = *next++;
-#endif
   }
   // base: the word of position 0
   __device__ __forceinline__ void seek(const uint32_t* base, uint32_t pos) {

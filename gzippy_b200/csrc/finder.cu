@@ -1,8 +1,9 @@
 // finder.cu -- deflate block-boundary finder (K1) and chunk linking.
 //
-// Each speculative chunk searches [guess_bit, limit_bit) for its first
-// block-start candidate (predicate and search in finder_core.cuh) with the
-// warps of one CTA.
+// Each speculative chunk's range [guess_bit, limit_bit) is searched for its first
+// block-start candidate (predicate in finder_core.cuh): stored blocks, then sync
+// starts in fixed blocks by a CTA per range, then dynamic headers by the warps of
+// a grid, a segment of a range each.
 #include <cstdint>
 
 #include "barrier.cuh"
@@ -14,7 +15,7 @@ namespace gzgpu {
 
 // Stored block starts, searched first for every speculative chunk: the first
 // one (by byte offset, hence by start bit) in [guess_bit, limit_bit) whose
-// successor passes stored_successor_ok becomes the chunk's start, and the
+// successor passes stored_successor becomes the chunk's start, and the
 // sync search and the block finder skip the chunk.  The successor check is
 // a heuristic: a false start needs two LEN/NLEN matches in a row, or a
 // LEN/NLEN match and a valid dynamic header, which is rare but possible.
@@ -519,12 +520,6 @@ __global__ void __launch_bounds__(kSyncOffsets)
   }
 }
 
-// stop_lo of each valid chunk = lo of the next valid chunk when that one is
-// speculative (member starts end their predecessor at BFINAL instead);
-// valid chunks are appended to the decode work list.
-// A speculative start may be a phantom whose garbage code table never fails;
-// such a chunk gives up `slack` bits past its stop and the chain walk
-// re-decodes the gap from the confirmed boundary instead.
 // Decode cost of a linked chunk: its compressed bytes.  Text and noisy
 // literals take the decoder 8.6 us per KB; stored data is a copy, a twentieth
 // of that (only the stored blocks themselves count so: chunks that begin with
@@ -550,6 +545,12 @@ __device__ float chunk_cost(const uint8_t* __restrict__ in, const ChunkDesc& d, 
   return fmaxf(span - 0.95f * (float)copied, 0.05f * span) * fmaxf(1.f, 0.5f * d.est_ratio);
 }
 
+// stop_lo of each valid chunk = lo of the next valid chunk when that one is
+// speculative (member starts end their predecessor at BFINAL instead);
+// valid chunks are appended to the decode work list.
+// A speculative start may be a phantom whose garbage code table never fails;
+// such a chunk gives up `slack` bits past its stop and the chain walk
+// re-decodes the gap from the confirmed boundary instead.
 __global__ void link_kernel(const uint8_t* __restrict__ in, ChunkDesc* descs, uint32_t n,
                             uint32_t* work, uint32_t* n_work, float* cost, uint64_t slack) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;

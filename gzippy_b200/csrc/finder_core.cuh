@@ -209,8 +209,8 @@ static __device__ __forceinline__ bool dyn_candidate_fast(const uint8_t* in, uin
 // predicate.  Not a rule of the reference's finder: it drops the false
 // LEN/NLEN matches (about one per 64 KiB of random bytes) that would
 // otherwise start speculative chunks inside stored data.  A true stored
-// block followed by a fixed-Huffman block is given up as a start.
-// stored_successor: all but that predicate (kSuccHeader: it decides).
+// block followed by a fixed-Huffman block is given up as a start.  All but that
+// predicate; kSuccHeader: it decides.
 enum : int { kSuccNo = 0, kSuccYes = 1, kSuccHeader = 2 };
 static __device__ __forceinline__ int stored_successor(const uint8_t* in, uint64_t nbytes, uint64_t n) {
   if (n >= nbytes) return kSuccNo;
@@ -228,12 +228,6 @@ static __device__ __forceinline__ int stored_successor(const uint8_t* in, uint64
   if (((h >> 3) & 31) > 29 || ((h >> 8) & 31) > 29) return kSuccNo;
   return kSuccHeader;
 }
-static __device__ __forceinline__ bool stored_successor_ok(const uint8_t* in, uint64_t nbytes,
-                                                           uint64_t n) {
-  const int s = stored_successor(in, nbytes, n);
-  return s == kSuccHeader ? dyn_candidate_full(in, nbytes, n * 8) : s == kSuccYes;
-}
-
 // Stored candidate test at byte offset `off` (find_uncompressed_blocks):
 // LEN == ~NLEN at the byte boundary, 3 zero header bits before it; the
 // candidate spans [byte_bit - zero_run, byte_bit - 3].

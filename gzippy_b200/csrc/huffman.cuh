@@ -121,19 +121,6 @@ struct BitReader {
       bc -= k;
     }
   }
-  __device__ __forceinline__ void consume_wide(int k) {  // 0 <= k < 128
-    if (k >= 64) {
-      bb = hi >> (k - 64);
-      hi = 0;
-      bc -= k;
-    } else {
-      consume(k);
-    }
-  }
-  // bits [i, i + 64) of the window, 0 <= i < 64
-  __device__ __forceinline__ uint64_t peek_at(int i) const {
-    return i ? (bb >> i) | (hi << (64 - i)) : bb;
-  }
   __device__ __forceinline__ uint64_t pos() const { return wpos * 32 - (uint64_t)bc; }
   __device__ __forceinline__ bool overrun() const { return wpos > limit_words; }
 };

@@ -9,13 +9,13 @@
 // instead (the zero window of chunk_fetcher.rs:696).
 //
 // Two kernels, same decode:
-//   pages (default) : one CTA of kCtaThreads threads per chunk.  A Huffman
-//                     block is cut into one bit range per thread, every
-//                     thread decodes its range, and the ranges are joined
-//                     once each starts where the one before it ended (see
-//                     "Block body" below).  Entries go straight into the
-//                     chunk's output pages in HBM, which are also its
-//                     history.
+//   pages (default) : one CTA per chunk, of kCtaThreads threads or, in jobs of
+//                     few chunks, kWideThreads.  A Huffman block is cut into
+//                     one bit range per thread, every thread decodes its
+//                     range, and the ranges are joined once each starts where
+//                     the one before it ended (block_cta.cuh).  Entries go
+//                     straight into the chunk's output pages in HBM, which
+//                     are also its history.
 //   ring            : one warp per chunk, serial decode, a 32 Ki-entry u16
 //                     ring per warp in shared memory (64 KB), flushed to the
 //                     pages in 8 Ki-entry units; 3 decoding warps per SM.
