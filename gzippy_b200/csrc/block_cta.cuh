@@ -99,6 +99,7 @@ struct CtaCtl {
   uint32_t hdr_move, hdr_end, hdr_last;
   uint32_t build_ok[2];
   uint32_t page_cur, page_prev, page_seq, n_pages;
+  uint64_t fail_o;          // where the page pool ran out
   uint32_t round_slots, round_lanes, round_kind, round_pos;
   int32_t carry_ms;         // match reaching into the next window: start (relative to it)
   uint32_t carry_len, carry_dist;
@@ -610,6 +611,7 @@ __device__ __forceinline__ bool cta_page(CtaSmem<LB, NT>* S, const PagePool& poo
       pool.seq[p] = (S->c.gen << kGenShift) | s;
     } else {
       p = kNoPage;
+      S->c.fail_o = w0;
     }
     S->c.page_prev = S->c.page_cur;
     S->c.page_cur = p;
@@ -635,9 +637,8 @@ __device__ __forceinline__ bool cta_page(CtaSmem<LB, NT>* S, const PagePool& poo
 // stage has two turns, so a window needs three barriers: its tokens are placed
 // (which also makes the window before it readable as history), its records are
 // read, its references are in place.
-// Returns kOk, or kPoolExhausted with S->c.o and round_slots as far as it got.
-// (No distance reaches beyond the window before
-// the chunk: a code names 32768 at most.)
+// Returns kOk, or kPoolExhausted (S->c.fail_o: the entries written).  (No
+// distance reaches beyond the window before the chunk: a code names 32768 at most.)
 template <int LB, int NT>
 __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB, NT>* S, const PagePool& pool, uint32_t n,
                                                  bool zero_window) {
@@ -689,14 +690,7 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB, NT>* S, const PageP
     uint32_t* const stage = S->stage[turn];
     uint32_t* const bm = S->bm[turn];
     const uint32_t wbase = lo & ~(kWin - 1), wend = wbase + kWin;
-    if (!cta_page(S, pool, base + wbase)) {
-      // what the larger pool is sized by: the entries written, and the slots that gave them
-      if (tid == 0) {
-        S->c.o = base + lo;
-        S->c.round_slots = b0 + (uint32_t)((uint64_t)kTokPer * NT * (lo - bpos) / (bend - bpos));
-      }
-      return kPoolExhausted;
-    }
+    if (!cta_page(S, pool, base + wbase)) return kPoolExhausted;
     // (the thread that wrote it in the window before sees it in time, which is
     // enough for the vote)
     uint32_t any_match = S->c.carry_len;
@@ -894,6 +888,29 @@ __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB, NT>* S, const PageP
   return kOk;
 }
 
+// The pool ran out in a round of n slots that ends at new_pos: move S->c.o to the
+// entries written and S->c.pos by the same share of the round, which the larger pool
+// is sized by.  (Apart from expand_tokens, whose loop is 5 % slower on byte runs
+// when it keeps count itself.)
+template <int LB, int NT>
+__device__ __noinline__ void cta_progress(CtaSmem<LB, NT>* S, uint32_t n, uint64_t new_pos) {
+  const uint32_t tid = threadIdx.x;
+  if (tid == 0) S->c.mark_max = 0;
+  cta_sync();
+  uint32_t sum = 0;  // entries of the round
+  for (uint32_t i = tid; i < n; i += NT) {
+    const uint32_t v = S->tok[i];
+    sum += v & kTokMatch ? v & 0x1FFu : (i && S->tok[i - 1] & kTokMatch ? 0u : 1u);
+  }
+  atomicAdd(&S->c.mark_max, sum);
+  cta_sync();
+  if (tid == 0 && S->c.fail_o > S->c.o) {
+    const float part = (float)(uint32_t)(S->c.fail_o - S->c.o) / (float)S->c.mark_max;
+    S->c.pos += (uint32_t)(fminf(part, 1.f) * (float)(uint32_t)(new_pos - S->c.pos));
+    S->c.o = S->c.fail_o;
+  }
+}
+
 // The body of one Huffman-coded block, tables in place.  On return (after a
 // barrier) S->c holds the new position and entry count, status, synced (at
 // the successor's sync start) or passed (went by the successor's start).
@@ -1016,10 +1033,8 @@ __device__ __forceinline__ void cta_block(const uint8_t* __restrict__ in, CtaSme
       const int32_t st = expand_tokens<LB, NT>(S, pool, n_slots, zero_window);
       if (st != kOk) {
         cta_sync();
-        if (tid == 0) {
-          S->c.status = st;
-          S->c.pos += (new_pos - pos) * min(S->c.round_slots, n_slots) / n_slots;
-        }
+        cta_progress<LB, NT>(S, n_slots, new_pos);
+        if (tid == 0) S->c.status = st;
         break;
       }
     }
