@@ -99,7 +99,7 @@ struct HostPinned {
 
 // Page-locked host memory of a context.  Locking or unlocking pages can stall
 // every stream of the device, so a context locks at most two blocks in its life
-// (reserve_tables: with its first job, and with its first large one) and unlocks
+// (reserve_tables: with its second job, and with its second large one) and unlocks
 // none before its end.  What outgrows them goes on in plain memory.
 struct TableArena {
   struct Block {
@@ -271,12 +271,17 @@ struct gzgpu_ctx {
   PinnedVec<ChunkDesc> hd{TableAlloc<ChunkDesc>(&arena)};
   PinnedVec<ChunkDesc> hd_cut{TableAlloc<ChunkDesc>(&arena)};  // the table with its partitions cut finer
   PinnedVec<ChunkResult> hr{TableAlloc<ChunkResult>(&arena)};
-  // Room for a job of total_in bytes: 1 MB (0.5 ms to lock), or from kLargeJob on
-  // 10 MB (5 ms), which is for 32,768 chunks, about 1.5 GiB.
+  // Room for jobs of the size of this one, once a second one comes: 1 MB, or for
+  // those above kLargeJob 10 MB, which is for 32,768 chunks, about 1.5 GiB.
+  // Locking takes 2.8 and 7 ms, more than a small call by itself (4 KiB: 0.25 ms),
+  // and saves a call 50 us: a context made for one call does not repay it.
   static constexpr uint64_t kLargeJob = 64ull << 20;
+  uint32_t n_jobs = 0, n_large = 0;
   int tables_for = 0;  // 1 small jobs, 2 large ones
   void reserve_tables(uint64_t total_in) {
-    const int want = total_in > kLargeJob ? 2 : 1;
+    n_jobs++;
+    n_large += total_in > kLargeJob;
+    const int want = n_large >= 2 ? 2 : (n_jobs >= 2 ? 1 : 0);
     if (want <= tables_for) return;
     tables_for = want;
     const size_t n = want == 2 ? 32768 : 3072;
