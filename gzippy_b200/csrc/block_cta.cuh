@@ -99,7 +99,6 @@ struct CtaCtl {
   uint32_t hdr_move, hdr_end, hdr_last;
   uint32_t build_ok[2];
   uint32_t page_cur, page_prev, page_seq, n_pages;
-  uint64_t fail_o;          // where the page pool ran out
   uint32_t round_slots, round_lanes, round_kind, round_pos;
   int32_t carry_ms;         // match reaching into the next window: start (relative to it)
   uint32_t carry_len, carry_dist;
@@ -611,7 +610,6 @@ __device__ __forceinline__ bool cta_page(CtaSmem<LB, NT>* S, const PagePool& poo
       pool.seq[p] = (S->c.gen << kGenShift) | s;
     } else {
       p = kNoPage;
-      S->c.fail_o = w0;
     }
     S->c.page_prev = S->c.page_cur;
     S->c.page_cur = p;
@@ -637,8 +635,8 @@ __device__ __forceinline__ bool cta_page(CtaSmem<LB, NT>* S, const PagePool& poo
 // stage has two turns, so a window needs three barriers: its tokens are placed
 // (which also makes the window before it readable as history), its records are
 // read, its references are in place.
-// Returns kOk, or kPoolExhausted (S->c.fail_o: the entries written).  (No
-// distance reaches beyond the window before the chunk: a code names 32768 at most.)
+// Returns kOk or kPoolExhausted.  (No distance reaches beyond the window before
+// the chunk: a code names 32768 at most.)
 template <int LB, int NT>
 __device__ __forceinline__ int32_t expand_tokens(CtaSmem<LB, NT>* S, const PagePool& pool, uint32_t n,
                                                  bool zero_window) {
@@ -904,10 +902,11 @@ __device__ __noinline__ void cta_progress(CtaSmem<LB, NT>* S, uint32_t n, uint64
   }
   atomicAdd(&S->c.mark_max, sum);
   cta_sync();
-  if (tid == 0 && S->c.fail_o > S->c.o) {
-    const float part = (float)(uint32_t)(S->c.fail_o - S->c.o) / (float)S->c.mark_max;
+  const uint64_t at = (uint64_t)S->c.page_seq * kPageEntries;  // the page there was none for
+  if (tid == 0 && at > S->c.o) {
+    const float part = (float)(uint32_t)(at - S->c.o) / (float)S->c.mark_max;
     S->c.pos += (uint32_t)(fminf(part, 1.f) * (float)(uint32_t)(new_pos - S->c.pos));
-    S->c.o = S->c.fail_o;
+    S->c.o = at;
   }
 }
 

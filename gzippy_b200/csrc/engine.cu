@@ -98,14 +98,14 @@ struct HostPinned {
 };
 
 // Page-locked host memory of a context.  Locking or unlocking pages can stall
-// every stream of the device, so a context locks at most two blocks in its life
-// (reserve_tables: with its second job, and with its second large one) and unlocks
-// none before its end.  What outgrows them goes on in plain memory.
+// every stream of the device, so a context locks at most four blocks in its life
+// (reserve_tables: each with the second job that wants it) and unlocks none before
+// its end.  What outgrows them goes on in plain memory.
 struct TableArena {
   struct Block {
     char* base;
     size_t cap, used;
-  } blocks[2];
+  } blocks[4];
   int n = 0;
   void add(size_t bytes) {
     Block& b = blocks[n];
@@ -271,21 +271,22 @@ struct gzgpu_ctx {
   PinnedVec<ChunkDesc> hd{TableAlloc<ChunkDesc>(&arena)};
   PinnedVec<ChunkDesc> hd_cut{TableAlloc<ChunkDesc>(&arena)};  // the table with its partitions cut finer
   PinnedVec<ChunkResult> hr{TableAlloc<ChunkResult>(&arena)};
-  // Room for jobs of the size of this one, once a second one comes: 1 MB, or for
-  // those above kLargeJob 10 MB, which is for 32,768 chunks, about 1.5 GiB.
-  // Locking takes 2.8 and 7 ms, more than a small call by itself (4 KiB: 0.25 ms),
-  // and saves a call 50 us: a context made for one call does not repay it.
-  static constexpr uint64_t kLargeJob = 64ull << 20;
-  uint32_t n_jobs = 0, n_large = 0;
-  int tables_for = 0;  // 1 small jobs, 2 large ones
-  void reserve_tables(uint64_t total_in) {
-    n_jobs++;
-    n_large += total_in > kLargeJob;
-    const int want = n_large >= 2 ? 2 : (n_jobs >= 2 ? 1 : 0);
-    if (want <= tables_for) return;
-    tables_for = want;
-    const size_t n = want == 2 ? 32768 : 3072;
-    const size_t scan_up = (sizeof(ScanUnit) + 16) * (want == 2 ? 8192 : 2048), down_n = want == 2 ? 1 << 18 : 1 << 16;
+  // Room for jobs of about n_chunks chunks, once a second one comes: 3,072 chunks
+  // (0.9 MB; inputs of up to 64 MiB), 12,288, 49,152 or 196,608 (60 MB).  Locking
+  // takes 2.8 ms for the first, more than a small call by itself (4 KiB: 0.25 ms),
+  // and saves that call 50 us: a context made for one call does not repay it.
+  // 64,418 chunks in plain memory cost a call of 50 ms three.
+  static constexpr size_t kRooms[4] = {3072, 12288, 49152, 196608};
+  uint32_t n_jobs[4] = {};  // jobs that wanted this room or more
+  int rooms = 0;            // [0, rooms) have been locked or passed over
+  void reserve_tables(uint64_t n_chunks) {
+    int want = 0;
+    for (int i = 0; i < 4; i++)
+      if ((!i || n_chunks > kRooms[i - 1]) && ++n_jobs[i] >= 2) want = i + 1;
+    if (want <= rooms) return;
+    rooms = want;
+    const size_t n = kRooms[want - 1];
+    const size_t scan_up = (sizeof(ScanUnit) + 16) * (2048 + n / 8), down_n = (1 << 16) + 4 * n;
     const size_t plan_up = (sizeof(PlacedChunk) + sizeof(CrcBlock) + 40) * n;
     arena.add(((1 + fine_split) * sizeof(ChunkDesc) + sizeof(ChunkResult) + 4) * n + scan_up + plan_up + down_n +
               8 * 64);
@@ -608,7 +609,7 @@ int gzgpu_ctx::run(const std::vector<StreamSpec>& S, std::vector<StreamOut>& R) 
     h_len[s] = S[s].len;
     total_in += S[s].len;
   }
-  reserve_tables(total_in);
+  reserve_tables(total_in / (chunk_bytes ? chunk_bytes : pick_chunk_bytes(total_in)) + ns);
   std::vector<ScanUnit> units;
   // one CTA per unit: small enough that every SM has several (1 MiB units left
   // all but 23 CTAs idle on a 23 MB stream: 113 us), 8 KiB (one load per
