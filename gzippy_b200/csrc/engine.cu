@@ -107,14 +107,27 @@ struct TableArena {
     size_t cap, used;
   } blocks[4];
   int n = 0;
-  void add(size_t bytes) {
+  std::vector<std::pair<void*, size_t>> spare;  // taken before and given back
+  bool add(size_t bytes) {
+    spare.reserve(64);
     Block& b = blocks[n];
     b = Block{nullptr, bytes, 0};
-    if (cudaMallocHost(reinterpret_cast<void**>(&b.base), bytes) == cudaSuccess) n++;
-    else cudaGetLastError();  // the tables stay in plain memory
+    if (cudaMallocHost(reinterpret_cast<void**>(&b.base), bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    n++;
+    return true;
   }
   void* take(size_t bytes) {
     bytes = (bytes + 63) & ~(size_t)63;
+    for (auto& s : spare)
+      if (s.second == bytes) {
+        void* const p = s.first;
+        s = spare.back();
+        spare.pop_back();
+        return p;
+      }
     if (!n || bytes > blocks[n - 1].cap - blocks[n - 1].used) return nullptr;
     Block& b = blocks[n - 1];
     b.used += bytes;
@@ -125,6 +138,7 @@ struct TableArena {
       if (p >= blocks[i].base && p < blocks[i].base + blocks[i].cap) return true;
     return false;
   }
+  void give_back(void* p, size_t bytes) { spare.emplace_back(p, (bytes + 63) & ~(size_t)63); }
   ~TableArena() {
     for (int i = 0; i < n; i++) cudaFreeHost(blocks[i].base);
   }
@@ -143,8 +157,9 @@ struct TableAlloc {
     void* p = arena->take(n * sizeof(T));
     return static_cast<T*>(p ? p : ::operator new(n * sizeof(T)));
   }
-  void deallocate(T* p, size_t) {
-    if (!arena->holds(p)) ::operator delete(p);
+  void deallocate(T* p, size_t n) {
+    if (arena->holds(p)) arena->give_back(p, n * sizeof(T));
+    else ::operator delete(p);
   }
   template <typename U>
   bool operator==(const TableAlloc<U>& o) const { return arena == o.arena; }
@@ -279,24 +294,38 @@ struct gzgpu_ctx {
   static constexpr size_t kRooms[4] = {3072, 12288, 49152, 196608};
   uint32_t n_jobs[4] = {};  // jobs that wanted this room or more
   int rooms = 0;            // [0, rooms) have been locked or passed over
+  bool can_lock = true;
   void reserve_tables(uint64_t n_chunks) {
+    // (a job may have more chunks than its size says; the one before tells)
+    n_chunks = std::max<uint64_t>(n_chunks, hd.size());
     int want = 0;
     for (int i = 0; i < 4; i++)
       if ((!i || n_chunks > kRooms[i - 1]) && ++n_jobs[i] >= 2) want = i + 1;
-    if (want <= rooms) return;
-    rooms = want;
-    const size_t n = kRooms[want - 1];
-    const size_t scan_up = (sizeof(ScanUnit) + 16) * (2048 + n / 8), down_n = (1 << 16) + 4 * n;
+    const bool more = want > rooms && can_lock;
+    if (more) rooms = want;
+    if (!rooms || n_chunks > kRooms[rooms - 1] || !can_lock) return;
+    const size_t n = kRooms[rooms - 1];
+    const size_t scan_up = (sizeof(ScanUnit) + 16) * (4096 + n / 4), down_n = (1 << 16) + 4 * n;
     const size_t plan_up = (sizeof(PlacedChunk) + sizeof(CrcBlock) + 40) * n;
-    arena.add(((1 + fine_split) * sizeof(ChunkDesc) + sizeof(ChunkResult) + 4) * n + scan_up + plan_up + down_n +
-              8 * 64);
-    hd.reserve(n);
-    if (fine_split) hd_cut.reserve(n);
-    hr.reserve(n);
-    h_spec.reserve(n);
-    up[0].reserve(scan_up);
-    up[1].reserve(plan_up);
-    down.reserve(down_n);
+    if (more)
+      can_lock = arena.add(((1 + fine_split) * sizeof(ChunkDesc) + sizeof(ChunkResult) + 4) * n + scan_up + plan_up +
+                           down_n + 8 * 64);
+    if (!can_lock) return;  // the tables stay where they are
+    // tables that had outgrown an earlier room come back into this one
+    seat(hd, n);
+    if (fine_split) seat(hd_cut, n);
+    seat(hr, n);
+    seat(h_spec, n);
+    seat(up[0], scan_up);
+    seat(up[1], plan_up);
+    seat(down, down_n);
+  }
+  template <typename T>
+  void seat(PinnedVec<T>& v, size_t n) {
+    if (v.capacity() >= n && arena.holds(v.data())) return;
+    PinnedVec<T> w{TableAlloc<T>(&arena)};
+    w.reserve(n);
+    v.swap(w);
   }
   uint32_t n_pages_used = 0;  // pages taken from the pool by the job's decodes
   cudaEvent_t ev[12];
