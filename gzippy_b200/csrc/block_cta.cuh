@@ -26,7 +26,7 @@
 // wrong start for 98 % of text, 88 % of byte runs and 59 % of noisy ramps
 // (codes nearly all of one length), measured on zlib level 6 streams.
 // Inflate kernel, before (one warp per chunk, steps of 64 bits decoded by the
-// whole warp) and now: 64 MiB text 6.9 -> 0.56 ms, 12 MiB ramps 4.6 -> 0.44,
+// whole warp) and now: 64 MiB text 6.9 -> 0.56 ms, 12 MiB ramps 4.6 -> 0.45,
 // 64 MiB byte runs 22 -> 0.45, 16 MiB of fixed codes 7.8 -> 0.25, a 4 KiB
 // stream 0.195 -> 0.044.  Where the cycles go (text; ramps): expansion 55 %;
 // 23 %, joining the ranges 12; 49, tokens 9; 7, guessed walks 8; 7, tables and
